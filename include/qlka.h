@@ -137,8 +137,9 @@ int qlka_abs_attention_forward(int kind, const float* q, const float* k, const f
 /* ---- weighted abs sum, forward ---------------------------------------------------------
  * out_w[p,m,c] = sum_{d,n} |k[p,d,n] - q[p,d,m]| v[p,n,c]           (P, M, C)
  * out_u[p,m]   = sum_{d,n} |k[p,d,n] - q[p,d,m]|                    (P, M), optional (NULL)
- * path: -1 auto, 0 global, 1 fused - kept for signature compatibility; the three values run
- * the same kernels here, but path == 1 with max(N, M) > 4096 is rejected as in the reference.
+ * path: -1 auto, 0 global, 1 fused, as in the reference. Here 0 takes the sorted walk whatever the size; the other two
+ * also take the pairwise kernels where those are faster (short sequences). path == 1 with max(N, M) > 4096 is rejected as
+ * in the reference.
  * Replaces weighted_abs_sum_forward / weighted_abs_sum_full_forward,
  * Weighted_Abs_Sum/csrc/binding.cpp:132-239. */
 int qlka_abs_forward_workspace_bytes(int P, int D, int N, int M, int C, size_t* bytes);

@@ -3,9 +3,12 @@
 // four operators. No allocation, no synchronisation, no torch types.
 #include "../../include/qlka.h"
 #include "qlka_common.cuh"
+#include "dense_tiles.cuh"
 
 #include <atomic>
+#include <algorithm>
 #include <climits>
+#include <cmath>
 
 namespace qlka {
 cudaError_t launch_sort_rank_small(const SortArgs& a, cudaStream_t stream);
@@ -17,6 +20,7 @@ int         walk_lanes_per_stream(int C4);
 int         walk_threads();
 int         laplace_agg_stride(int C4);
 int         prefix_agg_stride_host(int C4);
+cudaError_t launch_dense_forward(DenseArgs a, int kind, int sms, cudaStream_t stream);
 cudaError_t launch_colsum_d(const float* x, float* out, int P, int D, int L, cudaStream_t st);
 cudaError_t launch_rowstat(const float* w, const float* s, float* wsum, float* swsum, float* ssum, int P, int R, int C4, cudaStream_t st);
 cudaError_t launch_vecsum(const float* x, float* out, int P, int L, cudaStream_t st);
@@ -274,6 +278,56 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
     return cudaSuccess;
 }
 
+// ------------------------------------------------------------------ short sequences: pair by pair
+// Whether the pairwise kernels beat the sorted walk, from two cost estimates fitted to measurements on a B200 (1 to 256 heads,
+// 64 to 4096 keys, 32 and 64 features, 32 to 128 channels). Both are good to about a fifth, and around the line the two
+// paths cost the same, so a case on the wrong side of it loses little.
+double dense_us(int kind, double P, int D, int N, int M, int C) {
+    // picoseconds per pair and feature, and per pair and channel, with three CTAs on every SM
+    const double per_d = kind == DENSE_LAPLACE ? 0.155 : kind == DENSE_BUMP ? 0.115 : 0.090, per_c = 0.027;
+    const int    sms = sm_count();
+    const double tile = 4096e-6 * sms * (D * per_d + (C <= 32 ? 32 : C <= 64 ? 64 : 128) * per_c);     // us of one SM per 64 x 64 pairs
+    const int    nt = (N + 63) / 64;
+    const double ctas = P * ((M + 63) / 64);
+    double best = 1e300;
+    for (int s = 1; s <= 8 && s <= nt; s *= 2) {                       // the kernel's own choice of CTAs per query tile, about
+        const double per_sm = std::ceil(ctas * s / sms), alone = per_sm < 2 ? 2.2 : per_sm < 3 ? 1.25 : 1.0;
+        best = std::min(best, per_sm * alone * ((nt + s - 1) / s + 0.5) * tile);
+    }
+    return 8.0 + best;
+}
+double sorted_us(int kind, double P, int D, int N, int M, int C) {
+    const double segs = P * D, wide = C <= 32 ? 0.6 : C <= 64 ? 1.0 : 4.0;      // the walks move rows of 32, 64 or 128 channels
+    const double keys = N * (0.022 + 0.045 * wide), queries = M * (0.022 + 0.050 * wide) * (kind == DENSE_BUMP ? 5.0 : 1.0);
+    return 70.0 + segs * (30.0 + keys + queries) * 1e-3;               // (launches and tails; nanoseconds per segment)
+}
+bool dense_pays(int kind, long long P, int D, int N, int M, int C) {
+    if (D > DENSE_MAX_D) return false;
+    return dense_us(kind, (double)P, D, N, M, C) < sorted_us(kind, (double)P, D, N, M, C);
+}
+
+// scratch of the pairwise kernels where they are the ones to run
+size_t dense_bytes(int kind, int P, int D, int N, int M, int C) {
+    return dense_pays(kind, P, D, N, M, C) ? dense_workspace_bytes(kind, P, D, N, M) : 0;
+}
+
+DenseArgs dense_args(const float* q, const float* k, const float* v, float* out, float* out_u, void* ws, int P, int D, int N, int M, int C) {
+    DenseArgs a{};
+    a.q = q; a.k = k; a.v = v; a.out = out; a.out_u = out_u;
+    a.P = P; a.H = 1; a.D = D; a.N = N; a.M = M; a.C = C;
+    a.scale = 1.0f;
+    a.staged = static_cast<float*>(ws);
+    return a;
+}
+
+// the attention entry points: (B, H, S, D) rows, scaled, masked, normalised
+DenseArgs dense_attention_args(const float* q, const float* k, const float* v, const float* keep, float* out, float tau, void* ws,
+                               int P, int H, int S, int D, int C) {
+    DenseArgs a = dense_args(q, k, v, out, nullptr, ws, P, D, S, S, C);
+    a.keep = keep; a.H = H; a.scale = 1.0f / tau; a.eps = 1e-3f; a.clamp = 1e-6f; a.rows_layout = true; a.normalise = true;
+    return a;
+}
+
 // ------------------------------------------------------------------ Laplace forward
 struct LaplaceWs {
     float* vpad; float* opad; Records rec; LapWalkScratch walk; size_t bytes;
@@ -375,7 +429,7 @@ int qlka_laplace_forward_workspace_bytes(int P, int D, int N, int M, int C, size
     if (!bytes) return QLKA_ERR_NULL;
     int st = check_dims(P, D, N, M, C);
     if (st) return st;
-    *bytes = LaplaceWs(nullptr, P, D, N, M, C).bytes;
+    *bytes = std::max(LaplaceWs(nullptr, P, D, N, M, C).bytes, dense_bytes(DENSE_LAPLACE, P, D, N, M, C));
     return QLKA_OK;
 }
 
@@ -387,6 +441,12 @@ static int laplace_forward_impl(const float* q, const float* k, const float* v,
     if (st) return st;
     if (!q || !k || !v || !out_w || !out_u) return QLKA_ERR_NULL;
     if (!aligned16(v, out_w)) return QLKA_ERR_ALIGNMENT;
+    if (dense_pays(DENSE_LAPLACE, P, D, N, M, C) && ws_ok(workspace, workspace_bytes, dense_workspace_bytes(DENSE_LAPLACE, P, D, N, M))) {
+        if (ev) for (int i = 0; i < 3; i++) CU(cudaEventRecord(ev[i], stream));
+        CU(launch_dense_forward(dense_args(q, k, v, out_w, out_u, workspace, P, D, N, M, C), DENSE_LAPLACE, sm_count(), stream));
+        if (ev) CU(cudaEventRecord(ev[3], stream));
+        return QLKA_OK;
+    }
     LaplaceWs ws(workspace, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     const int C4 = round4(C), nseg = P * D;
@@ -526,7 +586,7 @@ int qlka_laplace_attention_workspace_bytes(int B, int H, int S, int D, int Dv, i
     if (!bytes) return QLKA_ERR_NULL;
     int st = attn_check(B, H, S, D, Dv);
     if (st) return st;
-    *bytes = LaplaceAttnWs(nullptr, B, H, S, D, Dv, masked != 0).bytes;
+    *bytes = std::max(LaplaceAttnWs(nullptr, B, H, S, D, Dv, masked != 0).bytes, dense_bytes(DENSE_LAPLACE, B * H, D, S, S, Dv));
     return QLKA_OK;
 }
 
@@ -539,6 +599,12 @@ int qlka_laplace_attention_forward(const float* q, const float* k, const float* 
     if (!q || !k || !v || !out) return QLKA_ERR_NULL;
     if (!aligned16(v, out)) return QLKA_ERR_ALIGNMENT;
     if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
+    if (dense_pays(DENSE_LAPLACE, (long long)B * H, D, S, S, Dv)) {
+        if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(DENSE_LAPLACE, B * H, D, S, S))) return QLKA_ERR_WORKSPACE;
+        CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, tau, workspace, B * H, H, S, D, Dv), DENSE_LAPLACE, sm_count(),
+                                reinterpret_cast<cudaStream_t>(stream_)));
+        return QLKA_OK;
+    }
     const bool masked = keep != nullptr;
     LaplaceAttnWs ws(workspace, B, H, S, D, Dv, masked);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
@@ -562,7 +628,7 @@ int qlka_laplace_attention_forward(const float* q, const float* k, const float* 
 // ---------------------------------------------------------------- add_riesz / add_bump attention on (B, H, S, D)
 static int abs_forward_impl(const float* q, const float* k, const float* v, float* out_w, float* out_u,
                             void* workspace, size_t workspace_bytes, int P, int D, int N, int M, int C,
-                            int ns, const float* shifts, const float* weights, cudaStream_t stream);
+                            int ns, const float* shifts, const float* weights, cudaStream_t stream, bool walk = false);
 namespace {
 constexpr float BUMP_SHIFTS[3]  = {0.0f, 1.0f, -1.0f};     // max(0, 1 - |x|) = |x + 1| / 2 + |x - 1| / 2 - |x|
 constexpr float BUMP_WEIGHTS[3] = {-1.0f, 0.5f, 0.5f};
@@ -598,7 +664,7 @@ int qlka_abs_attention_workspace_bytes(int kind, int B, int H, int S, int D, int
     if (!bytes) return QLKA_ERR_NULL;
     int st = abs_attn_check(kind, B, H, S, D, Dv);
     if (st) return st;
-    *bytes = AbsAttnWs(nullptr, B, H, S, D, Dv, masked != 0, kind == 1).bytes;
+    *bytes = std::max(AbsAttnWs(nullptr, B, H, S, D, Dv, masked != 0, kind == 1).bytes, dense_bytes(kind == 1 ? DENSE_BUMP : DENSE_RIESZ, B * H, D, S, S, Dv));
     return QLKA_OK;
 }
 
@@ -612,6 +678,12 @@ int qlka_abs_attention_forward(int kind, const float* q, const float* k, const f
     if (!aligned16(v, out)) return QLKA_ERR_ALIGNMENT;
     if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
     const bool masked = keep != nullptr, bump = kind == 1;
+    if (const int dk = bump ? DENSE_BUMP : DENSE_RIESZ; dense_pays(dk, (long long)B * H, D, S, S, Dv)) {
+        if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(dk, B * H, D, S, S))) return QLKA_ERR_WORKSPACE;
+        CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, tau, workspace, B * H, H, S, D, Dv), dk, sm_count(),
+                                reinterpret_cast<cudaStream_t>(stream_)));
+        return QLKA_OK;
+    }
     AbsAttnWs ws(workspace, B, H, S, D, Dv, masked, bump);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
@@ -694,15 +766,21 @@ int qlka_abs_forward_workspace_bytes(int P, int D, int N, int M, int C, size_t* 
     if (!bytes) return QLKA_ERR_NULL;
     int st = check_dims(P, D, N, M, C);
     if (st) return st;
-    *bytes = AbsFwdWs(nullptr, P, D, N, M, C).bytes;
+    *bytes = std::max(AbsFwdWs(nullptr, P, D, N, M, C).bytes, dense_bytes(DENSE_ABS, P, D, N, M, C));
     return QLKA_OK;
 }
 
-// ns == 0: the plain abs sum. ns >= 1: sum_s weights[s] * abs_sum(q + shifts[s]) from one sort of the keys.
+// ns == 0: the plain abs sum. ns >= 1: sum_s weights[s] * abs_sum(q + shifts[s]) from one sort of the keys. walk: by the sorted walk
+// whatever the size.
 static int abs_forward_impl(const float* q, const float* k, const float* v, float* out_w, float* out_u,
                             void* workspace, size_t workspace_bytes, int P, int D, int N, int M, int C,
-                            int ns, const float* shifts, const float* weights, cudaStream_t stream)
+                            int ns, const float* shifts, const float* weights, cudaStream_t stream, bool walk)
 {
+    if (!ns && !walk && dense_pays(DENSE_ABS, P, D, N, M, C)) {
+        if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(DENSE_ABS, P, D, N, M))) return QLKA_ERR_WORKSPACE;
+        CU(launch_dense_forward(dense_args(q, k, v, out_w, out_u, workspace, P, D, N, M, C), DENSE_ABS, sm_count(), stream));
+        return QLKA_OK;
+    }
     const int MQ = ns ? ns * M : M;                 // queries per segment
     AbsFwdWs ws(workspace, P, D, N, MQ, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
@@ -748,7 +826,7 @@ int qlka_weighted_abs_sum_forward(const float* q, const float* k, const float* v
     if (!q || !k || !v || !out_w) return QLKA_ERR_NULL;
     if (!aligned16(v, out_w)) return QLKA_ERR_ALIGNMENT;
     return abs_forward_impl(q, k, v, out_w, out_u, workspace, workspace_bytes, P, D, N, M, C, 0, nullptr, nullptr,
-                            reinterpret_cast<cudaStream_t>(stream_));
+                            reinterpret_cast<cudaStream_t>(stream_), path == 0);
 }
 
 int qlka_abs_shifted_forward_workspace_bytes(int P, int D, int N, int M, int C, int n_shifts, size_t* bytes) {
