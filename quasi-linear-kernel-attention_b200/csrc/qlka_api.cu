@@ -103,8 +103,8 @@ WalkPlan plan_walk(int nseg, int N, int C4, bool laplace) {
     const int lps      = walk_lanes_per_stream(C4);
     const int streams  = walk_threads() / lps;       // streams per CTA and work item
     const int sms      = sm_count();
-    const int cap2     = sms * (C4 <= 64 ? 2 : 1);    // resident CTAs of the emitting pass (registers and shared memory)
-    const int cap1     = sms * (C4 <= 64 ? 3 : 1);    // ... and of the lighter first pass
+    const int cap2     = sms * 2;                      // resident CTAs of the emitting pass (registers and shared memory)
+    const int cap1     = sms * 3;                      // ... and of the lighter first pass
     const int nbk      = nblocks(N);
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
@@ -161,9 +161,8 @@ WalkArgs walk_args(const Records& r, const float* rows, int nseg, int D, int N, 
     return a;
 }
 
-// channels as the kernels see them: padded to the lane granularity of the walk (4 floats up to 64
-// channels, 8 floats above, where a lane owns 8 channels)
-inline int round4(int C) { return C <= 64 ? (C + 3) & ~3 : (C + 7) & ~7; }
+// channels as the kernels see them: padded to the lane granularity of the walk
+inline int round4(int C) { return (C + 3) & ~3; }
 
 // The row matrices (v, g_w, g, out_w, grad_v, the attention output) are read and written with 16-byte copies,
 // loads and vector reductions: a pointer off that boundary would fault on the device, so it is refused here.

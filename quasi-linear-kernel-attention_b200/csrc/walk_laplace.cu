@@ -434,12 +434,12 @@ template <int EMIT>
 static cudaError_t launch_lap_c(const WalkArgs& a, int grid1, int grid2, cudaStream_t stream, cudaEvent_t mid) {
     if (a.C4 <= 32)  return launch_lap<8, 4, EMIT>(a, grid1, grid2, stream, mid);
     if (a.C4 <= 64)  return launch_lap<16, 4, EMIT>(a, grid1, grid2, stream, mid);
-    if (a.C4 <= 128) return launch_lap<16, 8, EMIT>(a, grid1, grid2, stream, mid);
+    if (a.C4 <= 128) return launch_lap<32, 4, EMIT>(a, grid1, grid2, stream, mid);      // (16 lanes of 8 channels left one CTA per SM: half the speed)
     return cudaErrorInvalidValue;
 }
 
 // lanes per stream for a padded channel count
-int walk_lanes_per_stream(int C4) { return C4 <= 32 ? 8 : 16; }
+int walk_lanes_per_stream(int C4) { return C4 <= 32 ? 8 : C4 <= 64 ? 16 : 32; }
 int walk_threads() { return WALK_THREADS; }
 
 int laplace_agg_stride(int C4) { return lap_agg_stride(C4); }

@@ -400,7 +400,7 @@ cudaError_t launch_prefix_walk(const WalkArgs& a, int emit, int grid1, int grid2
     if (emit != EMIT_ROWS && emit != EMIT_DOT && emit != EMIT_BOTH) return cudaErrorInvalidValue;
     if (a.C4 <= 32)  return launch_pw<8, 4>(a, emit, grid1, grid2, stream);
     if (a.C4 <= 64)  return launch_pw<16, 4>(a, emit, grid1, grid2, stream);
-    if (a.C4 <= 128) return launch_pw<16, 8>(a, emit, grid1, grid2, stream);
+    if (a.C4 <= 128) return launch_pw<32, 4>(a, emit, grid1, grid2, stream);
     return cudaErrorInvalidValue;
 }
 

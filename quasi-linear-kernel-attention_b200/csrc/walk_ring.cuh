@@ -221,18 +221,27 @@ struct Feeder {
         cp_async_commit();
     }
     // Partial dots of query n of the block in `slot`: LPS floats inside the stream's share (LPS x 16 bytes) of row
-    // (n mod 8) of the slot, at a word offset that puts the LPS lanes' reads of LPS different queries in different banks.
+    // (n mod 8) of the slot, placed so that the LPS lanes' reads of LPS different queries fall in different banks: shifted
+    // by n words, or, where a share has no room for that (LPS = 32), rotated by n. The two streams of a warp (LPS = 16)
+    // start half a query apart, so that they do not meet in a bank while a block has up to 8 queries.
     __device__ __forceinline__ uint32_t part_addr(const int slot, const uint32_t n) const {
-        return ring_s - ln * 16 + slot * ring_slot_bytes<CPL>() + (n & 7u) * (WALK_THREADS * 16) + ((n >> 3) * 32u + n) * 4u;
+        const uint32_t at = LPS == 32 ? (n >> 3) * (LPS * 4u) : ((n >> 3) * 32u + n) * 4u;
+        return ring_s - ln * 16 + slot * ring_slot_bytes<CPL>() + (n & 7u) * (WALK_THREADS * 16) + at;
     }
     __device__ __forceinline__ void put_part(const int slot, const uint32_t n, const float acc) const {
-        sts32f(part_addr(slot, n) + ln * 4, acc);
+        sts32f(part_addr(slot, n) + (LPS == 32 ? (ln + n) & (LPS - 1) : ln) * 4, acc);
     }
     __device__ __forceinline__ float sum_parts(const int slot, const uint32_t n) const {
         const uint32_t p = part_addr(slot, n);
         float s0 = 0.0f, s1 = 0.0f;
-        #pragma unroll
-        for (int k = 0; k < LPS; k += 2) { s0 += lds32f(p + 4 * k); s1 += lds32f(p + 4 * k + 4); }
+        if (LPS == 32) {
+            #pragma unroll
+            for (uint32_t k = 0; k < LPS; k += 2) { s0 += lds32f(p + ((k + n) & (LPS - 1)) * 4); s1 += lds32f(p + ((k + 1 + n) & (LPS - 1)) * 4); }
+        } else {
+            const uint32_t half = LPS == 16 ? (threadIdx.x & 16u) * 2u : 0u;          // bytes: 8 words for the second stream
+            #pragma unroll
+            for (int k = 0; k < LPS / 2; k++) { s0 += lds32f(p + half + 4 * k); s1 += lds32f(p - half + 4 * (k + LPS / 2)); }
+        }
         return s0 + s1;
     }
     __device__ __forceinline__ void read_g(const uint32_t n, Vec<CPL>& gq) const {
