@@ -62,6 +62,23 @@ struct SortArgs {
     int   rows_coef;          // abs mode: 1 = e1 is the key-sum coefficient -2 * weight of the row emission, 0 = e1 is a dot addend
 };
 
+// A long segment is cut by value into parts that the shared-memory sort/rank kernel holds (sort_rank_large.cu). Part i of a
+// segment has the keys of sorted positions ks .. ks + n - 1 and the queries of record positions qs .. qs + m - 1.
+constexpr int PART_CAP = 8192;              // keys per part
+struct PartInfo {
+    int   ks, n, qs, m;
+    float prevmax, nextmin;                 // largest key before the part, smallest after it
+    float lin, rin;                         // scalar scan state of the keys before (at prevmax) and after (at nextmin); abs: sum before
+};
+struct PartArgs {
+    const uint32_t* kkey;                   // [seg][N] keys (f2key) grouped by part, any order inside
+    const uint32_t* kidx;                   // [seg][N] their indices in the segment
+    const float*    qval;                   // [seg][M] queries grouped by part
+    const uint32_t* qidx;                   // [seg][M]
+    const PartInfo* info;                   // [seg][maxparts], n = 0 beyond the last part
+    int maxparts;
+};
+
 struct WalkArgs {
     const float*    rows;     // (P, N, C4) rows the stream points at; C4 = channels padded to 4 (<= 64) or 8 floats
     const uint32_t* xperm;

@@ -177,6 +177,18 @@ __device__ __forceinline__ void load_segment(const float* __restrict__ src, cons
     }
 }
 
+template <int THREADS, int E>
+__device__ __forceinline__ void load_part(const uint32_t* __restrict__ src, const int n, uint32_t (&key)[E], uint32_t (&idx)[E])
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    #pragma unroll
+    for (int s = 0; s < E; s++) {
+        const int pos = warp * 32 * E + s * 32 + lane;
+        key[s] = pos < n ? __ldg(src + pos) : 0xffffffffu;
+        idx[s] = pos;
+    }
+}
+
 // ------------------------------------------------------------------ block scans
 // x_j = A_j x_{j-1} + B_j, inclusive, x_{-1} = 0, over scan positions 0..n-1. Every thread owns
 // the contiguous run [i0, i1) and passes the coefficients of its run in registers
@@ -317,8 +329,8 @@ __host__ __device__ constexpr int sort_buckets(int threads, int e) {
     return threads == 1024 ? threads * e - threads * e / 32 : threads * e / 2;
 }
 
-template <int THREADS, int E, int VAR>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const SortArgs a)
+template <int THREADS, int E, int VAR, bool PART>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const SortArgs a, const PartArgs pa)
 {
     constexpr bool LAP = VAR == VAR_LAP || VAR == VAR_LAP_SIGNED, SIGNED = VAR == VAR_LAP_SIGNED, FOLD = VAR == VAR_ABS_FOLD;
     constexpr int CAP = THREADS * E;
@@ -337,17 +349,31 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     uint2*    tab  = reinterpret_cast<uint2*>(xs);                  // (mask, count) table of the radix sort (E = 16), idle by the time xs is filled
 
     const int tid = threadIdx.x;
-    const int seg = blockIdx.x;
+    const int seg = PART ? blockIdx.x / pa.maxparts : blockIdx.x;
     const int p   = seg / a.D;
-    const int N = a.N, M = a.M;
-    const int NP = npad(N), NBK = nblocks(N);
+    // a part: keys ks .. ks + N - 1 of the segment's sorted order, queries qs .. qs + M - 1 of its record order; the lists
+    // give each its index in the segment
+    PartInfo pi{};
+    if (PART) {
+        pi = pa.info[blockIdx.x];
+        if (pi.n == 0) return;
+    }
+    const int NG = a.N, MG = a.M;                                   // keys and queries of the whole segment
+    const int N = PART ? pi.n : NG, M = PART ? pi.m : MG, ks = PART ? pi.ks : 0, qs = PART ? pi.qs : 0;
+    const int NP = npad(NG), NBK = nblocks(NG);
+    const bool first = ks == 0, last = ks + N == NG;
+    const uint32_t* kkey = PART ? pa.kkey + (long long)seg * NG + ks : nullptr;
+    const uint32_t* kidx = PART ? pa.kidx + (long long)seg * NG + ks : nullptr;
+    const uint32_t* qidx = PART ? pa.qidx + (long long)seg * MG + qs : nullptr;
 
-    uint32_t* xperm  = a.xperm + (long long)seg * NP;
-    float*    xval   = a.xval + (long long)seg * xstride(N);
-    uint4*    yrec   = a.yrec + (long long)seg * (M + 1);
-    uint32_t* mstart = a.mstart + (long long)seg * mstride(N);
-    float*    su0    = a.su0 ? a.su0 + (long long)seg * (N + 1) : nullptr;
-    float*    su1    = a.su1 ? a.su1 + (long long)seg * (N + 1) : nullptr;
+    uint32_t* xperm  = a.xperm + (long long)seg * NP + ks;
+    float*    xval   = a.xval + (long long)seg * xstride(NG) + ks;
+    uint4*    yrec   = a.yrec + (long long)seg * (MG + 1) + qs;
+    uint32_t* mstart = a.mstart + (long long)seg * mstride(NG);
+    float*    su0    = a.su0 ? a.su0 + (long long)seg * (NG + 1) + ks : nullptr;
+    float*    su1    = a.su1 ? a.su1 + (long long)seg * (NG + 1) + ks : nullptr;
+    auto key_row = [&](const uint32_t i) -> uint32_t { return PART ? __ldg(kidx + i) : i; };
+    auto query_row = [&](const int m) -> int { return PART ? (int)__ldg(qidx + m) : m; };
     PHASE_BEGIN();
     // ---- (1) keys
     // NB equal-width value buckets between the smallest and the largest key; the bucket of a value is a monotone
@@ -364,7 +390,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     bool by_radix;
     {
         uint32_t key[E], idx[E];
-        load_segment<THREADS, E>(a.x + (long long)seg * N, N, key, idx);
+        if (PART) load_part<THREADS, E>(kkey, N, key, idx);
+        else      load_segment<THREADS, E>(a.x + (long long)seg * N, N, key, idx);
         PHASE_MARK(0);
         const int warp = tid >> 5, lane = tid & 31;
         uint32_t* hw = reinterpret_cast<uint32_t*>(bst);           // the bucket counters: NB + 1 of 16 bits, two to a word
@@ -474,7 +501,14 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         for (int t = bucket(key2f(skey[N - 1])) + 1 + tid; t <= NB; t += THREADS) bst[t] = (uint16_t)N;
     }
     __syncthreads();
-    for (int j = tid; j < NP; j += THREADS) xperm[j] = j < N ? (uint32_t)sidx[j] : 0u;
+    if (PART) {
+        // the list's indices through the idle sort buffer: scattered 4-byte reads of global memory cost about 2 cycles each per SM
+        #pragma unroll 4
+        for (int j = tid; j < N; j += THREADS) skey[j] = __ldg(kidx + j);
+        __syncthreads();
+    }
+    for (int j = tid; j < N; j += THREADS) xperm[j] = PART ? skey[sidx[j]] : (uint32_t)sidx[j];
+    if (last) for (int j = N + tid; j < NP - ks; j += THREADS) xperm[j] = 0u;
     __syncthreads();
     PHASE_MARK(2);
     // ---- (2) per-key scalars; my run of keys is [i0, i0 + cntk). The run length is odd so that the
@@ -500,9 +534,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
             for (int j = tid; j < N; j += THREADS) {
                 const float d = j > 0 ? decay_of(xs[skew(j)] - xs[skew(j - 1)]) : 0.0f;
                 stage[j] = d;
-                xval[j]  = d;
+                xval[j]  = PART && j == 0 && !first ? decay_of(xs[0] - pi.prevmax) : d;      // (the scans below start anew in each part)
             }
-            for (int j = N + tid; j < NP + KB; j += THREADS) xval[j] = 1.0f;
+            if (last) for (int j = N + tid; j < NP - ks + KB; j += THREADS) xval[j] = 1.0f;
             __syncthreads();
             #pragma unroll
             for (int k = 0; k <= R; k++) {
@@ -515,10 +549,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                 // (all ones without one). The scalars wait in the staging buffer, every thread touching only its own run,
                 // because su0s overwrites the index payload; the backward scan runs in place there and leaves through it.
                 {
-                    const float* us = a.us ? a.us + (long long)p * N : nullptr;
+                    const float* us = a.us ? a.us + (long long)p * NG : nullptr;
                     __syncthreads();                  // every thread has picked its decays out of the staging buffer
                     #pragma unroll
-                    for (int k = 0; k < R; k++) if (k < cntk) stage[i0 + k] = us ? us[sidx[i0 + k]] : 1.0f;
+                    for (int k = 0; k < R; k++) if (k < cntk) stage[i0 + k] = us ? us[key_row(sidx[i0 + k])] : 1.0f;
                 }
                 block_affine_scan_mem<THREADS, R, false, 0>(cntk, i0, dk, stage, su0s, wa, wb);
                 block_affine_scan_mem<THREADS, R, true, 1>(cntk, i0, dk, stage, stage, wa, wb);
@@ -538,16 +572,18 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                 flush(bx, su1);
             }
         } else {
-            if (a.mode == MODE_ABS)
-                for (int j = tid; j < NP + KB; j += THREADS) xval[j] = j < N ? xs[skew(j)] : 0.0f;
+            if (a.mode == MODE_ABS) {
+                for (int j = tid; j < N; j += THREADS) xval[j] = xs[skew(j)];
+                if (last) for (int j = N + tid; j < NP - ks + KB; j += THREADS) xval[j] = 0.0f;
+            }
             if (a.scal == SCAL_UNIT || a.scal == SCAL_PREFIX) {
                 // su0[j] = sum_{i<=j} k_i   or   sum_{i<=j} us[row of key i]
-                const float* us = a.scal == SCAL_PREFIX ? a.us + (long long)p * N : nullptr;
+                const float* us = a.scal == SCAL_PREFIX ? a.us + (long long)p * NG : nullptr;
                 float bx[R];
                 #pragma unroll
                 for (int k = 0; k <= R; k++) dk[k] = 1.0f;
                 #pragma unroll
-                for (int k = 0; k < R; k++) bx[k] = k < cntk ? (us ? us[sidx[i0 + k]] : xs[skew(i0 + k)]) : 0.0f;
+                for (int k = 0; k < R; k++) bx[k] = k < cntk ? (us ? us[key_row(sidx[i0 + k])] : xs[skew(i0 + k)]) : 0.0f;
                 block_affine_scan<THREADS, R, false, 0>(cntk, dk, bx, wa, wb);
                 flush(bx, su0);
             }
@@ -559,9 +595,48 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     uint32_t* hist = skey;                                         // N + 1 bins
     for (int i = tid; i <= N; i += THREADS) hist[i] = 0;
     __syncthreads();
-    const int    MR   = FOLD ? a.fold : M;            // distinct query values (and output rows) per segment
-    const float* ysrc = a.y + (long long)seg * MR;
+    const int    MR   = FOLD ? a.fold : MG;           // distinct query values (and output rows) per segment
+    const float* ysrc = PART ? pa.qval + (long long)seg * MG + qs : a.y + (long long)seg * MR;
     auto yval = [&](int m) -> float { return FOLD ? ysrc[m % MR] + a.shift[m / MR] : ysrc[m]; };
+    constexpr bool lap = LAP;
+    // e^{-gap} for the query weights: one ex2.approx (relative error ~ (2 + 1.2 gap) ulp; these weights enter each
+    // output once, unlike the step decays, which multiply into every prefix state and are taken with expm1)
+    auto wexp = [](const float gap) -> float { return __expf(-gap); };
+    // The scalar side channel of a query with value y and r keys of this part below it; su0 / su1 at r - 1 and r come from `s0`
+    // and `s1`. Parts add what lies beyond their ends: the state of the keys below, decayed from the last of them, and above.
+    const bool side = a.scal == SCAL_UNIT || (SIGNED && a.scal == SCAL_SIGNED);
+    auto side_channel = [&](const int m, const int row, const int r, const float y, const float* s0, const float* s1) {
+        const float wq = FOLD ? a.wgt[m / MR] : 1.0f;
+        if (lap) {
+            float t0 = r > 0 ? wexp(y - xs[skew(r - 1)]) * s0[r - 1] : 0.0f;
+            float t1 = r < N ? wexp(xs[skew(r)] - y) * s1[r] : 0.0f;
+            if (PART) {
+                if (!first) t0 += wexp(y - pi.prevmax) * pi.lin;
+                if (!last)  t1 += wexp(pi.nextmin - y) * pi.rin;
+            }
+            if (a.scal == SCAL_UNIT) atomicAdd(a.out_u + (long long)p * MR + row, t0 + t1);
+            else a.out_s[(long long)seg * MG + row] = (a.uq ? a.uq[(long long)p * MG + row] : 1.0f) * (t1 - t0);
+        } else {
+            float below = r > 0 ? s1[r - 1] : 0.0f;
+            if (PART) below += pi.lin;
+            atomicAdd(a.out_u + (long long)p * MR + row, wq * 2.0f * (y * (float)(ks + r) - below));
+        }
+    };
+    auto record = [&](const int m, const int row, const int r, const float y) -> uint4 {
+        const float wq = FOLD ? a.wgt[m / MR] : 1.0f;
+        float e0 = 0.0f, e1 = 0.0f;
+        if (lap) {
+            if (r > 0)                e0 = wexp(y - xs[skew(r - 1)]);
+            else if (PART && !first)  e0 = wexp(y - pi.prevmax);
+            if (r < N)                e1 = wexp(xs[skew(r)] - y);
+            else if (PART && !last)   e1 = wexp(pi.nextmin - y);
+        } else {
+            if (a.mode == MODE_ABS) { e0 = 2.0f * y * wq; e1 = a.rows_coef ? -2.0f * wq : 0.0f; }      // row emission: e0 * PV + e1 * PK
+            if (a.scal == SCAL_RANK)        e1 = a.uq[(long long)p * MG + row] * (2.0f * (float)(ks + r) - (float)NG);
+            else if (a.scal == SCAL_PREFIX) e1 = 2.0f * ((PART ? pi.lin : 0.0f) + (r > 0 ? su0[r - 1] : 0.0f)) - a.us_total[p];
+        }
+        return make_uint4(__float_as_uint(e0), __float_as_uint(e1), (uint32_t)row, (uint32_t)(ks + r));
+    };
     uint32_t rp[E];                                   // rank, later rank | position << 16 (both <= 16384)
     // Slot s of a thread is query tid + ((s + rot) mod E) * THREADS with rot the segment index: the D segments of a head
     // run at the same time and all add into the same out_u row, and with a common visiting order their atomics would
@@ -570,41 +645,83 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     auto mq = [&](const int s) -> int { return tid + ((s + rot) & (E - 1)) * THREADS; };
     // QI searches in flight per thread (the probes are latency bound); the loop runs until the thread's longest is done
     constexpr int QI = E >= 8 ? 8 : 4;
-    #pragma unroll
-    for (int s0 = 0; s0 < E; s0 += QI) {
-        int   lo[QI], hi[QI];
-        float yq[QI];
-        bool  open = false;
+    auto rank_queries = [&](const int c0) {           // rp = ranks of the queries c0 + mq(s)
         #pragma unroll
-        for (int t = 0; t < QI; t++) {
-            const int m = mq(s0 + t);
-            yq[t] = m < M ? yval(m) : 0.0f;
-            const int b = bucket(yq[t]);
-            lo[t] = bst[b]; hi[t] = bst[b + 1];
-            open |= lo[t] < hi[t];
-        }
-        while (open) {
-            open = false;
+        for (int s0 = 0; s0 < E; s0 += QI) {
+            int   lo[QI], hi[QI];
+            float yq[QI];
+            bool  open = false;
             #pragma unroll
             for (int t = 0; t < QI; t++) {
-                if (lo[t] < hi[t]) {
-                    const int mid = (lo[t] + hi[t]) >> 1;
-                    if (xs[skew(mid)] < yq[t]) lo[t] = mid + 1; else hi[t] = mid;
-                    open |= lo[t] < hi[t];
+                const int m = c0 + mq(s0 + t);
+                yq[t] = m < M ? yval(m) : 0.0f;
+                const int b = bucket(yq[t]);
+                lo[t] = bst[b]; hi[t] = bst[b + 1];
+                open |= lo[t] < hi[t];
+            }
+            while (open) {
+                open = false;
+                #pragma unroll
+                for (int t = 0; t < QI; t++) {
+                    if (lo[t] < hi[t]) {
+                        const int mid = (lo[t] + hi[t]) >> 1;
+                        if (xs[skew(mid)] < yq[t]) lo[t] = mid + 1; else hi[t] = mid;
+                        open |= lo[t] < hi[t];
+                    }
                 }
             }
+            #pragma unroll
+            for (int t = 0; t < QI; t++) rp[s0 + t] = (uint32_t)lo[t];       // number of keys strictly below the query
         }
+    };
+    // More queries than the kernel holds (only a part can have them: values far denser there than the keys): a first sweep
+    // counts them, a second ranks them again and writes side channel and records one by one.
+    auto count_ranks = [&](const int c0) {
         #pragma unroll
-        for (int t = 0; t < QI; t++) rp[s0 + t] = (uint32_t)lo[t];       // number of keys strictly below the query
+        for (int s = 0; s < E; s++) if (c0 + mq(s) < M) atomicAdd(&hist[rp[s]], 1u);
+    };
+    auto scan_ranks = [&]() {
+        __syncthreads();
+        block_exclusive_sum<THREADS, E>(hist, N + 1, wsum);
+        __syncthreads();
+        // mstart of every block that starts at one of this part's ranks: (ks, ks + N], and rank 0 in the first part
+        for (int b = (ks + (first ? 0 : 1) + KB - 1) / KB + tid; b * KB <= ks + N; b += THREADS) mstart[b] = (uint32_t)qs + hist[b * KB - ks];
+        if (first && tid == 0) {
+            mstart[NBK] = (uint32_t)MG;
+            a.yrec[(long long)seg * (MG + 1) + MG] = make_uint4(0u, 0u, 0u, 0xffffffffu);      // sentinel: a rank no key position has
+        }
+        __syncthreads();
+    };
+    if constexpr (!PART) {
+        rank_queries(0);
+        PHASE_MARK(4);
+        count_ranks(0);
+        scan_ranks();
+    } else {
+        const bool many = M > CAP;
+        #pragma unroll 1
+        for (int sweep = 0; sweep < (many ? 2 : 1); sweep++) {
+            #pragma unroll 1
+            for (int c0 = 0; c0 < M; c0 += CAP) {
+                rank_queries(c0);
+                if (sweep == 0) { count_ranks(c0); continue; }
+                #pragma unroll 1
+                for (int s = 0; s < E; s++) {
+                    const int m = c0 + mq(s);
+                    if (m >= M) continue;
+                    uint32_t rank = 0;
+                    #pragma unroll
+                    for (int t = 0; t < E; t++) if (t == s) rank = rp[t];
+                    const int   r = (int)rank, row = query_row(m);
+                    const float y = yval(m);
+                    if (side) side_channel(m, row, r, y, su0s, lap ? su1 : su0);
+                    yrec[atomicAdd(&hist[r], 1u)] = record(m, row, r, y);
+                }
+            }
+            if (sweep == 0) scan_ranks();
+        }
+        if (many) return;
     }
-    PHASE_MARK(4);
-    #pragma unroll
-    for (int s = 0; s < E; s++) if (mq(s) < M) atomicAdd(&hist[rp[s]], 1u);
-    __syncthreads();
-    block_exclusive_sum<THREADS, E>(hist, N + 1, wsum);
-    __syncthreads();
-    for (int b = tid; b <= NBK; b += THREADS) mstart[b] = b == NBK ? (uint32_t)M : hist[b * KB];     // b*KB <= N for b < NBK
-    __syncthreads();
     #pragma unroll
     for (int s = 0; s < E; s++)
         if (mq(s) < M) rp[s] |= atomicAdd(&hist[rp[s]], 1u) << 16;       // final position of the record
@@ -620,17 +737,13 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     //   B  the query's value and (index | rank << 16) go to shared memory at the record's position - the value into
     //      the forward-scan array, which step A was the last to read;
     //   C  in position order: weights from the two neighbouring keys, record written.
-    constexpr bool lap = LAP;
-    // e^{-gap} for the query weights: one ex2.approx (relative error ~ (2 + 1.2 gap) ulp; these weights enter each
-    // output once, unlike the step decays, which multiply into every prefix state and are taken with expm1)
-    auto wexp = [](const float gap) -> float { return __expf(-gap); };
     float yv[E];                                      // the thread's query values again, all loads in flight together
     #pragma unroll
     for (int s = 0; s < E; s++) {
         const int m = mq(s);
         yv[s] = m < M ? (FOLD ? __ldg(ysrc + m % MR) + a.shift[m / MR] : __ldg(ysrc + m)) : 0.0f;
     }
-    if (a.scal == SCAL_UNIT || (SIGNED && a.scal == SCAL_SIGNED)) {
+    if (side) {
         float*       suq   = reinterpret_cast<float*>(skey);
         const float* susrc = lap ? su1 : su0;
         #pragma unroll 8
@@ -639,23 +752,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         #pragma unroll
         for (int s = 0; s < E; s++) {
             const int m = mq(s);
-            if (m >= M) continue;
-            const int   r   = (int)(rp[s] & 0xffffu);
-            const float y   = yv[s];
-            const int   row = FOLD ? m % MR : m;
-            const float wq  = FOLD ? a.wgt[m / MR] : 1.0f;
-            if (lap) {
-                const float t0 = r > 0 ? wexp(y - xs[skew(r - 1)]) * su0s[r - 1] : 0.0f;
-                const float t1 = r < N ? wexp(xs[skew(r)] - y) * suq[r] : 0.0f;
-                if (a.scal == SCAL_UNIT) atomicAdd(a.out_u + (long long)p * MR + row, t0 + t1);
-                else a.out_s[(long long)seg * M + m] = (a.uq ? a.uq[(long long)p * M + m] : 1.0f) * (t1 - t0);
-            } else {
-                atomicAdd(a.out_u + (long long)p * MR + row, wq * 2.0f * (y * (float)r - (r > 0 ? suq[r - 1] : 0.0f)));
-            }
+            if (m < M) side_channel(m, FOLD ? m % MR : query_row(m), (int)(rp[s] & 0xffffu), yv[s], su0s, suq);
         }
     }
     __syncthreads();
     PHASE_MARK(8);
+    constexpr int WHO = PART ? 18 : 16;               // row (a part's: below 2^18) and rank (at most 16384, a part's 8192) in one word
     uint32_t* who  = skey;
     float*    ypos = su0s;
     #pragma unroll
@@ -663,7 +765,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         const int m = mq(s);
         if (m < M) {
             const uint32_t pos = rp[s] >> 16;
-            who[pos]  = (uint32_t)m | (rp[s] << 16);
+            who[pos]  = (uint32_t)(PART ? query_row(m) : m) | ((rp[s] & 0xffffu) << WHO);
             ypos[pos] = yv[s];
         }
     }
@@ -672,45 +774,41 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     #pragma unroll 4
     for (int pos = tid; pos < M; pos += THREADS) {
         const uint32_t w = who[pos];
-        const int      m = (int)(w & 0xffffu), r = (int)(w >> 16);
-        const float    y   = ypos[pos];
-        const int      row = FOLD ? m % MR : m;
-        const float    wq  = FOLD ? a.wgt[m / MR] : 1.0f;
-        float e0 = 0.0f, e1 = 0.0f;
-        if (lap) {
-            e0 = r > 0 ? wexp(y - xs[skew(r - 1)]) : 0.0f;
-            e1 = r < N ? wexp(xs[skew(r)] - y) : 0.0f;
-        } else {
-            if (a.mode == MODE_ABS) { e0 = 2.0f * y * wq; e1 = a.rows_coef ? -2.0f * wq : 0.0f; }      // row emission: e0 * PV + e1 * PK
-            if (a.scal == SCAL_RANK)        e1 = a.uq[(long long)p * M + m] * (2.0f * (float)r - (float)N);
-            else if (a.scal == SCAL_PREFIX) e1 = 2.0f * (r > 0 ? su0[r - 1] : 0.0f) - a.us_total[p];
-        }
-        yrec[pos] = make_uint4(__float_as_uint(e0), __float_as_uint(e1), (uint32_t)row, (uint32_t)r);
+        const int      m = (int)(w & ((1u << WHO) - 1u)), r = (int)(w >> WHO);
+        yrec[pos] = record(m, FOLD ? m % MR : m, r, ypos[pos]);
     }
-    if (tid == 0) yrec[M] = make_uint4(0u, 0u, 0u, 0xffffffffu);      // sentinel: a rank no key position has
     PHASE_MARK(6);
 }
 
 
 
-template <int THREADS, int E, int VAR>
-static cudaError_t launch_inst(const SortArgs& a, cudaStream_t stream) {
+template <int THREADS, int E, int VAR, bool PART>
+static cudaError_t launch_inst(const SortArgs& a, const PartArgs& pa, cudaStream_t stream) {
     constexpr int CAP = THREADS * E;
     constexpr int W   = THREADS / 32;
     const size_t smem = (size_t)CAP * 4 * 2 + 32 * 4 + (size_t)(CAP / 32 + 32) * 4 + (size_t)W * 256 * 4 + 256 * 4 + 32 * 4 * 3 + (size_t)CAP * 2
                       + (size_t)(sort_buckets(THREADS, E) + 8) * 2;
-    auto kern = sort_rank_small<THREADS, E, VAR>;
+    auto kern = sort_rank_small<THREADS, E, VAR, PART>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<a.nseg, THREADS, smem, stream>>>(a);
+    kern<<<PART ? a.nseg * pa.maxparts : a.nseg, THREADS, smem, stream>>>(a, pa);
     return cudaGetLastError();
 }
 
 template <int THREADS, int E>
 static cudaError_t launch_one(const SortArgs& a, cudaStream_t stream) {
+    const PartArgs none{};
     if (a.mode == MODE_LAPLACE)
-        return a.scal == SCAL_SIGNED ? launch_inst<THREADS, E, VAR_LAP_SIGNED>(a, stream) : launch_inst<THREADS, E, VAR_LAP>(a, stream);
-    return a.fold ? launch_inst<THREADS, E, VAR_ABS_FOLD>(a, stream) : launch_inst<THREADS, E, VAR_ABS>(a, stream);
+        return a.scal == SCAL_SIGNED ? launch_inst<THREADS, E, VAR_LAP_SIGNED, false>(a, none, stream) : launch_inst<THREADS, E, VAR_LAP, false>(a, none, stream);
+    return a.fold ? launch_inst<THREADS, E, VAR_ABS_FOLD, false>(a, none, stream) : launch_inst<THREADS, E, VAR_ABS, false>(a, none, stream);
+}
+
+// the parts of long segments (sort_rank_large.cu): up to PART_CAP keys each, two CTAs per SM
+cudaError_t launch_sort_rank_parts(const SortArgs& a, const PartArgs& pa, cudaStream_t stream) {
+    constexpr int T = 512, E = PART_CAP / T;
+    if (a.mode == MODE_LAPLACE)
+        return a.scal == SCAL_SIGNED ? launch_inst<T, E, VAR_LAP_SIGNED, true>(a, pa, stream) : launch_inst<T, E, VAR_LAP, true>(a, pa, stream);
+    return launch_inst<T, E, VAR_ABS, true>(a, pa, stream);
 }
 
 // max(N, M) <= 16384
