@@ -134,6 +134,22 @@ int qlka_abs_attention_forward(int kind, const float* q, const float* k, const f
                                float tau, float* out, void* workspace, size_t workspace_bytes,
                                int B, int H, int S, int D, int Dv, qlka_stream_t stream);
 
+/* The three attentions for training: kind 0 = add_riesz, 1 = add_bump, 2 = add_laplace. The forward call is the ones above and
+ * also writes den (B, H, S), the row sums before their floor (NULL: not wanted), which the backward call takes together with the
+ * output and its gradient. grad_q and grad_k (B, H, S, D), grad_v (B, H, S, Dv); masked keys get zero gradients. The derivative
+ * where a key equals a query (add_bump: or is exactly one away) is that of the operators' backward passes. The size query
+ * answers QLKA_ERR_UNSUPPORTED where there is no single call (long sequences of kinds 0 and 1): there the gradient is assembled
+ * from the abs sum's. */
+int qlka_attention_workspace_bytes(int kind, int B, int H, int S, int D, int Dv, int masked, size_t* bytes);
+int qlka_attention_forward(int kind, const float* q, const float* k, const float* v, const float* keep /* nullable */, float tau,
+                           float* out, float* den /* nullable */, void* workspace, size_t workspace_bytes,
+                           int B, int H, int S, int D, int Dv, qlka_stream_t stream);
+int qlka_attention_backward_workspace_bytes(int kind, int B, int H, int S, int D, int Dv, int masked, size_t* bytes);
+int qlka_attention_backward(int kind, const float* q, const float* k, const float* v, const float* keep /* nullable */, float tau,
+                            const float* out, const float* den, const float* grad_out,
+                            float* grad_q, float* grad_k, float* grad_v, void* workspace, size_t workspace_bytes,
+                            int B, int H, int S, int D, int Dv, qlka_stream_t stream);
+
 /* ---- weighted abs sum, forward ---------------------------------------------------------
  * out_w[p,m,c] = sum_{d,n} |k[p,d,n] - q[p,d,m]| v[p,n,c]           (P, M, C)
  * out_u[p,m]   = sum_{d,n} |k[p,d,n] - q[p,d,m]|                    (P, M), optional (NULL)

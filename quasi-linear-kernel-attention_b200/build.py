@@ -1,34 +1,55 @@
-"""Builds the CUDA library (libqlka.so, next to this file) for sm_100a with nvcc.
+"""Builds the CUDA library (libqlka.so, next to this file) for sm_100a with nvcc, and the torch binding over it
+(_qlka_torch.so) with g++.
 
     python quasi-linear-kernel-attention_b200/build.py [--force] [--verbose]
 
-Plain nvcc, no torch headers: the library's ABI is the C header include/qlka.h.
+The library is plain nvcc, no torch headers: its ABI is the C header include/qlka.h. The binding is the only file that
+sees torch.
 """
 
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libqlka.so")
-SOURCES = ["qlka_api.cu", "sort_rank.cu", "sort_rank_large.cu", "walk_laplace.cu", "walk_prefix.cu", "dense_tiles.cu", "aux_kernels.cu"]
+SOURCES = ["qlka_api.cu", "sort_rank.cu", "sort_rank_large.cu", "walk_laplace.cu", "walk_prefix.cu", "dense_tiles.cu", "dense_gradient.cu", "aux_kernels.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
          "-Xcompiler", "-fPIC", "--threads", "4"]
 
 
-def _stale():
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "qlka.h"), os.path.abspath(__file__)]
-    return any(os.path.getmtime(d) > t for d in deps)
+BINDING = os.path.join(HERE, "_qlka_torch.so")
+BINDING_SOURCE = os.path.join(CSRC, "torch_binding.cpp")
+HEADER = os.path.join(HERE, "..", "include", "qlka.h")
+
+
+def _stale(target, deps):
+    return not os.path.exists(target) or any(os.path.getmtime(d) > os.path.getmtime(target) for d in [*deps, HEADER, os.path.abspath(__file__)])
+
+
+def build_binding(force=False, verbose=False):
+    """Compile the torch binding; returns the path."""
+    if not force and not _stale(BINDING, [BINDING_SOURCE]):
+        return BINDING
+    import torch
+    from torch.utils import cpp_extension
+    libs = [d for d in cpp_extension.library_paths() if os.path.isdir(d)]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_qlka_torch", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in [*cpp_extension.include_paths(), "/usr/local/cuda/include", sysconfig.get_paths()["include"]]],
+           BINDING_SOURCE, "-o", BINDING, *[f"-L{d}" for d in libs], "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-ldl"]
+    if verbose:
+        print(" ".join(cmd))
+    subprocess.check_call(cmd)
+    return BINDING
 
 
 def build(force=False, verbose=False):
-    """Compile every .cu of csrc/ into libqlka.so; returns the path."""
-    if not force and not _stale():
+    """Compile every .cu of csrc/ into libqlka.so, and the torch binding; returns the library's path."""
+    build_binding(force, verbose)
+    if not force and not _stale(LIB, [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))]):
         return LIB
     objs = []
     procs = []

@@ -137,8 +137,62 @@ __global__ void __launch_bounds__(256) transpose_scale_kernel(const float* __res
     }
 }
 
-// dst[p, s, :] = src[p, s, :] * keep[p / H, s]
-__global__ void mask_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, const float* __restrict__ keep,
+// The way back for a gradient: dst[p, s, d] = (src[p, d, s] + c) * scale * (keep ? keep[p / H, s] : 1). With `qt` (the operator's
+// queries) c takes out what the masked keys, which sit at the origin, added through the row sum's gradient dd[p, s]:
+// c = n_pad[p / H] dd[p, s] sign(q) exp(-|q|).
+__global__ void __launch_bounds__(256) transpose_back_kernel(const float* __restrict__ src, float* __restrict__ dst,
+                                                             const float* __restrict__ keep, const float scale,
+                                                             const float* __restrict__ qt, const float* __restrict__ dd, const float* __restrict__ n_pad,
+                                                             const int S, const int D, const int H)
+{
+    __shared__ float tile[32][33];
+    const int stiles = (S + 31) / 32;
+    const int p  = blockIdx.x / stiles;
+    const int s0 = (blockIdx.x % stiles) * 32, d0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const float np = qt ? n_pad[p / H] : 0.0f;
+    #pragma unroll
+    for (int r = ty; r < 32; r += 8) {
+        const int d = d0 + r, s = s0 + tx;
+        float x = 0.0f;
+        if (d < D && s < S) {
+            const long long at = ((long long)p * D + d) * S + s;
+            x = src[at];
+            if (qt) { const float q = qt[at]; if (q != 0.0f) x += copysignf(np * __expf(-fabsf(q)), q) * dd[(long long)p * S + s]; }
+            x *= scale;
+            if (keep) x *= keep[(long long)(p / H) * S + s];
+        }
+        tile[r][tx] = x;
+    }
+    __syncthreads();
+    #pragma unroll
+    for (int r = ty; r < 32; r += 8) {
+        const int s = s0 + r, d = d0 + tx;
+        if (s < S && d < D) dst[((long long)p * S + s) * D + d] = tile[tx][r];
+    }
+}
+
+// dn[row, :] = g[row, :] / max(den[row], clamp),  dd[row] = den[row] >= clamp ? -<dn[row, :], out[row, :]> : 0; one warp per row
+__global__ void __launch_bounds__(256) attention_gradient_rows_kernel(const float* __restrict__ g, const float* __restrict__ out, const float* __restrict__ den,
+                                                                      float* __restrict__ dn, float* __restrict__ dd, const int C, const float clamp, const long long rows)
+{
+    const long long row  = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int       lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    const float d = den[row], inv = 1.0f / fmaxf(d, clamp);
+    float dot = 0.0f;
+    for (int c = lane; c < C; c += 32) {
+        const float x = g[row * C + c] * inv;
+        dn[row * C + c] = x;
+        dot = fmaf(x, out[row * C + c], dot);
+    }
+    #pragma unroll
+    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(FULL, dot, off);
+    if (lane == 0) dd[row] = d >= clamp ? -dot : 0.0f;
+}
+
+// dst[p, s, :] = src[p, s, :] * keep[p / H, s]   (src may be dst)
+__global__ void mask_rows_kernel(const float* src, float* dst, const float* __restrict__ keep,
                                  const int S, const int C, const int H, const long long total)
 {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -165,12 +219,13 @@ __global__ void __launch_bounds__(256) npad_kernel(const float* __restrict__ kee
 
 // out[p, m, :] /= max(out_u[p, m] - n_pad[p / H] * sum_d f(qt[p, d, m]), clamp): the row normalisation of _add_laplace
 // (BUMP = false, f(x) = exp(-|x|)) and of _add_bump (BUMP = true, f(x) = max(0, 1 - |x|)), with the row sum corrected for
-// the masked keys (each sits at k = 0 with v = 0 and adds f(q_d) per dimension). One warp per row.
+// the masked keys (each sits at k = 0 with v = 0 and adds f(q_d) per dimension); the corrected sum goes to den_out if given.
+// One warp per row.
 template <bool BUMP>
 __global__ void __launch_bounds__(256) normalise_kernel(float* __restrict__ out, const float* __restrict__ out_u,
                                                         const float* __restrict__ qt, const float* __restrict__ n_pad,
                                                         const int M, const int D, const int C, const int H,
-                                                        const float clamp, const long long rows)
+                                                        const float clamp, const long long rows, float* __restrict__ den_out)
 {
     const long long row  = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int       lane = threadIdx.x & 31;
@@ -190,6 +245,7 @@ __global__ void __launch_bounds__(256) normalise_kernel(float* __restrict__ out,
             den -= np * acc;
         }
     }
+    if (den_out && lane == 0) den_out[row] = den;
     const float inv = 1.0f / fmaxf(den, clamp);
     float* o = out + row * C;
     for (int c = lane; c < C; c += 32) o[c] *= inv;
@@ -203,7 +259,7 @@ __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__
                                                              const float* __restrict__ akv, const float* __restrict__ aksum,
                                                              const float* __restrict__ n_pad,
                                                              const int M, const int C, const int C4, const int H,
-                                                             const float eps, const float clamp, const long long rows)
+                                                             const float eps, const float clamp, const long long rows, float* __restrict__ den_out)
 {
     const long long row  = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int       lane = threadIdx.x & 31;
@@ -212,6 +268,7 @@ __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__
     const float a   = aq[row] + eps;
     const float np  = n_pad ? n_pad[p / H] : 0.0f;
     const float den = a * (float)M + aksum[p] - out_u[row] - eps * np;
+    if (den_out && lane == 0) den_out[row] = den;
     const float inv = 1.0f / fmaxf(den, clamp);
     float* o = out + row * C;
     for (int c = lane; c < C; c += 32) o[c] = (fmaf(a, vsum[p * C4 + c], akv[p * C4 + c]) - o[c]) * inv;
@@ -260,6 +317,16 @@ cudaError_t launch_transpose_scale(const float* src, float* dst, const float* ke
     transpose_scale_kernel<<<grid, 256, 0, st>>>(src, dst, keep, scale, S, D, H);
     return cudaGetLastError();
 }
+cudaError_t launch_transpose_back(const float* src, float* dst, const float* keep, float scale, const float* qt, const float* dd, const float* n_pad,
+                                  int P, int S, int D, int H, cudaStream_t st) {
+    dim3 grid((unsigned)((S + 31) / 32) * (unsigned)P, (D + 31) / 32);
+    transpose_back_kernel<<<grid, 256, 0, st>>>(src, dst, keep, scale, qt, dd, n_pad, S, D, H);
+    return cudaGetLastError();
+}
+cudaError_t launch_attention_gradient_rows(const float* g, const float* out, const float* den, float* dn, float* dd, long long rows, int C, float clamp, cudaStream_t st) {
+    attention_gradient_rows_kernel<<<blocks_for(rows, 8), 256, 0, st>>>(g, out, den, dn, dd, C, clamp, rows);
+    return cudaGetLastError();
+}
 cudaError_t launch_mask_rows(const float* src, float* dst, const float* keep, int P, int S, int C, int H, cudaStream_t st) {
     const long long total = (long long)P * S * C;
     mask_rows_kernel<<<blocks_for(total, 256), 256, 0, st>>>(src, dst, keep, S, C, H, total);
@@ -270,17 +337,17 @@ cudaError_t launch_npad(const float* keep, float* n_pad, int B, int S, cudaStrea
     return cudaGetLastError();
 }
 cudaError_t launch_normalise(float* out, const float* out_u, const float* qt, const float* n_pad,
-                             int P, int M, int D, int C, int H, float clamp, bool bump, cudaStream_t st) {
+                             int P, int M, int D, int C, int H, float clamp, bool bump, float* den_out, cudaStream_t st) {
     const long long rows = (long long)P * M;
-    if (bump) normalise_kernel<true><<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows);
-    else      normalise_kernel<false><<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows);
+    if (bump) normalise_kernel<true><<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows, den_out);
+    else      normalise_kernel<false><<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows, den_out);
     return cudaGetLastError();
 }
 cudaError_t launch_riesz_epilogue(float* out, const float* out_u, const float* aq, const float* vsum, const float* akv,
                                   const float* aksum, const float* n_pad, int P, int M, int C, int C4, int H,
-                                  float eps, float clamp, cudaStream_t st) {
+                                  float eps, float clamp, float* den_out, cudaStream_t st) {
     const long long rows = (long long)P * M;
-    riesz_epilogue_kernel<<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, aq, vsum, akv, aksum, n_pad, M, C, C4, H, eps, clamp, rows);
+    riesz_epilogue_kernel<<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, aq, vsum, akv, aksum, n_pad, M, C, C4, H, eps, clamp, rows, den_out);
     return cudaGetLastError();
 }
 

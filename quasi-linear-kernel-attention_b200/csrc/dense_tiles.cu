@@ -38,7 +38,6 @@ namespace qlka {
 constexpr int TM = 64, TN = 64, DT_THREADS = 128;
 constexpr int AT_LD = TM + 4;                 // row pitch of the transposed A tile: 16-byte stores of a warp hit all banks
 constexpr int KSTAGES = 3;                    // chunks of the key tile in shared memory: one in use, two on their way
-constexpr float LAP_RANGE = 80.0f;
 
 namespace {
 
@@ -364,13 +363,14 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
         #pragma unroll
         for (int off = 4; off < 32; off <<= 1) rs[i] += __shfl_xor_sync(FULL, rs[i], off);
     }
+    auto row_weight = [&](const int m) -> float { return a.row_keep ? __ldg(a.row_keep + (long long)(p / a.H) * M + m) : 1.0f; };
     auto finish = [&](const float den) -> float { return a.normalise ? 1.0f / fmaxf(den, a.clamp) : 1.0f; };
     if (split == 1) {
         #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int m = m0 + mg * 4 + i;
             if (m >= M) continue;
-            const float f = finish(rs[i]);
+            const float f = finish(rs[i]) * row_weight(m);
             if (a.out_u && ng == 0) a.out_u[(long long)p * M + m] = rs[i];
             float* dst = a.out + ((long long)p * M + m) * C;
             #pragma unroll
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
                 den += cl.map_shared_rank(rsum, b)[r];
             }
             if (m0 + r < M) {
-                a.out[((long long)p * M + m0 + r) * C + c] = s * finish(den);
+                a.out[((long long)p * M + m0 + r) * C + c] = s * (finish(den) * row_weight(m0 + r));
                 if (a.out_u && c == 0) a.out_u[(long long)p * M + m0 + r] = den;
             }
         }
@@ -447,22 +447,8 @@ static cudaError_t launch_dense_c(const DenseArgs& a, cudaStream_t stream) {
     return launch_dense_inst<KIND, 16>(a, stream);
 }
 
-// CTAs that share one query tile: the count that gives the busiest SM the fewest key tiles, a CTA's own start and end counted
-// as one more tile
-static int dense_split(const DenseArgs& a, int sms) {
-    const long long ctas = (long long)a.P * ((a.M + TM - 1) / TM);
-    const int ntiles = (a.N + TN - 1) / TN;
-    int best = 1;
-    double best_cost = 1e300;
-    for (int s = 1; s <= 8 && s <= ntiles; s *= 2) {
-        const double cost = (double)((ctas * s + sms - 1) / sms) * ((ntiles + s - 1) / s + 1.0);
-        if (cost < best_cost * 0.97) { best = s; best_cost = cost; }
-    }
-    return best;
-}
-
 cudaError_t launch_dense_forward(DenseArgs a, int kind, int sms, cudaStream_t stream) {
-    a.split = dense_split(a, sms);
+    a.split = dense_split((long long)a.P * ((a.M + TM - 1) / TM), (a.N + TN - 1) / TN, sms);
     a.vec = a.rows_layout && (a.D & 3) == 0 && ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k)) & 15) == 0;
     switch (kind) {
         case DENSE_LAPLACE: return launch_dense_c<DENSE_LAPLACE>(a, stream);

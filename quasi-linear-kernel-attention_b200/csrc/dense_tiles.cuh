@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 namespace qlka {
 
 enum DenseKind : int { DENSE_LAPLACE = 0, DENSE_ABS = 1, DENSE_BUMP = 2, DENSE_RIESZ = 3 };
@@ -11,11 +13,12 @@ struct DenseArgs {
     const float* k;          // (P, D, N), or (P, N, D)
     const float* v;          // (P, N, C), 16-byte aligned
     const float* keep;       // (P / H, N) key weights 0 / 1, or null
+    const float* row_keep;   // (P / H, M) weights of the output rows 0 / 1, or null
     float*       staged;     // dense_workspace_bytes() of scratch
     float*       out;        // (P, M, C), 16-byte aligned
     float*       out_u;      // (P, M) row sums, or null
     int   P, H, D, N, M, C;
-    float scale;             // applied to q and k
+    float scale;             // applied to q and k: 1 / tau rounded, as torch divides by a scalar (ties between q and k depend on it)
     float eps;               // RIESZ: added to every A_mn
     float clamp;             // floor of the row sum when normalising
     bool  rows_layout, normalise;
@@ -23,8 +26,40 @@ struct DenseArgs {
     int   split;             // (set by the launcher) CTAs per query tile
 };
 
-size_t dense_workspace_bytes(int kind, int P, int D, int N, int M);
+size_t      dense_workspace_bytes(int kind, int P, int D, int N, int M);
+cudaError_t launch_dense_forward(DenseArgs a, int kind, int sms, cudaStream_t stream);
 
+// Gradients of the same sums, dense_gradient.cu.
+struct DenseGradArgs {
+    const float *q, *k, *v;  // as in DenseArgs; attention: rows layout, scaled
+    const float* a;          // (P, M, C) upstream gradient of the sums (attention: of the normalised output)
+    const float* s;          // (P, M) upstream gradient of the row sums, or null (attention: unused)
+    const float *out, *den;  // attention: (P, M, C) output and (P, M) row sums of the forward call
+    const float* keep;       // (P / H, N) or null
+    float *grad_q, *grad_k;  // in the layout of q and k
+    float* grad_v;           // (P, N, C), 16-byte aligned
+    float* staged;           // dense_gradient_workspace_bytes()
+    int   P, H, D, N, M, C;
+    float scale, eps, clamp;
+    bool  attention;
+    int   split;             // (set by the launcher)
+};
+size_t      dense_gradient_workspace_bytes(int kind, int P, int D, int N, int M, int C, bool attention);
+cudaError_t launch_dense_gradient(const DenseGradArgs& g, int kind, int sms, cudaStream_t stream);
+
+// CTAs that share one tile of 64 rows: the count that gives the busiest SM the fewest tiles of the other side, a CTA's own start
+// and end counted as one more tile
+inline int dense_split(long long ctas, int ntiles, int sms) {
+    int best = 1;
+    double best_cost = 1e300;
+    for (int s = 1; s <= 8 && s <= ntiles; s *= 2) {
+        const double cost = (double)((ctas * s + sms - 1) / sms) * ((ntiles + s - 1) / s + 1.0);
+        if (cost < best_cost * 0.97) { best = s; best_cost = cost; }
+    }
+    return best;
+}
+
+constexpr float LAP_RANGE = 80.0f;     // largest |value| whose exponentials the Laplace kernels multiply
 constexpr int DENSE_MAX_D = 128;      // the query tile of all features stays in shared memory
 
 }  // namespace qlka

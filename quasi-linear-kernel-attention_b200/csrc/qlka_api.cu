@@ -20,7 +20,6 @@ int         walk_lanes_per_stream(int C4);
 int         walk_threads();
 int         laplace_agg_stride(int C4);
 int         prefix_agg_stride_host(int C4);
-cudaError_t launch_dense_forward(DenseArgs a, int kind, int sms, cudaStream_t stream);
 cudaError_t launch_colsum_d(const float* x, float* out, int P, int D, int L, cudaStream_t st);
 cudaError_t launch_rowstat(const float* w, const float* s, float* wsum, float* swsum, float* ssum, int P, int R, int C4, cudaStream_t st);
 cudaError_t launch_vecsum(const float* x, float* out, int P, int L, cudaStream_t st);
@@ -29,14 +28,17 @@ cudaError_t launch_abs_init(const float* ktot, const float* vsum, const float* q
 cudaError_t launch_pad_rows(const float* src, float* dst, long long rows, int C, int C4, cudaStream_t st);
 cudaError_t launch_unpad_rows(const float* src, float* dst, long long rows, int C, int C4, cudaStream_t st);
 cudaError_t launch_transpose_scale(const float* src, float* dst, const float* keep, float scale, int P, int S, int D, int H, cudaStream_t st);
+cudaError_t launch_transpose_back(const float* src, float* dst, const float* keep, float scale, const float* qt, const float* dd, const float* n_pad,
+                                  int P, int S, int D, int H, cudaStream_t st);
+cudaError_t launch_attention_gradient_rows(const float* g, const float* out, const float* den, float* dn, float* dd, long long rows, int C, float clamp, cudaStream_t st);
 cudaError_t launch_mask_rows(const float* src, float* dst, const float* keep, int P, int S, int C, int H, cudaStream_t st);
 cudaError_t launch_npad(const float* keep, float* n_pad, int B, int S, cudaStream_t st);
 cudaError_t launch_normalise(float* out, const float* out_u, const float* qt, const float* n_pad,
-                             int P, int M, int D, int C, int H, float clamp, bool bump, cudaStream_t st);
+                             int P, int M, int D, int C, int H, float clamp, bool bump, float* den_out, cudaStream_t st);
 cudaError_t launch_abscolsum_d(const float* x, float* out, int P, int D, int L, cudaStream_t st);
 cudaError_t launch_riesz_epilogue(float* out, const float* out_u, const float* aq, const float* vsum, const float* akv,
                                   const float* aksum, const float* n_pad, int P, int M, int C, int C4, int H,
-                                  float eps, float clamp, cudaStream_t st);
+                                  float eps, float clamp, float* den_out, cudaStream_t st);
 }  // namespace qlka
 
 using namespace qlka;
@@ -296,13 +298,27 @@ double dense_us(int kind, double P, int D, int N, int M, int C) {
     return 8.0 + best;
 }
 double sorted_us(int kind, double P, int D, int N, int M, int C) {
-    const double segs = P * D, wide = C <= 32 ? 0.6 : C <= 64 ? 1.0 : 4.0;      // the walks move rows of 32, 64 or 128 channels
+    const double segs = P * D, wide = C <= 32 ? 0.6 : C <= 64 ? 1.0 : 1.4;      // the walks move rows of 32, 64 or 128 channels
     const double keys = N * (0.022 + 0.045 * wide), queries = M * (0.022 + 0.050 * wide) * (kind == DENSE_BUMP ? 5.0 : 1.0);
     return 70.0 + segs * (30.0 + keys + queries) * 1e-3;               // (launches and tails; nanoseconds per segment)
 }
 bool dense_pays(int kind, long long P, int D, int N, int M, int C) {
     if (D > DENSE_MAX_D) return false;
     return dense_us(kind, (double)P, D, N, M, C) < sorted_us(kind, (double)P, D, N, M, C);
+}
+
+// The same for the gradients: three kernels of the same tiling against two sorts and three walks (Laplace 0.43 ns per feature
+// and key, abs 0.30, measured at 4096 keys; the bump's are three abs gradients put together op by op).
+bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C) {
+    if (D > DENSE_MAX_D) return false;
+    const double grad_d = kind == DENSE_LAPLACE ? 0.50 : kind == DENSE_BUMP ? 0.68 : 0.26, grad_c = 0.054;
+    const int    cw = C <= 32 ? 32 : C <= 64 ? 64 : 128;
+    const double tile = 4096e-6 * sm_count() * (D * grad_d + cw * grad_c);
+    const double per_sm = std::ceil((double)P * ((M + N + 127) / 128) / sm_count());
+    const double dense = 20.0 + std::max(per_sm, 1.0) * ((M + N + 127) / 128) * tile * (per_sm < 2 ? 0.5 : 1.0) + dense_us(kind, (double)P, D, M, N, C);
+    const double wide = C <= 32 ? 0.8 : C <= 64 ? 1.0 : 1.4, pair = kind == DENSE_LAPLACE ? 0.43 : kind == DENSE_BUMP ? 1.45 : 0.30;
+    const double sorted = (kind == DENSE_BUMP ? 250.0 : 110.0) + (double)P * D * (60.0 + pair * wide * 0.5 * (N + M)) * 1e-3;
+    return dense < sorted;
 }
 
 // scratch of the pairwise kernels where they are the ones to run
@@ -319,10 +335,25 @@ DenseArgs dense_args(const float* q, const float* k, const float* v, float* out,
     return a;
 }
 
+size_t dense_gradient_bytes(int kind, int P, int D, int N, int M, int C, bool attention) {
+    return dense_gradient_pays(kind, P, D, N, M, C) ? dense_gradient_workspace_bytes(kind, P, D, N, M, C, attention) : 0;
+}
+
+DenseGradArgs dense_grad_args(const float* q, const float* k, const float* v, const float* g_w, const float* g_u,
+                              float* grad_q, float* grad_k, float* grad_v, void* ws, int P, int D, int N, int M, int C) {
+    DenseGradArgs g{};
+    g.q = q; g.k = k; g.v = v; g.a = g_w; g.s = g_u;
+    g.grad_q = grad_q; g.grad_k = grad_k; g.grad_v = grad_v;
+    g.staged = static_cast<float*>(ws);
+    g.P = P; g.H = 1; g.D = D; g.N = N; g.M = M; g.C = C;
+    g.scale = 1.0f;
+    return g;
+}
+
 // the attention entry points: (B, H, S, D) rows, scaled, masked, normalised
-DenseArgs dense_attention_args(const float* q, const float* k, const float* v, const float* keep, float* out, float tau, void* ws,
+DenseArgs dense_attention_args(const float* q, const float* k, const float* v, const float* keep, float* out, float* den, float tau, void* ws,
                                int P, int H, int S, int D, int C) {
-    DenseArgs a = dense_args(q, k, v, out, nullptr, ws, P, D, S, S, C);
+    DenseArgs a = dense_args(q, k, v, out, den, ws, P, D, S, S, C);
     a.keep = keep; a.H = H; a.scale = 1.0f / tau; a.eps = 1e-3f; a.clamp = 1e-6f; a.rows_layout = true; a.normalise = true;
     return a;
 }
@@ -506,7 +537,7 @@ int qlka_laplace_backward_workspace_bytes(int P, int D, int N, int M, int C, siz
     if (!bytes) return QLKA_ERR_NULL;
     int st = check_dims(P, D, N, M, C);
     if (st) return st;
-    *bytes = LaplaceBwdWs(nullptr, P, D, N, M, C).bytes;
+    *bytes = std::max(LaplaceBwdWs(nullptr, P, D, N, M, C).bytes, dense_gradient_bytes(DENSE_LAPLACE, P, D, N, M, C, false));
     return QLKA_OK;
 }
 
@@ -520,6 +551,12 @@ int qlka_weighted_laplace_sum_backward(const float* q, const float* k, const flo
     if (st) return st;
     if (!q || !k || !v || !g_w || !grad_q || !grad_k || !grad_v) return QLKA_ERR_NULL;
     if (!aligned16(v, g_w, grad_v)) return QLKA_ERR_ALIGNMENT;
+    if (dense_gradient_pays(DENSE_LAPLACE, P, D, N, M, C)) {
+        if (!ws_ok(workspace, workspace_bytes, dense_gradient_workspace_bytes(DENSE_LAPLACE, P, D, N, M, C, false))) return QLKA_ERR_WORKSPACE;
+        CU(launch_dense_gradient(dense_grad_args(q, k, v, g_w, g_u, grad_q, grad_k, grad_v, workspace, P, D, N, M, C), DENSE_LAPLACE, sm_count(),
+                                 reinterpret_cast<cudaStream_t>(stream_)));
+        return QLKA_OK;
+    }
     LaplaceBwdWs ws(workspace, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
@@ -589,9 +626,10 @@ int qlka_laplace_attention_workspace_bytes(int B, int H, int S, int D, int Dv, i
     return QLKA_OK;
 }
 
-int qlka_laplace_attention_forward(const float* q, const float* k, const float* v, const float* keep, float tau,
-                                   float* out, void* workspace, size_t workspace_bytes,
-                                   int B, int H, int S, int D, int Dv, qlka_stream_t stream_)
+// den: row sums (before the floor) for the backward pass, or null
+static int laplace_attention_impl(const float* q, const float* k, const float* v, const float* keep, float tau,
+                                  float* out, float* den, void* workspace, size_t workspace_bytes,
+                                  int B, int H, int S, int D, int Dv, cudaStream_t stream)
 {
     int st = attn_check(B, H, S, D, Dv);
     if (st) return st;
@@ -600,14 +638,12 @@ int qlka_laplace_attention_forward(const float* q, const float* k, const float* 
     if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
     if (dense_pays(DENSE_LAPLACE, (long long)B * H, D, S, S, Dv)) {
         if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(DENSE_LAPLACE, B * H, D, S, S))) return QLKA_ERR_WORKSPACE;
-        CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, tau, workspace, B * H, H, S, D, Dv), DENSE_LAPLACE, sm_count(),
-                                reinterpret_cast<cudaStream_t>(stream_)));
+        CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, den, tau, workspace, B * H, H, S, D, Dv), DENSE_LAPLACE, sm_count(), stream));
         return QLKA_OK;
     }
     const bool masked = keep != nullptr;
     LaplaceAttnWs ws(workspace, B, H, S, D, Dv, masked);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
-    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int P = B * H;
 
     CU(launch_transpose_scale(q, ws.qt, nullptr, 1.0f / tau, P, S, D, H, stream));
@@ -620,8 +656,15 @@ int qlka_laplace_attention_forward(const float* q, const float* k, const float* 
     }
     st = laplace_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, stream, nullptr);
     if (st) return st;
-    CU(launch_normalise(out, ws.out_u, ws.qt, ws.n_pad, P, S, D, Dv, H, 1e-6f, false, stream));
+    CU(launch_normalise(out, ws.out_u, ws.qt, ws.n_pad, P, S, D, Dv, H, 1e-6f, false, den, stream));
     return QLKA_OK;
+}
+
+int qlka_laplace_attention_forward(const float* q, const float* k, const float* v, const float* keep, float tau,
+                                   float* out, void* workspace, size_t workspace_bytes,
+                                   int B, int H, int S, int D, int Dv, qlka_stream_t stream_)
+{
+    return laplace_attention_impl(q, k, v, keep, tau, out, nullptr, workspace, workspace_bytes, B, H, S, D, Dv, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 // ---------------------------------------------------------------- add_riesz / add_bump attention on (B, H, S, D)
@@ -667,9 +710,9 @@ int qlka_abs_attention_workspace_bytes(int kind, int B, int H, int S, int D, int
     return QLKA_OK;
 }
 
-int qlka_abs_attention_forward(int kind, const float* q, const float* k, const float* v, const float* keep, float tau,
-                               float* out, void* workspace, size_t workspace_bytes,
-                               int B, int H, int S, int D, int Dv, qlka_stream_t stream_)
+static int abs_attention_impl(int kind, const float* q, const float* k, const float* v, const float* keep, float tau,
+                              float* out, float* den, void* workspace, size_t workspace_bytes,
+                              int B, int H, int S, int D, int Dv, cudaStream_t stream)
 {
     int st = abs_attn_check(kind, B, H, S, D, Dv);
     if (st) return st;
@@ -679,13 +722,11 @@ int qlka_abs_attention_forward(int kind, const float* q, const float* k, const f
     const bool masked = keep != nullptr, bump = kind == 1;
     if (const int dk = bump ? DENSE_BUMP : DENSE_RIESZ; dense_pays(dk, (long long)B * H, D, S, S, Dv)) {
         if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(dk, B * H, D, S, S))) return QLKA_ERR_WORKSPACE;
-        CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, tau, workspace, B * H, H, S, D, Dv), dk, sm_count(),
-                                reinterpret_cast<cudaStream_t>(stream_)));
+        CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, den, tau, workspace, B * H, H, S, D, Dv), dk, sm_count(), stream));
         return QLKA_OK;
     }
     AbsAttnWs ws(workspace, B, H, S, D, Dv, masked, bump);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
-    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int P = B * H;
 
     CU(launch_transpose_scale(q, ws.qt, nullptr, 1.0f / tau, P, S, D, H, stream));
@@ -700,7 +741,7 @@ int qlka_abs_attention_forward(int kind, const float* q, const float* k, const f
         // numerator and row sum of the three shifted abs sums from one sort, then the row normalisation
         st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, 3, BUMP_SHIFTS, BUMP_WEIGHTS, stream);
         if (st) return st;
-        CU(launch_normalise(out, ws.out_u, ws.qt, ws.n_pad, P, S, D, Dv, H, 1e-6f, true, stream));
+        CU(launch_normalise(out, ws.out_u, ws.qt, ws.n_pad, P, S, D, Dv, H, 1e-6f, true, den, stream));
     } else {
         // A_ij = |q_i|_1 + |k_j|_1 - |q_i - k_j|_1 + eps: rank-1 terms from column and row statistics, the abs sum from the walk
         float* vsum  = ws.sums;
@@ -710,10 +751,106 @@ int qlka_abs_attention_forward(int kind, const float* q, const float* k, const f
         CU(launch_abscolsum_d(ws.kt, ws.ak, P, D, S, stream));
         CU(cudaMemsetAsync(ws.sums, 0, sizeof(float) * ((size_t)P * Dv * 2 + P), stream));
         CU(launch_rowstat(rows, ws.ak, vsum, akv, aksum, P, S, Dv, stream));
-        st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, 0, nullptr, nullptr, stream);
+        st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, 0, nullptr, nullptr, stream, true);
         if (st) return st;
-        CU(launch_riesz_epilogue(out, ws.out_u, ws.aq, vsum, akv, aksum, ws.n_pad, P, S, Dv, Dv, H, 1e-3f, 1e-6f, stream));
+        CU(launch_riesz_epilogue(out, ws.out_u, ws.aq, vsum, akv, aksum, ws.n_pad, P, S, Dv, Dv, H, 1e-3f, 1e-6f, den, stream));
     }
+    return QLKA_OK;
+}
+
+int qlka_abs_attention_forward(int kind, const float* q, const float* k, const float* v, const float* keep, float tau,
+                               float* out, void* workspace, size_t workspace_bytes,
+                               int B, int H, int S, int D, int Dv, qlka_stream_t stream_)
+{
+    return abs_attention_impl(kind, q, k, v, keep, tau, out, nullptr, workspace, workspace_bytes, B, H, S, D, Dv, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+// ---------------------------------------------------------------- attention, training: row sums kept, backward
+namespace {
+constexpr int ATTN_LAPLACE = 2;
+int dense_kind_of(int kind) { return kind == ATTN_LAPLACE ? DENSE_LAPLACE : kind == 1 ? DENSE_BUMP : DENSE_RIESZ; }
+
+struct LaplaceAttnBwdWs {
+    float *qt, *kt, *vm, *dn, *dd, *gqt, *gkt, *n_pad; void* inner; size_t inner_bytes, bytes;
+    LaplaceAttnBwdWs(void* base, int B, int H, int S, int D, int C, bool masked) {
+        Bump b(base);
+        const size_t P = (size_t)B * H;
+        qt    = b.take<float>(P * D * S);
+        kt    = b.take<float>(P * D * S);
+        gqt   = b.take<float>(P * D * S);
+        gkt   = b.take<float>(P * D * S);
+        vm    = masked ? b.take<float>(P * S * C) : nullptr;
+        dn    = b.take<float>(P * S * C);
+        dd    = b.take<float>(P * S);
+        n_pad = masked ? b.take<float>((size_t)B) : nullptr;
+        inner_bytes = LaplaceBwdWs(nullptr, (int)P, D, S, S, C).bytes;
+        inner = b.take<unsigned char>(inner_bytes);
+        bytes = (b.off + 255) & ~size_t(255);
+    }
+};
+}  // namespace
+
+int qlka_attention_forward(int kind, const float* q, const float* k, const float* v, const float* keep, float tau,
+                           float* out, float* den, void* workspace, size_t workspace_bytes,
+                           int B, int H, int S, int D, int Dv, qlka_stream_t stream_)
+{
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    if (kind == ATTN_LAPLACE) return laplace_attention_impl(q, k, v, keep, tau, out, den, workspace, workspace_bytes, B, H, S, D, Dv, stream);
+    return abs_attention_impl(kind, q, k, v, keep, tau, out, den, workspace, workspace_bytes, B, H, S, D, Dv, stream);
+}
+
+int qlka_attention_workspace_bytes(int kind, int B, int H, int S, int D, int Dv, int masked, size_t* bytes) {
+    if (kind == ATTN_LAPLACE) return qlka_laplace_attention_workspace_bytes(B, H, S, D, Dv, masked, bytes);
+    return qlka_abs_attention_workspace_bytes(kind, B, H, S, D, Dv, masked, bytes);
+}
+
+int qlka_attention_backward_workspace_bytes(int kind, int B, int H, int S, int D, int Dv, int masked, size_t* bytes) {
+    if (!bytes) return QLKA_ERR_NULL;
+    int st = kind == ATTN_LAPLACE ? attn_check(B, H, S, D, Dv) : abs_attn_check(kind, B, H, S, D, Dv);
+    if (st) return st;
+    const int dk = dense_kind_of(kind);
+    if (dense_gradient_pays(dk, (long long)B * H, D, S, S, Dv)) *bytes = dense_gradient_workspace_bytes(dk, B * H, D, S, S, Dv, true);
+    else if (kind == ATTN_LAPLACE)                              *bytes = LaplaceAttnBwdWs(nullptr, B, H, S, D, Dv, masked != 0).bytes;
+    else                                                        return QLKA_ERR_UNSUPPORTED;
+    return QLKA_OK;
+}
+
+int qlka_attention_backward(int kind, const float* q, const float* k, const float* v, const float* keep, float tau,
+                            const float* out, const float* den, const float* grad_out,
+                            float* grad_q, float* grad_k, float* grad_v, void* workspace, size_t workspace_bytes,
+                            int B, int H, int S, int D, int Dv, qlka_stream_t stream_)
+{
+    const bool masked = keep != nullptr;
+    size_t need = 0;
+    int st = qlka_attention_backward_workspace_bytes(kind, B, H, S, D, Dv, masked, &need);
+    if (st) return st;
+    if (!q || !k || !v || !out || !den || !grad_out || !grad_q || !grad_k || !grad_v) return QLKA_ERR_NULL;
+    if (!aligned16(v, out, grad_out, grad_v)) return QLKA_ERR_ALIGNMENT;
+    if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
+    if (!ws_ok(workspace, workspace_bytes, need)) return QLKA_ERR_WORKSPACE;
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    const int P = B * H, dk = dense_kind_of(kind);
+    if (dense_gradient_pays(dk, P, D, S, S, Dv)) {
+        DenseGradArgs g = dense_grad_args(q, k, v, grad_out, nullptr, grad_q, grad_k, grad_v, workspace, P, D, S, S, Dv);
+        g.attention = true; g.H = H; g.scale = 1.0f / tau; g.eps = 1e-3f; g.clamp = 1e-6f; g.keep = keep; g.out = out; g.den = den;
+        CU(launch_dense_gradient(g, dk, sm_count(), stream));
+        return QLKA_OK;
+    }
+    LaplaceAttnBwdWs ws(workspace, B, H, S, D, Dv, masked);
+    CU(launch_transpose_scale(q, ws.qt, nullptr, 1.0f / tau, P, S, D, H, stream));
+    CU(launch_transpose_scale(k, ws.kt, keep, 1.0f / tau, P, S, D, H, stream));
+    const float* rows = v;
+    if (masked) {
+        CU(launch_mask_rows(v, ws.vm, keep, P, S, Dv, H, stream));
+        CU(launch_npad(keep, ws.n_pad, B, S, stream));
+        rows = ws.vm;
+    }
+    CU(launch_attention_gradient_rows(grad_out, out, den, ws.dn, ws.dd, (long long)P * S, Dv, 1e-6f, stream));
+    st = qlka_weighted_laplace_sum_backward(ws.qt, ws.kt, rows, ws.dn, ws.dd, ws.gqt, ws.gkt, grad_v, ws.inner, ws.inner_bytes, P, D, S, S, Dv, stream_);
+    if (st) return st;
+    CU(launch_transpose_back(ws.gqt, grad_q, nullptr, 1.0f / tau, masked ? ws.qt : nullptr, ws.dd, ws.n_pad, P, S, D, H, stream));
+    CU(launch_transpose_back(ws.gkt, grad_k, keep, 1.0f / tau, nullptr, nullptr, nullptr, P, S, D, H, stream));
+    if (masked) CU(launch_mask_rows(grad_v, grad_v, keep, P, S, Dv, H, stream));
     return QLKA_OK;
 }
 
@@ -858,7 +995,7 @@ int qlka_abs_backward_workspace_bytes(int P, int D, int N, int M, int C, size_t*
     if (!bytes) return QLKA_ERR_NULL;
     int st = check_dims(P, D, N, M, C);
     if (st) return st;
-    *bytes = AbsBwdWs(nullptr, P, D, N, M, C).bytes;
+    *bytes = std::max(AbsBwdWs(nullptr, P, D, N, M, C).bytes, dense_gradient_bytes(DENSE_ABS, P, D, N, M, C, false));
     return QLKA_OK;
 }
 
@@ -872,6 +1009,12 @@ int qlka_weighted_abs_sum_backward(const float* q, const float* k, const float* 
     if (st) return st;
     if (!q || !k || !v || !g_w || !grad_q || !grad_k || !grad_v) return QLKA_ERR_NULL;
     if (!aligned16(v, g_w, grad_v)) return QLKA_ERR_ALIGNMENT;
+    if (dense_gradient_pays(DENSE_ABS, P, D, N, M, C)) {
+        if (!ws_ok(workspace, workspace_bytes, dense_gradient_workspace_bytes(DENSE_ABS, P, D, N, M, C, false))) return QLKA_ERR_WORKSPACE;
+        CU(launch_dense_gradient(dense_grad_args(q, k, v, g_w, g_u, grad_q, grad_k, grad_v, workspace, P, D, N, M, C), DENSE_ABS, sm_count(),
+                                 reinterpret_cast<cudaStream_t>(stream_)));
+        return QLKA_OK;
+    }
     AbsBwdWs ws(workspace, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);

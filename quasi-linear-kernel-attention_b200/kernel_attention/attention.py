@@ -6,9 +6,10 @@ efficient evaluation goes through the sorted-walk operators: add_laplace, add_ri
 the reference's own file also runs unchanged on top of the two operator packages of this library.
 
 Two routes:
-* no gradient needed - one native call per attention (`qlka_native.fused_attention`): layout change, tau,
+* one native call forward and, where gradients are wanted, one backward (`qlka_native.attention`): layout change, tau,
   masking, the sums and the normalisation all happen inside the library;
-* gradients needed - the sums are assembled here from the differentiable operators. Every kernel is described
+* the cases without such a call (gradients of add_riesz and add_bump at long lengths, add_bump beyond 5461 keys) - the sums are
+  assembled here from the differentiable operators. Every kernel is described
   by two small functions: `sums` returns the unnormalised numerator sum_j A_ij v_j and row sum sum_j A_ij over
   ALL S keys, and `at_origin` returns A(q_i, 0), the weight a key placed at the origin has. Masked keys are moved
   to the origin with a zero value row, so they add nothing to the numerator and exactly `at_origin` each to the
@@ -79,10 +80,10 @@ def attention(q, k, v, kernel, tau, keep=None):
     if kernel not in _ROUTES:
         raise ValueError(f"kernel must be one of {tuple(_ROUTES)}, got {kernel!r}")
     B, H, S, D = q.shape
-    wants_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
-    fused_fits = kernel != "add_bump" or 3 * S <= 16384      # the fused add_bump shares one shared-memory sort between its three shifts
-    if not wants_grad and fused_fits:
-        return _native.fused_attention(kernel, q, k, v, tau, keep)
+    if kernel != "add_bump" or 3 * S <= 16384:      # the fused add_bump shares one shared-memory sort between its three shifts
+        out = _native.attention(kernel, q, k, v, tau, keep)
+        if out is not None:
+            return out
 
     sums, at_origin = _ROUTES[kernel]
     heads = B * H

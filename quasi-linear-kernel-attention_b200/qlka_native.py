@@ -1,4 +1,5 @@
-"""ctypes binding of libqlka.so (the C ABI of include/qlka.h) for torch tensors.
+"""Bindings of libqlka.so (the C ABI of include/qlka.h) for torch tensors: the operators and their autograd through the
+compiled _qlka_torch.so (csrc/torch_binding.cpp), the diagnostics and the host pipeline through ctypes.
 
 torch is used for device memory and the current stream only; the kernels are the
 library's. There is no fallback: a missing library or a non-CUDA tensor raises.
@@ -8,13 +9,17 @@ The tensor checks and their messages follow the reference's host code
 """
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libqlka.so")
+EXT_PATH = os.path.join(_HERE, "_qlka_torch.so")
 _lib = None
+_ext = None
 
 _vp, _sz, _i = ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int
 
@@ -69,6 +74,22 @@ def lib():
     return _lib
 
 
+def ext():
+    """The compiled torch binding, over the library at LIB_PATH; raises if it has not been built."""
+    global _ext
+    if _ext is None:
+        if not (os.path.exists(EXT_PATH) and os.path.exists(LIB_PATH)):
+            raise RuntimeError(
+                f"{EXT_PATH} or {LIB_PATH} is missing: build them with `python {os.path.join(_HERE, 'build.py')}` "
+                "(nvcc, sm_100a, g++). There is no CPU or PyTorch fallback for these operators.")
+        loader = importlib.machinery.ExtensionFileLoader("_qlka_torch", EXT_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_qlka_torch", loader))
+        loader.exec_module(mod)
+        mod.load(LIB_PATH)
+        _ext = mod
+    return _ext
+
+
 def _raise(status):
     L = lib()
     msg = L.qlka_status_string(status).decode()
@@ -120,18 +141,8 @@ def _stream():
 
 
 def laplace_forward(q, k, v):
-    P, D, N, M, C = dims = check_qkv(q, k, v)
-    v = _aligned(v)
-    L = lib()
-    with torch.cuda.device(q.device):
-        ws, n = _workspace(L.qlka_laplace_forward_workspace_bytes, dims, q.device)
-        out_w = torch.empty(P, M, C, dtype=torch.float32, device=q.device)
-        out_u = torch.empty(P, M, dtype=torch.float32, device=q.device)
-        st = L.qlka_weighted_laplace_sum_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), out_w.data_ptr(), out_u.data_ptr(),
-                                                 ws.data_ptr(), n, P, D, N, M, C, _stream())
-    if st:
-        _raise(st)
-    return out_w, out_u
+    """(out_w, out_u) of the weighted Laplace sum, without autograd."""
+    return ext().laplace_forward(q, k, v)
 
 
 def laplace_forward_noalloc(q, k, v, out_w=None, out_u=None):
@@ -253,19 +264,8 @@ def laplace_stage_times(q, k, v, reps=5):
 
 
 def abs_forward(q, k, v, full, path=-1):
-    P, D, N, M, C = dims = check_qkv(q, k, v, "q, k, and v")
-    v = _aligned(v)
-    L = lib()
-    with torch.cuda.device(q.device):
-        ws, n = _workspace(L.qlka_abs_forward_workspace_bytes, dims, q.device)
-        out_w = torch.empty(P, M, C, dtype=torch.float32, device=q.device)
-        out_u = torch.empty(P, M, dtype=torch.float32, device=q.device) if full else None
-        st = L.qlka_weighted_abs_sum_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), out_w.data_ptr(),
-                                             out_u.data_ptr() if full else None,
-                                             ws.data_ptr(), n, P, D, N, M, C, int(path), _stream())
-    if st:
-        _raise(st)
-    return out_w, out_u
+    """(out_w, out_u or None) of the weighted abs sum, without autograd."""
+    return ext().abs_forward(q, k, v, full, path)
 
 
 def abs_shifted_forward(q, k, v, shifts, weights, full=True):
@@ -294,104 +294,36 @@ def abs_shifted_forward(q, k, v, shifts, weights, full=True):
 
 
 def abs_backward(q, k, v, g_w, g_u=None):
-    P, D, N, M, C = dims = check_qkv(q, k, v, "q, k, and v")
-    _check_like(g_w, "g_w", (P, M, C), q)
-    if g_u is not None:
-        _check_like(g_u, "g_u", (P, M), q)
-    v, g_w = _aligned(v), _aligned(g_w)
-    L = lib()
-    with torch.cuda.device(q.device):
-        ws, n = _workspace(L.qlka_abs_backward_workspace_bytes, dims, q.device)
-        gq = torch.empty(P, D, M, dtype=torch.float32, device=q.device)
-        gk = torch.empty(P, D, N, dtype=torch.float32, device=q.device)
-        gv = torch.empty(P, N, C, dtype=torch.float32, device=q.device)
-        st = L.qlka_weighted_abs_sum_backward(q.data_ptr(), k.data_ptr(), v.data_ptr(), g_w.data_ptr(),
-                                              None if g_u is None else g_u.data_ptr(),
-                                              gq.data_ptr(), gk.data_ptr(), gv.data_ptr(),
-                                              ws.data_ptr(), n, P, D, N, M, C, _stream())
-    if st:
-        _raise(st)
-    return gq, gk, gv
-
-
-ATTENTION_KINDS = {"add_laplace": -1, "add_riesz": 0, "add_bump": 1}
-
-
-def fused_attention(kernel, q, k, v, tau, keep=None):
-    """Normalised additive-kernel attention on (B, H, S, D) / (B, H, S, Dv) tensors in one native call (forward only)."""
-    kind = ATTENTION_KINDS[kernel]
-    _check(q.is_cuda and k.is_cuda and v.is_cuda, "q, k, and v must be CUDA tensors")
-    _check(q.dtype == k.dtype == v.dtype == torch.float32, "q, k, and v must be float32")
-    _check(q.dim() == 4 and k.shape == q.shape and v.dim() == 4 and v.shape[:3] == q.shape[:3],
-           "expected q, k (B, H, S, D) and v (B, H, S, Dv)")
-    q, k, v = q.contiguous(), k.contiguous(), _aligned(v.contiguous())
-    B, H, S, D = q.shape
-    Dv = v.shape[3]
-    if keep is not None:
-        _check(keep.shape == (B, S), "keep must be (B, S)")
-        keep = keep.to(device=q.device, dtype=torch.float32).contiguous()
-    L = lib()
-    with torch.cuda.device(q.device):
-        n = _sz(0)
-        if kind < 0:
-            st = L.qlka_laplace_attention_workspace_bytes(B, H, S, D, Dv, int(keep is not None), ctypes.byref(n))
-        else:
-            st = L.qlka_abs_attention_workspace_bytes(kind, B, H, S, D, Dv, int(keep is not None), ctypes.byref(n))
-        if st:
-            _raise(st)
-        ws = torch.empty(max(int(n.value), 1), dtype=torch.uint8, device=q.device)
-        out = torch.empty(B, H, S, Dv, dtype=torch.float32, device=q.device)
-        kp = None if keep is None else keep.data_ptr()
-        if kind < 0:
-            st = L.qlka_laplace_attention_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), kp, float(tau), out.data_ptr(),
-                                                  ws.data_ptr(), int(n.value), B, H, S, D, Dv, _stream())
-        else:
-            st = L.qlka_abs_attention_forward(kind, q.data_ptr(), k.data_ptr(), v.data_ptr(), kp, float(tau), out.data_ptr(),
-                                              ws.data_ptr(), int(n.value), B, H, S, D, Dv, _stream())
-    if st:
-        _raise(st)
-    return out
-
-
-def laplace_attention(q, k, v, tau, keep=None):
-    return fused_attention("add_laplace", q, k, v, tau, keep)
+    """Gradients (grad_q, grad_k, grad_v) of sum(out_w * g_w) + sum(out_u * g_u) of the abs sum."""
+    return ext().abs_backward(q, k, v, g_w, g_u)
 
 
 def laplace_backward(q, k, v, g_w, g_u=None):
     """Gradients (grad_q, grad_k, grad_v) of sum(out_w * g_w) + sum(out_u * g_u) of the Laplace sum."""
-    P, D, N, M, C = dims = check_qkv(q, k, v, "q, k, and v")
-    _check_like(g_w, "g_w", (P, M, C), q)
-    if g_u is not None:
-        _check_like(g_u, "g_u", (P, M), q)
-    v, g_w = _aligned(v), _aligned(g_w)
-    L = lib()
-    with torch.cuda.device(q.device):
-        ws, n = _workspace(L.qlka_laplace_backward_workspace_bytes, dims, q.device)
-        gq = torch.empty(P, D, M, dtype=torch.float32, device=q.device)
-        gk = torch.empty(P, D, N, dtype=torch.float32, device=q.device)
-        gv = torch.empty(P, N, C, dtype=torch.float32, device=q.device)
-        st = L.qlka_weighted_laplace_sum_backward(q.data_ptr(), k.data_ptr(), v.data_ptr(), g_w.data_ptr(),
-                                                  None if g_u is None else g_u.data_ptr(),
-                                                  gq.data_ptr(), gk.data_ptr(), gv.data_ptr(),
-                                                  ws.data_ptr(), n, P, D, N, M, C, _stream())
-    if st:
-        _raise(st)
-    return gq, gk, gv
+    return ext().laplace_backward(q, k, v, g_w, g_u)
 
 
 def sgn_forward(q, k, v, g):
-    P, D, N, M, C = dims = check_qkv(q, k, v, "q, k, and v")
-    _check_like(g, "g", (P, M, C), q)
-    v, g = _aligned(v), _aligned(g)
-    L = lib()
-    with torch.cuda.device(q.device):
-        ws, n = _workspace(L.qlka_sgn_forward_workspace_bytes, dims, q.device)
-        out = torch.empty(P, D, M, dtype=torch.float32, device=q.device)
-        st = L.qlka_weighted_sgn_sum_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), out.data_ptr(),
-                                             ws.data_ptr(), n, P, D, N, M, C, _stream())
-    if st:
-        _raise(st)
-    return out
+    return ext().sgn_forward(q, k, v, g)
+
+
+ATTENTION_KINDS = {"add_riesz": 0, "add_bump": 1, "add_laplace": 2}
+
+
+def fused_attention(kernel, q, k, v, tau, keep=None):
+    """Normalised additive-kernel attention on (B, H, S, D) / (B, H, S, Dv) tensors in one native call (forward only)."""
+    with torch.no_grad():
+        return ext().attention(ATTENTION_KINDS[kernel], q, k, v, float(tau), keep)
+
+
+def attention(kernel, q, k, v, tau, keep=None):
+    """The same, differentiable: one native call forward and one backward. None where inputs want a gradient and there is no
+    single backward call (long sequences of add_riesz and add_bump)."""
+    return ext().attention(ATTENTION_KINDS[kernel], q, k, v, float(tau), keep)
+
+
+def laplace_attention(q, k, v, tau, keep=None):
+    return fused_attention("add_laplace", q, k, v, tau, keep)
 
 
 def sort_rank_records(x, y, mode):

@@ -8,8 +8,6 @@ kernels, which cover short sequences as well; "keops" is accepted and means "the
 beyond 4096 elements fails as it does in the reference.
 """
 
-import torch
-
 import qlka_native as _native
 
 _BACKENDS = ("auto", "keops", "cuda", "cuda-fused", "cuda-global")
@@ -33,55 +31,18 @@ def _resolve(backend):
     return _PATH[backend]
 
 
-class _WeightedAbsSum(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, path):
-        ctx.save_for_backward(q, k, v)
-        ctx.set_materialize_grads(False)
-        return _native.abs_forward(q, k, v, full=False, path=path)[0]
-
-    @staticmethod
-    def backward(ctx, g_w):
-        q, k, v = ctx.saved_tensors
-        if g_w is None:
-            return None, None, None, None
-        grad_q, grad_k, grad_v = _native.abs_backward(q, k, v, g_w.contiguous())
-        return grad_q, grad_k, grad_v, None
-
-
-class _WeightedAbsSumFull(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, path):
-        ctx.save_for_backward(q, k, v)
-        ctx.set_materialize_grads(False)
-        return _native.abs_forward(q, k, v, full=True, path=path)
-
-    @staticmethod
-    def backward(ctx, g_w, g_u):
-        q, k, v = ctx.saved_tensors
-        if g_w is None and g_u is None:
-            return None, None, None, None
-        if g_u is None:     # nothing flowed back into the row sums: the native call skips their scalar terms
-            grad_q, grad_k, grad_v = _native.abs_backward(q, k, v, g_w.contiguous())
-        else:
-            if g_w is None:
-                g_w = torch.zeros(q.shape[0], q.shape[2], v.shape[2], device=q.device, dtype=q.dtype)
-            grad_q, grad_k, grad_v = _native.abs_backward(q, k, v, g_w.contiguous(), g_u.contiguous())
-        return grad_q, grad_k, grad_v, None
-
-
 def weighted_abs_sum(q, k, v, backend="auto"):
     """out[p,m,c] = sum_{n,d} |k[p,d,n] - q[p,d,m]| * v[p,n,c]
 
     q: (P, D, M), k: (P, D, N), v: (P, N, C) -> (P, M, C). Differentiable.
     """
-    return _WeightedAbsSum.apply(q, k, v, _resolve(backend))
+    return _native.ext().abs_sum(q, k, v, False, _resolve(backend))[0]
 
 
 def weighted_abs_sum_full(q, k, v, backend="auto"):
     """Returns (out_w, out_u): the weighted abs sum (P, M, C) and the unweighted abs sum
     out_u[p,m] = sum_{n,d} |k[p,d,n] - q[p,d,m]| (P, M). Differentiable in both outputs."""
-    return _WeightedAbsSumFull.apply(q, k, v, _resolve(backend))
+    return tuple(_native.ext().abs_sum(q, k, v, True, _resolve(backend)))
 
 
 def weighted_abs_sum_shifted(q, k, v, shifts, weights):

@@ -6,26 +6,7 @@ backward runs the same sort and walk kernels with the roles of queries and keys 
 under `torch.no_grad()` or with inputs that need no gradient it is exactly the reference's call.
 """
 
-import torch
-
 import qlka_native as _native
-
-
-class _WeightedLaplaceSum(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v):
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(q, k, v)
-        return _native.laplace_forward(q, k, v)
-
-    @staticmethod
-    def backward(ctx, g_w, g_u):
-        q, k, v = ctx.saved_tensors
-        if g_w is None and g_u is None:
-            return None, None, None
-        if g_w is None:
-            g_w = torch.zeros(q.shape[0], q.shape[2], v.shape[2], device=q.device, dtype=q.dtype)
-        return _native.laplace_backward(q, k, v, g_w.contiguous(), None if g_u is None else g_u.contiguous())
 
 
 def weighted_laplace_sum(q, k, v):
@@ -38,9 +19,7 @@ def weighted_laplace_sum(q, k, v):
     Differentiable in both outputs (where a key equals a query the one-sided derivative of the walk's
     tie side is taken). Padded keys: zero k and v there and subtract n_pad * sum_d exp(-|q_d|) from out_u.
     """
-    if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
-        return _WeightedLaplaceSum.apply(q, k, v)
-    return _native.laplace_forward(q, k, v)
+    return _native.ext().laplace_sum(q, k, v)
 
 
 def weighted_laplace_sum_backward(q, k, v, g_w, g_u=None):
