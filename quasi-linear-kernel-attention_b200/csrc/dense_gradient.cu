@@ -145,6 +145,7 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
     float* yw = Gs + GT * G_LD;                          // [64] weight of y: keep mask, 0 beyond the last
     float* ys = yw + GT;                                 // [64] scalar of y
     float* rg = ys + GT;                                 // [2][64] row sums of G (RIESZ)
+    int*   list = reinterpret_cast<int*>(rg + 2 * GT);   // [ytiles + 1] with a keep mask over y: its active tiles and their number
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int mg = (warp & 3) * 4 + (lane & 3), ng = (warp >> 2) * 8 + (lane >> 2);
@@ -158,11 +159,17 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
     const float* xt_g = g.staged + (keys ? gv.vt : gv.at) + (long long)xtile * C4 * GT;
     const float* yt_g = g.staged + (keys ? gv.at : gv.vt) + (long long)p * ytiles * C4 * GT;
     const float* keep = g.keep ? g.keep + (long long)(p / g.H) * g.N : nullptr;
-    const int t0 = (int)((long long)rank * ytiles / split), t1 = (int)((long long)(rank + 1) * ytiles / split);
+    const int active = keep && !keys ? active_tiles(keep, g.N, list, list + ytiles) : ytiles;
+    int t0 = (int)((long long)rank * active / split), t1 = (int)((long long)(rank + 1) * active / split);
+    if (keep && keys) {                                  // x that all are masked
+        const bool on = tid < GT && x0 + tid < Lx && __ldg(keep + x0 + tid) != 0.0f;
+        if (!__syncthreads_or(on)) t1 = t0;
+    }
+    auto tile_at = [&](const int t) -> int { return keep && !keys ? list[t] : t; };
 
     auto copy = [&](float* dst, const float* src, const int n) { for (int i = tid * 4; i < n; i += G_THREADS * 4) cp16(dst + i, src + i); };
-    auto issue_yt = [&](const int t) { if (t < t1) copy(yt, yt_g + (long long)t * C4 * GT, C4 * GT); cp_commit(); };
-    auto issue_yr = [&](const int t) { if (t < t1) copy(yr, yr_g + (long long)t * RA * GT * DP, RA * GT * DP); cp_commit(); };
+    auto issue_yt = [&](const int t) { if (t < t1) copy(yt, yt_g + (long long)tile_at(t) * C4 * GT, C4 * GT); cp_commit(); };
+    auto issue_yr = [&](const int t) { if (t < t1) copy(yr, yr_g + (long long)tile_at(t) * RA * GT * DP, RA * GT * DP); cp_commit(); };
     copy(xt, xt_g, C4 * GT);
     issue_yt(t0);
     issue_yr(t0);
@@ -184,8 +191,8 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
     }
     const int* flag = reinterpret_cast<const int*>(g.staged) + gv.flag;
     const long long fx = keys ? g.P * (long long)ytiles : 0, fy = keys ? 0 : g.P * (long long)xtiles;       // flags of the x and of the y side
-    for (int t = t0; t < t1; t++) {
-        const int y0 = t * GT;
+    for (int step = t0; step < t1; step++) {
+        const int t = tile_at(step), y0 = t * GT;
         const bool plain = KIND == DENSE_LAPLACE && (__ldg(flag + fx + xtile) | __ldg(flag + fy + (long long)p * ytiles + t)) != 0;
         if (tid < GT) {
             yw[tid] = y0 + tid < Ly ? (keep && !keys ? __ldg(keep + y0 + tid) : 1.0f) : 0.0f;
@@ -226,7 +233,7 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
         }
         cp_wait<0>();
         __syncthreads();
-        issue_yt(t + 1);                                 // (everybody has left this tile's)
+        issue_yt(step + 1);                                 // (everybody has left this tile's)
         // ---- contraction over y
         #pragma unroll
         for (int h = 0; h < ND; h++) {
@@ -290,7 +297,7 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
             }
         }
         __syncthreads();                                 // the y rows and G are free again
-        issue_yr(t + 1);
+        issue_yr(step + 1);
     }
     cp_wait<0>();
     if (KIND == DENSE_RIESZ) {                           // |x|_1 in every A: sign(x) times the row sum of G
@@ -315,25 +322,29 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
         for (int i = 0; i < 4; i++)
             *reinterpret_cast<float4*>(part + (mg * 4 + i) * DP + h * 64 + ng * 4) = make_float4(acc[h][i][0], acc[h][i][1], acc[h][i][2], acc[h][i][3]);
     if (split > 1) cl_g.sync(); else __syncthreads();
-    const int r0 = GT * rank / split, r1 = GT * (rank + 1) / split, rn = r1 - r0;
-    for (int i = tid; i < rn * D; i += G_THREADS) {
-        const int r = r0 + (g.attention ? i / D : i % rn), d = g.attention ? i % D : i / rn;
-        if (x0 + r >= Lx) continue;
-        float s = 0.0f, G = 0.0f;
-        if (split > 1) {
-            for (int b = 0; b < split; b++) {
-                s += cl_g.map_shared_rank(part, b)[r * DP + d];
-                if (KIND == DENSE_RIESZ) { const float* q = cl_g.map_shared_rank(rg, b); G += q[r] + q[GT + r]; }
-            }
-        } else {
-            s = part[r * DP + d];
-            if (KIND == DENSE_RIESZ) G = rg[r] + rg[GT + r];
+    // this CTA's rows, as float4s of features, lanes along the contiguous direction of the gradient
+    const int r0 = GT * rank / split, rn = GT / split, d4 = (D + 3) >> 2;
+    #pragma unroll 4
+    for (int i = tid; i < rn * d4; i += G_THREADS) {
+        const int r = r0 + (g.attention ? i / d4 : i % rn), d = (g.attention ? i % d4 : i / rn) * 4;
+        float y[4] = {0.f, 0.f, 0.f, 0.f}, G = 0.0f;
+        #pragma unroll
+        for (int b = 0; b < 8; b++) {
+            if (b >= split) break;
+            const float4 v = *reinterpret_cast<const float4*>((split > 1 ? cl_g.map_shared_rank(part, b) : part) + r * DP + d);
+            y[0] += v.x; y[1] += v.y; y[2] += v.z; y[3] += v.w;
+            if (KIND == DENSE_RIESZ) { const float* q = split > 1 ? cl_g.map_shared_rank(rg, b) : rg; G += q[r] + q[GT + r]; }
         }
-        s *= sign;
-        if (KIND == DENSE_RIESZ) { const float x = __ldg(xr_g + r * DP + d); s += x > 0.0f ? G : x < 0.0f ? -G : 0.0f; }
-        if (g.attention) s *= g.scale;
-        if (keys && keep) { const float w = __ldg(keep + x0 + r); s = w != 0.0f ? s * w : 0.0f; }
-        grad[(x0 + r) * s_row + d * s_d] = s;
+        if (x0 + r >= Lx) continue;
+        const float w = keys && keep ? __ldg(keep + x0 + r) : 1.0f;
+        #pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if (d + e >= D) continue;
+            float s = y[e] * sign;
+            if (KIND == DENSE_RIESZ) { const float x = __ldg(xr_g + r * DP + d + e); s += x > 0.0f ? G : x < 0.0f ? -G : 0.0f; }
+            if (g.attention) s *= g.scale;
+            grad[(x0 + r) * s_row + (d + e) * s_d] = w != 0.0f ? s * w : 0.0f;
+        }
     }
     if (split > 1) cl_g.sync();                          // nobody leaves while its shared memory is still read
 }
@@ -345,6 +356,7 @@ static cudaError_t launch_gradient_inst(DenseGradArgs g, int sms, cudaStream_t s
     size_t smem = sizeof(float) * ((size_t)2 * c4 * GT + row_arrays<KIND>() * GT * ND * 64 + GT * G_LD + 2 * GT + 2 * GT);
     const size_t need = sizeof(float) * ((size_t)c4 * GT + GT * ND * 64 + 2 * GT);       // (the partial result overlies the y tile)
     if (smem < need) smem = need;
+    if (g.keep) smem += sizeof(int) * ((g.N + GT - 1) / GT + 1);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     for (int keys = 0; keys < 2; keys++) {

@@ -145,10 +145,10 @@ __global__ void __launch_bounds__(256) dense_stage(const DenseArgs a)
     }
 }
 
-// shared memory of the main kernel, in floats: q tile | k chunks | A tile | v tile | key weights | key norms | row sums
+// shared memory of the main kernel, in floats: q tile | k chunks | A tile | v tile | key weights | key norms | row sums | tile list
 template <int KIND, int CT>
-static size_t dense_smem_bytes(int D) {
-    return sizeof(float) * ((size_t)D * TM + KSTAGES * kind_arrays<KIND>() * kind_chunk<KIND>() * TN + TN * AT_LD + TN * CT * 8 + 2 * TN + TM);
+static size_t dense_smem_bytes(int D, int list) {
+    return sizeof(float) * (list + (size_t)D * TM + KSTAGES * kind_arrays<KIND>() * kind_chunk<KIND>() * TN + TN * AT_LD + TN * CT * 8 + 2 * TN + TM);
 }
 
 // CT: channels per thread (C <= 8 CT). Thread (mg, ng) of 16 x 8 owns the pairs of queries 4 mg .. 4 mg + 3 with the keys
@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
     float* kw = vs + TN * CP;                            // [TN] weight of a key: keep mask, 0 beyond the last key
     float* kns = kw + TN;                                // [TN] |k|_1 (RIESZ)
     float* rsum = kns + TN;                              // [TM]
+    int*   list = reinterpret_cast<int*>(rsum + TM);     // [ntiles + 1] with a keep mask: its active tiles and their number
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int mg = warp * 4 + (lane & 3), ng = lane >> 2;
@@ -178,7 +179,13 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
     const float* kst = a.staged + sv.k + (long long)p * ntiles * NA * D * TN;
     const float* v = a.v + (long long)p * N * C;
     const float* keep = a.keep ? a.keep + (long long)(p / a.H) * N : nullptr;
-    const int tile0 = (int)((long long)rank * ntiles / split), tile1 = (int)((long long)(rank + 1) * ntiles / split);
+    const int active = keep ? active_tiles(keep, N, list, list + ntiles) : ntiles;
+    int tile0 = (int)((long long)rank * active / split), tile1 = (int)((long long)(rank + 1) * active / split);
+    if (a.row_keep) {                                    // rows that all are masked
+        const bool on = tid < TM && m0 + tid < M && __ldg(a.row_keep + (long long)(p / a.H) * M + m0 + tid) != 0.0f;
+        if (!__syncthreads_or(on)) tile1 = tile0;
+    }
+    auto tile_at = [&](const int t) -> int { return keep ? list[t] : t; };
     const int nchunks = (D + DK - 1) / DK;
 
     // chunk c of this CTA's sequence (tile tile0 + c / nchunks, features DK (c mod nchunks) on) into its stage
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
     auto issue_chunk = [&]() {
         if (it < tile1) {
             const int d0 = ic * DK, n4 = min(DK, D - d0) * (TN / 4);         // float4s per array
-            const float* src = kst + ((long long)it * NA * D + d0) * TN;
+            const float* src = kst + ((long long)tile_at(it) * NA * D + d0) * TN;
             float* dst = ks + istage * CHUNK;
             #pragma unroll
             for (int b = 0; b < NA; b++)
@@ -221,8 +228,8 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
         for (int c = 0; c < CT / 2; c++) o[i][c] = 0ull;
     }
     int stage = 0;
-    for (int t = tile0; t < tile1; t++) {
-        const int n0 = t * TN;
+    for (int i = tile0; i < tile1; i++) {
+        const int t = tile_at(i), n0 = t * TN;
         float acc[4][8];
         #pragma unroll
         for (int i = 0; i < 4; i++)
@@ -400,18 +407,31 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
                 *reinterpret_cast<ulonglong2*>(part + (mg * 4 + i) * CP + h * 32 + ng * 4) = make_ulonglong2(o[i][2 * h], o[i][2 * h + 1]);
         }
         cl.sync();
-        const int r0 = TM * rank / split, r1 = TM * (rank + 1) / split;
-        for (int i = tid; i < (r1 - r0) * C; i += DT_THREADS) {
-            const int r = r0 + i / C, c = i % C;
-            float s = 0.0f, den = 0.0f;
-            for (int b = 0; b < split; b++) {
-                s   += cl.map_shared_rank(part, b)[r * CP + c];
+        // (float4s, a few at a time: every remote load takes some hundred cycles)
+        const int r0 = TM * rank / split, rn = TM / split, c4 = (C + 3) >> 2;
+        #pragma unroll 4
+        for (int i = tid; i < rn * c4; i += DT_THREADS) {
+            const int r = r0 + i / c4, c = (i % c4) * 4;
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            float  den = 0.0f;
+            #pragma unroll
+            for (int b = 0; b < 8; b++) {
+                if (b >= split) break;
+                const float4 x = *reinterpret_cast<const float4*>(cl.map_shared_rank(part, b) + r * CP + c);
+                s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
                 den += cl.map_shared_rank(rsum, b)[r];
             }
-            if (m0 + r < M) {
-                a.out[((long long)p * M + m0 + r) * C + c] = s * (finish(den) * row_weight(m0 + r));
-                if (a.out_u && c == 0) a.out_u[(long long)p * M + m0 + r] = den;
+            if (m0 + r >= M) continue;
+            const float f = finish(den) * row_weight(m0 + r);
+            float* dst = a.out + ((long long)p * M + m0 + r) * C + c;
+            if ((C & 3) == 0) {
+                *reinterpret_cast<float4*>(dst) = make_float4(s.x * f, s.y * f, s.z * f, s.w * f);
+            } else {
+                const float y[4] = {s.x * f, s.y * f, s.z * f, s.w * f};
+                #pragma unroll
+                for (int e = 0; e < 4; e++) if (c + e < C) dst[e] = y[e];
             }
+            if (a.out_u && c == 0) a.out_u[(long long)p * M + m0 + r] = den;
         }
         cl.sync();                                       // nobody leaves while its shared memory is still read
     }
@@ -420,7 +440,7 @@ __global__ void __launch_bounds__(DT_THREADS, CT > 8 ? 2 : 3) dense_forward(cons
 template <int KIND, int CT>
 static cudaError_t launch_dense_inst(const DenseArgs& a, cudaStream_t stream) {
     auto kern = dense_forward<KIND, CT>;
-    const size_t smem = dense_smem_bytes<KIND, CT>(a.D);
+    const size_t smem = dense_smem_bytes<KIND, CT>(a.D, a.keep ? (a.N + TN - 1) / TN + 1 : 0);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
@@ -428,7 +448,7 @@ static cudaError_t launch_dense_inst(const DenseArgs& a, cudaStream_t stream) {
     cfg.blockDim = dim3(DT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at{};
+    cudaLaunchAttribute at{};                            // (a programmatic launch that overlaps dense_stage was measured slower: its CTAs take the room)
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = a.split; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at; cfg.numAttrs = 1;

@@ -47,17 +47,47 @@ struct DenseGradArgs {
 size_t      dense_gradient_workspace_bytes(int kind, int P, int D, int N, int M, int C, bool attention);
 cudaError_t launch_dense_gradient(const DenseGradArgs& g, int kind, int sms, cudaStream_t stream);
 
-// CTAs that share one tile of 64 rows: the count that gives the busiest SM the fewest tiles of the other side, a CTA's own start
-// and end counted as one more tile
+// CTAs that share one tile of 64 rows: the count that takes the busiest SM the least time, in tiles of the other side; a CTA's own
+// start and end count as one and a half more, and an SM with one or two of these CTAs leaves a half or a fifth of itself idle.
+inline double dense_sm_cost(long long ctas, int ntiles, int split, int sms) {
+    const long long per_sm = (ctas * split + sms - 1) / sms;
+    return per_sm * (per_sm < 2 ? 2.2 : per_sm < 3 ? 1.25 : 1.0) * ((ntiles + split - 1) / split + 1.5);
+}
 inline int dense_split(long long ctas, int ntiles, int sms) {
     int best = 1;
-    double best_cost = 1e300;
-    for (int s = 1; s <= 8 && s <= ntiles; s *= 2) {
-        const double cost = (double)((ctas * s + sms - 1) / sms) * ((ntiles + s - 1) / s + 1.0);
-        if (cost < best_cost * 0.97) { best = s; best_cost = cost; }
-    }
+    for (int s = 2; s <= 8 && s <= ntiles; s *= 2)
+        if (dense_sm_cost(ctas, ntiles, s, sms) < 0.97 * dense_sm_cost(ctas, ntiles, best, sms)) best = s;
     return best;
 }
+
+#ifdef __CUDACC__
+// The tiles of 64 keys that hold an unmasked one, in order, into `list` (shared memory, one entry per tile); returns their number.
+// Padding at the end of a sequence costs nothing that way. All threads of the block call it; `keep` has N entries.
+__device__ __forceinline__ int active_tiles(const float* __restrict__ keep, const int N, int* list, int* count) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, tiles = (N + 63) / 64;
+    for (int t = warp; t < tiles; t += warps) {
+        const int  n = t * 64 + lane;
+        const bool on = (n < N && __ldg(keep + n) != 0.0f) || (n + 32 < N && __ldg(keep + n + 32) != 0.0f);
+        const bool any = __any_sync(0xffffffffu, on);
+        if (lane == 0) list[t] = any;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int n = 0;
+        for (int t0 = 0; t0 < tiles; t0 += 32) {
+            const bool     on = t0 + lane < tiles && list[t0 + lane];
+            const unsigned b  = __ballot_sync(0xffffffffu, on);
+            __syncwarp();
+            if (on) list[n + __popc(b & ((1u << lane) - 1u))] = t0 + lane;      // (never ahead of the entries still to be read)
+            n += __popc(b);
+            __syncwarp();
+        }
+        if (lane == 0) *count = n;
+    }
+    __syncthreads();
+    return *count;
+}
+#endif
 
 constexpr float LAP_RANGE = 80.0f;     // largest |value| whose exponentials the Laplace kernels multiply
 constexpr int DENSE_MAX_D = 128;      // the query tile of all features stays in shared memory

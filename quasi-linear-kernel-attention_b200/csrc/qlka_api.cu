@@ -289,12 +289,10 @@ double dense_us(int kind, double P, int D, int N, int M, int C) {
     const int    sms = sm_count();
     const double tile = 4096e-6 * sms * (D * per_d + (C <= 32 ? 32 : C <= 64 ? 64 : 128) * per_c);     // us of one SM per 64 x 64 pairs
     const int    nt = (N + 63) / 64;
-    const double ctas = P * ((M + 63) / 64);
-    double best = 1e300;
-    for (int s = 1; s <= 8 && s <= nt; s *= 2) {                       // the kernel's own choice of CTAs per query tile, about
-        const double per_sm = std::ceil(ctas * s / sms), alone = per_sm < 2 ? 2.2 : per_sm < 3 ? 1.25 : 1.0;
-        best = std::min(best, per_sm * alone * ((nt + s - 1) / s + 0.5) * tile);
-    }
+    const long long ctas = (long long)P * ((M + 63) / 64);
+    const int split = dense_split(ctas, nt, sms);
+    const double per_sm = std::ceil((double)ctas * split / sms), alone = per_sm < 2 ? 2.2 : per_sm < 3 ? 1.25 : 1.0;
+    const double best = per_sm * alone * ((nt + split - 1) / split + 0.5) * tile;
     return 8.0 + best;
 }
 double sorted_us(int kind, double P, int D, int N, int M, int C) {
@@ -302,14 +300,16 @@ double sorted_us(int kind, double P, int D, int N, int M, int C) {
     const double keys = N * (0.022 + 0.045 * wide), queries = M * (0.022 + 0.050 * wide) * (kind == DENSE_BUMP ? 5.0 : 1.0);
     return 70.0 + segs * (30.0 + keys + queries) * 1e-3;               // (launches and tails; nanoseconds per segment)
 }
-bool dense_pays(int kind, long long P, int D, int N, int M, int C) {
+// A key mask lets the pairwise kernels skip whole tiles of padding (a seventh is assumed) and costs the sorted path its bucket
+// sort: masked keys are zeros, too many in one bucket.
+bool dense_pays(int kind, long long P, int D, int N, int M, int C, bool masked = false) {
     if (D > DENSE_MAX_D) return false;
-    return dense_us(kind, (double)P, D, N, M, C) < sorted_us(kind, (double)P, D, N, M, C);
+    return dense_us(kind, (double)P, D, N, M, C) * (masked ? 0.85 : 1.0) < sorted_us(kind, (double)P, D, N, M, C) * (masked ? 1.25 : 1.0);
 }
 
 // The same for the gradients: three kernels of the same tiling against two sorts and three walks (Laplace 0.43 ns per feature
 // and key, abs 0.30, measured at 4096 keys; the bump's are three abs gradients put together op by op).
-bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C) {
+bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C, bool masked = false) {
     if (D > DENSE_MAX_D) return false;
     const double grad_d = kind == DENSE_LAPLACE ? 0.50 : kind == DENSE_BUMP ? 0.68 : 0.26, grad_c = 0.054;
     const int    cw = C <= 32 ? 32 : C <= 64 ? 64 : 128;
@@ -318,12 +318,12 @@ bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C) {
     const double dense = 20.0 + std::max(per_sm, 1.0) * ((M + N + 127) / 128) * tile * (per_sm < 2 ? 0.5 : 1.0) + dense_us(kind, (double)P, D, M, N, C);
     const double wide = C <= 32 ? 0.8 : C <= 64 ? 1.0 : 1.4, pair = kind == DENSE_LAPLACE ? 0.43 : kind == DENSE_BUMP ? 1.45 : 0.30;
     const double sorted = (kind == DENSE_BUMP ? 250.0 : 110.0) + (double)P * D * (60.0 + pair * wide * 0.5 * (N + M)) * 1e-3;
-    return dense < sorted;
+    return dense * (masked ? 0.85 : 1.0) < sorted * (masked ? 1.25 : 1.0);
 }
 
 // scratch of the pairwise kernels where they are the ones to run
-size_t dense_bytes(int kind, int P, int D, int N, int M, int C) {
-    return dense_pays(kind, P, D, N, M, C) ? dense_workspace_bytes(kind, P, D, N, M) : 0;
+size_t dense_bytes(int kind, int P, int D, int N, int M, int C, bool masked = false) {
+    return dense_pays(kind, P, D, N, M, C, masked) ? dense_workspace_bytes(kind, P, D, N, M) : 0;
 }
 
 DenseArgs dense_args(const float* q, const float* k, const float* v, float* out, float* out_u, void* ws, int P, int D, int N, int M, int C) {
@@ -622,7 +622,7 @@ int qlka_laplace_attention_workspace_bytes(int B, int H, int S, int D, int Dv, i
     if (!bytes) return QLKA_ERR_NULL;
     int st = attn_check(B, H, S, D, Dv);
     if (st) return st;
-    *bytes = std::max(LaplaceAttnWs(nullptr, B, H, S, D, Dv, masked != 0).bytes, dense_bytes(DENSE_LAPLACE, B * H, D, S, S, Dv));
+    *bytes = std::max(LaplaceAttnWs(nullptr, B, H, S, D, Dv, masked != 0).bytes, dense_bytes(DENSE_LAPLACE, B * H, D, S, S, Dv, masked != 0));
     return QLKA_OK;
 }
 
@@ -636,7 +636,7 @@ static int laplace_attention_impl(const float* q, const float* k, const float* v
     if (!q || !k || !v || !out) return QLKA_ERR_NULL;
     if (!aligned16(v, out)) return QLKA_ERR_ALIGNMENT;
     if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
-    if (dense_pays(DENSE_LAPLACE, (long long)B * H, D, S, S, Dv)) {
+    if (dense_pays(DENSE_LAPLACE, (long long)B * H, D, S, S, Dv, keep != nullptr)) {
         if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(DENSE_LAPLACE, B * H, D, S, S))) return QLKA_ERR_WORKSPACE;
         CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, den, tau, workspace, B * H, H, S, D, Dv), DENSE_LAPLACE, sm_count(), stream));
         return QLKA_OK;
@@ -706,7 +706,7 @@ int qlka_abs_attention_workspace_bytes(int kind, int B, int H, int S, int D, int
     if (!bytes) return QLKA_ERR_NULL;
     int st = abs_attn_check(kind, B, H, S, D, Dv);
     if (st) return st;
-    *bytes = std::max(AbsAttnWs(nullptr, B, H, S, D, Dv, masked != 0, kind == 1).bytes, dense_bytes(kind == 1 ? DENSE_BUMP : DENSE_RIESZ, B * H, D, S, S, Dv));
+    *bytes = std::max(AbsAttnWs(nullptr, B, H, S, D, Dv, masked != 0, kind == 1).bytes, dense_bytes(kind == 1 ? DENSE_BUMP : DENSE_RIESZ, B * H, D, S, S, Dv, masked != 0));
     return QLKA_OK;
 }
 
@@ -720,7 +720,7 @@ static int abs_attention_impl(int kind, const float* q, const float* k, const fl
     if (!aligned16(v, out)) return QLKA_ERR_ALIGNMENT;
     if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
     const bool masked = keep != nullptr, bump = kind == 1;
-    if (const int dk = bump ? DENSE_BUMP : DENSE_RIESZ; dense_pays(dk, (long long)B * H, D, S, S, Dv)) {
+    if (const int dk = bump ? DENSE_BUMP : DENSE_RIESZ; dense_pays(dk, (long long)B * H, D, S, S, Dv, masked)) {
         if (!ws_ok(workspace, workspace_bytes, dense_workspace_bytes(dk, B * H, D, S, S))) return QLKA_ERR_WORKSPACE;
         CU(launch_dense_forward(dense_attention_args(q, k, v, keep, out, den, tau, workspace, B * H, H, S, D, Dv), dk, sm_count(), stream));
         return QLKA_OK;
@@ -809,7 +809,7 @@ int qlka_attention_backward_workspace_bytes(int kind, int B, int H, int S, int D
     int st = kind == ATTN_LAPLACE ? attn_check(B, H, S, D, Dv) : abs_attn_check(kind, B, H, S, D, Dv);
     if (st) return st;
     const int dk = dense_kind_of(kind);
-    if (dense_gradient_pays(dk, (long long)B * H, D, S, S, Dv)) *bytes = dense_gradient_workspace_bytes(dk, B * H, D, S, S, Dv, true);
+    if (dense_gradient_pays(dk, (long long)B * H, D, S, S, Dv, masked != 0)) *bytes = dense_gradient_workspace_bytes(dk, B * H, D, S, S, Dv, true);
     else if (kind == ATTN_LAPLACE)                              *bytes = LaplaceAttnBwdWs(nullptr, B, H, S, D, Dv, masked != 0).bytes;
     else                                                        return QLKA_ERR_UNSUPPORTED;
     return QLKA_OK;
@@ -830,7 +830,7 @@ int qlka_attention_backward(int kind, const float* q, const float* k, const floa
     if (!ws_ok(workspace, workspace_bytes, need)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int P = B * H, dk = dense_kind_of(kind);
-    if (dense_gradient_pays(dk, P, D, S, S, Dv)) {
+    if (dense_gradient_pays(dk, P, D, S, S, Dv, masked)) {
         DenseGradArgs g = dense_grad_args(q, k, v, grad_out, nullptr, grad_q, grad_k, grad_v, workspace, P, D, S, S, Dv);
         g.attention = true; g.H = H; g.scale = 1.0f / tau; g.eps = 1e-3f; g.clamp = 1e-6f; g.keep = keep; g.out = out; g.den = den;
         CU(launch_dense_gradient(g, dk, sm_count(), stream));
