@@ -199,6 +199,32 @@ int qlka_weighted_sgn_sum_forward(const float* q, const float* k, const float* v
                                   void* workspace, size_t workspace_bytes,
                                   int P, int D, int N, int M, int C, qlka_stream_t stream);
 
+/* ---- linear layers of the encoder --------------------------------------------------------
+ * fp32 matrix products on the bf16 tensor cores without loss of precision: every operand is cut into three bf16 parts that
+ * add up to it (24 bits), six products of parts are summed in fp32 (the three left out are below 2^-24 of the product). `parts`
+ * of a (rows, K) matrix are three bf16 (rows, K) matrices one after the other, 6 * rows * K bytes. Weights are (N, K) row-major as
+ * in torch.nn.Linear; K and N must be multiples of 32 (QLKA_ERR_UNSUPPORTED otherwise), all pointers 16-byte aligned; the
+ * workspace takes the weight's parts.
+ *   split_rows       parts of x (rows, K), after a layer norm when its weight and bias are given (K % 4 == 0)
+ *   split_heads      parts of the (B, S, H * D) matrix whose heads are o (B, H, S, D)
+ *   linear_qkv       y = A W^T + bias with N = 3 * H * 64: q, k, v (B, H, S, 64), q and k turned by rotary position embedding,
+ *                    pairs (i, i + 32), cosines and sines in table (S, 32, 2)
+ *   linear_gelu      parts of GELU(A W^T + bias)
+ *   linear_residual  x += A W^T + bias
+ * linear_error waits for the device and reports whether a kernel of these has ever given up on a barrier (0: none has).
+ * No counterpart in the reference, which uses torch.nn.Linear. */
+size_t qlka_linear_workspace_bytes(int N, int K);
+int qlka_split_rows(const float* x, const float* ln_weight /* nullable */, const float* ln_bias /* nullable */, float eps, void* parts,
+                    int rows, int K, qlka_stream_t stream);
+int qlka_split_heads(const float* o, void* parts, int B, int H, int S, int D, qlka_stream_t stream);
+int qlka_linear_qkv(const void* parts, const float* weight, const float* bias, const float* table, float* q, float* k, float* v,
+                    void* workspace, size_t workspace_bytes, int B, int S, int H, int K, qlka_stream_t stream);
+int qlka_linear_gelu(const void* parts, const float* weight, const float* bias, void* out_parts, void* workspace, size_t workspace_bytes,
+                     int M, int N, int K, qlka_stream_t stream);
+int qlka_linear_residual(const void* parts, const float* weight, const float* bias, float* x, void* workspace, size_t workspace_bytes,
+                         int M, int N, int K, qlka_stream_t stream);
+int qlka_linear_error(int* error);
+
 /* ---- diagnostic: the sort/rank stage alone ---------------------------------------------
  * Sorts x (P, D, N) as the key stream and ranks y (P, D, M) against it, writing the walk
  * records: xperm (P*D, NP) uint32, xval (P*D, NP + 8) float, yrec (P*D, M + 1) 4 x uint32

@@ -20,6 +20,13 @@ int         walk_lanes_per_stream(int C4);
 int         walk_threads();
 int         laplace_agg_stride(int C4);
 int         prefix_agg_stride_host(int C4);
+cudaError_t launch_split_rows(const float* x, const float* w, const float* b, void* out, long long rows, int K, float eps, cudaStream_t st);
+cudaError_t launch_split_heads(const float* o, void* out, int B, int H, int S, int D, cudaStream_t st);
+cudaError_t launch_linear_qkv(const void* a3, const void* w3, const float* bias, const float* table, float* q, float* k, float* v,
+                              int B, int S, int H, int K, int sms, cudaStream_t st);
+cudaError_t launch_linear_gelu(const void* a3, const void* w3, const float* bias, void* out3, int M, int N, int K, int sms, cudaStream_t st);
+cudaError_t launch_linear_residual(const void* a3, const void* w3, const float* bias, float* x, int M, int N, int K, int sms, cudaStream_t st);
+cudaError_t read_linear_error(int* error);
 cudaError_t launch_colsum_d(const float* x, float* out, int P, int D, int L, cudaStream_t st);
 cudaError_t launch_rowstat(const float* w, const float* s, float* wsum, float* swsum, float* ssum, int P, int R, int C4, cudaStream_t st);
 cudaError_t launch_vecsum(const float* x, float* out, int P, int L, cudaStream_t st);
@@ -1097,6 +1104,79 @@ int qlka_weighted_sgn_sum_forward(const float* q, const float* k, const float* v
     WalkArgs w = walk_args(ws.rec, vrows, nseg, D, N, M, C4);
     w.g = grows; w.wtotal = vsum; w.out_s = out; w.sign = -1.0f; w.agg = ws.agg;
     CU(prefix_walk_chunked(w, EMIT_DOT, P, stream));
+    return QLKA_OK;
+}
+
+// ---------------------------------------------------------------- linear layers of the encoder
+int qlka_split_rows(const float* x, const float* ln_weight, const float* ln_bias, float eps, void* parts, int rows, int K, qlka_stream_t stream) {
+    if (rows <= 0 || K <= 0) return QLKA_ERR_BAD_SHAPE;
+    if (!x || !parts || !ln_weight != !ln_bias) return QLKA_ERR_NULL;
+    if (K % 4) return QLKA_ERR_UNSUPPORTED;
+    if (!aligned16(x, parts, ln_weight, ln_bias)) return QLKA_ERR_ALIGNMENT;
+    CU(launch_split_rows(x, ln_weight, ln_bias, parts, rows, K, eps, reinterpret_cast<cudaStream_t>(stream)));
+    return QLKA_OK;
+}
+
+int qlka_split_heads(const float* o, void* parts, int B, int H, int S, int D, qlka_stream_t stream) {
+    if (B <= 0 || H <= 0 || S <= 0 || D <= 0) return QLKA_ERR_BAD_SHAPE;
+    if (!o || !parts) return QLKA_ERR_NULL;
+    if (D % 4) return QLKA_ERR_UNSUPPORTED;
+    if (!aligned16(o, parts)) return QLKA_ERR_ALIGNMENT;
+    CU(launch_split_heads(o, parts, B, H, S, D, reinterpret_cast<cudaStream_t>(stream)));
+    return QLKA_OK;
+}
+
+size_t qlka_linear_workspace_bytes(int N, int K) { return (size_t)6 * N * K; }
+
+// the checks shared by the three layers, and the weight's parts in the workspace
+static int linear_begin(const void* parts, const float* weight, const float* bias, void* workspace, size_t workspace_bytes, int M, int N, int K, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || K <= 0) return QLKA_ERR_BAD_SHAPE;
+    if (!parts || !weight || !bias) return QLKA_ERR_NULL;
+    if (K % 32 || N % 32) return QLKA_ERR_UNSUPPORTED;
+    if (!aligned16(parts, weight, bias)) return QLKA_ERR_ALIGNMENT;
+    if (!ws_ok(workspace, workspace_bytes, qlka_linear_workspace_bytes(N, K))) return QLKA_ERR_WORKSPACE;
+    CU(launch_split_rows(weight, nullptr, nullptr, workspace, N, K, 0.0f, stream));
+    return QLKA_OK;
+}
+
+int qlka_linear_qkv(const void* parts, const float* weight, const float* bias, const float* table, float* q, float* k, float* v,
+                    void* workspace, size_t workspace_bytes, int B, int S, int H, int K, qlka_stream_t stream_) {
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    if (B <= 0 || S <= 0 || H <= 0) return QLKA_ERR_BAD_SHAPE;
+    if ((long long)B * S > INT_MAX || (long long)H * 192 > INT_MAX) return QLKA_ERR_INT32;
+    if (!table || !q || !k || !v) return QLKA_ERR_NULL;
+    if (!aligned16(table, q, k, v)) return QLKA_ERR_ALIGNMENT;
+    int st = linear_begin(parts, weight, bias, workspace, workspace_bytes, B * S, 3 * H * 64, K, stream);
+    if (st) return st;
+    CU(launch_linear_qkv(parts, workspace, bias, table, q, k, v, B, S, H, K, sm_count(), stream));
+    return QLKA_OK;
+}
+
+int qlka_linear_gelu(const void* parts, const float* weight, const float* bias, void* out_parts, void* workspace, size_t workspace_bytes,
+                     int M, int N, int K, qlka_stream_t stream_) {
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    if (!out_parts) return QLKA_ERR_NULL;
+    if (!aligned16(out_parts)) return QLKA_ERR_ALIGNMENT;
+    int st = linear_begin(parts, weight, bias, workspace, workspace_bytes, M, N, K, stream);
+    if (st) return st;
+    CU(launch_linear_gelu(parts, workspace, bias, out_parts, M, N, K, sm_count(), stream));
+    return QLKA_OK;
+}
+
+int qlka_linear_residual(const void* parts, const float* weight, const float* bias, float* x, void* workspace, size_t workspace_bytes,
+                         int M, int N, int K, qlka_stream_t stream_) {
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    if (!x) return QLKA_ERR_NULL;
+    if (!aligned16(x)) return QLKA_ERR_ALIGNMENT;
+    int st = linear_begin(parts, weight, bias, workspace, workspace_bytes, M, N, K, stream);
+    if (st) return st;
+    CU(launch_linear_residual(parts, workspace, bias, x, M, N, K, sm_count(), stream));
+    return QLKA_OK;
+}
+
+int qlka_linear_error(int* error) {
+    if (!error) return QLKA_ERR_NULL;
+    CU(read_linear_error(error));
     return QLKA_OK;
 }
 

@@ -38,6 +38,13 @@ struct Api {
     QLKA_FN(qlka_attention_forward);
     QLKA_FN(qlka_attention_backward_workspace_bytes);
     QLKA_FN(qlka_attention_backward);
+    QLKA_FN(qlka_linear_workspace_bytes);
+    QLKA_FN(qlka_split_rows);
+    QLKA_FN(qlka_split_heads);
+    QLKA_FN(qlka_linear_qkv);
+    QLKA_FN(qlka_linear_gelu);
+    QLKA_FN(qlka_linear_residual);
+    QLKA_FN(qlka_linear_error);
 #undef QLKA_FN
 } api;
 
@@ -63,6 +70,13 @@ void load(const std::string& path) {
     QLKA_FN(qlka_attention_forward);
     QLKA_FN(qlka_attention_backward_workspace_bytes);
     QLKA_FN(qlka_attention_backward);
+    QLKA_FN(qlka_linear_workspace_bytes);
+    QLKA_FN(qlka_split_rows);
+    QLKA_FN(qlka_split_heads);
+    QLKA_FN(qlka_linear_qkv);
+    QLKA_FN(qlka_linear_gelu);
+    QLKA_FN(qlka_linear_residual);
+    QLKA_FN(qlka_linear_error);
 #undef QLKA_FN
 }
 
@@ -310,6 +324,77 @@ std::optional<Tensor> attention(const int64_t kind, const Tensor& q_, const Tens
     return Attention::apply(q, k, v, keep.defined() ? std::optional<Tensor>(keep) : std::nullopt, kind, tau);
 }
 
+// ------------------------------------------------------------------ linear layers of the encoder (inference)
+const Tensor& check_matrix(const Tensor& t, const char* name, const at::IntArrayRef shape) {
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.sizes() == shape, name, " must be a contiguous float32 CUDA tensor of shape ", shape);
+    return t;
+}
+
+Tensor parts_of(const int64_t rows, const int64_t K, const Tensor& like) { return at::detail::empty_cuda({3, rows, K}, at::kBFloat16, like.device(), std::nullopt); }
+
+Tensor split_rows(const Tensor& x, const Tensor& ln_weight, const Tensor& ln_bias, const double eps) {
+    const int64_t rows = x.size(0), K = x.size(1);
+    check_matrix(x, "x", {rows, K});
+    check_matrix(ln_weight, "ln_weight", {K});
+    check_matrix(ln_bias, "ln_bias", {K});
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor parts = parts_of(rows, K, x);
+    check_status(api.qlka_split_rows(ptr(x), ptr(ln_weight), ptr(ln_bias), (float)eps, parts.mutable_data_ptr(), (int)rows, (int)K, current_stream()));
+    return parts;
+}
+
+Tensor split_heads(const Tensor& o) {
+    const int64_t B = o.size(0), H = o.size(1), S = o.size(2), D = o.size(3);
+    check_matrix(o, "o", {B, H, S, D});
+    const c10::cuda::CUDAGuard guard(o.device());
+    Tensor parts = parts_of(B * S, H * D, o);
+    check_status(api.qlka_split_heads(ptr(o), parts.mutable_data_ptr(), (int)B, (int)H, (int)S, (int)D, current_stream()));
+    return parts;
+}
+
+struct Layer { int M, N, K; Tensor ws; size_t bytes; };
+Layer layer(const Tensor& parts, const Tensor& weight, const Tensor& bias) {
+    TORCH_CHECK(parts.is_cuda() && parts.scalar_type() == at::kBFloat16 && parts.is_contiguous() && parts.dim() == 3 && parts.size(0) == 3, "parts must come from split_rows or split_heads");
+    const int64_t M = parts.size(1), K = parts.size(2), N = weight.size(0);
+    check_matrix(weight, "weight", {N, K});
+    check_matrix(bias, "bias", {N});
+    Layer l{(int)M, (int)N, (int)K, Tensor(), api.qlka_linear_workspace_bytes((int)N, (int)K)};
+    l.ws = at::detail::empty_cuda({(int64_t)l.bytes}, at::kByte, parts.device(), std::nullopt);
+    return l;
+}
+
+std::tuple<Tensor, Tensor, Tensor> linear_qkv(const Tensor& parts, const Tensor& weight, const Tensor& bias, const Tensor& table, const int64_t B, const int64_t S, const int64_t H) {
+    const c10::cuda::CUDAGuard guard(parts.device());
+    const Layer l = layer(parts, weight, bias);
+    TORCH_CHECK(l.M == B * S && l.N == 3 * H * 64, "expected B * S rows and 3 * H * 64 columns");
+    check_matrix(table, "table", {S, 32, 2});
+    Tensor q = floats({B, H, S, 64}, parts), k = floats({B, H, S, 64}, parts), v = floats({B, H, S, 64}, parts);
+    check_status(api.qlka_linear_qkv(parts.const_data_ptr(), ptr(weight), ptr(bias), ptr(table), out_ptr(q), out_ptr(k), out_ptr(v),
+                                     l.ws.mutable_data_ptr(), l.bytes, (int)B, (int)S, (int)H, l.K, current_stream()));
+    return {q, k, v};
+}
+
+Tensor linear_gelu(const Tensor& parts, const Tensor& weight, const Tensor& bias) {
+    const c10::cuda::CUDAGuard guard(parts.device());
+    const Layer l = layer(parts, weight, bias);
+    Tensor out = parts_of(l.M, l.N, parts);
+    check_status(api.qlka_linear_gelu(parts.const_data_ptr(), ptr(weight), ptr(bias), out.mutable_data_ptr(), l.ws.mutable_data_ptr(), l.bytes, l.M, l.N, l.K, current_stream()));
+    return out;
+}
+
+void linear_residual(const Tensor& parts, const Tensor& weight, const Tensor& bias, const Tensor& x) {
+    const c10::cuda::CUDAGuard guard(parts.device());
+    const Layer l = layer(parts, weight, bias);
+    check_matrix(x, "x", {l.M, l.N});
+    check_status(api.qlka_linear_residual(parts.const_data_ptr(), ptr(weight), ptr(bias), out_ptr(x), l.ws.mutable_data_ptr(), l.bytes, l.M, l.N, l.K, current_stream()));
+}
+
+int linear_error() {
+    int e = 0;
+    check_status(api.qlka_linear_error(&e));
+    return e;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -322,4 +407,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("abs_sum", &abs_sum);
     m.def("sgn_forward", &sgn_forward);
     m.def("attention", &attention);
+    m.def("split_rows", &split_rows);
+    m.def("split_heads", &split_heads);
+    m.def("linear_qkv", &linear_qkv);
+    m.def("linear_gelu", &linear_gelu);
+    m.def("linear_residual", &linear_residual);
+    m.def("linear_error", &linear_error);
 }

@@ -21,13 +21,18 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 
+def rotary_angles(S, half, device, base=10000.0):
+    """(cos, sin) of the rotary position embedding, (S, half) each."""
+    freq = base ** (-torch.arange(half, device=device, dtype=torch.float32) / half)
+    ang = torch.arange(S, device=device, dtype=torch.float32)[:, None] * freq[None, :]
+    return ang.cos(), ang.sin()
+
+
 def rotary(x, base=10000.0):
     """Rotary position embedding on (B, H, S, Dh), pairs (i, i + Dh/2)."""
     B, H, S, Dh = x.shape
     half = Dh // 2
-    freq = base ** (-torch.arange(half, device=x.device, dtype=torch.float32) / half)
-    ang = torch.arange(S, device=x.device, dtype=torch.float32)[:, None] * freq[None, :]      # (S, half)
-    cos, sin = ang.cos()[None, None], ang.sin()[None, None]
+    cos, sin = (t[None, None] for t in rotary_angles(S, half, x.device, base))
     x1, x2 = x[..., :half], x[..., half:]
     return torch.cat([x1 * cos - x2 * sin, x1 * sin + x2 * cos], dim=-1)
 
@@ -56,6 +61,33 @@ class Block(nn.Module):
         x = x + self.attend(self.ln1(x), keep)
         return x + self.fc2(F.gelu(self.fc1(self.ln2(x))))
 
+    def fits_native(self, x):
+        """Whether `forward_native` takes this block: fp32 on CUDA, heads of 64, sizes in steps of 32, parameters as torch allocates
+        them - and full fp32 products wanted (a caller who allows TF32 gets torch's TF32 products)."""
+        hidden = x.shape[-1]
+        return (x.is_cuda and x.dtype == torch.float32 and x.numel() > 0 and hidden == self.heads * 64 and self.fc1.out_features % 32 == 0
+                and not torch.backends.cuda.matmul.allow_tf32
+                and all(p.dtype == torch.float32 and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0 for p in self.parameters()))
+
+    def forward_native(self, x, table, keep=None):
+        """The block on x (B, S, hidden) in place, without autograd: layer norms, linear layers with their bias, rotary, GELU and
+        residual in the library's kernels (fp32 accuracy), table (S, 32, 2) the rotary cosines and sines."""
+        import qlka_native
+        from kernel_attention.attention import attention
+        native = qlka_native.ext()
+        B, S, hidden = x.shape
+        flat = x.view(B * S, hidden)
+        h = native.split_rows(flat, self.ln1.weight, self.ln1.bias, self.ln1.eps)
+        q, k, v = native.linear_qkv(h, self.qkv.weight, self.qkv.bias, table, B, S, self.heads)
+        if self.kernel == "softmax":
+            o = F.scaled_dot_product_attention(q, k, v, attn_mask=None if keep is None else keep[:, None, None, :])
+        else:
+            o = attention(q, k, v, self.kernel, self.tau, keep)
+        native.linear_residual(native.split_heads(o.contiguous()), self.proj.weight, self.proj.bias, flat)
+        h = native.split_rows(flat, self.ln2.weight, self.ln2.bias, self.ln2.eps)
+        native.linear_residual(native.linear_gelu(h, self.fc1.weight, self.fc1.bias), self.fc2.weight, self.fc2.bias, flat)
+        return x
+
 
 class Encoder(nn.Module):
     def __init__(self, kernel="add_laplace", tau=None, layers=12, hidden=768, heads=12, mlp=3072, vocab=30528):
@@ -69,8 +101,14 @@ class Encoder(nn.Module):
     @torch.no_grad()
     def forward(self, ids, keep=None):
         x = self.embed(ids)
+        table = None
         for blk in self.blocks:
-            x = blk(x, keep)
+            if blk.fits_native(x):
+                if table is None:
+                    table = torch.stack(rotary_angles(x.shape[1], 32, x.device), dim=-1).contiguous()
+                x = blk.forward_native(x, table, keep)
+            else:
+                x = blk(x, keep)
         return self.ln(x)
 
 
