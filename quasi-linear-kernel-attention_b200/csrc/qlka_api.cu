@@ -14,10 +14,8 @@ namespace qlka {
 cudaError_t launch_sort_rank_small(const SortArgs& a, cudaStream_t stream);
 cudaError_t launch_sort_rank_large(const SortArgs& a, void* scratch, cudaStream_t stream);
 size_t      sort_rank_large_scratch_bytes(int nseg, int N, int M);
-cudaError_t launch_laplace_walk(const WalkArgs& a, int emit, int grid1, int grid2, cudaStream_t stream, cudaEvent_t mid);
-cudaError_t launch_prefix_walk(const WalkArgs& a, int emit, int grid1, int grid2, cudaStream_t stream);
-int         walk_lanes_per_stream(int C4);
-int         walk_threads();
+cudaError_t launch_laplace_walk(const WalkArgs& a, int emit, int sms, cudaStream_t stream, cudaEvent_t mid);
+cudaError_t launch_prefix_walk(const WalkArgs& a, int emit, int sms, cudaStream_t stream);
 int         laplace_agg_stride(int C4);
 int         prefix_agg_stride_host(int C4);
 cudaError_t launch_split_rows(const float* x, const float* w, const float* b, void* out, long long rows, int K, float eps, cudaStream_t st);
@@ -100,31 +98,23 @@ int sm_count() {
     return n;
 }
 
-// How a walk over `nseg` segments of N keys is cut into streams, work items and CTAs. Streams are independent
-// work units (the passes exchange their states through memory), so a segment may be cut into any number of them:
+// How a walk over `nseg` segments of N keys is cut into streams and work items (a CTA's worth of streams, one per warp). Streams are
+// independent work units (the passes exchange their states through memory), so a segment may be cut into any number of them:
 // more streams until the persistent CTAs of the second pass get about sixteen items each, as long as a stream
 // keeps at least sixteen key blocks (the staging ring needs a few blocks to fill) - eight while there are fewer
 // items than CTAs. The prefix walks need no first pass with one stream per segment, which pays as soon as whole
 // segments alone give every CTA a few items.
-struct WalkPlan { int sps, nitems, grid1, grid2; };
+struct WalkPlan { int sps, nitems; };
 
 WalkPlan plan_walk(int nseg, int N, int C4, bool laplace) {
-    const int lps      = walk_lanes_per_stream(C4);
-    const int streams  = walk_threads() / lps;       // streams per CTA and work item
-    const int sms      = sm_count();
-    const int cap2     = sms * 2;                      // resident CTAs of the emitting pass (registers and shared memory)
-    const int cap1     = sms * 3;                      // ... and of the lighter first pass
-    const int nbk      = nblocks(N);
+    constexpr int streams = 8;                        // warps of a walk CTA
+    const int cap = sm_count() * 4;                    // resident CTAs, about
+    const int nbk = nblocks(N);
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
-    if (laplace || items(1) < 2LL * cap2)
-        while (items(sps) < 16LL * cap2 && nbk / (sps * 2) >= (items(sps) < cap2 ? 8 : 16) && sps < 4096) sps *= 2;
-    WalkPlan w;
-    w.sps    = sps;
-    w.nitems = (int)items(sps);
-    w.grid1  = w.nitems < cap1 ? w.nitems : cap1;
-    w.grid2  = w.nitems < cap2 ? w.nitems : cap2;
-    return w;
+    if (laplace || items(1) < 2LL * cap)
+        while (items(sps) < 16LL * cap && nbk / (sps * 2) >= (items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
+    return {sps, (int)items(sps)};
 }
 
 // per-stream aggregate table and (Laplace) per-segment checkpoint arrays of a planned walk
@@ -140,7 +130,7 @@ struct Records {
         large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(nseg, N, M)) : nullptr;
         xperm  = b.take<uint32_t>((size_t)nseg * npad(N));
         xval   = b.take<float>((size_t)nseg * xstride(N));
-        yrec   = b.take<uint4>((size_t)nseg * (M + 1));
+        yrec   = b.take<uint4>((size_t)nseg * (M + 1) + 16);      // (the walks stage 16 records from a block's first one on)
         mstart = b.take<uint32_t>((size_t)nseg * mstride(N));
         su0    = b.take<float>((size_t)nseg * (N + 1));
         su1    = b.take<float>((size_t)nseg * (N + 1));
@@ -225,7 +215,7 @@ cudaError_t prefix_walk_chunked(WalkArgs w, int emit, int P, cudaStream_t stream
         w.wtotal = all.wtotal ? all.wtotal + (size_t)p0 * all.C4 : nullptr;
         w.out_s  = all.out_s ? all.out_s + s0 * all.M : nullptr;
         w.nseg = pc * all.D; w.sps = plan.sps; w.nitems = plan.nitems;
-        cudaError_t e = launch_prefix_walk(w, emit, plan.grid1, plan.grid2, stream);
+        cudaError_t e = launch_prefix_walk(w, emit, sm_count(), stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -280,7 +270,7 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
         a.out_s = out_s ? out_s + s0 * M : nullptr;
         a.nseg = nseg; a.D = D; a.N = N; a.M = M; a.C4 = C4; a.sps = plan.sps; a.nitems = plan.nitems;
         a.sign = 1.0f; a.Mrows = M;
-        cudaError_t e = launch_laplace_walk(a, emit, plan.grid1, plan.grid2, stream, p0 == 0 ? mid : nullptr);
+        cudaError_t e = launch_laplace_walk(a, emit, sm_count(), stream, p0 == 0 ? mid : nullptr);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

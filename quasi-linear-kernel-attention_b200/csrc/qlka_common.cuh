@@ -80,7 +80,7 @@ struct PartArgs {
 };
 
 struct WalkArgs {
-    const float*    rows;     // (P, N, C4) rows the stream points at; C4 = channels padded to 4 (<= 64) or 8 floats
+    const float*    rows;     // (P, N, C4) rows the stream points at; C4 = channels padded to 4 floats
     const uint32_t* xperm;
     const float*    xval;
     const uint4*    yrec;
@@ -93,7 +93,7 @@ struct WalkArgs {
     const float*    wtotal;   // emit dot, prefix walk: (P, C4) column sums of rows
     float*          out_s;    // emit dot: (P, D, M); plain stores in the prefix walk, added to in the Laplace walk
     float           sign;     // emit dot, prefix walk: output scale (+1 gradients, -1 public sgn op)
-    int nseg, D, N, M, C4, sps, nitems;   // sps streams per segment, nitems work items of WALK_THREADS / LPS streams
+    int nseg, D, N, M, C4, sps, nitems;   // sps streams per segment, nitems work items of a CTA (one stream per warp)
     int Mrows;                // rows of `out` per p (= M unless the queries are folded)
 };
 

@@ -1,49 +1,42 @@
 // Asynchronous staging shared by the walk kernels.
 //
-// Every thread owns a private ring of RING_DEPTH slots in shared memory; a slot holds the
-// thread's CPL-channel slice of the KB rows of one key block. Rows are fetched with cp.async
-// (global -> shared, no registers, L2 only) one block ahead of their use, one commit group
-// per block, so the L2 latency of the row gather is hidden without extra warps. A thread only
-// ever reads the rows it copied itself, so cp.async.wait_group is all the rows need.
+// Emitting passes (Feeder): one warp walks one stream (a contiguous run of key blocks of a segment). Lane l owns the CPL
+// consecutive channels from l * CPL on, with CPL = 1, 2 or 4 for up to 32, 64 or 128 channels, so that every loop below is uniform
+// over the warp (two or four streams per warp, with 4 channels per lane whatever the width, spent half of their instructions on
+// diverged emission loops and left room for two CTAs per SM instead of three or four: Laplace backward at 48 heads x 4096 keys 5.6 ->
+// 4.1 ms, abs backward with 32 channels 4.2 -> 2.8 ms).
+// First passes (SumFeeder), which have nothing that diverges, keep 4 channels per lane and 1, 2 or 4 streams per warp: they are
+// bound by instruction issue, and a warp per stream took 1.35 instead of 1.02 ms at 48 heads x 16384 keys.
 //
-// Per stream (LPS lanes) and slot, two more things ride in the same commit group: the block's
-// per-key scalars (12 floats of which 9 are used, copied by lanes 0-2) and the LPS query records
-// from the block's first one on (one 16-byte record per lane; a block with fewer than LPS
-// queries finds all of them there, followed by a record of a later block or the segment's
-// sentinel). Both are read by every lane of the stream after a sub-warp barrier; a sub-warp
-// barrier at the top of the next iteration lets the slot be refilled. The block's query range
-// travels in registers. Shared memory is addressed with 32-bit shared-window addresses throughout.
+// Every warp owns a ring of DEPTH slots in shared memory; a slot holds the KB rows of one key block, the block's per-key
+// scalars (12 floats of which 9 are used) and its first QCAP query records. All of it is fetched with cp.async (global ->
+// shared, no registers, L2 only) DEPTH - 1 blocks ahead of its use, one commit group per block: 16 bytes per lane, so that
+// 32 / (8 CPL) rows travel with one instruction. cp.async.wait_group and a warp barrier make the copies readable by every lane;
+// a warp barrier at the top of the next iteration lets the slot be refilled. Blocks with QCAP queries or more read the further
+// records into the same place. The blocks' query ranges travel in registers. Shared memory is addressed with 32-bit
+// shared-window addresses throughout.
 //
-// Walks that contract their state with a row of a second matrix per query (the dot emissions)
-// need that row, whose index is only known once the query's record has arrived. Fetching it when
-// the record is emitted puts one L2 round trip on every query of a stream; instead each thread
-// copies its slice of the rows of up to G_SLOTS of the block's queries into a private third area
-// as soon as the block's records are readable, and emits after the block's arithmetic.
-//
-// The dot of a query is a sum over the lanes of its stream. Warp shuffles inside the emission loop
-// would split a warp that carries two or four streams (their loops have different trip counts) for good,
-// so each lane parks its partial sum in shared memory - in the stream's part of the row slot in use,
-// whose rows are in registers by then - and after the loop lane n adds up the partials of query n and
-// writes the result: no shuffle, one writer per query, and the writes of a block go out together.
+// Walks that contract their state with a row of a second matrix per query (the dot emissions) need that row, whose index is
+// only known once the query's record has arrived: the rows of up to G_SLOTS of the block's queries are copied into a third area
+// as soon as the block's records are readable, ahead of the next block's copies, and land during the block's arithmetic.
+// The dot of a query is a sum over the warp: each lane parks its part in shared memory (in the row slot in use, whose rows are
+// in registers by then), and after every G_SLOTS queries four lanes add up the parts of one query each: 16 instructions for 8
+// queries, where a shuffle tree per query takes 80.
 #pragma once
 #include "qlka_common.cuh"
 
 namespace qlka {
 
-constexpr int WALK_THREADS  = 256;
-constexpr int WALK_MIN_CTAS = 2;     // resident CTAs per SM the narrow (4 channels per lane) walks are compiled for
-constexpr int RING_DEPTH    = 2;     // blocks in flight: the one in use and RING_DEPTH - 1 prefetched
-constexpr int RING_AHEAD   = RING_DEPTH - 1;
+constexpr int WALK_THREADS = 256;
+constexpr int WALK_STREAMS = WALK_THREADS / 32;      // streams per CTA
 constexpr int SX_STRIDE    = 12;     // floats per staged scalar slot: 8 decays / keys and the next four
-constexpr int G_SLOTS      = 8;      // emit-side rows staged per batch (a power of two)
+constexpr int QCAP         = 16;     // query records staged per block
+constexpr int G_SLOTS      = 8;      // emit-side rows staged per batch
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void cp_async16(const uint32_t dst, const void* gmem_src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(const uint32_t dst, const void* gmem_src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -59,11 +52,6 @@ __device__ __forceinline__ uint32_t lds32u(const uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ float lds32f(const uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
-}
 __device__ __forceinline__ void sts32f(const uint32_t addr, const float v) {
     asm volatile("st.shared.f32 [%0], %1;" :: "r"(addr), "f"(v) : "memory");
 }
@@ -75,32 +63,8 @@ __device__ __forceinline__ uint4 lds128u(const uint32_t addr) {
 __device__ __forceinline__ void sts128u(const uint32_t addr, const uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ void sts64u(const uint32_t addr, const uint32_t a, const uint32_t b) {
-    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(addr), "r"(a), "r"(b) : "memory");
-}
 
-// d = a * b + c on two packed floats (one instruction on sm_100)
-__device__ __forceinline__ void fma2(float& d0, float& d1, const float a0, const float a1, const float b0, const float b1,
-                                     const float c0, const float c1) {
-    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
-        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
-__device__ __forceinline__ void mul2(float& d0, float& d1, const float a0, const float a1, const float b0, const float b1) {
-    asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
-        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-        "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-
-__device__ __forceinline__ void add2(float& d0, float& d1, const float a0, const float a1, const float b0, const float b1) {
-    asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
-        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-        "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-
+// ------------------------------------------------------------------ a lane's channels
 template <int CPL>
 struct Vec {
     float x[CPL];
@@ -110,169 +74,373 @@ struct Vec {
     }
 };
 
-template <int CPL> __host__ __device__ constexpr int    ring_slot_bytes() { return KB * (CPL / 4) * WALK_THREADS * 16; }
-template <int CPL> __host__ __device__ constexpr size_t ring_bytes()      { return (size_t)RING_DEPTH * ring_slot_bytes<CPL>(); }
-// dynamic shared memory of a walk kernel: row ring | record slots | scalar slots
-template <int LPS, int CPL> __host__ __device__ constexpr size_t walk_smem_bytes() {
-    return ring_bytes<CPL>() + (size_t)(WALK_THREADS / LPS) * RING_DEPTH * LPS * sizeof(uint4)
-         + (size_t)(WALK_THREADS / LPS) * RING_DEPTH * SX_STRIDE * sizeof(float);
+// d = a * x + y. Two packed floats per instruction where a lane has 4 channels; with fewer, pairing the broadcast factor costs
+// the instruction it saves.
+template <int CPL>
+__device__ __forceinline__ void axpy(Vec<CPL>& d, const float a, const Vec<CPL>& x, const Vec<CPL>& y) {
+    if constexpr (CPL == 4) {
+        #pragma unroll
+        for (int c = 0; c < CPL; c += 2)
+            asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+                "mov.b64 ra, {%2, %2};\n\tmov.b64 rb, {%3, %4};\n\tmov.b64 rc, {%5, %6};\n\t"
+                "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+                : "=f"(d.x[c]), "=f"(d.x[c + 1]) : "f"(a), "f"(x.x[c]), "f"(x.x[c + 1]), "f"(y.x[c]), "f"(y.x[c + 1]));
+    } else {
+        #pragma unroll
+        for (int c = 0; c < CPL; c++) d.x[c] = fmaf(a, x.x[c], y.x[c]);
+    }
 }
-// a first pass stages rows and per-key scalars only: row ring | scalar slots
-template <int LPS, int CPL> __host__ __device__ constexpr size_t pass1_smem_bytes() {
-    return ring_bytes<CPL>() + (size_t)(WALK_THREADS / LPS) * RING_DEPTH * SX_STRIDE * sizeof(float);
+// d = a * x
+template <int CPL>
+__device__ __forceinline__ void scale(Vec<CPL>& d, const float a, const Vec<CPL>& x) {
+    if constexpr (CPL == 4) {
+        #pragma unroll
+        for (int c = 0; c < CPL; c += 2)
+            asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+                "mov.b64 ra, {%2, %2};\n\tmov.b64 rb, {%3, %4};\n\t"
+                "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+                : "=f"(d.x[c]), "=f"(d.x[c + 1]) : "f"(a), "f"(x.x[c]), "f"(x.x[c + 1]));
+    } else {
+        #pragma unroll
+        for (int c = 0; c < CPL; c++) d.x[c] = a * x.x[c];
+    }
 }
-// the emit-side row area of the dot emissions follows: [G_SLOTS][CPL/4][WALK_THREADS] x 16 B
-template <int CPL> __host__ __device__ constexpr size_t g_area_bytes() { return (size_t)G_SLOTS * (CPL / 4) * WALK_THREADS * 16; }
+// d += x
+template <int CPL>
+__device__ __forceinline__ void vadd(Vec<CPL>& d, const Vec<CPL>& x) {
+    if constexpr (CPL >= 2) {
+        #pragma unroll
+        for (int c = 0; c < CPL; c += 2)
+            asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+                "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+                "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+                : "=f"(d.x[c]), "=f"(d.x[c + 1]) : "f"(d.x[c]), "f"(d.x[c + 1]), "f"(x.x[c]), "f"(x.x[c + 1]));
+    } else {
+        d.x[0] += x.x[0];
+    }
+}
 
-// what one stream needs to stage its blocks
-template <int LPS, int CPL>
+template <int CPL>
+__device__ __forceinline__ Vec<CPL> vload_shared(const uint32_t addr) {
+    Vec<CPL> v;
+    if constexpr (CPL == 4)      { const float4 t = lds128(addr); v.x[0] = t.x; v.x[1] = t.y; v.x[2] = t.z; v.x[3] = t.w; }
+    else if constexpr (CPL == 2) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x[0]), "=f"(v.x[1]) : "r"(addr));
+    else                         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v.x[0]) : "r"(addr));
+    return v;
+}
+template <int CPL>
+__device__ __forceinline__ Vec<CPL> vload(const float* p) {
+    Vec<CPL> v;
+    if constexpr (CPL == 4)      { const float4 t = ldg4(p); v.x[0] = t.x; v.x[1] = t.y; v.x[2] = t.z; v.x[3] = t.w; }
+    else if constexpr (CPL == 2) { const float2 t = __ldg(reinterpret_cast<const float2*>(p)); v.x[0] = t.x; v.x[1] = t.y; }
+    else                         v.x[0] = __ldg(p);
+    return v;
+}
+// loads and stores of data that is used once, long after or long before
+template <int CPL>
+__device__ __forceinline__ Vec<CPL> vload_once(const float* p) {
+    Vec<CPL> v;
+    if constexpr (CPL == 4)      { const float4 t = __ldcs(reinterpret_cast<const float4*>(p)); v.x[0] = t.x; v.x[1] = t.y; v.x[2] = t.z; v.x[3] = t.w; }
+    else if constexpr (CPL == 2) { const float2 t = __ldcs(reinterpret_cast<const float2*>(p)); v.x[0] = t.x; v.x[1] = t.y; }
+    else                         v.x[0] = __ldcs(p);
+    return v;
+}
+template <int CPL>
+__device__ __forceinline__ void vstore_once(float* p, const Vec<CPL>& v) {
+    if constexpr (CPL == 4)      __stcs(reinterpret_cast<float4*>(p), make_float4(v.x[0], v.x[1], v.x[2], v.x[3]));
+    else if constexpr (CPL == 2) __stcs(reinterpret_cast<float2*>(p), make_float2(v.x[0], v.x[1]));
+    else                         __stcs(p, v.x[0]);
+}
+template <int CPL>
+__device__ __forceinline__ void vstore(float* p, const Vec<CPL>& v) {
+    if constexpr (CPL == 4)      *reinterpret_cast<float4*>(p) = make_float4(v.x[0], v.x[1], v.x[2], v.x[3]);
+    else if constexpr (CPL == 2) *reinterpret_cast<float2*>(p) = make_float2(v.x[0], v.x[1]);
+    else                         *p = v.x[0];
+}
+// vector reduction into global memory (no return value): a row of the output per warp
+template <int CPL>
+__device__ __forceinline__ void vred(float* p, const Vec<CPL>& v) {
+    if constexpr (CPL == 4)      red_add4(p, v.x[0], v.x[1], v.x[2], v.x[3]);
+    else if constexpr (CPL == 2) asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" :: "l"(p), "f"(v.x[0]), "f"(v.x[1]) : "memory");
+    else                         asm volatile("red.global.add.f32 [%0], %1;" :: "l"(p), "f"(v.x[0]) : "memory");
+}
+
+// ------------------------------------------------------------------ shared memory of a warp
+template <int CPL> __host__ __device__ constexpr int row_pitch()  { return 128 * CPL; }
+template <int CPL> __host__ __device__ constexpr int slot_bytes() { return KB * row_pitch<CPL>(); }
+// row slots | scalar slots | record slots, and one more: a read may look one ahead | emit-side rows (dot emissions)
+template <int CPL, int DEPTH> __host__ __device__ constexpr int sx_offset()  { return DEPTH * slot_bytes<CPL>(); }
+template <int CPL, int DEPTH> __host__ __device__ constexpr int rec_offset() { return sx_offset<CPL, DEPTH>() + DEPTH * SX_STRIDE * 4; }
+template <int CPL, int DEPTH> __host__ __device__ constexpr int g_offset()   { return rec_offset<CPL, DEPTH>() + (DEPTH * QCAP + 1) * 16; }
+template <int CPL, int DEPTH> __host__ __device__ constexpr int warp_bytes(const bool dots) {
+    return g_offset<CPL, DEPTH>() + (dots ? G_SLOTS * row_pitch<CPL>() : 0);
+}
+
+// the warp's index in its CTA, in a form the compiler knows to be uniform
+__device__ __forceinline__ int warp_index() { return __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0); }
+
+// What a stream of an emitting pass needs to stage its blocks, in order. The pointers run along.
+template <int CPL, bool WITH_X, int DEPTH>
 struct Feeder {
-    uint32_t        ring_s;    // shared address of this thread's float4 in row 0 of slot 0
-    uint32_t        qs_s;      // shared address of this stream's record slots [RING_DEPTH][LPS] x 16 B
-    uint32_t        sx_s;      // shared address of this stream's scalar slots [RING_DEPTH][SX_STRIDE] x 4 B
-    const float*    rows;      // + p*N*C4 + lane channel offset
-    const float*    xval;
-    const uint32_t* xperm;
-    const uint32_t* mstart;
-    const uint4*    yrec;
+    static constexpr int AHEAD = DEPTH - 1;
+    static constexpr int LR = 8 * CPL, RPC = 32 / LR, NCP = KB / RPC;     // lanes per row, rows per copy instruction, copies per lane and block
+    uint32_t        area;      // shared address of the warp's area
+    uint32_t        copy_dst;  // + my first row and my 16 bytes of it
     uint32_t        row_bytes; // C4 * 4
-    int             N, M, ln;
-    bool            with_x, with_q;
-    uint32_t        g_s;       // dot emissions: shared address of this thread's float4 in emit-side slot 0
-    const float*    grows;     //                + p*M*C4 + lane channel offset
+    bool            copy_on;   // my 16 bytes lie inside the row
+    int             lane, N;
+    const char*     rows;      // + p * N * row_bytes + my 16 bytes
+    const float*    xval;      // of the next block to start, + my 16 bytes (lanes 16 .. 18)
+    const uint32_t* xperm;     // of the next block to prefetch, + my first row
+    const uint32_t* mstart;    // of the next block to prefetch
+    const uint4*    yrec;      // + my record of a block
+    const char*     grows;     // dot emissions: + p * M * row_bytes + my 16 bytes
     // prefetched one block before its issue
-    uint4    p0, p1;
-    uint32_t ms0, ms1;
-    // query range [lo, hi) of the block in use and of the blocks in flight (all lanes load the same two words)
-    uint32_t m_lo, m_hi, mq_lo[RING_AHEAD], mq_hi[RING_AHEAD];
+    uint32_t idx[NCP], ms0, ms1;
+    // query range of the block in use and of the blocks in flight
+    uint32_t m_lo, m_hi, mq_lo[AHEAD], mq_hi[AHEAD];
 
-    __device__ __forceinline__ void prefetch_index(const int b) {
-        p0 = __ldg(reinterpret_cast<const uint4*>(xperm + b * KB));
-        p1 = __ldg(reinterpret_cast<const uint4*>(xperm + b * KB + 4));
-        if (with_q) { ms0 = __ldg(mstart + b); ms1 = __ldg(mstart + b + 1); }
+    __device__ __forceinline__ void init(const uint32_t area_, const int lane_, const int N_, const int C4) {
+        area = area_; lane = lane_; N = N_;
+        row_bytes = (uint32_t)C4 * 4u;
+        copy_on   = (uint32_t)(lane % LR) * 16u < row_bytes;
+        copy_dst  = area + (lane / LR) * NCP * row_pitch<CPL>() + (lane % LR) * 16;
+    }
+    // a stream of segment sg (head p) that starts at block b
+    __device__ __forceinline__ void start(const WalkArgs& a, const int sg, const int p, const int b) {
+        xperm = a.xperm + (long long)sg * npad(a.N) + b * KB + (lane / LR) * NCP;
+        if (WITH_X) xval = a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * (lane - 16);
+        rows  = reinterpret_cast<const char*>(a.rows + (long long)p * a.N * a.C4) + (lane % LR) * 16;
+        mstart = a.mstart + (long long)sg * mstride(a.N) + b;
+        yrec   = a.yrec + (long long)sg * (a.M + 1) + lane;
+    }
+    __device__ __forceinline__ void start_dots(const WalkArgs& a, const int p) {
+        grows = reinterpret_cast<const char*>(a.g + (long long)p * a.M * a.C4) + (lane % LR) * 16;
     }
 
-    // start the copies of key block b (whose indices were prefetched) into `slot`; one commit group
-    __device__ __forceinline__ void issue(const int slot, const int b, const int ahead) {
-        mq_lo[ahead] = ms0; mq_hi[ahead] = ms1;
-        const int      j0    = b * KB;
-        const uint32_t pr[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-        const uint32_t dst   = ring_s + slot * ring_slot_bytes<CPL>();
-        const char*    rb    = reinterpret_cast<const char*>(rows);
-        #pragma unroll
-        for (int i = 0; i < KB; i++) {                 // (positions past the last key point at row 0; read_rows zeroes them)
-            const char* src = rb + (size_t)pr[i] * row_bytes;
+    __device__ __forceinline__ void prefetch_index() {
+        if constexpr (NCP == 2) { const uint2 t = __ldg(reinterpret_cast<const uint2*>(xperm)); idx[0] = t.x; idx[1] = t.y; }
+        else {
             #pragma unroll
-            for (int h = 0; h < CPL / 4; h++) cp_async16(dst + (i * (CPL / 4) + h) * WALK_THREADS * 16, src + 16 * h);
+            for (int i = 0; i < NCP; i += 4) {
+                const uint4 t = __ldg(reinterpret_cast<const uint4*>(xperm + i));
+                idx[i] = t.x; idx[i + 1] = t.y; idx[i + 2] = t.z; idx[i + 3] = t.w;
+            }
         }
-        const uint32_t sx = sx_s + slot * SX_STRIDE * 4;
-        if (with_x && ln < 3) cp_async16(sx + 16 * ln, xval + j0 + 4 * ln);       // (the array is padded by KB floats)
-        if (with_q) {
-            // the LPS records from the block's first on (clamped to the segment's sentinel): a block with fewer than
-            // LPS queries finds all of them here, followed by a record of a later block or the sentinel
-            const uint32_t r = min(ms0 + (uint32_t)ln, (uint32_t)M);
-            cp_async16(qs_s + (slot * LPS + ln) * 16, yrec + r);
+        xperm += KB;
+        ms0 = __ldg(mstart); ms1 = __ldg(mstart + 1); mstart++;
+    }
+
+    // start the copies of the block whose indices were prefetched last into `slot`; one commit group
+    __device__ __forceinline__ void issue(const int slot, const int ahead) {
+        mq_lo[ahead] = ms0; mq_hi[ahead] = ms1;
+        const uint32_t dst = copy_dst + slot * slot_bytes<CPL>();
+        if (copy_on) {                                 // (positions past the last key point at row 0; read_rows zeroes them)
+            #pragma unroll
+            for (int i = 0; i < NCP; i++) cp_async16(dst + i * row_pitch<CPL>(), rows + (unsigned long long)idx[i] * row_bytes);
+        }
+        // lanes 0..15 the first QCAP records from the block's first one on (the array is padded by QCAP records), lanes 16..18 the scalars
+        if (lane < QCAP) cp_async16(area + rec_offset<CPL, DEPTH>() + (slot * QCAP + lane) * 16, yrec + ms0);
+        if (WITH_X) {                                  // (the array is padded by KB floats)
+            if (lane >= 16 && lane < 19) cp_async16(area + sx_offset<CPL, DEPTH>() + slot * SX_STRIDE * 4 + (lane - 16) * 16, xval);
+            xval += KB;
         }
         cp_async_commit();
     }
 
-    // Blocks are visited in steps t = 0 .. nblk-1, block of step t = bfirst + dir * t, slot of step t = t mod RING_DEPTH.
-    // prologue: start the first RING_AHEAD blocks; step: start block t + RING_AHEAD, then wait for block t.
-    __device__ __forceinline__ void prologue(const int bfirst, const int dir, const int nblk) {
+    // Blocks are visited in steps t = 0 .. nblk-1; slot of step t = t mod DEPTH.
+    __device__ __forceinline__ void prologue(const int nblk) {
         #pragma unroll
-        for (int s = 0; s < RING_AHEAD; s++) {
-            if (s < nblk) { prefetch_index(bfirst + dir * s); issue(s, bfirst + dir * s, s); }
+        for (int i = 0; i < AHEAD; i++) {
+            if (i < nblk) { prefetch_index(); issue(i, i); }
             else cp_async_commit();
         }
-        if (RING_AHEAD < nblk) prefetch_index(bfirst + dir * RING_AHEAD);
+        if (AHEAD < nblk) prefetch_index();
     }
     // first thing of every step: the oldest block in flight becomes the block in use
     __device__ __forceinline__ void advance_range() {
         m_lo = mq_lo[0]; m_hi = mq_hi[0];
         #pragma unroll
-        for (int s = 0; s + 1 < RING_AHEAD; s++) { mq_lo[s] = mq_lo[s + 1]; mq_hi[s] = mq_hi[s + 1]; }
+        for (int i = 0; i + 1 < AHEAD; i++) { mq_lo[i] = mq_lo[i + 1]; mq_hi[i] = mq_hi[i + 1]; }
     }
-    __device__ __forceinline__ void step_issue(const int t, const int cur, const int bfirst, const int dir, const int nblk) {
-        if (t + RING_AHEAD < nblk) issue(cur == 0 ? RING_DEPTH - 1 : cur - 1, bfirst + dir * (t + RING_AHEAD), RING_AHEAD - 1);
+    __device__ __forceinline__ void step_issue(const int t, const int cur, const int nblk) {
+        if (t + AHEAD < nblk) issue(cur == 0 ? DEPTH - 1 : cur - 1, AHEAD - 1);
         else cp_async_commit();
-        if (t + RING_AHEAD + 1 < nblk) prefetch_index(bfirst + dir * (t + RING_AHEAD + 1));
+        if (t + AHEAD + 1 < nblk) prefetch_index();
     }
-    __device__ __forceinline__ void step(const int t, const int cur, const int bfirst, const int dir, const int nblk) {
-        advance_range();
-        step_issue(t, cur, bfirst, dir, nblk);
-        cp_async_wait<RING_AHEAD>();
-    }
+    __device__ __forceinline__ static int next_slot(const int cur) { return cur == DEPTH - 1 ? 0 : cur + 1; }
 
-    // start the copies of this thread's slice of the emit-side rows of the staged records n0 .. n1-1 of `slot`
-    // (n1 - n0 <= G_SLOTS; record n lands in emit-side slot n mod G_SLOTS); one commit group
-    __device__ __forceinline__ void issue_g(const int slot, const uint32_t n0, const uint32_t n1) {
-        const char* gb = reinterpret_cast<const char*>(grows);
-        #pragma unroll
-        for (int i = 0; i < G_SLOTS; i++) {
-            const uint32_t n = n0 + i;
-            if (n < n1) {
-                const uint32_t row = lds32u(qs_s + (slot * LPS + n) * 16 + 8);
-                const char*    src = gb + (size_t)row * row_bytes;
-                #pragma unroll
-                for (int h = 0; h < CPL / 4; h++)
-                    cp_async16(g_s + ((n & (G_SLOTS - 1)) * (CPL / 4) + h) * WALK_THREADS * 16, src + 16 * h);
-            }
-        }
-        cp_async_commit();
-    }
-    // Partial dots of query n of the block in `slot`: LPS floats inside the stream's share (LPS x 16 bytes) of row
-    // (n mod 8) of the slot, placed so that the LPS lanes' reads of LPS different queries fall in different banks: shifted
-    // by n words, or, where a share has no room for that (LPS = 32), rotated by n. The two streams of a warp (LPS = 16)
-    // start half a query apart, so that they do not meet in a bank while a block has up to 8 queries.
-    __device__ __forceinline__ uint32_t part_addr(const int slot, const uint32_t n) const {
-        const uint32_t at = LPS == 32 ? (n >> 3) * (LPS * 4u) : ((n >> 3) * 32u + n) * 4u;
-        return ring_s - ln * 16 + slot * ring_slot_bytes<CPL>() + (n & 7u) * (WALK_THREADS * 16) + at;
-    }
-    __device__ __forceinline__ void put_part(const int slot, const uint32_t n, const float acc) const {
-        sts32f(part_addr(slot, n) + (LPS == 32 ? (ln + n) & (LPS - 1) : ln) * 4, acc);
-    }
-    __device__ __forceinline__ float sum_parts(const int slot, const uint32_t n) const {
-        const uint32_t p = part_addr(slot, n);
-        float s0 = 0.0f, s1 = 0.0f;
-        if (LPS == 32) {
-            #pragma unroll
-            for (uint32_t k = 0; k < LPS; k += 2) { s0 += lds32f(p + ((k + n) & (LPS - 1)) * 4); s1 += lds32f(p + ((k + 1 + n) & (LPS - 1)) * 4); }
-        } else {
-            const uint32_t half = LPS == 16 ? (threadIdx.x & 16u) * 2u : 0u;          // bytes: 8 words for the second stream
-            #pragma unroll
-            for (int k = 0; k < LPS / 2; k++) { s0 += lds32f(p + half + 4 * k); s1 += lds32f(p - half + 4 * (k + LPS / 2)); }
-        }
-        return s0 + s1;
-    }
-    __device__ __forceinline__ void read_g(const uint32_t n, Vec<CPL>& gq) const {
-        #pragma unroll
-        for (int h = 0; h < CPL / 4; h++) {
-            const float4 t = lds128(g_s + ((n & (G_SLOTS - 1)) * (CPL / 4) + h) * WALK_THREADS * 16);
-            gq.x[4 * h] = t.x; gq.x[4 * h + 1] = t.y; gq.x[4 * h + 2] = t.z; gq.x[4 * h + 3] = t.w;
-        }
-    }
-
-    // this thread's slice of the block's rows from `slot`; rows at positions >= N read as zero
+    // this lane's slice of the block's rows from `slot`; rows at positions >= N read as zero
     __device__ __forceinline__ void read_rows(const int slot, const int j0, Vec<CPL> (&v)[KB]) const {
-        const uint32_t src = ring_s + slot * ring_slot_bytes<CPL>();
+        const uint32_t src = area + slot * slot_bytes<CPL>() + lane * (4 * CPL);
         #pragma unroll
-        for (int i = 0; i < KB; i++) {
-            #pragma unroll
-            for (int h = 0; h < CPL / 4; h++) {
-                const float4 t = lds128(src + (i * (CPL / 4) + h) * WALK_THREADS * 16);
-                v[i].x[4 * h] = t.x; v[i].x[4 * h + 1] = t.y; v[i].x[4 * h + 2] = t.z; v[i].x[4 * h + 3] = t.w;
-            }
-        }
+        for (int i = 0; i < KB; i++) v[i] = vload_shared<CPL>(src + i * row_pitch<CPL>());
         if (j0 + KB > N) {
             #pragma unroll
             for (int i = 0; i < KB; i++) if (j0 + i >= N) v[i].zero();
         }
     }
-
     // the block's nine scalars, from `slot`
     __device__ __forceinline__ void read_scalars(const int slot, float (&av)[KB + 1]) const {
-        const uint32_t sx = sx_s + slot * SX_STRIDE * 4;
+        const uint32_t sx = area + sx_offset<CPL, DEPTH>() + slot * SX_STRIDE * 4;
         const float4 a0 = lds128(sx), a1 = lds128(sx + 16), a2 = lds128(sx + 32);
+        av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
+        av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
+        av[8] = a2.x;
+    }
+
+    __device__ __forceinline__ uint32_t records(const int slot) const { return area + rec_offset<CPL, DEPTH>() + slot * QCAP * 16; }
+
+    // start the copies of the emit-side rows of the staged records n0 .. n1-1 of `slot` (n1 - n0 <= G_SLOTS); one commit group
+    __device__ __forceinline__ void issue_g(const int slot, const uint32_t n0, const uint32_t n1) const {
+        const uint32_t g = area + g_offset<CPL, DEPTH>() + (lane / LR) * NCP * row_pitch<CPL>() + (lane % LR) * 16;
+        const uint32_t n = n0 + (lane / LR) * NCP;
+        #pragma unroll
+        for (int i = 0; i < NCP; i++)
+            if (copy_on && n + i < n1) cp_async16(g + i * row_pitch<CPL>(), grows + (unsigned long long)lds32u(records(slot) + (n + i) * 16 + 8) * row_bytes);
+        cp_async_commit();
+    }
+    // lane addresses of the emit-side row of query 0 of a batch and of this lane's part of its dot; query n: + n pitches, + n * 128
+    __device__ __forceinline__ uint32_t g_lane() const { return area + g_offset<CPL, DEPTH>() + lane * (4 * CPL); }
+    __device__ __forceinline__ uint32_t part_lane(const int slot) const { return area + slot * slot_bytes<CPL>() + lane * 4; }
+    // the dot of the batch's query lane / 4, in each of its four lanes
+    __device__ __forceinline__ float sum_parts(const int slot) const {
+        const int      q = lane >> 2, k = (lane & 3) ^ ((q & 1) * 4);      // (odd queries start in the other half: no bank conflicts)
+        const uint32_t p = area + slot * slot_bytes<CPL>() + q * 128;
+        const float4   a = lds128(p + k * 16), b = lds128(p + (k ^ 4) * 16);
+        float s = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+        s += __shfl_xor_sync(FULL, s, 1);
+        return s + __shfl_xor_sync(FULL, s, 2);
+    }
+};
+
+// The queries of a block, in rank order: emit(i, rec, n128) for the queries that precede key i, n128 = 128 * (query's place in its
+// batch of G_SLOTS); finish(n0, n1) after every G_SLOTS queries and at the end (dot emissions; n0 counts from the staged records).
+// The staged records are followed by one of a later block (or the segment's sentinel), so a record's rank alone says where the
+// block ends; blocks with QCAP queries or more go QCAP - 1 at a time, with a terminator of their own.
+template <bool DO_DOT, class F, class Emit, class Finish>
+__device__ __forceinline__ void for_queries(const F& f, const int slot, const int j0, const uint32_t cnt, Emit emit, Finish finish) {
+    constexpr uint32_t BATCH = QCAP - 1;
+    const uint32_t recs = f.records(slot);
+    uint32_t left = cnt;                                   // queries from the staged records on
+    uint32_t at   = f.m_lo;
+    while (true) {
+        const bool more = left > BATCH;
+        if (more) {
+            __syncwarp();
+            if (f.lane == 0) sts32f(recs + BATCH * 16 + 12, __uint_as_float(0xffffffffu));
+            __syncwarp();
+        }
+        uint32_t qa = recs, n128 = 0, n0 = 0;
+        uint4    rec = lds128u(qa);
+        uint32_t key = rec.w - (uint32_t)j0;
+        #pragma unroll
+        for (int i = 0; i < KB; i++) {
+            while (key == (uint32_t)i) {
+                emit(i, rec, n128);
+                qa += 16;
+                rec = lds128u(qa);
+                key = rec.w - (uint32_t)j0;
+                if (DO_DOT) {
+                    n128 += 128;
+                    if (n128 == G_SLOTS * 128) {
+                        __syncwarp();
+                        finish(n0, n0 + G_SLOTS);
+                        __syncwarp();
+                        n0 += G_SLOTS;
+                        n128 = 0;
+                        f.issue_g(slot, n0, min(left, min(n0 + G_SLOTS, BATCH)));
+                        cp_async_wait<0>();
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+        if (DO_DOT && n128 != 0) {
+            __syncwarp();
+            finish(n0, n0 + (n128 >> 7));
+        }
+        if (!more) break;
+        left -= BATCH;
+        at   += BATCH;
+        __syncwarp();
+        if (f.lane < QCAP) sts128u(recs + f.lane * 16, __ldg(f.yrec + at));
+        __syncwarp();
+        if (DO_DOT) {
+            f.issue_g(slot, 0u, min(left, (uint32_t)G_SLOTS));
+            cp_async_wait<0>();
+            __syncwarp();
+        }
+    }
+}
+
+// The first passes' staging: LPS lanes per stream (8, 16 or 32 for up to 32, 64 or 128 channels), 4 channels per lane. Every lane
+// copies its own 16 bytes of each row into a private ring of two slots, and reads only those; the block's scalars are shared by
+// the lanes of the stream.
+constexpr int SUM_SLOT_BYTES = KB * WALK_THREADS * 16;
+template <int LPS> __host__ __device__ constexpr int sum_smem_bytes() { return 2 * SUM_SLOT_BYTES + (WALK_THREADS / LPS) * 2 * SX_STRIDE * 4; }
+
+template <int LPS, bool WITH_X, int DIR>
+struct SumFeeder {
+    uint32_t        ring, sx;  // shared addresses: this lane's 16 bytes of row 0 of slot 0, the stream's scalar slots
+    uint32_t        row_bytes;
+    int             ln, N;
+    bool            on;        // this lane's 16 bytes lie inside the row
+    const char*     rows;      // + p * N * row_bytes + my 16 bytes
+    const float*    xval;      // of the next block to start, + my 16 bytes (lanes 0 .. 2)
+    const uint32_t* xperm;     // of the next block to prefetch
+    uint4           p0, p1;    // prefetched one block before its issue
+
+    __device__ __forceinline__ void init(const uint32_t smem, const int N_, const int C4) {
+        ring = smem + threadIdx.x * 16;
+        sx   = smem + 2 * SUM_SLOT_BYTES + (threadIdx.x / LPS) * 2 * SX_STRIDE * 4;
+        ln   = threadIdx.x % LPS; N = N_;
+        on   = ln * 4 < C4;
+        row_bytes = (uint32_t)C4 * 4u;
+    }
+    __device__ __forceinline__ void start(const WalkArgs& a, const int sg, const int p, const int b) {
+        xperm = a.xperm + (long long)sg * npad(a.N) + b * KB;
+        if (WITH_X) xval = a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * ln;
+        rows = reinterpret_cast<const char*>(a.rows + (long long)p * a.N * a.C4) + ln * 16;
+    }
+    __device__ __forceinline__ void prefetch_index() {
+        p0 = __ldg(reinterpret_cast<const uint4*>(xperm));
+        p1 = __ldg(reinterpret_cast<const uint4*>(xperm + 4));
+        xperm += DIR * KB;
+    }
+    __device__ __forceinline__ void issue(const int slot) {
+        const uint32_t pr[KB] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+        if (on) {
+            #pragma unroll
+            for (int i = 0; i < KB; i++) cp_async16(ring + slot * SUM_SLOT_BYTES + i * WALK_THREADS * 16, rows + (unsigned long long)pr[i] * row_bytes);
+        }
+        if (WITH_X) {
+            if (ln < 3) cp_async16(sx + slot * SX_STRIDE * 4 + 16 * ln, xval);
+            xval += DIR * KB;
+        }
+        cp_async_commit();
+    }
+    __device__ __forceinline__ void prologue(const int nblk) {
+        if (nblk > 0) { prefetch_index(); issue(0); }
+        if (nblk > 1) prefetch_index();
+    }
+    __device__ __forceinline__ void step(const int t, const int cur, const int nblk) {
+        if (t + 1 < nblk) issue(cur ^ 1);
+        else cp_async_commit();
+        if (t + 2 < nblk) prefetch_index();
+        cp_async_wait<1>();
+    }
+    __device__ __forceinline__ void read_rows(const int slot, const int j0, Vec<4> (&v)[KB]) const {
+        #pragma unroll
+        for (int i = 0; i < KB; i++) v[i] = vload_shared<4>(ring + slot * SUM_SLOT_BYTES + i * WALK_THREADS * 16);
+        if (j0 + KB > N) {
+            #pragma unroll
+            for (int i = 0; i < KB; i++) if (j0 + i >= N) v[i].zero();
+        }
+    }
+    __device__ __forceinline__ void read_scalars(const int slot, float (&av)[KB + 1]) const {
+        const uint32_t s = sx + slot * SX_STRIDE * 4;
+        const float4 a0 = lds128(s), a1 = lds128(s + 16), a2 = lds128(s + 32);
         av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
         av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
         av[8] = a2.x;
@@ -285,6 +453,20 @@ __device__ __forceinline__ void stream_blocks(const int s, const int SPS, const 
     b1 = (int)((long long)(s + 1) * NBK / SPS);
 }
 
-__device__ __forceinline__ int ring_next(const int cur) { return cur == RING_DEPTH - 1 ? 0 : cur + 1; }
+// the stream of a warp: segment, block range
+struct StreamOf {
+    long long g; bool on; int sg, p, b0, b1, nblk;
+    // stream `i` of the `streams` of work item `item`
+    __device__ __forceinline__ StreamOf(const WalkArgs& a, const int item, const int i, const int NBK, const int streams = WALK_STREAMS) {
+        g  = (long long)item * streams + i;
+        on = g < (long long)a.nseg * a.sps;
+        const long long gg = on ? g : 0;
+        sg = (int)(gg / a.sps);
+        const int s = (int)(gg - (long long)sg * a.sps);
+        p  = sg / a.D;
+        stream_blocks(s, a.sps, NBK, b0, b1);
+        nblk = on ? b1 - b0 : 0;
+    }
+};
 
 }  // namespace qlka
