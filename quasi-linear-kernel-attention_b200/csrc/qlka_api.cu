@@ -130,7 +130,7 @@ struct Records {
         large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(nseg, N, M)) : nullptr;
         xperm  = b.take<uint32_t>((size_t)nseg * npad(N));
         xval   = b.take<float>((size_t)nseg * xstride(N));
-        yrec   = b.take<uint4>((size_t)nseg * (M + 1) + 16);      // (the walks stage 16 records from a block's first one on)
+        yrec   = b.take<uint4>((size_t)nseg * (M + 1));
         mstart = b.take<uint32_t>((size_t)nseg * mstride(N));
         su0    = b.take<float>((size_t)nseg * (N + 1));
         su1    = b.take<float>((size_t)nseg * (N + 1));

@@ -30,10 +30,10 @@ namespace qlka {
 
 enum { LAP_ROWS = 0, LAP_DOT = 1, LAP_BOTH = 2 };
 
-// resident CTAs per SM that the emitting pass is compiled for, and blocks in its rings: three for the rows (two: 3.34 instead of 3.02 ms at
-// 48 heads x 16384 keys), two where the emit-side rows want shared memory and copies of their own (three: backward 4.1 -> 4.4 ms
-// at 48 x 4096). A fourth CTA leaves 64 registers: 4.1 ms.
-constexpr int LAP_CTAS1 = 3;
+// resident CTAs per SM that the emitting pass is compiled for, and blocks in its rings: three CTAs with one stream per warp (two: 3.34
+// instead of 3.02 ms at 48 heads x 16384 keys; four leave 64 registers: 4.1 ms); two blocks where the emit-side rows want
+// shared memory and copies of their own (three: backward 4.1 -> 4.4 ms at 48 x 4096).
+constexpr int LAP_CTAS1 = 3, LAP_CTAS_ROWS = 2;
 __host__ __device__ constexpr int lap_ctas2(int cpl) { return cpl == 4 ? 2 : 3; }
 __host__ __device__ constexpr int lap_depth2(int emit) { return emit == LAP_ROWS ? 3 : 2; }
 
@@ -179,13 +179,12 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
         int cur = 0, j0 = b0 * KB;
         for (int t = 0; t < nblk; t++, j0 += KB, cur = F2::next_slot(cur)) {
             f.advance_range();
-            const uint32_t cnt = f.m_hi - f.m_lo;
             if (DO_DOT) {
                 // the block's copies have had whole iterations; once its records are readable the emit-side rows
                 // of its first G_SLOTS queries start, ahead of the next block's copies, and land during the arithmetic
                 cp_async_wait<F2::AHEAD - 1>();
                 __syncwarp();
-                f.issue_g(cur, 0u, min(cnt, (uint32_t)G_SLOTS));
+                f.issue_g(cur, j0, 0u);
             } else {
                 __syncwarp();
             }
@@ -240,28 +239,119 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
                 const uint32_t n   = n0 + (lane >> 2);
                 if ((lane & 3) == 0 && n < n1) atomicAdd(out_s + lds32u(f.records(cur) + n * 16 + 8), sum);
             };
-            for_queries<DO_DOT>(f, cur, j0, cnt, emit, finish);
+            for_queries<DO_DOT>(f, cur, j0, emit, finish);
         }
         cp_async_wait<0>();
     }
 }
 
+// The second pass's row emission with 4 channels per lane (RowFeeder; rows_by_quads says when). Two CTAs per SM: its state takes
+// some 120 registers. Bound by the L2 traffic of one row gathered and one row reduced per key and query (2.4 of its 2.8 ms
+// at 48 heads x 16384 keys and queries; with one stream per warp it took 3.0).
+template <int LPS>
+__global__ void __launch_bounds__(WALK_THREADS, LAP_CTAS_ROWS) laplace_rows(const WalkArgs a)
+{
+    constexpr int STREAMS = WALK_THREADS / LPS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x, ln = tid % LPS, c0 = ln * 4;
+    const int N = a.N, C4 = a.C4, NBK = nblocks(N);
+    const bool lane_on = c0 < C4;
+    const int  c0l     = lane_on ? c0 : 0;
+    const unsigned gmask = LPS == 32 ? FULL : (((1u << (LPS & 31)) - 1u) << ((tid & 31) & ~(LPS - 1)));
+
+    RowFeeder<LPS> f;
+    f.init(smem_u32(smem), N, a.M, C4);
+
+    const int items = (int)(((long long)a.nseg * a.sps + STREAMS - 1) / STREAMS);
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const StreamOf st(a, item, tid / LPS, NBK, STREAMS);
+        const int nblk = st.nblk;
+        f.start(a, st.sg, st.p, st.b0);
+        char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
+        const float* ck = a.ckpt + ((long long)st.sg * NBK + st.b0 + 1) * C4 + c0l;      // of the next block to fetch
+        const float* wk = a.wck + (long long)st.sg * NBK + st.b0 + 1;
+        const float* ag = a.agg + (st.on ? st.g : 0) * lap_agg_stride(C4) + c0l;
+        Vec<4> L = vload<4>(ag), Rin = vload<4>(ag + C4);
+
+        __syncwarp(gmask);                         // every lane has left the previous item's slots
+        f.prologue(nblk);
+        Vec<4> cnext; cnext.zero();
+        float  wnext = 0.0f;
+        auto load_ckpt = [&]() { wnext = *wk++; cnext = vload_once<4>(ck); ck += C4; };
+        if (nblk > 1) load_ckpt();
+        int cur = 0, j0 = st.b0 * KB;
+        for (int t = 0; t < nblk; t++, j0 += KB, cur ^= 1) {
+            __syncwarp(gmask);                     // every lane is done with the slot refilled below
+            // suffix state entering the block from above: corrected checkpoint, or the stream's incoming state
+            Vec<4> Rn = Rin;
+            if (t + 1 < nblk) axpy(Rn, wnext, Rin, cnext);
+            if (t + 2 < nblk) load_ckpt();
+            f.step(t, cur, nblk);
+            __syncwarp(gmask);
+            float av[KB + 1];
+            f.read_scalars(cur, av);
+            Vec<4> v[KB], Rb[KB];
+            f.read_rows(cur, j0, v);
+            #pragma unroll
+            for (int i = KB - 1; i >= 0; i--) {
+                axpy(Rn, av[i + 1], Rn, v[i]);
+                Rb[i] = Rn;
+            }
+            // prefix state before each key, in place of the rows
+            #pragma unroll
+            for (int i = 0; i < KB; i++) {
+                const Vec<4> row = v[i];
+                v[i] = L;
+                axpy(L, av[i], L, row);
+            }
+            f.for_queries(cur, j0, [&](const int i, const uint4& rec) {
+                Vec<4> r;
+                scale(r, __uint_as_float(rec.y), Rb[i]);
+                axpy(r, __uint_as_float(rec.x), v[i], r);
+                if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
+            });
+        }
+        cp_async_wait<0>();
+    }
+}
+
+template <int LPS>
+static cudaError_t launch_lap_rows(const WalkArgs& a, int sms, cudaStream_t stream) {
+    constexpr int smem = row_smem_bytes<LPS>();
+    cudaError_t e = cudaFuncSetAttribute(laplace_rows<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const long long items = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
+    const int cap = sms * LAP_CTAS_ROWS;
+    laplace_rows<LPS><<<items < cap ? (int)items : cap, WALK_THREADS, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+template <int CPL, int EMIT>
+static cudaError_t launch_lap_pass2(const WalkArgs& a, int sms, cudaStream_t stream) {
+    constexpr int smem = WALK_STREAMS * warp_bytes<CPL, lap_depth2(EMIT)>(EMIT != LAP_ROWS);
+    cudaError_t e = cudaFuncSetAttribute(laplace_pass2<CPL, EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int cap = sms * lap_ctas2(CPL);
+    laplace_pass2<CPL, EMIT><<<a.nitems < cap ? a.nitems : cap, WALK_THREADS, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
 template <int LPS, int CPL, int EMIT>
 static cudaError_t launch_lap(const WalkArgs& a, int sms, cudaStream_t stream, cudaEvent_t mid) {
-    auto k1 = laplace_pass1<LPS>;
-    auto k2 = laplace_pass2<CPL, EMIT>;
-    constexpr int smem1 = sum_smem_bytes<LPS>(), smem2 = WALK_STREAMS * warp_bytes<CPL, lap_depth2(EMIT)>(EMIT != LAP_ROWS);
-    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
+    constexpr int smem1 = sum_smem_bytes<LPS>();
+    cudaError_t e = cudaFuncSetAttribute(laplace_pass1<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
     if (e != cudaSuccess) return e;
     const long long items1 = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
-    const int cap1 = sms * LAP_CTAS1, cap2 = sms * lap_ctas2(CPL);
-    k1<<<items1 < cap1 ? (int)items1 : cap1, WALK_THREADS, smem1, stream>>>(a);
+    const int cap1 = sms * LAP_CTAS1;
+    laplace_pass1<LPS><<<items1 < cap1 ? (int)items1 : cap1, WALK_THREADS, smem1, stream>>>(a);
     laplace_fold<<<(unsigned)(((long long)a.nseg * a.C4 + 255) / 256), 256, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4);
-    if (mid) { e = cudaEventRecord(mid, stream); if (e != cudaSuccess) return e; }
-    k2<<<a.nitems < cap2 ? a.nitems : cap2, WALK_THREADS, smem2, stream>>>(a);
-    return cudaGetLastError();
+    e = cudaGetLastError();
+    if (e == cudaSuccess && mid) e = cudaEventRecord(mid, stream);
+    if (e != cudaSuccess) return e;
+    if constexpr (EMIT == LAP_ROWS) {
+        if (CPL == 4 || rows_by_quads(a)) return launch_lap_rows<LPS>(a, sms, stream);
+    }
+    if constexpr (EMIT != LAP_ROWS || CPL < 4) return launch_lap_pass2<CPL, EMIT>(a, sms, stream);
 }
 
 template <int EMIT>

@@ -23,7 +23,7 @@ namespace qlka {
 enum { EMIT_ROWS = 0, EMIT_DOT = 1, EMIT_BOTH = 2 };
 
 // resident CTAs per SM that the passes are compiled for, and blocks in the emitting pass's rings (as in the Laplace walk)
-constexpr int PREFIX_CTAS1 = 3;
+constexpr int PREFIX_CTAS1 = 3, PREFIX_CTAS_ROWS = 2;
 __host__ __device__ constexpr int prefix_ctas2(int cpl, int emit) { return cpl == 4 ? 2 : emit == EMIT_BOTH ? 3 : 4; }
 __host__ __device__ constexpr int prefix_depth2(int emit) { return emit == EMIT_ROWS ? 3 : 2; }
 
@@ -145,13 +145,12 @@ __global__ void __launch_bounds__(WALK_THREADS, prefix_ctas2(CPL, EMIT)) prefix_
         int cur = 0, j0 = st.b0 * KB;
         for (int t = 0; t < st.nblk; t++, j0 += KB, cur = F2::next_slot(cur)) {
             f.advance_range();
-            const uint32_t cnt = f.m_hi - f.m_lo;
             if (DO_DOT) {
                 // the block's copies have had whole iterations; once its records are readable the emit-side rows
                 // of its first G_SLOTS queries start, ahead of the next block's copies, and land during the arithmetic
                 cp_async_wait<F2::AHEAD - 1>();
                 __syncwarp();
-                f.issue_g(cur, 0u, min(cnt, (uint32_t)G_SLOTS));
+                f.issue_g(cur, j0, 0u);
                 f.step_issue(t, cur, st.nblk);
             } else {
                 __syncwarp();
@@ -203,10 +202,79 @@ __global__ void __launch_bounds__(WALK_THREADS, prefix_ctas2(CPL, EMIT)) prefix_
                     out_s[r.z] = a.sign * (sum + __uint_as_float(r.y));
                 }
             };
-            for_queries<DO_DOT>(f, cur, j0, cnt, emit, finish);
+            for_queries<DO_DOT>(f, cur, j0, emit, finish);
         }
         cp_async_wait<0>();
     }
+}
+
+// Row emission with 4 channels per lane (RowFeeder; walk_ring.cuh's rows_by_quads says when)
+template <int LPS>
+__global__ void __launch_bounds__(WALK_THREADS, PREFIX_CTAS_ROWS) prefix_rows(const WalkArgs a)
+{
+    constexpr int STREAMS = WALK_THREADS / LPS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x, ln = tid % LPS, c0 = ln * 4;
+    const int N = a.N, C4 = a.C4, NBK = nblocks(N);
+    const bool lane_on = c0 < C4;
+    const int  c0l     = lane_on ? c0 : 0;
+    const unsigned gmask = LPS == 32 ? FULL : (((1u << (LPS & 31)) - 1u) << ((tid & 31) & ~(LPS - 1)));
+
+    RowFeeder<LPS> f;
+    f.init(smem_u32(smem), N, a.M, C4);
+
+    const int items = (int)(((long long)a.nseg * a.sps + STREAMS - 1) / STREAMS);
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const StreamOf st(a, item, tid / LPS, NBK, STREAMS);
+        f.start(a, st.sg, st.p, st.b0);
+        char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
+        Vec<4> PV, PK;
+        PV.zero(); PK.zero();
+        if (a.sps > 1) {        // incoming prefix sums (prefix_fold left them in the aggregate table)
+            const float* ag = a.agg + (st.on ? st.g : 0) * prefix_agg_stride(C4) + c0l;
+            PV = vload<4>(ag);
+            PK = vload<4>(ag + C4);
+        }
+        __syncwarp(gmask);                         // every lane has left the previous item's slots
+        f.prologue(st.nblk);
+        int cur = 0, j0 = st.b0 * KB;
+        for (int t = 0; t < st.nblk; t++, j0 += KB, cur ^= 1) {
+            __syncwarp(gmask);                     // every lane is done with the slot refilled below
+            f.step(t, cur, st.nblk);
+            __syncwarp(gmask);
+            float kv[KB + 1];
+            f.read_scalars(cur, kv);
+            Vec<4> v[KB], kb[KB];
+            f.read_rows(cur, j0, v);
+            // prefix states before each key, in place of the rows
+            #pragma unroll
+            for (int i = 0; i < KB; i++) {
+                const Vec<4> row = v[i];
+                v[i]  = PV;
+                kb[i] = PK;
+                vadd(PV, row);
+                axpy(PK, kv[i], row, PK);
+            }
+            f.for_queries(cur, j0, [&](const int i, const uint4& rec) {
+                Vec<4> r;
+                scale(r, __uint_as_float(rec.y), kb[i]);
+                axpy(r, __uint_as_float(rec.x), v[i], r);
+                if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
+            });
+        }
+        cp_async_wait<0>();
+    }
+}
+
+template <int LPS>
+static cudaError_t launch_rows(const WalkArgs& a, int sms, cudaStream_t stream) {
+    constexpr int smem = row_smem_bytes<LPS>();
+    cudaError_t e = cudaFuncSetAttribute(prefix_rows<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const long long items = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
+    const int cap = sms * PREFIX_CTAS_ROWS;
+    prefix_rows<LPS><<<items < cap ? (int)items : cap, WALK_THREADS, smem, stream>>>(a);
+    return cudaGetLastError();
 }
 
 template <int CPL, int EMIT>
@@ -239,7 +307,10 @@ static cudaError_t launch_pw(const WalkArgs& a, int emit, int sms, cudaStream_t 
         cudaError_t e = emit == EMIT_DOT ? launch_pass1<LPS, false>(a, sms, stream) : launch_pass1<LPS, true>(a, sms, stream);
         if (e != cudaSuccess) return e;
     }
-    if (emit == EMIT_ROWS) return launch_pass2<CPL, EMIT_ROWS>(a, sms, stream);
+    if (emit == EMIT_ROWS) {
+        if (CPL == 4 || rows_by_quads(a)) return launch_rows<LPS>(a, sms, stream);
+        if constexpr (CPL < 4) return launch_pass2<CPL, EMIT_ROWS>(a, sms, stream);
+    }
     if (emit == EMIT_DOT)  return launch_pass2<CPL, EMIT_DOT>(a, sms, stream);
     return launch_pass2<CPL, EMIT_BOTH>(a, sms, stream);
 }

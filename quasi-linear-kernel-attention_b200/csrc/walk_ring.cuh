@@ -52,6 +52,11 @@ __device__ __forceinline__ uint32_t lds32u(const uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
+__device__ __forceinline__ uint2 lds64u(const uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ void sts32f(const uint32_t addr, const float v) {
     asm volatile("st.shared.f32 [%0], %1;" :: "r"(addr), "f"(v) : "memory");
 }
@@ -188,63 +193,66 @@ struct Feeder {
     uint32_t        copy_dst;  // + my first row and my 16 bytes of it
     uint32_t        row_bytes; // C4 * 4
     bool            copy_on;   // my 16 bytes lie inside the row
-    int             lane, N;
+    int             lane, N, M;
     const char*     rows;      // + p * N * row_bytes + my 16 bytes
-    const float*    xval;      // of the next block to start, + my 16 bytes (lanes 16 .. 18)
-    const uint32_t* xperm;     // of the next block to prefetch, + my first row
-    const uint32_t* mstart;    // of the next block to prefetch
-    const uint4*    yrec;      // + my record of a block
+    const uint32_t* xperm;     // of the stream's first block, + my first row
+    const uint32_t* mstart;    // of the stream's first block
+    const char*     aux;       // lanes 0 .. 15: the segment's records; lanes 16 .. 18: the first block's scalars, + my 16 bytes
+    uint32_t        aux_dst;   // shared address they go to in slot 0
+    const uint4*    yrec;      // the segment's records
     const char*     grows;     // dot emissions: + p * M * row_bytes + my 16 bytes
     // prefetched one block before its issue
-    uint32_t idx[NCP], ms0, ms1;
-    // query range of the block in use and of the blocks in flight
-    uint32_t m_lo, m_hi, mq_lo[AHEAD], mq_hi[AHEAD];
+    uint32_t idx[NCP], ms;
+    // first query of the block in use and of the blocks in flight
+    uint32_t m_lo, mq_lo[AHEAD];
 
     __device__ __forceinline__ void init(const uint32_t area_, const int lane_, const int N_, const int C4) {
         area = area_; lane = lane_; N = N_;
         row_bytes = (uint32_t)C4 * 4u;
         copy_on   = (uint32_t)(lane % LR) * 16u < row_bytes;
         copy_dst  = area + (lane / LR) * NCP * row_pitch<CPL>() + (lane % LR) * 16;
+        aux_dst   = area + (lane < QCAP ? rec_offset<CPL, DEPTH>() + lane * 16 : sx_offset<CPL, DEPTH>() + (lane - QCAP) * 16);
     }
     // a stream of segment sg (head p) that starts at block b
     __device__ __forceinline__ void start(const WalkArgs& a, const int sg, const int p, const int b) {
-        xperm = a.xperm + (long long)sg * npad(a.N) + b * KB + (lane / LR) * NCP;
-        if (WITH_X) xval = a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * (lane - 16);
-        rows  = reinterpret_cast<const char*>(a.rows + (long long)p * a.N * a.C4) + (lane % LR) * 16;
+        xperm  = a.xperm + (long long)sg * npad(a.N) + b * KB + (lane / LR) * NCP;
+        rows   = reinterpret_cast<const char*>(a.rows + (long long)p * a.N * a.C4) + (lane % LR) * 16;
         mstart = a.mstart + (long long)sg * mstride(a.N) + b;
-        yrec   = a.yrec + (long long)sg * (a.M + 1) + lane;
+        yrec   = a.yrec + (long long)sg * (a.M + 1);
+        M      = a.M;
+        aux    = lane < QCAP ? reinterpret_cast<const char*>(yrec)
+                             : reinterpret_cast<const char*>(WITH_X ? a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * (lane - QCAP) : nullptr);
     }
     __device__ __forceinline__ void start_dots(const WalkArgs& a, const int p) {
         grows = reinterpret_cast<const char*>(a.g + (long long)p * a.M * a.C4) + (lane % LR) * 16;
     }
 
-    __device__ __forceinline__ void prefetch_index() {
-        if constexpr (NCP == 2) { const uint2 t = __ldg(reinterpret_cast<const uint2*>(xperm)); idx[0] = t.x; idx[1] = t.y; }
+    // t: the block's place in the stream
+    __device__ __forceinline__ void prefetch_index(const uint32_t t) {
+        const uint32_t* at = xperm + t * KB;
+        if constexpr (NCP == 2) { const uint2 u = __ldg(reinterpret_cast<const uint2*>(at)); idx[0] = u.x; idx[1] = u.y; }
         else {
             #pragma unroll
             for (int i = 0; i < NCP; i += 4) {
-                const uint4 t = __ldg(reinterpret_cast<const uint4*>(xperm + i));
-                idx[i] = t.x; idx[i + 1] = t.y; idx[i + 2] = t.z; idx[i + 3] = t.w;
+                const uint4 u = __ldg(reinterpret_cast<const uint4*>(at + i));
+                idx[i] = u.x; idx[i + 1] = u.y; idx[i + 2] = u.z; idx[i + 3] = u.w;
             }
         }
-        xperm += KB;
-        ms0 = __ldg(mstart); ms1 = __ldg(mstart + 1); mstart++;
+        ms = __ldg(mstart + t);
     }
 
     // start the copies of the block whose indices were prefetched last into `slot`; one commit group
-    __device__ __forceinline__ void issue(const int slot, const int ahead) {
-        mq_lo[ahead] = ms0; mq_hi[ahead] = ms1;
+    __device__ __forceinline__ void issue(const int slot, const int ahead, const uint32_t t) {
+        mq_lo[ahead] = ms;
         const uint32_t dst = copy_dst + slot * slot_bytes<CPL>();
         if (copy_on) {                                 // (positions past the last key point at row 0; read_rows zeroes them)
             #pragma unroll
             for (int i = 0; i < NCP; i++) cp_async16(dst + i * row_pitch<CPL>(), rows + (unsigned long long)idx[i] * row_bytes);
         }
-        // lanes 0..15 the first QCAP records from the block's first one on (the array is padded by QCAP records), lanes 16..18 the scalars
-        if (lane < QCAP) cp_async16(area + rec_offset<CPL, DEPTH>() + (slot * QCAP + lane) * 16, yrec + ms0);
-        if (WITH_X) {                                  // (the array is padded by KB floats)
-            if (lane >= 16 && lane < 19) cp_async16(area + sx_offset<CPL, DEPTH>() + slot * SX_STRIDE * 4 + (lane - 16) * 16, xval);
-            xval += KB;
-        }
+        // lanes 0..15 the first QCAP records from the block's first one on (past the segment's end: its sentinel, whose rank no block
+        // has), lanes 16..18 the scalars (padded by KB floats)
+        if (lane < (WITH_X ? QCAP + 3 : QCAP))
+            cp_async16(aux_dst + slot * (lane < QCAP ? QCAP * 16 : SX_STRIDE * 4), aux + (unsigned long long)(lane < QCAP ? min(ms + lane, (uint32_t)M) * 16ull : t * (KB * 4ull)));
         cp_async_commit();
     }
 
@@ -252,21 +260,21 @@ struct Feeder {
     __device__ __forceinline__ void prologue(const int nblk) {
         #pragma unroll
         for (int i = 0; i < AHEAD; i++) {
-            if (i < nblk) { prefetch_index(); issue(i, i); }
+            if (i < nblk) { prefetch_index(i); issue(i, i, i); }
             else cp_async_commit();
         }
-        if (AHEAD < nblk) prefetch_index();
+        if (AHEAD < nblk) prefetch_index(AHEAD);
     }
     // first thing of every step: the oldest block in flight becomes the block in use
     __device__ __forceinline__ void advance_range() {
-        m_lo = mq_lo[0]; m_hi = mq_hi[0];
+        m_lo = mq_lo[0];
         #pragma unroll
-        for (int i = 0; i + 1 < AHEAD; i++) { mq_lo[i] = mq_lo[i + 1]; mq_hi[i] = mq_hi[i + 1]; }
+        for (int i = 0; i + 1 < AHEAD; i++) mq_lo[i] = mq_lo[i + 1];
     }
     __device__ __forceinline__ void step_issue(const int t, const int cur, const int nblk) {
-        if (t + AHEAD < nblk) issue(cur == 0 ? DEPTH - 1 : cur - 1, AHEAD - 1);
+        if (t + AHEAD < nblk) issue(cur == 0 ? DEPTH - 1 : cur - 1, AHEAD - 1, t + AHEAD);
         else cp_async_commit();
-        if (t + AHEAD + 1 < nblk) prefetch_index();
+        if (t + AHEAD + 1 < nblk) prefetch_index(t + AHEAD + 1);
     }
     __device__ __forceinline__ static int next_slot(const int cur) { return cur == DEPTH - 1 ? 0 : cur + 1; }
 
@@ -291,13 +299,16 @@ struct Feeder {
 
     __device__ __forceinline__ uint32_t records(const int slot) const { return area + rec_offset<CPL, DEPTH>() + slot * QCAP * 16; }
 
-    // start the copies of the emit-side rows of the staged records n0 .. n1-1 of `slot` (n1 - n0 <= G_SLOTS); one commit group
-    __device__ __forceinline__ void issue_g(const int slot, const uint32_t n0, const uint32_t n1) const {
-        const uint32_t g = area + g_offset<CPL, DEPTH>() + (lane / LR) * NCP * row_pitch<CPL>() + (lane % LR) * 16;
-        const uint32_t n = n0 + (lane / LR) * NCP;
+    // start the copies of the emit-side rows of the G_SLOTS staged records from n0 on, as far as they belong to the block of key j0;
+    // one commit group
+    __device__ __forceinline__ void issue_g(const int slot, const int j0, const uint32_t n0) const {
+        const uint32_t g   = area + g_offset<CPL, DEPTH>() + (lane / LR) * NCP * row_pitch<CPL>() + (lane % LR) * 16;
+        const uint32_t rec = records(slot) + (n0 + (lane / LR) * NCP) * 16;
         #pragma unroll
-        for (int i = 0; i < NCP; i++)
-            if (copy_on && n + i < n1) cp_async16(g + i * row_pitch<CPL>(), grows + (unsigned long long)lds32u(records(slot) + (n + i) * 16 + 8) * row_bytes);
+        for (int i = 0; i < NCP; i++) {
+            const uint2 zw = lds64u(rec + i * 16 + 8);
+            if (copy_on && zw.y - (uint32_t)j0 < (uint32_t)KB) cp_async16(g + i * row_pitch<CPL>(), grows + (unsigned long long)zw.x * row_bytes);
+        }
         cp_async_commit();
     }
     // lane addresses of the emit-side row of query 0 of a batch and of this lane's part of its dot; query n: + n pitches, + n * 128
@@ -314,33 +325,39 @@ struct Feeder {
     }
 };
 
-// The queries of a block, in rank order: emit(i, rec, n128) for the queries that precede key i, n128 = 128 * (query's place in its
-// batch of G_SLOTS); finish(n0, n1) after every G_SLOTS queries and at the end (dot emissions; n0 counts from the staged records).
-// The staged records are followed by one of a later block (or the segment's sentinel), so a record's rank alone says where the
-// block ends; blocks with QCAP queries or more go QCAP - 1 at a time, with a terminator of their own.
+// The queries of the block of key j0, in rank order: emit(i, rec, n128) for the queries that precede key i, n128 = 128 * (query's place
+// in its batch of G_SLOTS); finish(n0, n1) after every G_SLOTS queries and at the end (dot emissions; n0 counts from the staged
+// records). The staged records are followed by one of a later block (or the segment's sentinel), so a record's rank alone says
+// where the block ends; when the last staged record is still the block's, it goes QCAP - 1 queries at a time, with a terminator.
+// (Dots carry only the next query's rank: carrying its record costs them four moves a query; rows, with fewer registers in use,
+// are 3 % faster with the record.)
 template <bool DO_DOT, class F, class Emit, class Finish>
-__device__ __forceinline__ void for_queries(const F& f, const int slot, const int j0, const uint32_t cnt, Emit emit, Finish finish) {
+__device__ __forceinline__ void for_queries(const F& f, const int slot, const int j0, Emit emit, Finish finish) {
     constexpr uint32_t BATCH = QCAP - 1;
     const uint32_t recs = f.records(slot);
-    uint32_t left = cnt;                                   // queries from the staged records on
-    uint32_t at   = f.m_lo;
+    uint32_t at = f.m_lo;
     while (true) {
-        const bool more = left > BATCH;
+        const bool more = lds32u(recs + BATCH * 16 + 12) - (uint32_t)j0 < (uint32_t)KB;
         if (more) {
             __syncwarp();
             if (f.lane == 0) sts32f(recs + BATCH * 16 + 12, __uint_as_float(0xffffffffu));
             __syncwarp();
         }
         uint32_t qa = recs, n128 = 0, n0 = 0;
-        uint4    rec = lds128u(qa);
-        uint32_t key = rec.w - (uint32_t)j0;
+        uint4    rec;
+        uint32_t key;
+        auto fetch = [&]() {
+            if (DO_DOT) key = lds32u(qa + 12) - (uint32_t)j0;
+            else      { rec = lds128u(qa); key = rec.w - (uint32_t)j0; }
+        };
+        fetch();
         #pragma unroll
         for (int i = 0; i < KB; i++) {
             while (key == (uint32_t)i) {
-                emit(i, rec, n128);
+                const uint4 now = DO_DOT ? lds128u(qa) : rec;
                 qa += 16;
-                rec = lds128u(qa);
-                key = rec.w - (uint32_t)j0;
+                if (DO_DOT) { fetch(); emit(i, now, n128); }
+                else        { emit(i, now, n128); fetch(); }
                 if (DO_DOT) {
                     n128 += 128;
                     if (n128 == G_SLOTS * 128) {
@@ -349,7 +366,7 @@ __device__ __forceinline__ void for_queries(const F& f, const int slot, const in
                         __syncwarp();
                         n0 += G_SLOTS;
                         n128 = 0;
-                        f.issue_g(slot, n0, min(left, min(n0 + G_SLOTS, BATCH)));
+                        f.issue_g(slot, j0, n0);
                         cp_async_wait<0>();
                         __syncwarp();
                     }
@@ -361,13 +378,12 @@ __device__ __forceinline__ void for_queries(const F& f, const int slot, const in
             finish(n0, n0 + (n128 >> 7));
         }
         if (!more) break;
-        left -= BATCH;
-        at   += BATCH;
+        at += BATCH;
         __syncwarp();
-        if (f.lane < QCAP) sts128u(recs + f.lane * 16, __ldg(f.yrec + at));
+        if (f.lane < QCAP) sts128u(recs + f.lane * 16, __ldg(f.yrec + min(at + f.lane, (uint32_t)f.M)));
         __syncwarp();
         if (DO_DOT) {
-            f.issue_g(slot, 0u, min(left, (uint32_t)G_SLOTS));
+            f.issue_g(slot, j0, 0u);
             cp_async_wait<0>();
             __syncwarp();
         }
@@ -446,6 +462,84 @@ struct SumFeeder {
         av[8] = a2.x;
     }
 };
+
+// The same mapping with the queries' records, for row emission where queries are few beside the keys or the rows are wide: what a
+// block costs besides its queries is then what counts, and 4 channels per lane halve (LPS = 16) or quarter (LPS = 8) it. The
+// streams of a warp go through their queries side by side, each in its own loop.
+template <int LPS> __host__ __device__ constexpr int row_smem_bytes() { return sum_smem_bytes<LPS>() + WALK_THREADS * 2 * 16; }
+
+template <int LPS>
+struct RowFeeder : SumFeeder<LPS, true, 1> {
+    using Base = SumFeeder<LPS, true, 1>;
+    uint32_t        recs;      // shared address of the stream's record slots [2][LPS]
+    const uint4*    yrec;      // the segment's records
+    const uint32_t* mstart;    // of the next block to prefetch
+    uint32_t        ms, m_lo, m_next, M;     // first query: of the block prefetched, in use, in flight
+
+    __device__ __forceinline__ void init(const uint32_t smem, const int N_, const int M_, const int C4) {
+        Base::init(smem, N_, C4);
+        recs = smem + sum_smem_bytes<LPS>() + (threadIdx.x / LPS) * 2 * LPS * 16;
+        M = (uint32_t)M_;
+    }
+    __device__ __forceinline__ void start(const WalkArgs& a, const int sg, const int p, const int b) {
+        Base::start(a, sg, p, b);
+        yrec   = a.yrec + (long long)sg * (a.M + 1);
+        mstart = a.mstart + (long long)sg * mstride(a.N) + b;
+    }
+    __device__ __forceinline__ void prefetch() { Base::prefetch_index(); ms = __ldg(mstart++); }
+    // (a block with fewer than LPS queries finds all of them staged, followed by a record of a later block or the sentinel)
+    __device__ __forceinline__ void issue_with_records(const int slot) {
+        m_next = ms;
+        cp_async16(recs + (slot * LPS + this->ln) * 16, yrec + min(ms + (uint32_t)this->ln, M));
+        Base::issue(slot);
+    }
+    __device__ __forceinline__ void prologue(const int nblk) {
+        if (nblk > 0) { prefetch(); issue_with_records(0); }
+        if (nblk > 1) prefetch();
+    }
+    __device__ __forceinline__ void step(const int t, const int cur, const int nblk) {
+        m_lo = m_next;
+        if (t + 1 < nblk) issue_with_records(cur ^ 1);
+        else cp_async_commit();
+        if (t + 2 < nblk) prefetch();
+        cp_async_wait<1>();
+    }
+    // emit(i, rec) for the queries of the block of key j0 that precede key i, in rank order
+    template <class Emit>
+    __device__ __forceinline__ void for_queries(const int slot, const int j0, Emit emit) const {
+        uint32_t qa = recs + slot * LPS * 16;
+        if (lds32u(qa + (LPS - 1) * 16 + 12) - (uint32_t)j0 >= (uint32_t)KB) {
+            uint4 rec = lds128u(qa);
+            #pragma unroll
+            for (int i = 0; i < KB; i++) {
+                while (rec.w == (uint32_t)(j0 + i)) {
+                    qa += 16;
+                    const uint4 next = lds128u(qa);
+                    emit(i, rec);
+                    rec = next;
+                }
+            }
+        } else {                                       // more queries than the slot holds: read them from memory
+            const uint4* yp  = yrec + m_lo;
+            uint4        rec = __ldg(yp);
+            #pragma unroll
+            for (int i = 0; i < KB; i++) {
+                while (rec.w == (uint32_t)(j0 + i)) {
+                    const uint4 next = __ldg(++yp);    // at most the segment's sentinel
+                    emit(i, rec);
+                    rec = next;
+                }
+            }
+        }
+    }
+};
+
+// Which mapping emits rows: at 33 .. 64 channels a warp per stream is the faster one once queries outnumber keys (48 heads x 1024
+// keys x 8192 queries 2.52 -> 1.70 ms; at equal numbers Laplace 5.47 -> 5.53 ms at 16384, abs 1.33 -> 1.37 ms at 4096; at 15847 keys
+// x 2522 queries 3.88 -> 4.13 ms), at up to 32 from a quarter as many queries as keys on (4096 x 4096: 1.32 -> 1.05 ms, x 512
+// queries: 0.68 -> 0.79 ms); wider rows leave one stream per warp either way, with shared-memory copies of its own in favour
+// of this one (abs at 8192: 1.49 against 1.55 ms).
+inline bool rows_by_quads(const WalkArgs& a) { return a.C4 > 64 || (a.C4 > 32 ? a.M <= a.N : 4LL * a.M <= a.N); }
 
 // the key blocks [b0, b1) that stream s of the SPS streams of a segment owns (NBK blocks per segment)
 __device__ __forceinline__ void stream_blocks(const int s, const int SPS, const int NBK, int& b0, int& b1) {
