@@ -100,7 +100,8 @@ int sm_count() {
 
 // How a walk over `nseg` segments of N keys is cut into streams and work items (a CTA's worth of streams, one per warp). Streams are
 // independent work units (the passes exchange their states through memory), so a segment may be cut into any number of them:
-// more streams until the persistent CTAs of the second pass get about sixteen items each, as long as a stream
+// more streams until the persistent CTAs of the second pass get about eight items each (sixteen: more aggregates to write, fold and read,
+// Laplace backward at 48 heads x 4096 keys 4.0 instead of 3.9 ms; four: tails, abs at 16 x 65536 8.45 instead of 8.25 ms), as long as a stream
 // keeps at least sixteen key blocks (the staging ring needs a few blocks to fill) - eight while there are fewer
 // items than CTAs. The prefix walks need no first pass with one stream per segment, which pays as soon as whole
 // segments alone give every CTA a few items.
@@ -113,7 +114,7 @@ WalkPlan plan_walk(int nseg, int N, int C4, bool laplace) {
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
     if (laplace || items(1) < 2LL * cap)
-        while (items(sps) < 16LL * cap && nbk / (sps * 2) >= (items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
+        while (items(sps) < 8LL * cap && nbk / (sps * 2) >= (items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
     return {sps, (int)items(sps)};
 }
 

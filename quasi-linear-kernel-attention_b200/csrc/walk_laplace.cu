@@ -100,39 +100,54 @@ __global__ void __launch_bounds__(WALK_THREADS, LAP_CTAS1) laplace_pass1(const W
 
 // Between the passes: per segment and channel, the aggregates of the SPS streams become the states entering each
 // stream - in place, forward aggregate -> prefix state before the stream (L = decay * L + aggregate over the earlier
-// streams), backward aggregate -> suffix state after it. One thread per (segment, channel), serial over the streams.
-__global__ void __launch_bounds__(256) laplace_fold(float* __restrict__ agg, const int nseg, const int SPS, const int C4)
+// streams), backward aggregate -> suffix state after it. A warp's share of the streams is one such step itself: its aggregate and the
+// product of its decays.
+__global__ void __launch_bounds__(32 * FOLD_WARPS) laplace_fold(float* __restrict__ agg, const int nseg, const int SPS, const int C4, const int warps)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nseg * C4) return;
-    const int sg = (int)(i / C4), c = (int)(i - (long long)sg * C4);
-    const int AGS = lap_agg_stride(C4);
-    float* ag = agg + (long long)sg * SPS * AGS;
-    constexpr int CH = 16;                     // streams per chunk: their loads are issued together, then the serial part
-    float L = 0.0f;
-    for (int t0 = 0; t0 < SPS; t0 += CH) {
-        float fv[CH], af[CH];
+    __shared__ float4 total[FOLD_WARPS][32];       // forward and backward aggregate, forward and backward decay of a share
+    const FoldOf f(nseg, SPS, C4, warps);
+    const int lane = threadIdx.x & 31, c = f.c, first = f.first, last = f.last, AGS = lap_agg_stride(C4);
+    float* ag = agg + f.sg * SPS * AGS;
+    float L = 0.0f, R = 0.0f;
+    if (warps > 1) {
+        float dl = 1.0f, dr = 1.0f;
+        #pragma unroll FOLD_CHUNK
+        for (int t = first; t < last; t++) {           // (the backward aggregates forwards: R = b + d * (next b + next d * (...)))
+            const float* at = ag + (long long)t * AGS;
+            const float  af = at[2 * C4], ab = at[2 * C4 + 1];
+            L = fmaf(af, L, at[c]);
+            R = fmaf(dr, at[C4 + c], R);
+            dl *= af; dr *= ab;
+        }
+        total[threadIdx.x >> 5][lane] = make_float4(L, R, dl, dr);
+        __syncthreads();
+        L = R = 0.0f;
+        for (int u = f.group; u < f.group + f.share; u++)             { const float4 t = total[u][lane]; L = fmaf(t.z, L, t.x); }
+        for (int u = f.group + warps - 1; u > f.group + f.share; u--) { const float4 t = total[u][lane]; R = fmaf(t.w, R, t.y); }
+    }
+    if (!f.on) return;
+    for (int t0 = first; t0 < last; t0 += FOLD_CHUNK) {
+        float fv[FOLD_CHUNK], af[FOLD_CHUNK];
         #pragma unroll
-        for (int k = 0; k < CH; k++) {
-            const float* at = ag + (long long)min(t0 + k, SPS - 1) * AGS;
+        for (int k = 0; k < FOLD_CHUNK; k++) {
+            const float* at = ag + (long long)min(t0 + k, last - 1) * AGS;
             fv[k] = at[c]; af[k] = at[2 * C4];
         }
         #pragma unroll
-        for (int k = 0; k < CH; k++) {
-            if (t0 + k < SPS) { ag[(long long)(t0 + k) * AGS + c] = L; L = fmaf(af[k], L, fv[k]); }
+        for (int k = 0; k < FOLD_CHUNK; k++) {
+            if (t0 + k < last) { ag[(long long)(t0 + k) * AGS + c] = L; L = fmaf(af[k], L, fv[k]); }
         }
     }
-    float R = 0.0f;
-    for (int t0 = SPS - 1; t0 >= 0; t0 -= CH) {
-        float bv[CH], ab[CH];
+    for (int t0 = last - 1; t0 >= first; t0 -= FOLD_CHUNK) {
+        float bv[FOLD_CHUNK], ab[FOLD_CHUNK];
         #pragma unroll
-        for (int k = 0; k < CH; k++) {
-            const float* at = ag + (long long)max(t0 - k, 0) * AGS;
+        for (int k = 0; k < FOLD_CHUNK; k++) {
+            const float* at = ag + (long long)max(t0 - k, first) * AGS;
             bv[k] = at[C4 + c]; ab[k] = at[2 * C4 + 1];
         }
         #pragma unroll
-        for (int k = 0; k < CH; k++) {
-            if (t0 - k >= 0) { ag[(long long)(t0 - k) * AGS + C4 + c] = R; R = fmaf(ab[k], R, bv[k]); }
+        for (int k = 0; k < FOLD_CHUNK; k++) {
+            if (t0 - k >= first) { ag[(long long)(t0 - k) * AGS + C4 + c] = R; R = fmaf(ab[k], R, bv[k]); }
         }
     }
 }
@@ -344,7 +359,7 @@ static cudaError_t launch_lap(const WalkArgs& a, int sms, cudaStream_t stream, c
     const long long items1 = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
     const int cap1 = sms * LAP_CTAS1;
     laplace_pass1<LPS><<<items1 < cap1 ? (int)items1 : cap1, WALK_THREADS, smem1, stream>>>(a);
-    laplace_fold<<<(unsigned)(((long long)a.nseg * a.C4 + 255) / 256), 256, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4);
+    laplace_fold<<<fold_grid(a), 32 * FOLD_WARPS, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4, fold_share_warps(a));
     e = cudaGetLastError();
     if (e == cudaSuccess && mid) e = cudaEventRecord(mid, stream);
     if (e != cudaSuccess) return e;

@@ -79,25 +79,36 @@ __global__ void __launch_bounds__(WALK_THREADS, PREFIX_CTAS1) prefix_pass1(const
 }
 
 // Between the launches: per segment and channel, exclusive prefix sums of the stream aggregates, in place.
-__global__ void __launch_bounds__(256) prefix_fold(float* __restrict__ agg, const int nseg, const int SPS, const int C4, const int with_k)
+__global__ void __launch_bounds__(32 * FOLD_WARPS) prefix_fold(float* __restrict__ agg, const int nseg, const int SPS, const int C4, const int warps, const int with_k)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nseg * C4) return;
-    const int sg = (int)(i / C4), c = (int)(i - (long long)sg * C4);
-    const int AGS = prefix_agg_stride(C4);
-    float* ag = agg + (long long)sg * SPS * AGS;
-    constexpr int CH = 16;                     // streams per chunk: their loads are issued together, then the serial part
+    __shared__ float total[2][FOLD_WARPS][32];
+    const FoldOf f(nseg, SPS, C4, warps);
+    const int lane = threadIdx.x & 31, c = f.c, first = f.first, last = f.last, AGS = prefix_agg_stride(C4);
+    float* ag = agg + f.sg * SPS * AGS;
     float pv = 0.0f, pk = 0.0f;
-    for (int t0 = 0; t0 < SPS; t0 += CH) {
-        float v[CH], k[CH];
+    if (warps > 1) {
+        #pragma unroll FOLD_CHUNK
+        for (int t = first; t < last; t++) {
+            pv += ag[(long long)t * AGS + c];
+            if (with_k) pk += ag[(long long)t * AGS + C4 + c];
+        }
+        total[0][threadIdx.x >> 5][lane] = pv;
+        total[1][threadIdx.x >> 5][lane] = pk;
+        __syncthreads();
+        pv = pk = 0.0f;
+        for (int u = f.group; u < f.group + f.share; u++) { pv += total[0][u][lane]; pk += total[1][u][lane]; }
+    }
+    if (!f.on) return;
+    for (int t0 = first; t0 < last; t0 += FOLD_CHUNK) {
+        float v[FOLD_CHUNK], k[FOLD_CHUNK];
         #pragma unroll
-        for (int j = 0; j < CH; j++) {
-            const float* at = ag + (long long)min(t0 + j, SPS - 1) * AGS;
+        for (int j = 0; j < FOLD_CHUNK; j++) {
+            const float* at = ag + (long long)min(t0 + j, last - 1) * AGS;
             v[j] = at[c]; k[j] = with_k ? at[C4 + c] : 0.0f;
         }
         #pragma unroll
-        for (int j = 0; j < CH; j++) {
-            if (t0 + j < SPS) {
+        for (int j = 0; j < FOLD_CHUNK; j++) {
+            if (t0 + j < last) {
                 float* at = ag + (long long)(t0 + j) * AGS;
                 at[c] = pv; pv += v[j];
                 if (with_k) { at[C4 + c] = pk; pk += k[j]; }
@@ -297,7 +308,7 @@ static cudaError_t launch_pass1(const WalkArgs& a, int sms, cudaStream_t stream)
     const long long items1 = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
     const int cap1 = sms * PREFIX_CTAS1;
     k1<<<items1 < cap1 ? (int)items1 : cap1, WALK_THREADS, smem1, stream>>>(a);
-    prefix_fold<<<(unsigned)(((long long)a.nseg * a.C4 + 255) / 256), 256, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4, WITH_K ? 1 : 0);
+    prefix_fold<<<fold_grid(a), 32 * FOLD_WARPS, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4, fold_share_warps(a), WITH_K ? 1 : 0);
     return cudaGetLastError();
 }
 

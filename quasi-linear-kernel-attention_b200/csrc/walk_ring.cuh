@@ -547,6 +547,32 @@ __device__ __forceinline__ void stream_blocks(const int s, const int SPS, const 
     b1 = (int)((long long)(s + 1) * NBK / SPS);
 }
 
+// The kernels between the passes: a lane per segment and channel. From 32 streams per segment on, 2, 4 or 8 warps share a column:
+// each folds its share of the streams, the totals go through shared memory, then each writes the states entering its
+// streams. (One thread per column whatever the number: a serial chain through memory, 0.38 instead of 0.32 ms for a whole
+// Laplace sum of 16 segments of 65536 keys; sharing fewer streams only reads them twice.)
+constexpr int FOLD_WARPS = 8, FOLD_CHUNK = 16;     // warps per CTA; loads of FOLD_CHUNK streams are in flight together
+inline int      fold_share_warps(const WalkArgs& a) { return a.sps < 32 ? 1 : a.sps < 64 ? 2 : a.sps < 128 ? 4 : FOLD_WARPS; }
+inline unsigned fold_grid(const WalkArgs& a) {
+    const int columns = 32 * FOLD_WARPS / fold_share_warps(a);                     // per CTA
+    return (unsigned)(((long long)a.nseg * a.C4 + columns - 1) / columns);
+}
+// where a thread of a fold stands: segment and channel (the last column's for lanes past the end), its share [first, last) of the
+// SPS streams, and which share of how many that is
+struct FoldOf {
+    bool on; long long sg; int c, first, last, share, group;      // group: first warp of the CTA that works on the column
+    __device__ __forceinline__ FoldOf(const int nseg, const int SPS, const int C4, const int warps) {
+        const int w = threadIdx.x >> 5;
+        share = w % warps; group = w - share;
+        const long long col = ((long long)blockIdx.x * (FOLD_WARPS / warps) + w / warps) * 32 + (threadIdx.x & 31), all = (long long)nseg * C4;
+        on = col < all;
+        const long long i = on ? col : all - 1;
+        sg = i / C4; c = (int)(i - sg * C4);
+        const int per = (SPS + warps - 1) / warps;
+        first = min(share * per, SPS); last = min(first + per, SPS);
+    }
+};
+
 // the stream of a warp: segment, block range
 struct StreamOf {
     long long g; bool on; int sg, p, b0, b1, nblk;
