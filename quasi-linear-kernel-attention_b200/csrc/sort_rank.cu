@@ -388,6 +388,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     float blo, bsc;
     auto bucket = [&](const float val) -> int { return (int)fminf(fmaxf((val - blo) * bsc, 0.0f), (float)(NB - 1)); };
     bool by_radix;
+    uint16_t*  sorted  = reinterpret_cast<uint16_t*>(cnt);         // the keys' indices in sorted order ...
+    const bool scalars = a.us != nullptr;                          // ... needed here only to look up per-key scalars
     {
         uint32_t key[E], idx[E];
         if (PART) load_part<THREADS, E>(kkey, N, key, idx);
@@ -460,8 +462,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
             }
             __syncthreads();
             // final place of the key at p: start of its bucket + the keys of the bucket that sort before it (equal keys in
-            // the order of their original index, as the radix sort leaves them)
-            uint16_t* sidx2 = reinterpret_cast<uint16_t*>(cnt);
+            // the order of their original index, as the radix sort leaves them). The lanes of a warp work on neighbouring buckets, so
+            // the permutation leaves from here, a line or two per store.
             #pragma unroll 2
             for (int s = 0; s < E; s++) {
                 const int pp = warp * 32 * E + s * 32 + lane;
@@ -477,15 +479,15 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                         if (kk == k && j != pp) c += sidx[j] < mine;
                     }
                     xs[skew(lo + c)] = x;
-                    sidx2[lo + c]    = (uint16_t)mine;
+                    if (!PART) xperm[lo + c] = mine;
+                    if (PART || scalars) sorted[lo + c] = (uint16_t)mine;
                 }
             }
-            __syncthreads();
-            for (int j = tid; j < N; j += THREADS) sidx[j] = sidx2[j];
         } else {
             #pragma unroll
             for (int s = 0; s < E; s++) idx[s] = warp * 32 * E + s * 32 + lane;
             block_radix_sort<THREADS, E>(key, idx, skey, sidx, cnt, base, wsum, tab);
+            sorted = sidx;
         }
     }
     PHASE_MARK(1);
@@ -507,7 +509,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         for (int j = tid; j < N; j += THREADS) skey[j] = __ldg(kidx + j);
         __syncthreads();
     }
-    for (int j = tid; j < N; j += THREADS) xperm[j] = PART ? skey[sidx[j]] : (uint32_t)sidx[j];
+    if (PART || by_radix) for (int j = tid; j < N; j += THREADS) xperm[j] = PART ? skey[sorted[j]] : (uint32_t)sorted[j];
     if (last) for (int j = N + tid; j < NP - ks; j += THREADS) xperm[j] = 0u;
     __syncthreads();
     PHASE_MARK(2);
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                     const float* us = a.us ? a.us + (long long)p * NG : nullptr;
                     __syncthreads();                  // every thread has picked its decays out of the staging buffer
                     #pragma unroll
-                    for (int k = 0; k < R; k++) if (k < cntk) stage[i0 + k] = us ? us[key_row(sidx[i0 + k])] : 1.0f;
+                    for (int k = 0; k < R; k++) if (k < cntk) stage[i0 + k] = us ? us[key_row(sorted[i0 + k])] : 1.0f;
                 }
                 block_affine_scan_mem<THREADS, R, false, 0>(cntk, i0, dk, stage, su0s, wa, wb);
                 block_affine_scan_mem<THREADS, R, true, 1>(cntk, i0, dk, stage, stage, wa, wb);
@@ -583,7 +585,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                 #pragma unroll
                 for (int k = 0; k <= R; k++) dk[k] = 1.0f;
                 #pragma unroll
-                for (int k = 0; k < R; k++) bx[k] = k < cntk ? (us ? us[key_row(sidx[i0 + k])] : xs[skew(i0 + k)]) : 0.0f;
+                for (int k = 0; k < R; k++) bx[k] = k < cntk ? (us ? us[key_row(sorted[i0 + k])] : xs[skew(i0 + k)]) : 0.0f;
                 block_affine_scan<THREADS, R, false, 0>(cntk, dk, bx, wa, wb);
                 flush(bx, su0);
             }
