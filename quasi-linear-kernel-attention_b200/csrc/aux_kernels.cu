@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(256) vecsum_kernel(const float* __restrict__ x
 }
 
 // out[p, m, c] = A * ktot[p, c] - (A * qsum[p, m] + Bq) * vsum[p, c];  out_u[p, m] = A * ksr[p] - Nk * (A * qsum[p, m] + Bq)
-// (A = 1, Bq = 0 for the plain abs sum; a folded sum over shifted queries has A = sum of weights, Bq = D * sum w_s shift_s)
+// (A = 1, Bq = 0 for the plain abs sum; a folded sum over shifted queries has A = sum of weights, Bq = D * sum w_s shift_s; without
+// qsum the query terms are left out)
 __global__ void abs_init_kernel(
     const float* __restrict__ ktot, const float* __restrict__ vsum, const float* __restrict__ qsum,
     const float* __restrict__ ksr, float* __restrict__ out, float* __restrict__ out_u,
@@ -84,7 +85,7 @@ __global__ void abs_init_kernel(
     const long long p  = pm / M;
     const float4 kt = *reinterpret_cast<const float4*>(ktot + p * C4 + c);
     const float4 vs = *reinterpret_cast<const float4*>(vsum + p * C4 + c);
-    const float  qs = fmaf(A, qsum[pm], Bq);
+    const float  qs = qsum ? fmaf(A, qsum[pm], Bq) : 0.0f;
     *reinterpret_cast<float4*>(out + pm * C4 + c) =
         make_float4(fmaf(-qs, vs.x, A * kt.x), fmaf(-qs, vs.y, A * kt.y), fmaf(-qs, vs.z, A * kt.z), fmaf(-qs, vs.w, A * kt.w));
     if (out_u && c == 0) out_u[pm] = A * ksr[p] - Nk * qs;

@@ -408,7 +408,7 @@ struct AbsFwdWs {
 // ------------------------------------------------------------------ abs backward / sgn
 struct AbsBwdWs {
     float *vpad, *gpad, *gvpad; Records rec;
-    float *qsumd, *ksumd, *sums /* vsum | gwsum | qtotg | gu_total */, *agg;
+    float *qsumd, *sums /* vsum | gwsum | qtotg | gu_total */, *agg;
     size_t bytes;
     AbsBwdWs(void* base, int P, int D, int N, int M, int C) {
         Bump b(base);
@@ -419,7 +419,6 @@ struct AbsBwdWs {
         const int mx = N > M ? N : M;
         rec.carve(b, nseg, mx, mx);
         qsumd = b.take<float>((size_t)P * M);
-        ksumd = b.take<float>((size_t)P * N);
         sums  = b.take<float>((size_t)P * C4 * 3 + P);
         const size_t agg_k = prefix_agg_floats(P, D, N, C4), agg_q = prefix_agg_floats(P, D, M, C4);
         agg   = b.take<float>(agg_k > agg_q ? agg_k : agg_q);
@@ -1032,7 +1031,6 @@ int qlka_weighted_abs_sum_backward(const float* q, const float* k, const float* 
     float* qtotg    = gwsum + (size_t)P * C4;
     float* gu_total = qtotg + (size_t)P * C4;
     CU(launch_colsum_d(q, ws.qsumd, P, D, M, stream));
-    CU(launch_colsum_d(k, ws.ksumd, P, D, N, stream));
     CU(cudaMemsetAsync(ws.sums, 0, sizeof(float) * ((size_t)P * C4 * 3 + P), stream));
     CU(launch_rowstat(vrows, nullptr, vsum, nullptr, nullptr, P, N, C4, stream));
     CU(launch_rowstat(grows, ws.qsumd, gwsum, qtotg, nullptr, P, M, C4, stream));
@@ -1051,8 +1049,8 @@ int qlka_weighted_abs_sum_backward(const float* q, const float* k, const float* 
         s.us = g_u; s.us_total = gu_total;
         CU(launch_sort_rank(s, ws.rec, stream));
         // one walk for both: grad_v = abs sum with keys q, weights g_w, evaluated at the keys k (row reductions on
-        // top of its rank-1 initial value); grad_k = prefix of g_w rows contracted with v rows (+ the g_u term in e1)
-        CU(launch_abs_init(qtotg, gwsum, ws.ksumd, nullptr, gv, nullptr, P, N, C4, M, 1.0f, 0.0f, stream));
+        // top of a constant row per head); grad_k = prefix of g_w rows contracted with v rows (+ the g_u term in e1)
+        CU(launch_abs_init(qtotg, gwsum, nullptr, nullptr, gv, nullptr, P, N, C4, M, 1.0f, 0.0f, stream));
         WalkArgs w = walk_args(ws.rec, grows, nseg, D, M, N, C4);
         w.g = vrows; w.wtotal = gwsum; w.out_s = grad_k; w.out = gv; w.agg = ws.agg;
         CU(prefix_walk_chunked(w, EMIT_BOTH, P, stream));

@@ -330,8 +330,8 @@ struct Feeder {
 // records). The staged records are followed by one of a later block (or the segment's sentinel), so a record's rank alone says
 // where the block ends; when the last staged record is still the block's, it goes QCAP - 1 queries at a time, with a terminator.
 // (Dots carry only the next query's rank: carrying its record costs them four moves a query; rows, with fewer registers in use,
-// are 3 % faster with the record.)
-template <bool DO_DOT, class F, class Emit, class Finish>
+// are 3 % faster with the record. REC false: emit has no use for the record.)
+template <bool DO_DOT, bool REC = true, class F, class Emit, class Finish>
 __device__ __forceinline__ void for_queries(const F& f, const int slot, const int j0, Emit emit, Finish finish) {
     constexpr uint32_t BATCH = QCAP - 1;
     const uint32_t recs = f.records(slot);
@@ -354,7 +354,7 @@ __device__ __forceinline__ void for_queries(const F& f, const int slot, const in
         #pragma unroll
         for (int i = 0; i < KB; i++) {
             while (key == (uint32_t)i) {
-                const uint4 now = DO_DOT ? lds128u(qa) : rec;
+                const uint4 now = DO_DOT ? (REC ? lds128u(qa) : make_uint4(0u, 0u, 0u, 0u)) : rec;
                 qa += 16;
                 if (DO_DOT) { fetch(); emit(i, now, n128); }
                 else        { emit(i, now, n128); fetch(); }
