@@ -221,7 +221,7 @@ def run_abs_fwd_bwd(args):
             "dtype": "f32", "data": "synthetic",
             "config": {"workload": "weighted_abs_sum_full forward+backward B=8 H=12 N=M=4096 D=64 Dv=64 fp32 (q,k~0.5*N(0,1), v,g~N(0,1), seed 0)",
                        "l2": "inputs larger than L2"},
-            "clocks": clocks.summary(), "gpu_launches": 16 * args.steps,      # 6 kernels of the forward, 10 of the backward
+            "clocks": clocks.summary(), "gpu_launches": 21 * args.steps,      # 8 kernels of the forward, 13 of the backward
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None, "peak_source": which, "algorithmic_bytes": algo, "kernel": "whole forward+backward step"}}
     print(json.dumps(line), flush=True)
@@ -434,7 +434,7 @@ def run_ours(args, rank, world, local_rank):
         "gpu_launches": 4 * args.steps,          # sort/rank, first walk pass, fold, second walk pass
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_source": which, "algorithmic_bytes": ab,
-                     "kernel": "laplace_pass2 (dominant kernel; launch time from CUDA events on the launching stream)",
+                     "kernel": "laplace_rows (dominant kernel; launch time from CUDA events on the launching stream)",
                      "operator_achieved": achieved_op, "operator_frac": achieved_op / peak,
                      "stage_ms": stage,
                      # ceilings of this formulation that sit far below the HBM one (per launch, this rank's heads):
@@ -453,10 +453,10 @@ def run_ours(args, rank, world, local_rank):
     print(json.dumps(line), flush=True)
 
 
-# figures from a profiler capture of the dominant kernel (dram__bytes_read + dram__bytes_write of one laplace_pass2 launch over
-# 12 heads: 845.7 MB + 43.3 MB) and from a bare gather / reduction loop with the walk's access pattern (two row gathers and one
+# figures from a profiler capture of the dominant kernel (dram__bytes_read + dram__bytes_write of one laplace_rows launch over
+# 12 heads: 837.6 MB + 41.3 MB) and from a bare gather / reduction loop with the walk's access pattern (two row gathers and one
 # row reduction per segment, 48 heads: 3.03 ms), both on a B200
-WALK_DRAM_BYTES_PER_HEAD = (845.66e6 + 43.32e6) / 12
+WALK_DRAM_BYTES_PER_HEAD = (837.61e6 + 41.28e6) / 12
 L2_FLOOR_MS_PER_HEAD = 3.034 / 48
 
 
