@@ -109,7 +109,9 @@ struct WalkPlan { int sps, nitems; };
 
 WalkPlan plan_walk(int nseg, int N, int C4, bool laplace) {
     constexpr int streams = 8;                        // warps of a walk CTA
-    const int cap = sm_count() * 4;                    // resident CTAs, about
+    // resident CTAs, about (above 64 channels two per SM; planned for four, Laplace at 16 heads x 8191 keys x 1030 queries took 1.08
+    // instead of 1.03 ms, its backward at 16 x 8192 4.71 instead of 4.45 ms)
+    const int cap = sm_count() * (C4 > 64 ? 2 : 4);
     const int nbk = nblocks(N);
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
