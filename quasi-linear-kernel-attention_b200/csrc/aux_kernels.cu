@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) transpose_scale_kernel(const float* __res
 
 // The way back for a gradient: dst[p, s, d] = (src[p, d, s] + c) * scale * (keep ? keep[p / H, s] : 1). With `qt` (the operator's
 // queries) c takes out what the masked keys, which sit at the origin, added through the row sum's gradient dd[p, s]:
-// c = n_pad[p / H] dd[p, s] sign(q) exp(-|q|).
+// c = n_pad[p / H] dd[p, s] sign(q) exp(-|q|), the sign at 0 as the walk has it: a key equal to the query counts as above it, derivative +1.
 __global__ void __launch_bounds__(256) transpose_back_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                              const float* __restrict__ keep, const float scale,
                                                              const float* __restrict__ qt, const float* __restrict__ dd, const float* __restrict__ n_pad,
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) transpose_back_kernel(const float* __rest
         if (d < D && s < S) {
             const long long at = ((long long)p * D + d) * S + s;
             x = src[at];
-            if (qt) { const float q = qt[at]; if (q != 0.0f) x += copysignf(np * __expf(-fabsf(q)), q) * dd[(long long)p * S + s]; }
+            if (qt) { const float q = qt[at], w = np * __expf(-fabsf(q)); x += (q > 0.0f ? w : -w) * dd[(long long)p * S + s]; }
             x *= scale;
             if (keep) x *= keep[(long long)(p / H) * S + s];
         }

@@ -13,7 +13,8 @@ Two routes:
   by two small functions: `sums` returns the unnormalised numerator sum_j A_ij v_j and row sum sum_j A_ij over
   ALL S keys, and `at_origin` returns A(q_i, 0), the weight a key placed at the origin has. Masked keys are moved
   to the origin with a zero value row, so they add nothing to the numerator and exactly `at_origin` each to the
-  row sum, which is subtracted again.
+  row sum, which is subtracted again. Where a query coordinate lies on a kink there, `at_origin` has the operators' derivative
+  (of |q - k| with respect to q: -1 at 0), not torch's, so that the gradients cancel too.
 """
 
 import torch
@@ -33,7 +34,7 @@ def _laplace_sums(q, k, v):
 
 
 def _laplace_at_origin(q):
-    return torch.exp(-q.abs()).sum(dim=1)
+    return torch.exp(torch.where(q > 0, -q, q)).sum(dim=1)
 
 
 # ---- add_riesz: A_ij = |q_i|_1 + |k_j|_1 - |q_i - k_j|_1 + EPS; the two norms are rank-1 terms around the abs sum
@@ -49,7 +50,7 @@ def _riesz_sums(q, k, v):
 
 
 def _riesz_at_origin(q):
-    return torch.full_like(q[:, 0, :], EPS)               # the norms cancel against |q - 0|_1
+    return (q.abs() - torch.where(q > 0, q, -q)).sum(dim=1) + EPS          # the norm cancels against |q - 0|_1; the derivatives differ at 0
 
 
 # ---- add_bump: A_ij = sum_d max(0, 1 - |x|), x = q_id - k_jd, and max(0, 1 - |x|) = (|x + 1| + |x - 1|) / 2 - |x|
@@ -66,7 +67,8 @@ def _bump_sums(q, k, v):
 
 
 def _bump_at_origin(q):
-    return (1.0 - q.abs()).clamp_min(0.0).sum(dim=1)
+    # (the derivative of the three terms: +1 at 0, -1 at 1, 0 at -1; clamp_min hands the gradient on at its bound, relu does not)
+    return torch.where(q > 0, (1.0 - q).clamp_min(0.0), torch.relu(1.0 + q)).sum(dim=1)
 
 
 _ROUTES = {"add_laplace": (_laplace_sums, _laplace_at_origin),

@@ -1,0 +1,70 @@
+"""The sorted route of the attention entry points: layout change, masking, sums, normalisation and the gradients around the walks.
+More features than the pairwise kernels take (128), so that no estimate of times decides which route runs; where a call must not
+depend on the route, 16 features beside them, which run pair by pair at these lengths."""
+
+import pytest
+import torch
+
+from util import rel_err
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = ["add_laplace", "add_riesz", "add_bump"]
+SORTED, PAIRWISE = 130, 16       # features
+
+
+def dense_attention(q, k, v, kernel, tau, keep):
+    """The attention by its definition in float64, differentiable; masked keys are left out."""
+    q, k, v = q.double() / tau, k.double() / tau, v.double()
+    x = (q[..., :, None, :] - k[..., None, :, :]).abs()
+    if kernel == "add_laplace":
+        A = torch.exp(-x).sum(-1)
+    elif kernel == "add_bump":
+        A = (1 - x).clamp_min(0).sum(-1)
+    else:
+        A = q.abs().sum(-1)[..., :, None] + k.abs().sum(-1)[..., None, :] - x.sum(-1) + 1e-3
+    if keep is not None:
+        A = A * keep[:, None, None, :].double()
+    return (A @ v) / A.sum(-1, keepdim=True).clamp_min(1e-6)
+
+
+def two_norm(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+def inputs(B, H, S, D, C, masked, seed):
+    g = torch.Generator().manual_seed(seed)
+    q, k, v = (torch.randn(B, H, S, n, generator=g).cuda() for n in (D, D, C))
+    grad = torch.randn(B, H, S, C, generator=g).cuda()
+    keep = None
+    if masked:
+        keep = (torch.rand(B, S, generator=g) > 0.4).cuda()
+        keep[:, 0] = True
+    return q, k, v, grad, keep
+
+
+def call(q, k, v, grad, kernel, tau, keep, fn=None):
+    """Output and gradients."""
+    if fn is None:
+        from kernel_attention import attention as fn
+    q, k, v = (t.detach().clone().requires_grad_(True) for t in (q, k, v))
+    out = fn(q, k, v, kernel, tau, keep)
+    return (out.detach(), *torch.autograd.grad(out, (q, k, v), grad.to(out.dtype)))
+
+
+@pytest.mark.parametrize("D", [SORTED, PAIRWISE])
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_queries_at_zero_beside_masked_keys(kernel, D):
+    """The sorted route moves masked keys to the origin: what they add where a query's coordinate is 0 (or, for the bump, one
+    width from 0) has to be taken out with the derivative that the walk gave them there."""
+    tau = 0.5
+    q, k, v, grad, keep = inputs(2, 2, 150, D, 16, True, D)
+    q[:, :, ::5, :7] = 0.0
+    q[:, :, 3::5, 2:5] = -0.0
+    q[:, :, 1::5, 3] = tau
+    q[:, :, 2::5, 4] = -tau
+    got = call(q, k, v, grad, kernel, tau, keep)
+    want = call(q, k, v, grad, kernel, tau, keep, dense_attention)
+    assert rel_err(got[0], want[0]) < 1e-4
+    for a, b in zip(got[1:], want[1:]):
+        assert two_norm(a, b) < 2e-4, two_norm(a, b)
