@@ -114,6 +114,7 @@ int qlka_weighted_laplace_sum_backward(const float* q, const float* k, const flo
 /* ---- add_laplace attention on the caller's layout ---------------------------------------
  * out[b,h,i,:] = sum_j A_ij v[b,h,j,:] / max(sum_j A_ij, 1e-6),  A_ij = sum_d exp(-|q[b,h,i,d] - k[b,h,j,d]| / tau),
  * with q, k (B, H, S, D), v and out (B, H, S, Dv) contiguous and keep (B, S) an optional key-keep mask of 0 / 1 floats
+ * (the rows of masked keys may hold anything, NaN included)
  * (NULL: all keys kept). One call does what the reference spreads over attention() and _add_laplace
  * (Experiments/kernel_attention/attention.py:67-72, 95-126) around its operator: the layout change to (P, D, S) fused
  * with the division by tau and the zeroing of masked keys, the Laplace sum accumulated straight into `out`, and the

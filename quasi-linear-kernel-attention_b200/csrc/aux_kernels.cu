@@ -107,8 +107,11 @@ __global__ void unpad_rows_kernel(const float* __restrict__ src, float* __restri
 }
 
 // ---- the caller's side of add_laplace attention (Experiments/kernel_attention/attention.py:67-72, 95-126) ----
+// x under a key mask: what stands in a masked place counts nothing, NaN and infinities too
+__device__ __forceinline__ float weighted(const float x, const float keep) { return keep != 0.0f ? x * keep : 0.0f; }
+
 // dst[p, d, s] = src[p, s, d] * scale * (keep ? keep[p / H, s] : 1): the (B, H, S, D) -> (P, D, S) layout change of
-// attention(), the division by tau and the zeroing of masked keys in one pass; 32 x 32 tiles through shared memory
+// attention(), the division by tau and the zeroing of masked keys (whatever they hold) in one pass; 32 x 32 tiles through shared memory
 __global__ void __launch_bounds__(256) transpose_scale_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                               const float* __restrict__ keep, const float scale,
                                                               const int S, const int D, const int H)
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(256) transpose_scale_kernel(const float* __res
         float x = 0.0f;
         if (s < S && d < D) {
             x = sp[(long long)s * D + d] * scale;
-            if (keep) x *= keep[(long long)(p / H) * S + s];
+            if (keep) x = weighted(x, keep[(long long)(p / H) * S + s]);
         }
         tile[r][tx] = x;
     }
@@ -161,7 +164,7 @@ __global__ void __launch_bounds__(256) transpose_back_kernel(const float* __rest
             x = src[at];
             if (qt) { const float q = qt[at], w = np * __expf(-fabsf(q)); x += (q > 0.0f ? w : -w) * dd[(long long)p * S + s]; }
             x *= scale;
-            if (keep) x *= keep[(long long)(p / H) * S + s];
+            if (keep) x = weighted(x, keep[(long long)(p / H) * S + s]);
         }
         tile[r][tx] = x;
     }
@@ -200,7 +203,7 @@ __global__ void mask_rows_kernel(const float* src, float* dst, const float* __re
     if (i >= total) return;
     const long long ps = i / C;
     const long long p = ps / S, s = ps % S;
-    dst[i] = src[i] * keep[(p / H) * S + s];
+    dst[i] = weighted(src[i], keep[(p / H) * S + s]);
 }
 
 // n_pad[b] = S - sum_s keep[b, s]; one CTA per b

@@ -83,19 +83,22 @@ __global__ void __launch_bounds__(256) dense_stage_gradient(const DenseGradArgs 
     const int  L = keys ? g.N : g.M, tiles = keys ? nt : mt;
     const int  p = tile / tiles, r0 = (tile % tiles) * GT, rows = min(GT, L - r0);
     constexpr int RA = row_arrays<KIND>();
+    // masked keys are staged as zeros, their rows of v too: what stands there reaches no gradient
+    const float* keep = keys && g.keep ? g.keep + (long long)(p / g.H) * L + r0 : nullptr;
+    auto present = [&](const int r) -> bool { return r < rows && (!keep || __ldg(keep + r) != 0.0f); };
 
     // ---- rows of q or k
     const float* src = (keys ? g.k : g.q) + (long long)p * L * D;
     float*       dst = g.staged + (keys ? gv.kr : gv.qr) + (long long)tile * RA * GT * DP;
     if (!g.attention) {                                  // (P, D, L): through shared memory
-        for (int d = sub; d < D; d += 4) tr[row * (D + 1) + d] = row < rows ? __ldg(src + (long long)d * L + r0 + row) : 0.0f;
+        for (int d = sub; d < D; d += 4) tr[row * (D + 1) + d] = present(row) ? __ldg(src + (long long)d * L + r0 + row) : 0.0f;
         __syncthreads();
     }
     int bad = 0;
     for (int i = tid; i < GT * DP; i += 256) {
         const int r = i / DP, d = i % DP;
         float x = 0.0f;
-        if (r < rows && d < D) x = g.attention ? __ldg(src + (long long)(r0 + r) * D + d) * g.scale : tr[r * (D + 1) + d];
+        if (d < D && present(r)) x = g.attention ? __ldg(src + (long long)(r0 + r) * D + d) * g.scale : tr[r * (D + 1) + d];
         dst[i] = x;
         if (KIND == DENSE_LAPLACE) { dst[GT * DP + i] = expf(x); dst[2 * GT * DP + i] = expf(-x); bad |= !(fabsf(x) <= LAP_RANGE); }
     }
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(256) dense_stage_gradient(const DenseGradArgs 
             if (lane == 0) g.staged[gv.s + (long long)tile * GT + r] = r < rows && den >= g.clamp ? -dot : 0.0f;
         }
     } else {
-        for (int i = tid; i < GT * C; i += 256) tr[(i % C) * 65 + i / C] = i / C < rows ? __ldg(w + i) : 0.0f;
+        for (int i = tid; i < GT * C; i += 256) tr[(i % C) * 65 + i / C] = present(i / C) ? __ldg(w + i) : 0.0f;
         if (!keys && tid < GT) g.staged[gv.s + (long long)tile * GT + tid] = g.s && tid < rows ? __ldg(g.s + (long long)p * g.M + r0 + tid) : 0.0f;
     }
     __syncthreads();
@@ -165,7 +168,7 @@ __global__ void __launch_bounds__(G_THREADS, KIND == DENSE_LAPLACE && ND == 2 ? 
         const bool on = tid < GT && x0 + tid < Lx && __ldg(keep + x0 + tid) != 0.0f;
         if (!__syncthreads_or(on)) t1 = t0;
     }
-    auto tile_at = [&](const int t) -> int { return keep && !keys ? list[t] : t; };
+    auto tile_at = [&](const int t) -> int { return keep && !keys ? list[t] >> 1 : t; };
 
     auto copy = [&](float* dst, const float* src, const int n) { for (int i = tid * 4; i < n; i += G_THREADS * 4) cp16(dst + i, src + i); };
     auto issue_yt = [&](const int t) { if (t < t1) copy(yt, yt_g + (long long)tile_at(t) * C4 * GT, C4 * GT); cp_commit(); };

@@ -61,24 +61,25 @@ inline int dense_split(long long ctas, int ntiles, int sms) {
 }
 
 #ifdef __CUDACC__
-// The tiles of 64 keys that hold an unmasked one, in order, into `list` (shared memory, one entry per tile); returns their number.
+// The tiles of 64 keys that hold an unmasked one, in order, into `list` (shared memory, one entry per tile: twice the tile, plus 1 if
+// masked or absent keys are in it too); returns their number.
 // Padding at the end of a sequence costs nothing that way. All threads of the block call it; `keep` has N entries.
 __device__ __forceinline__ int active_tiles(const float* __restrict__ keep, const int N, int* list, int* count) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, tiles = (N + 63) / 64;
     for (int t = warp; t < tiles; t += warps) {
         const int  n = t * 64 + lane;
-        const bool on = (n < N && __ldg(keep + n) != 0.0f) || (n + 32 < N && __ldg(keep + n + 32) != 0.0f);
-        const bool any = __any_sync(0xffffffffu, on);
-        if (lane == 0) list[t] = any;
+        const bool a = n < N && __ldg(keep + n) != 0.0f, b = n + 32 < N && __ldg(keep + n + 32) != 0.0f;
+        const bool any = __any_sync(0xffffffffu, a || b), all = __all_sync(0xffffffffu, a && b);
+        if (lane == 0) list[t] = any ? (all ? 2 : 1) : 0;
     }
     __syncthreads();
     if (warp == 0) {
         int n = 0;
         for (int t0 = 0; t0 < tiles; t0 += 32) {
-            const bool     on = t0 + lane < tiles && list[t0 + lane];
-            const unsigned b  = __ballot_sync(0xffffffffu, on);
+            const int      s = t0 + lane < tiles ? list[t0 + lane] : 0;
+            const unsigned b = __ballot_sync(0xffffffffu, s != 0);
             __syncwarp();
-            if (on) list[n + __popc(b & ((1u << lane) - 1u))] = t0 + lane;      // (never ahead of the entries still to be read)
+            if (s) list[n + __popc(b & ((1u << lane) - 1u))] = 2 * (t0 + lane) + (s == 1);      // (never ahead of the entries still to be read)
             n += __popc(b);
             __syncwarp();
         }

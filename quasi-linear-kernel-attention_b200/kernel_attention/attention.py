@@ -94,7 +94,8 @@ def attention(q, k, v, kernel, tau, keep=None):
     vs = v.reshape(heads, S, v.shape[3])
     if keep is not None:
         kept = keep.to(q.dtype).repeat_interleave(H, dim=0)                       # (P, S)
-        ks, vs = ks * kept.unsqueeze(1), vs * kept.unsqueeze(2)
+        gone = kept == 0                                                          # (whatever stands there: 0 times NaN would be NaN)
+        ks, vs = (ks * kept.unsqueeze(1)).masked_fill(gone.unsqueeze(1), 0.0), (vs * kept.unsqueeze(2)).masked_fill(gone.unsqueeze(2), 0.0)
     num, row = sums(qs, ks.contiguous(), vs.contiguous())
     if keep is not None:
         row = row - (S - kept.sum(dim=1, keepdim=True)) * at_origin(qs)

@@ -68,3 +68,23 @@ def test_queries_at_zero_beside_masked_keys(kernel, D):
     assert rel_err(got[0], want[0]) < 1e-4
     for a, b in zip(got[1:], want[1:]):
         assert two_norm(a, b) < 2e-4, two_norm(a, b)
+
+
+@pytest.mark.parametrize("D", [SORTED, PAIRWISE])
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_masked_values_are_never_looked_at(kernel, D):
+    """Whatever stands in the masked rows of k and v, NaN and infinities too: the results are those of zeros there, and the masked
+    rows get no gradient."""
+    q, k, v, grad, keep = inputs(2, 2, 150, D, 16, True, 7 * D)
+    junk = torch.tensor([float("nan"), float("inf"), -float("inf"), 3e38], device="cuda").repeat(38)[:150]
+    off = ~keep[:, None, :, None]
+    kj = torch.where(off, junk[:, None], k)
+    vj = torch.where(off, junk[:, None].flip(0), v)
+    got = call(q, kj, vj, grad, kernel, 0.5, keep)
+    want = call(q, k.masked_fill(off, 0.0), v.masked_fill(off, 0.0), grad, kernel, 0.5, keep)
+    for a, b in zip(got, want):      # (the same sums, in the order of the atomics)
+        assert two_norm(a, b) < 1e-5, two_norm(a, b)
+    for a in got[2:]:
+        assert a.masked_select(off.expand_as(a)).abs().max().item() == 0.0
+    from kernel_attention import attention
+    assert two_norm(attention(q, kj, vj, kernel, 0.5, keep), want[0]) < 1e-5

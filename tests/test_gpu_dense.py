@@ -26,7 +26,7 @@ def test_operators(shape):
 @pytest.mark.parametrize("kernel", ["add_laplace", "add_riesz", "add_bump"])
 @pytest.mark.parametrize("shape", [(2, 2, 64, 16, 64), (1, 3, 129, 30, 33), (2, 1, 513, 128, 16), (3, 20, 190, 65, 100)])
 def test_attention_masked(kernel, shape):
-    """Padded and scattered masks; a masked key counts nothing even if its values are not finite."""
+    """Scattered masks."""
     from kernel_attention import attention
     B, H, S, D, C = shape
     g = torch.Generator().manual_seed(S)
