@@ -45,7 +45,8 @@ enum qlka_status {
     QLKA_ERR_CUDA = 9,             /* a CUDA runtime call failed; see qlka_last_cuda_error */
     QLKA_ERR_UNSUPPORTED = 10,     /* a size inside the limits that this build has no kernel for */
     QLKA_ERR_NO_ALLOC_LIMIT = 11,  /* problem too large for the fixed scratch of the *_noalloc entry point */
-    QLKA_ERR_ALIGNMENT = 12        /* a row matrix (v, g_w, g, out_w, grad_v, attention out) is not 16-byte aligned */
+    QLKA_ERR_ALIGNMENT = 12,       /* a row matrix (v, g_w, g, out_w, grad_v, attention out) is not 16-byte aligned */
+    QLKA_ERR_GAVE_UP = 13          /* the kernel of an earlier qlka_linear_* call on this device gave up on a barrier wait */
 };
 
 /* Human-readable text of a status code (static storage). */
@@ -212,7 +213,9 @@ int qlka_weighted_sgn_sum_forward(const float* q, const float* k, const float* v
  *                    pairs (i, i + 32), cosines and sines in table (S, 32, 2)
  *   linear_gelu      parts of GELU(A W^T + bias)
  *   linear_residual  x += A W^T + bias
- * linear_error waits for the device and reports whether a kernel of these has ever given up on a barrier (0: none has).
+ * A kernel that gives up on a barrier wait writes NaN where its results belong and sets its device's error word, which is in host
+ * memory: the next linear_* call on the device answers QLKA_ERR_GAVE_UP, launches nothing and clears it. linear_error waits for
+ * the device, reports the word (0: no kernel has given up) and clears it; linear_error_word gives its address, to watch without a call.
  * No counterpart in the reference, which uses torch.nn.Linear. */
 size_t qlka_linear_workspace_bytes(int N, int K);
 int qlka_split_rows(const float* x, const float* ln_weight /* nullable */, const float* ln_bias /* nullable */, float eps, void* parts,
@@ -225,6 +228,7 @@ int qlka_linear_gelu(const void* parts, const float* weight, const float* bias, 
 int qlka_linear_residual(const void* parts, const float* weight, const float* bias, float* x, void* workspace, size_t workspace_bytes,
                          int M, int N, int K, qlka_stream_t stream);
 int qlka_linear_error(int* error);
+int qlka_linear_error_word(volatile int** word);
 
 /* ---- diagnostic: the sort/rank stage alone ---------------------------------------------
  * Sorts x (P, D, N) as the key stream and ranks y (P, D, M) against it, writing the walk

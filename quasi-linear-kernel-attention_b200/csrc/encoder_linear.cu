@@ -16,12 +16,16 @@
 // is what keeps the L2 out of the way: 48 bytes per clock and SM for six products instead of 96 each.
 // Bound by the tensor pipe (and, in long runs, by the power limit): 16384 x 3072 x 768 with GELU 414 us (1120 TFLOP/s of bf16
 // products), torch's fp32 linear on the FP32 pipe 1492 us without the GELU.
+//
+// Every barrier wait has a limit. A CTA that reaches one sets the device's error word, writes NaN to the tiles it has left, waits for
+// its copies and products in flight and ends. The word is in host memory: the next call sees it without waiting for the device.
 #include "qlka_common.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <atomic>
+#include <mutex>
 
 namespace qlka {
 
@@ -45,9 +49,8 @@ struct LinearArgs {
     float *q, *k, *v;            // QKV: (B, H, S, 64), M = B * S rows, N = 3 * H * 64 columns
     const float2* table;         // QKV: (S, 32) cos, sin
     int S, H;
+    int* error;                  // set to 1 by a CTA that gave up on a barrier
 };
-
-__device__ int g_linear_error;   // set by a kernel that gave up on a barrier
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(const uint32_t b, const uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(b), "r"(n) : "memory"); }
@@ -106,10 +109,10 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)STAGES * STAGE_BYTES);       // full[STAGES] empty[STAGES] acc_full small_empty main_empty
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 3);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)STAGES * STAGE_BYTES);       // full[STAGES] empty[STAGES] acc_full small_empty main_empty drained
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t full = smem_addr(bars), empty = full + STAGES * 8, acc_full = empty + STAGES * 8, small_empty = acc_full + 8, main_empty = small_empty + 8;
+    const uint32_t full = smem_addr(bars), empty = full + STAGES * 8, acc_full = empty + STAGES * 8, small_empty = acc_full + 8, main_empty = small_empty + 8, drained = main_empty + 8;
     const int mt = (g.M + BM - 1) / BM, nt = (g.N + BN - 1) / BN, tiles = mt * nt, ksteps = g.K / BK;
 
     if (warp == 0) {
@@ -121,6 +124,7 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
         bar_init(acc_full, 1);
         bar_init(small_empty, EPI_WARPS);
         bar_init(main_empty, EPI_WARPS);
+        bar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -186,6 +190,8 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
                     if ((ks + 1) % KCHUNK_STEPS == 0 || ks + 1 == ksteps) mma_commit(acc_full);
                 }
             }
+            mma_commit(drained);                         // no product is in flight any more when TMEM is handed back
+            ok &= bar_wait(drained, 0);
         }
     } else {                                             // ---- results: warp w has rows 32 (w mod 4) .. + 31 and 128 of the 256 columns
         uint32_t parity = 0;
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
                 for (int j = 0; j < 32; j++) r[c][j] = 0.0f;
             #pragma unroll 1
             for (int ks = 0; ks < ksteps && ok; ks += KCHUNK_STEPS) {
-                if (!(ok = bar_wait(acc_full, parity))) break;
+                if (!(ok = __all_sync(FULL, bar_wait(acc_full, parity)))) break;
                 parity ^= 1;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 #pragma unroll
@@ -216,7 +222,12 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
                     if (lane == 0) bar_arrive(which ? small_empty : main_empty);
                 }
             }
-            if (!ok) break;
+            if (!ok) {                                   // (this tile and all that follow)
+                #pragma unroll
+                for (int c = 0; c < 4; c++)
+                    #pragma unroll
+                    for (int j = 0; j < 32; j++) r[c][j] = __int_as_float(0x7fffffff);
+            }
             const int row = tile / nt * BM + row_in, n0 = tile % nt * BN + col_in;
             if (EPI == EPI_QKV) {
                 // 64 columns are one head of q, k or v; pairs (i, i + 32) turn by the angle of the position
@@ -286,7 +297,10 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
             }
         }
     }
-    if (!ok) g_linear_error = 1;
+    if (!ok) {
+        *reinterpret_cast<volatile int*>(g.error) = 1;
+        __threadfence_system();
+    }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -370,7 +384,39 @@ cudaError_t launch_split_heads(const float* o, void* out, int B, int H, int S, i
     return cudaGetLastError();
 }
 
-cudaError_t read_linear_error(int* error) { return cudaMemcpyFromSymbol(error, g_linear_error, sizeof(int)); }
+// The current device's error word, in pinned host memory that kernels can write to: allocated at the first use, one word per device,
+// for as long as the process runs.
+cudaError_t linear_error_word(int** host, int** device) {
+    constexpr int MAX_DEV = 64;
+    static std::mutex        lock;
+    static std::atomic<int*> words;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= MAX_DEV) return cudaErrorInvalidDevice;
+    int* base = words.load(std::memory_order_acquire);
+    if (!base) {
+        std::lock_guard<std::mutex> hold(lock);
+        base = words.load(std::memory_order_relaxed);
+        if (!base) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;        // (the first call may be under capture: this allocation is not part of it)
+            e = cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return e;
+            void* p = nullptr;
+            e = cudaHostAlloc(&p, MAX_DEV * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return e;
+            base = static_cast<int*>(p);
+            for (int i = 0; i < MAX_DEV; i++) base[i] = 0;
+            words.store(base, std::memory_order_release);
+        }
+    }
+    *host = base + dev;
+    void* d = nullptr;
+    e = cudaHostGetDevicePointer(&d, base, 0);
+    *device = static_cast<int*>(d) + dev;
+    return e;
+}
 
 // (3, rows, K) bf16 parts, boxes of `box_rows` rows x 32 columns x 3 parts with the 64-byte swizzle
 static cudaError_t make_map(CUtensorMap* map, const void* base, long long rows, int K, int box_rows) {
@@ -393,9 +439,11 @@ static cudaError_t make_map(CUtensorMap* map, const void* base, long long rows, 
 }
 
 template <int EPI>
-static cudaError_t launch_linear(const LinearArgs& g, const void* a3, const void* w3, int sms, cudaStream_t st) {
+static cudaError_t launch_linear(LinearArgs g, const void* a3, const void* w3, int sms, cudaStream_t st) {
     CUtensorMap ma, mb;
-    cudaError_t e = make_map(&ma, a3, g.M, g.K, BM);
+    int* word;
+    cudaError_t e = linear_error_word(&word, &g.error);
+    if (e == cudaSuccess) e = make_map(&ma, a3, g.M, g.K, BM);
     if (e == cudaSuccess) e = make_map(&mb, w3, g.N, g.K, BN);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(linear_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_SMEM);

@@ -24,7 +24,7 @@ cudaError_t launch_linear_qkv(const void* a3, const void* w3, const float* bias,
                               int B, int S, int H, int K, int sms, cudaStream_t st);
 cudaError_t launch_linear_gelu(const void* a3, const void* w3, const float* bias, void* out3, int M, int N, int K, int sms, cudaStream_t st);
 cudaError_t launch_linear_residual(const void* a3, const void* w3, const float* bias, float* x, int M, int N, int K, int sms, cudaStream_t st);
-cudaError_t read_linear_error(int* error);
+cudaError_t linear_error_word(int** host, int** device);
 cudaError_t launch_colsum_d(const float* x, float* out, int P, int D, int L, cudaStream_t st);
 cudaError_t launch_rowstat(const float* w, const float* s, float* wsum, float* swsum, float* ssum, int P, int R, int C4, cudaStream_t st);
 cudaError_t launch_vecsum(const float* x, float* out, int P, int L, cudaStream_t st);
@@ -447,6 +447,7 @@ const char* qlka_status_string(int status) {
         case QLKA_ERR_UNSUPPORTED:       return "no kernel in this build for these sizes (shifted abs sum: N and n_shifts * M must be <= 16384)";
         case QLKA_ERR_NO_ALLOC_LIMIT:    return "problem needs more scratch than the fixed 32 MiB of the no-allocation entry point; use the workspace variant";
         case QLKA_ERR_ALIGNMENT:         return "v, g_w, g, out_w, grad_v and the attention output must be 16-byte aligned";
+        case QLKA_ERR_GAVE_UP:           return "an earlier linear layer gave up on a barrier wait: what it wrote is NaN";
         default:                         return "unknown status";
     }
 }
@@ -1126,6 +1127,9 @@ static int linear_begin(const void* parts, const float* weight, const float* bia
     if (K % 32 || N % 32) return QLKA_ERR_UNSUPPORTED;
     if (!aligned16(parts, weight, bias)) return QLKA_ERR_ALIGNMENT;
     if (!ws_ok(workspace, workspace_bytes, qlka_linear_workspace_bytes(N, K))) return QLKA_ERR_WORKSPACE;
+    volatile int* word = nullptr;
+    if (int st = qlka_linear_error_word(&word)) return st;
+    if (*word) { *word = 0; return QLKA_ERR_GAVE_UP; }        // an earlier call's kernel: reported once
     CU(launch_split_rows(weight, nullptr, nullptr, workspace, N, K, 0.0f, stream));
     return QLKA_OK;
 }
@@ -1165,9 +1169,22 @@ int qlka_linear_residual(const void* parts, const float* weight, const float* bi
     return QLKA_OK;
 }
 
+int qlka_linear_error_word(volatile int** word) {
+    if (!word) return QLKA_ERR_NULL;
+    int *host = nullptr, *device = nullptr;
+    CU(linear_error_word(&host, &device));
+    *word = host;
+    return QLKA_OK;
+}
+
 int qlka_linear_error(int* error) {
     if (!error) return QLKA_ERR_NULL;
-    CU(read_linear_error(error));
+    CU(cudaDeviceSynchronize());
+    volatile int* word = nullptr;
+    int st = qlka_linear_error_word(&word);
+    if (st) return st;
+    *error = *word;
+    *word = 0;
     return QLKA_OK;
 }
 

@@ -46,3 +46,24 @@ def test_qkv_rotary_layout():
     q, k, v = F.linear(parts.double().sum(0).float(), w, b).view(B, S, 3, H, 64).permute(2, 0, 3, 1, 4)
     for a, want in zip(got, (rotary(q), rotary(k), v)):
         assert two_norm(a, want.double()) < 1e-6
+
+
+def test_a_kernel_that_gave_up_is_reported():
+    """The error word as a kernel would leave it (no kernel is made to give up): the next layer raises, once."""
+    import ctypes
+    import qlka_native
+    from kernel_attention.encoder import Encoder
+    word = ctypes.POINTER(ctypes.c_int)()
+    assert qlka_native.lib().qlka_linear_error_word(ctypes.byref(word)) == 0
+    model = Encoder("add_laplace", layers=1, hidden=128, heads=2, mlp=256, vocab=100).cuda().eval()
+    ids = torch.randint(0, 100, (1, 40), device="cuda")
+    want = model(ids)
+    torch.cuda.synchronize()
+    assert word[0] == 0
+    word[0] = 1
+    with pytest.raises(RuntimeError, match="gave up"):
+        model(ids)
+    assert word[0] == 0
+    word[0] = 1
+    assert qlka_native.ext().linear_error() == 1 and qlka_native.ext().linear_error() == 0
+    assert torch.equal(model(ids), want)
