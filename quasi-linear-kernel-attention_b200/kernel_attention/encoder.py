@@ -37,6 +37,19 @@ def rotary(x, base=10000.0):
     return torch.cat([x1 * cos - x2 * sin, x1 * sin + x2 * cos], dim=-1)
 
 
+def _calls_are_plain():
+    """Whether calling a module does nothing but compute its fp32 output right now: nothing traces, transforms, watches or casts."""
+    hooks = torch.nn.modules.module
+    return not (torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack()
+                or torch._C._functorch.maybe_current_level() is not None or hooks._global_forward_hooks or hooks._global_forward_pre_hooks)
+
+
+def _is_plain(module, kind):
+    """Whether a call of `module` is `kind.forward` and nothing else (no subclass, parametrisation, hook or override)."""
+    return (type(module) is kind and not module._forward_hooks and not module._forward_pre_hooks and module._compiled_call_impl is None
+            and "forward" not in module.__dict__)
+
+
 class Block(nn.Module):
     def __init__(self, hidden, heads, mlp, kernel, tau):
         super().__init__()
@@ -62,12 +75,22 @@ class Block(nn.Module):
         return x + self.fc2(F.gelu(self.fc1(self.ln2(x))))
 
     def fits_native(self, x):
-        """Whether `forward_native` takes this block: fp32 on CUDA, heads of 64, sizes in steps of 32, parameters as torch allocates
-        them - and full fp32 products wanted (a caller who allows TF32 gets torch's TF32 products)."""
-        hidden = x.shape[-1]
-        return (x.is_cuda and x.dtype == torch.float32 and x.numel() > 0 and hidden == self.heads * 64 and self.fc1.out_features % 32 == 0
-                and not torch.backends.cuda.matmul.allow_tf32
-                and all(p.dtype == torch.float32 and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0 for p in self.parameters()))
+        """Whether `forward_native` computes what a call of this block does: fp32 on CUDA, heads of 64, sizes in steps of 32, layer norms and
+        linear layers as torch has them, with their biases, and full fp32 products wanted (a caller who allows TF32 gets torch's)."""
+        if not (type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and x.numel() > 0 and _is_plain(self, Block) and "attend" not in self.__dict__
+                and torch.backends.cuda.matmul.fp32_precision in ("ieee", "none")):
+            return False
+        hidden, mlp = x.shape[-1], getattr(self.fc1, "out_features", 0)
+        if hidden != self.heads * 64 or mlp % 32:
+            return False
+        for m, kind, shape in ((self.ln1, nn.LayerNorm, (hidden,)), (self.ln2, nn.LayerNorm, (hidden,)), (self.qkv, nn.Linear, (3 * hidden, hidden)),
+                               (self.proj, nn.Linear, (hidden, hidden)), (self.fc1, nn.Linear, (mlp, hidden)), (self.fc2, nn.Linear, (hidden, mlp))):
+            if not _is_plain(m, kind) or m.weight is None or m.bias is None or m.weight.shape != shape or m.bias.shape != shape[:1]:
+                return False
+            for p in (m.weight, m.bias):
+                if type(p) not in (nn.Parameter, torch.Tensor) or p.dtype != torch.float32 or p.device != x.device or not p.is_contiguous() or p.data_ptr() % 16:
+                    return False
+        return True
 
     def forward_native(self, x, table, keep=None):
         """The block on x (B, S, hidden) in place, without autograd: layer norms, linear layers with their bias, rotary, GELU and
@@ -101,14 +124,15 @@ class Encoder(nn.Module):
     @torch.no_grad()
     def forward(self, ids, keep=None):
         x = self.embed(ids)
-        table = None
+        plain, table = _calls_are_plain(), None
+        own = _is_plain(self.embed, nn.Embedding)        # nobody else holds x: the native block may write to it
         for blk in self.blocks:
-            if blk.fits_native(x):
+            if plain and isinstance(blk, Block) and blk.fits_native(x):
                 if table is None:
                     table = torch.stack(rotary_angles(x.shape[1], 32, x.device), dim=-1).contiguous()
-                x = blk.forward_native(x, table, keep)
+                x, own = blk.forward_native(x if own else x.clone(memory_format=torch.contiguous_format), table, keep), True
             else:
-                x = blk(x, keep)
+                x, own = blk(x, keep), False
         return self.ln(x)
 
 
