@@ -397,20 +397,23 @@ int linear_error() {
 
 }  // namespace
 
+// Every call that enqueues work lets go of Python's lock: a launch can wait for room in its stream's queue, and other threads drive
+// other streams and GPUs.
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    using Unlocked = py::call_guard<py::gil_scoped_release>;
     m.def("load", &load);
-    m.def("laplace_forward", &laplace_forward);
-    m.def("laplace_backward", &laplace_backward, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("g_w"), py::arg("g_u") = py::none());
-    m.def("laplace_sum", &laplace_sum);
-    m.def("abs_forward", &abs_forward);
-    m.def("abs_backward", &abs_backward, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("g_w"), py::arg("g_u") = py::none());
-    m.def("abs_sum", &abs_sum);
-    m.def("sgn_forward", &sgn_forward);
-    m.def("attention", &attention);
-    m.def("split_rows", &split_rows);
-    m.def("split_heads", &split_heads);
-    m.def("linear_qkv", &linear_qkv);
-    m.def("linear_gelu", &linear_gelu);
-    m.def("linear_residual", &linear_residual);
-    m.def("linear_error", &linear_error);
+    m.def("laplace_forward", &laplace_forward, Unlocked());
+    m.def("laplace_backward", &laplace_backward, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("g_w"), py::arg("g_u") = py::none(), Unlocked());
+    m.def("laplace_sum", &laplace_sum, Unlocked());
+    m.def("abs_forward", &abs_forward, Unlocked());
+    m.def("abs_backward", &abs_backward, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("g_w"), py::arg("g_u") = py::none(), Unlocked());
+    m.def("abs_sum", &abs_sum, Unlocked());
+    m.def("sgn_forward", &sgn_forward, Unlocked());
+    m.def("attention", &attention, Unlocked());
+    m.def("split_rows", &split_rows, Unlocked());
+    m.def("split_heads", &split_heads, Unlocked());
+    m.def("linear_qkv", &linear_qkv, Unlocked());
+    m.def("linear_gelu", &linear_gelu, Unlocked());
+    m.def("linear_residual", &linear_residual, Unlocked());
+    m.def("linear_error", &linear_error, Unlocked());
 }
