@@ -281,6 +281,14 @@ Tensor attention_forward(const int64_t kind, const Tensor& q, const Tensor& k, c
     return out;
 }
 
+// The output's version when the forward pass ended, without its memory.
+struct OutputVersion : torch::CustomClassHolder {
+    c10::VariableVersion counter;
+    const uint32_t       at;
+    explicit OutputVersion(const Tensor& out) : counter(out.unsafeGetTensorImpl()->version_counter()), at(counter.current_version()) {}
+    bool changed() const { return counter.current_version() != at; }
+};
+
 class Attention : public torch::autograd::Function<Attention> {
 public:
     static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& mask, const int64_t kind, const double tau) {
@@ -288,7 +296,10 @@ public:
         const AttnDims d{(int)q.size(0), (int)q.size(1), (int)q.size(2), (int)q.size(3), (int)v.size(3)};
         Tensor den;
         Tensor out = attention_forward(kind, q, k, v, keep, tau, d, &den);
-        ctx->save_for_backward({q, k, v, keep, out, den});
+        // The gradient needs the output, but a caller may change it in place, as after any division. So it is saved with a version of
+        // its own, which no such change fails on, and computed again by the backward pass if there was one.
+        ctx->save_for_backward({q, k, v, keep, out.variable_data(), den});
+        ctx->saved_data["out"]  = c10::IValue::make_capsule(c10::make_intrusive<OutputVersion>(out));
         ctx->saved_data["kind"] = kind;
         ctx->saved_data["tau"]  = tau;
         return out;
@@ -300,9 +311,12 @@ public:
         const AttnDims d{(int)q.size(0), (int)q.size(1), (int)q.size(2), (int)q.size(3), (int)v.size(3)};
         const c10::cuda::CUDAGuard guard(q.device());
         const Tensor grad = aligned(g[0].contiguous());
+        const double tau = ctx->saved_data["tau"].toDouble();
+        const bool   changed = static_cast<const OutputVersion*>(ctx->saved_data["out"].toCapsule().get())->changed();
+        const Tensor out = changed ? attention_forward(kind, q, k, v, keep, tau, d, nullptr) : s[4];
         const Workspace ws = workspace(q, api.qlka_attention_backward_workspace_bytes, kind, d.B, d.H, d.S, d.D, d.C, (int)keep.defined());
         Tensor gq = floats(q.sizes(), q), gk = floats(k.sizes(), q), gv = floats(v.sizes(), q);
-        check_status(api.qlka_attention_backward(kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)ctx->saved_data["tau"].toDouble(), ptr(s[4]), ptr(s[5]), ptr(grad),
+        check_status(api.qlka_attention_backward(kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, ptr(out), ptr(s[5]), ptr(grad),
                                                  out_ptr(gq), out_ptr(gk), out_ptr(gv), ws.ptr(), ws.bytes, d.B, d.H, d.S, d.D, d.C, current_stream()));
         return {gq, gk, gv, Tensor(), Tensor(), Tensor()};
     }
