@@ -260,6 +260,7 @@ struct AttnDims { int B, H, S, D, C; };
 
 AttnDims check_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& keep) {
     TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda(), "q, k, and v must be CUDA tensors");
+    TORCH_CHECK(q.device() == k.device() && q.device() == v.device(), "q, k, and v must be on one device");
     TORCH_CHECK(q.scalar_type() == at::kFloat && k.scalar_type() == at::kFloat && v.scalar_type() == at::kFloat, "q, k, and v must be float32");
     TORCH_CHECK(q.dim() == 4 && k.sizes() == q.sizes() && v.dim() == 4 && v.sizes().slice(0, 3) == q.sizes().slice(0, 3),
                 "expected q, k (B, H, S, D) and v (B, H, S, Dv)");
@@ -306,17 +307,22 @@ public:
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list g) {
         const auto s = ctx->get_saved_variables();
-        const Tensor &q = s[0], &k = s[1], &v = s[2], &keep = s[3];
+        // (hooks on saved tensors may hand back other tensors: any strides, any place)
         const int kind = (int)ctx->saved_data["kind"].toInt();
-        const AttnDims d{(int)q.size(0), (int)q.size(1), (int)q.size(2), (int)q.size(3), (int)v.size(3)};
-        const c10::cuda::CUDAGuard guard(q.device());
+        const AttnDims d = check_attention(s[0], s[1], s[2], s[3].defined() ? std::optional<Tensor>(s[3]) : std::nullopt);
+        const c10::cuda::CUDAGuard guard(s[0].device());
+        const Tensor q = s[0].contiguous(), k = s[1].contiguous(), v = aligned(s[2].contiguous()), keep = s[3].defined() ? s[3].contiguous() : s[3];
+        const Tensor saved_out = aligned(s[4].contiguous()), den = s[5].contiguous();
+        if (keep.defined()) check_like(keep, "keep", {d.B, d.S}, q);
+        check_like(saved_out, "the saved output", {d.B, d.H, d.S, d.C}, q);
+        check_like(den, "the saved row sums", {d.B, d.H, d.S}, q);
         const Tensor grad = aligned(g[0].contiguous());
         const double tau = ctx->saved_data["tau"].toDouble();
         const bool   changed = static_cast<const OutputVersion*>(ctx->saved_data["out"].toCapsule().get())->changed();
-        const Tensor out = changed ? attention_forward(kind, q, k, v, keep, tau, d, nullptr) : s[4];
+        const Tensor out = changed ? attention_forward(kind, q, k, v, keep, tau, d, nullptr) : saved_out;
         const Workspace ws = workspace(q, api.qlka_attention_backward_workspace_bytes, kind, d.B, d.H, d.S, d.D, d.C, (int)keep.defined());
         Tensor gq = floats(q.sizes(), q), gk = floats(k.sizes(), q), gv = floats(v.sizes(), q);
-        check_status(api.qlka_attention_backward(kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, ptr(out), ptr(s[5]), ptr(grad),
+        check_status(api.qlka_attention_backward(kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, ptr(out), ptr(den), ptr(grad),
                                                  out_ptr(gq), out_ptr(gk), out_ptr(gv), ws.ptr(), ws.bytes, d.B, d.H, d.S, d.D, d.C, current_stream()));
         return {gq, gk, gv, Tensor(), Tensor(), Tensor()};
     }
@@ -339,18 +345,18 @@ std::optional<Tensor> attention(const int64_t kind, const Tensor& q_, const Tens
 }
 
 // ------------------------------------------------------------------ linear layers of the encoder (inference)
-const Tensor& check_matrix(const Tensor& t, const char* name, const at::IntArrayRef shape) {
-    TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.sizes() == shape, name, " must be a contiguous float32 CUDA tensor of shape ", shape);
-    return t;
+void check_matrix(const Tensor& t, const char* name, const at::IntArrayRef shape, const Tensor& like) {
+    TORCH_CHECK(t.is_cuda() && t.device() == like.device() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.sizes() == shape,
+                name, " must be a contiguous float32 CUDA tensor of shape ", shape, " on the input's device");
 }
 
 Tensor parts_of(const int64_t rows, const int64_t K, const Tensor& like) { return at::detail::empty_cuda({3, rows, K}, at::kBFloat16, like.device(), std::nullopt); }
 
 Tensor split_rows(const Tensor& x, const Tensor& ln_weight, const Tensor& ln_bias, const double eps) {
     const int64_t rows = x.size(0), K = x.size(1);
-    check_matrix(x, "x", {rows, K});
-    check_matrix(ln_weight, "ln_weight", {K});
-    check_matrix(ln_bias, "ln_bias", {K});
+    check_matrix(x, "x", {rows, K}, x);
+    check_matrix(ln_weight, "ln_weight", {K}, x);
+    check_matrix(ln_bias, "ln_bias", {K}, x);
     const c10::cuda::CUDAGuard guard(x.device());
     Tensor parts = parts_of(rows, K, x);
     check_status(api.qlka_split_rows(ptr(x), ptr(ln_weight), ptr(ln_bias), (float)eps, parts.mutable_data_ptr(), (int)rows, (int)K, current_stream()));
@@ -359,7 +365,7 @@ Tensor split_rows(const Tensor& x, const Tensor& ln_weight, const Tensor& ln_bia
 
 Tensor split_heads(const Tensor& o) {
     const int64_t B = o.size(0), H = o.size(1), S = o.size(2), D = o.size(3);
-    check_matrix(o, "o", {B, H, S, D});
+    check_matrix(o, "o", {B, H, S, D}, o);
     const c10::cuda::CUDAGuard guard(o.device());
     Tensor parts = parts_of(B * S, H * D, o);
     check_status(api.qlka_split_heads(ptr(o), parts.mutable_data_ptr(), (int)B, (int)H, (int)S, (int)D, current_stream()));
@@ -370,8 +376,8 @@ struct Layer { int M, N, K; Tensor ws; size_t bytes; };
 Layer layer(const Tensor& parts, const Tensor& weight, const Tensor& bias) {
     TORCH_CHECK(parts.is_cuda() && parts.scalar_type() == at::kBFloat16 && parts.is_contiguous() && parts.dim() == 3 && parts.size(0) == 3, "parts must come from split_rows or split_heads");
     const int64_t M = parts.size(1), K = parts.size(2), N = weight.size(0);
-    check_matrix(weight, "weight", {N, K});
-    check_matrix(bias, "bias", {N});
+    check_matrix(weight, "weight", {N, K}, parts);
+    check_matrix(bias, "bias", {N}, parts);
     Layer l{(int)M, (int)N, (int)K, Tensor(), api.qlka_linear_workspace_bytes((int)N, (int)K)};
     l.ws = at::detail::empty_cuda({(int64_t)l.bytes}, at::kByte, parts.device(), std::nullopt);
     return l;
@@ -381,7 +387,7 @@ std::tuple<Tensor, Tensor, Tensor> linear_qkv(const Tensor& parts, const Tensor&
     const c10::cuda::CUDAGuard guard(parts.device());
     const Layer l = layer(parts, weight, bias);
     TORCH_CHECK(l.M == B * S && l.N == 3 * H * 64, "expected B * S rows and 3 * H * 64 columns");
-    check_matrix(table, "table", {S, 32, 2});
+    check_matrix(table, "table", {S, 32, 2}, parts);
     Tensor q = floats({B, H, S, 64}, parts), k = floats({B, H, S, 64}, parts), v = floats({B, H, S, 64}, parts);
     check_status(api.qlka_linear_qkv(parts.const_data_ptr(), ptr(weight), ptr(bias), ptr(table), out_ptr(q), out_ptr(k), out_ptr(v),
                                      l.ws.mutable_data_ptr(), l.bytes, (int)B, (int)S, (int)H, l.K, current_stream()));
@@ -399,7 +405,7 @@ Tensor linear_gelu(const Tensor& parts, const Tensor& weight, const Tensor& bias
 void linear_residual(const Tensor& parts, const Tensor& weight, const Tensor& bias, const Tensor& x) {
     const c10::cuda::CUDAGuard guard(parts.device());
     const Layer l = layer(parts, weight, bias);
-    check_matrix(x, "x", {l.M, l.N});
+    check_matrix(x, "x", {l.M, l.N}, parts);
     check_status(api.qlka_linear_residual(parts.const_data_ptr(), ptr(weight), ptr(bias), out_ptr(x), l.ws.mutable_data_ptr(), l.bytes, l.M, l.N, l.K, current_stream()));
 }
 

@@ -57,3 +57,25 @@ def test_backward_twice_and_no_reference_cycle():
         assert gone() is None and torch.cuda.memory_allocated() <= before - size
     finally:
         gc.enable()
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_saved_tensor_hooks_that_hand_back_other_layouts(kernel):
+    from kernel_attention import attention
+    q, k, v, up = inputs(PAIRWISE)
+    keep = (torch.arange(100, device="cuda")[None] < torch.tensor([[100], [60]], device="cuda"))
+    want = torch.autograd.grad(attention(q, k, v, kernel, 0.5, keep), (q, k, v), up)
+
+    def unpack(t):      # the same values, every other element of a new tensor, off its 16-byte boundary
+        store = torch.full((2 * t.numel() + 1,), float("nan"), device="cuda")
+        return store[1:].view(*t.shape[:-1], 2 * t.shape[-1])[..., ::2].copy_(t)
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().cpu(), unpack):
+        out = attention(q, k, v, kernel, 0.5, keep)
+    out.mul_(1.0)
+    for a, b in zip(torch.autograd.grad(out, (q, k, v), up), want):
+        assert two_norm(a, b) < 1e-5
+    from torch.utils.checkpoint import checkpoint
+    out = checkpoint(lambda *x: attention(*x, kernel, 0.5, keep), q, k, v, use_reentrant=False)
+    for a, b in zip(torch.autograd.grad(out, (q, k, v), up), want):
+        assert two_norm(a, b) < 1e-5
