@@ -8,7 +8,8 @@ the reference's own file also runs unchanged on top of the two operator packages
 Two routes:
 * one native call forward and, where gradients are wanted, one backward (`qlka_native.attention`): layout change, tau,
   masking, the sums and the normalisation all happen inside the library;
-* the cases without such a call (gradients of add_riesz and add_bump at long lengths, add_bump beyond 5461 keys) - the sums are
+* the cases without such a call (gradients of add_riesz and add_bump at long lengths, add_bump beyond 5461 keys, training with a
+  temperature that is a tensor to broadcast or to train, or that is not above 0, or with a mask that wants a gradient) - the sums are
   assembled here from the differentiable operators. Every kernel is described
   by two small functions: `sums` returns the unnormalised numerator sum_j A_ij v_j and row sum sum_j A_ij over
   ALL S keys, and `at_origin` returns A(q_i, 0), the weight a key placed at the origin has. Masked keys are moved
@@ -76,13 +77,22 @@ _ROUTES = {"add_laplace": (_laplace_sums, _laplace_at_origin),
            "add_bump": (_bump_sums, _bump_at_origin)}
 
 
+def _needs_operators(q, k, v, tau, keep):
+    """Whether a call asks for gradients that the native backward pass does not give, or for a temperature it does not take."""
+    by_tensor = isinstance(tau, torch.Tensor)
+    trained = (by_tensor and tau.requires_grad) or (keep is not None and keep.requires_grad)
+    if not (trained or q.requires_grad or k.requires_grad or v.requires_grad) or not torch.is_grad_enabled():
+        return False
+    return trained or (by_tensor and tau.numel() != 1) or not tau > 0
+
+
 def attention(q, k, v, kernel, tau, keep=None):
     """q, k (B, H, S, D), v (B, H, S, Dv) fp32 CUDA; keep (B, S) bool/float key-keep mask or None -> (B, H, S, Dv)."""
     assert q.dtype == k.dtype == v.dtype == torch.float32, "kernel attention runs in fp32 only"
     if kernel not in _ROUTES:
         raise ValueError(f"kernel must be one of {tuple(_ROUTES)}, got {kernel!r}")
     B, H, S, D = q.shape
-    if kernel != "add_bump" or 3 * S <= 16384:      # the fused add_bump shares one shared-memory sort between its three shifts
+    if (kernel != "add_bump" or 3 * S <= 16384) and not _needs_operators(q, k, v, tau, keep):      # the fused add_bump shares one shared-memory sort between its three shifts
         out = _native.attention(kernel, q, k, v, tau, keep)
         if out is not None:
             return out

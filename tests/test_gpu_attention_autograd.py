@@ -79,3 +79,32 @@ def test_saved_tensor_hooks_that_hand_back_other_layouts(kernel):
     out = checkpoint(lambda *x: attention(*x, kernel, 0.5, keep), q, k, v, use_reentrant=False)
     for a, b in zip(torch.autograd.grad(out, (q, k, v), up), want):
         assert two_norm(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("tau", ["per head", "trained", "negative", "one element"])
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_temperatures(kernel, tau):
+    from kernel_attention import attention
+    q, k, v, up = inputs(PAIRWISE, S=60)
+    tau = {"per head": torch.tensor([0.5, 0.8], device="cuda").view(1, 2, 1, 1), "trained": torch.tensor(0.7, device="cuda", requires_grad=True),
+           "negative": -0.5, "one element": torch.tensor([0.6], device="cuda")}[tau]
+    wrt = (q, k, v, tau) if isinstance(tau, torch.Tensor) and tau.requires_grad else (q, k, v)
+    out, ref = attention(q, k, v, kernel, tau), dense_attention(q, k, v, kernel, tau, None)
+    assert two_norm(out, ref) < 1e-5
+    got, want = torch.autograd.grad(out, wrt, up), torch.autograd.grad(ref, wrt, up.double())
+    for a, b in zip(got[:3], want[:3]):
+        assert two_norm(a, b) < 2e-4
+    if len(wrt) == 4:       # -(<grad_q, q> + <grad_k, k>) / tau, where the terms nearly cancel (add_riesz depends on tau through EPS only)
+        bound = 2e-4 * sum((g.norm() * x.norm()).item() for g, x in zip(want[:2], (q, k))) / tau.item()
+        assert (got[3] - want[3]).abs().item() < bound
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_mask_that_wants_a_gradient(kernel):
+    """A 0 / 1 mask of floats: kept keys get one, in the operators' sense."""
+    from kernel_attention import attention
+    q, k, v, up = inputs(PAIRWISE, S=60)
+    keep = (torch.arange(60, device="cuda")[None] < torch.tensor([[60], [40]], device="cuda")).float().requires_grad_(True)
+    out = attention(q, k, v, kernel, 0.5, keep)
+    assert two_norm(out, dense_attention(q, k, v, kernel, 0.5, keep)) < 1e-5
+    assert torch.autograd.grad(out, keep, up)[0].abs().max().item() > 0
