@@ -236,8 +236,10 @@ public:
     }
 };
 
+// Whether a call has to go through its autograd node. Forward-mode tangents do too: the nodes have no rule for them and say so.
 bool wants_grad(const Tensor& q, const Tensor& k, const Tensor& v) {
-    return at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
+    auto dual = [](const Tensor& t) { return t._fw_grad(/*level=*/0).defined(); };
+    return (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) || dual(q) || dual(k) || dual(v);
 }
 
 std::tuple<Tensor, Tensor> laplace_sum(const Tensor& q, const Tensor& k, const Tensor& v) {

@@ -108,3 +108,25 @@ def test_mask_that_wants_a_gradient(kernel):
     out = attention(q, k, v, kernel, 0.5, keep)
     assert two_norm(out, dense_attention(q, k, v, kernel, 0.5, keep)) < 1e-5
     assert torch.autograd.grad(out, keep, up)[0].abs().max().item() > 0
+
+
+def test_transforms_without_a_rule_are_refused():
+    """Forward-mode derivatives, vmap and the functional transforms: an error, not a result without the derivative."""
+    import torch.autograd.forward_ad as forward_ad
+    from kernel_attention import attention
+    from weighted_abs_sum import weighted_abs_sum, weighted_abs_sum_full
+    from weighted_laplace_sum import weighted_laplace_sum
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, v, x = (torch.randn(*s, generator=g, device="cuda") for s in ((1, 2, 64), (1, 64, 4), (1, 2, 64, 4)))
+    ops = [(f, (q, q + 1, v)) for f in (weighted_abs_sum, weighted_abs_sum_full, weighted_laplace_sum)]
+    ops += [(lambda a, b, c, kernel=kernel: attention(a, b, c, kernel, 0.5), (x, x + 1, x)) for kernel in KERNELS]
+    for f, args in ops:
+        for grad_mode in (True, False):
+            with torch.set_grad_enabled(grad_mode), forward_ad.dual_level(), pytest.raises(RuntimeError, match="jvp"):
+                f(forward_ad.make_dual(args[0], torch.ones_like(args[0])), *args[1:])
+        with pytest.raises(Exception):
+            torch.func.vmap(f)(*(a[None] for a in args))
+        with pytest.raises(Exception):
+            torch.func.jvp(lambda a: f(a, *args[1:]), (args[0],), (args[0],))
+        with pytest.raises(Exception):
+            torch.func.grad(lambda a: sum(t.sum() for t in f(a, *args[1:])))(args[0])
