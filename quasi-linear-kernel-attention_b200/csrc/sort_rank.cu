@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
             for (int t = 0; t < QI; t++) rp[s0 + t] = (uint32_t)lo[t];       // number of keys strictly below the query
         }
     };
-    // More queries than the kernel holds (only a part can have them: values far denser there than the keys): a first sweep
+    // More queries than the kernel holds (only a part can have them: far more of them between two keys than elsewhere): a first sweep
     // counts them, a second ranks them again and writes side channel and records one by one.
     auto count_ranks = [&](const int c0) {
         #pragma unroll

@@ -8,7 +8,8 @@
 //   count_bins        per tile of 4096 keys or queries: the bin of every element (binary search over the splitters), kept as
 //                     a byte; counts per bin. A query's bin is chosen so that every key below it lies in its own bin or an
 //                     earlier one and every key of a later bin is not below it.
-//   merge_bins        per segment: consecutive bins are merged into parts while they stay within PART_CAP keys; starts.
+//   merge_bins        per segment: consecutive bins are merged into parts while they stay within PART_CAP keys (and as many queries,
+//                     where there are more queries than keys); starts.
 //   scatter_parts     per tile: elements to their parts, through shared memory so that the lists are written in runs.
 //   part_stats        per part: smallest and largest key and the part's own scalar sums; the last CTA of a segment chains them
 //                     into what enters each part from below and from above.
@@ -32,9 +33,20 @@ namespace {
 constexpr int MAX_BINS = 256, SAMPLES_PER_BIN = 8;
 constexpr int TILE = 4096, TILE_THREADS = 256, TILE_E = TILE / TILE_THREADS;
 
-__host__ __device__ inline int bins_of(int N)  { int b = 32; while (b < MAX_BINS && b * 512 < N) b *= 2; return b; }
-__host__ __device__ inline int max_parts(int N) { return 2 * (N / PART_CAP) + 2; }        // two neighbouring parts hold more than PART_CAP keys
-constexpr int MAX_PARTS = 2 * (262144 / PART_CAP) + 2;
+// With more queries than keys, parts are cut by their queries as well, and the bins are made finer as far as there are samples: a part is
+// one CTA's, and one that has more than PART_CAP queries ranks them twice, with a scattered record per thread and turn. Laplace sums
+// with and without (ms): 1 head x 64 features, 8192 keys, 262144 queries 1.59 / 2.88; 16 heads, 8192 x 65536, 5.5 / 6.4; 130 features,
+// 1000 x 262144, 5.28 / 5.55. Below 512 keys the parts get too few keys for what a CTA costs: 24 heads x 130 features, 300 x 32768, 9.3 / 8.7.
+inline bool cut_by_queries(int N, int M) { return M > N && N >= 512; }
+inline int bins_of(int N, int M) {
+    int b = 32;
+    while (b < MAX_BINS && (b * 512 < N || (cut_by_queries(N, M) && b * 512 < M && b * 2 * SAMPLES_PER_BIN <= N))) b *= 2;
+    return b;
+}
+// two neighbouring parts hold more than PART_CAP keys, or queries
+inline int max_parts(int N, int M) { return 2 * (N / PART_CAP) + (cut_by_queries(N, M) ? 2 * (M / PART_CAP) : 0) + 2; }
+constexpr int MAX_PARTS = 4 * (262144 / PART_CAP) + 2;
+static_assert(MAX_PARTS <= 256, "parts are bytes, and one thread each in part_stats");
 __host__ __device__ inline int tiles_of(int n) { return (n + TILE - 1) / TILE; }
 
 // key order with the two zeros equal, as the float comparisons of the rank search see them
@@ -52,11 +64,12 @@ struct Lists {
     float4   *stats;                // [seg][maxparts] smallest key, largest key, sum seen from the largest, sum seen from the smallest
     uint32_t *done;                 // [seg] parts whose stats are written
     size_t   bytes;
-    Lists(void* base, int nseg, int N, int M) {
+    int      bins, mp, qcap;        // bins and (at most) parts per segment, queries that a part may collect
+    Lists(void* base, int nseg, int N, int M) : bins(bins_of(N, M)), mp(max_parts(N, M)), qcap(cut_by_queries(N, M) ? PART_CAP : M) {
         char*  b = static_cast<char*>(base);
         size_t off = 0;
         auto take = [&](size_t n) { char* p = b ? b + off : nullptr; off += (n + 255) & ~size_t(255); return p; };
-        const size_t s = nseg, mp = max_parts(N);
+        const size_t s = nseg, mp = this->mp;
         bin_keys    = reinterpret_cast<uint32_t*>(take(s * MAX_BINS * 4));        // zeroed together: bin_keys, bin_queries, done
         bin_queries = reinterpret_cast<uint32_t*>(take(s * MAX_BINS * 4));
         done        = reinterpret_cast<uint32_t*>(take(s * 4));
@@ -84,7 +97,7 @@ __device__ __forceinline__ uint32_t mix(uint32_t x) {
 __global__ void __launch_bounds__(512) sample_splitters(const SortArgs a, const Lists l)
 {
     __shared__ unsigned long long s[MAX_BINS * SAMPLES_PER_BIN];
-    const int N = a.N, bins = bins_of(N), n = bins * SAMPLES_PER_BIN;
+    const int N = a.N, bins = l.bins, n = bins * SAMPLES_PER_BIN;
     const long long seg = blockIdx.x;
     const float* x = a.x + seg * N;
     for (int i = threadIdx.x; i < n; i += 512) {
@@ -123,12 +136,12 @@ struct Tile {
 // of a warp, at different nodes of one level, meet in a bank only on the two last levels. In the sorted array, whose level with
 // step s has its entries 2 s words apart, the last five levels cost 4 to 8 passes each: 0.34 ms for 128 segments of
 // 262144 keys and queries.
-__global__ void __launch_bounds__(TILE_THREADS) count_bins(const SortArgs a, const Lists l)
+__global__ void __launch_bounds__(TILE_THREADS, 8) count_bins(const SortArgs a, const Lists l)
 {
     __shared__ uint32_t value[MAX_BINS], index[MAX_BINS];          // first (value, index) of every bin
     __shared__ uint32_t count[MAX_BINS], tree[MAX_BINS];           // node j's children are 2 j and 2 j + 1, the root is 1
     const Tile t(a);
-    const int  bins = bins_of(a.N), tid = threadIdx.x;
+    const int  bins = l.bins, tid = threadIdx.x;
     for (int b = tid; b < bins; b += TILE_THREADS) {
         const unsigned long long c = l.split[t.seg * MAX_BINS + b];
         value[b] = (uint32_t)(c >> 32); index[b] = (uint32_t)c; count[b] = 0;
@@ -178,7 +191,7 @@ __global__ void __launch_bounds__(MAX_BINS) merge_bins(const SortArgs a, const L
     __shared__ uint32_t nk[MAX_BINS], nq[MAX_BINS];
     __shared__ uint8_t  part[MAX_BINS];
     const long long seg = blockIdx.x;
-    const int bins = bins_of(a.N), mp = max_parts(a.N), tid = threadIdx.x;
+    const int bins = l.bins, mp = l.mp, tid = threadIdx.x;
     if (tid < bins) { nk[tid] = l.bin_keys[seg * MAX_BINS + tid]; nq[tid] = l.bin_queries[seg * MAX_BINS + tid]; }
     for (int i = tid; i < mp; i += MAX_BINS) l.info[seg * mp + i].n = 0;
     __syncthreads();
@@ -194,7 +207,7 @@ __global__ void __launch_bounds__(MAX_BINS) merge_bins(const SortArgs a, const L
             np++; ks += k; qs += q; k = q = 0;
         };
         for (int b = 0; b < bins; b++) {
-            if (k > 0 && k + (int)nk[b] > PART_CAP) close();       // (a part without keys takes the next bin's)
+            if (k > 0 && nk[b] > 0 && (k + (int)nk[b] > PART_CAP || q + (int)nq[b] > l.qcap)) close();       // (every part has keys)
             part[b] = (uint8_t)np;
             k += nk[b]; q += nq[b];
         }
@@ -210,7 +223,7 @@ __global__ void __launch_bounds__(TILE_THREADS) scatter_parts(const SortArgs a, 
     __shared__ uint8_t  spart[TILE], part_of[MAX_BINS];
     __shared__ uint32_t count[MAX_PARTS], start[MAX_PARTS], gofs[MAX_PARTS];
     const Tile t(a);
-    const int  tid = threadIdx.x, mp = max_parts(a.N), lane = tid & 31;
+    const int  tid = threadIdx.x, mp = l.mp, lane = tid & 31;
     const float*   src = t.keys ? a.x + t.seg * a.N + t.t0 : a.y + t.seg * a.M + t.t0;
     const uint8_t* bin = t.keys ? l.kbin + t.seg * a.N + t.t0 : l.qbin + t.seg * a.M + t.t0;
     float    x[TILE_E];
@@ -221,7 +234,7 @@ __global__ void __launch_bounds__(TILE_THREADS) scatter_parts(const SortArgs a, 
         x[s]  = i < t.n ? src[i] : 0.0f;
         pr[s] = i < t.n ? bin[i] : 0u;
     }
-    part_of[tid] = tid < bins_of(a.N) ? l.part_of[t.seg * MAX_BINS + tid] : 0;
+    part_of[tid] = tid < l.bins ? l.part_of[t.seg * MAX_BINS + tid] : 0;
     if (tid < mp) count[tid] = 0;
     __syncthreads();
     #pragma unroll
@@ -287,7 +300,7 @@ __global__ void __launch_bounds__(256) part_stats(const SortArgs a, const Lists 
     __shared__ float  red[8];
     __shared__ float4 st[MAX_PARTS];
     __shared__ bool   finish;
-    const int mp = max_parts(a.N), tid = threadIdx.x, N = a.N;
+    const int mp = l.mp, tid = threadIdx.x, N = a.N;
     const long long seg = blockIdx.x / mp;
     const int part = blockIdx.x % mp;
     const PartInfo pi = l.info[seg * mp + part];
@@ -361,7 +374,7 @@ cudaError_t launch_sort_rank_large(const SortArgs& a, void* scratch, cudaStream_
     const Lists l(scratch, a.nseg, a.N, a.M);
     cudaError_t e = cudaMemsetAsync(scratch, 0, l.zeroed, stream);
     if (e != cudaSuccess) return e;
-    const unsigned tiles = (unsigned)a.nseg * (unsigned)(tiles_of(a.N) + tiles_of(a.M)), parts = (unsigned)a.nseg * (unsigned)max_parts(a.N);
+    const unsigned tiles = (unsigned)a.nseg * (unsigned)(tiles_of(a.N) + tiles_of(a.M)), parts = (unsigned)a.nseg * (unsigned)l.mp;
     sample_splitters<<<a.nseg, 512, 0, stream>>>(a, l);
     count_bins<<<tiles, TILE_THREADS, 0, stream>>>(a, l);
     merge_bins<<<a.nseg, MAX_BINS, 0, stream>>>(a, l);
@@ -370,7 +383,7 @@ cudaError_t launch_sort_rank_large(const SortArgs& a, void* scratch, cudaStream_
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     PartArgs pa{};
-    pa.kkey = l.kkey; pa.kidx = l.kidx; pa.qval = l.qval; pa.qidx = l.qidx; pa.info = l.info; pa.maxparts = max_parts(a.N);
+    pa.kkey = l.kkey; pa.kidx = l.kidx; pa.qval = l.qval; pa.qidx = l.qidx; pa.info = l.info; pa.maxparts = l.mp;
     return launch_sort_rank_parts(a, pa, stream);
 }
 

@@ -86,6 +86,27 @@ def test_records_long_segments(shape, mode):
     check_records(x, y, mode)
 
 
+# More queries than keys: parts are cut by their queries too, down to a few keys each, and a part whose queries crowd between two keys
+# has more of them than a CTA holds.
+@pytest.mark.parametrize("kind", ["plain", "narrow", "equal", "few_values", "one_key_value"])
+@pytest.mark.parametrize("shape", [(1, 2, 1, 16385), (2, 1, 5, 40000), (1, 2, 300, 33000), (1, 1, 512, 70000), (1, 1, 2000, 262144), (1, 1, 8192, 100000), (1, 1, 20000, 30001)])
+def test_records_more_queries_than_keys(shape, kind):
+    P, D, N, M = shape
+    g = torch.Generator().manual_seed(N + M)
+    x, y = torch.randn(P, D, N, generator=g), torch.randn(P, D, M, generator=g)
+    if kind == "narrow":
+        y *= 0.01
+    elif kind == "equal":
+        y[:] = 0.3
+        y[:, :, 7] = x[:, :, 0]
+    elif kind == "few_values":
+        x, y = (x * 2).round() / 2, (y * 2).round() / 2
+    elif kind == "one_key_value":
+        x[:] = 0.25
+    for mode in (0, 1):
+        check_records(x, y, mode)
+
+
 def check_records(x, y, mode):
     import qlka_native
     P, D, N = x.shape
