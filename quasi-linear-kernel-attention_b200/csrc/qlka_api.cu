@@ -53,7 +53,7 @@ namespace {
 thread_local int g_last_cuda = 0;
 
 constexpr int SMALL_MAX = 16384;     // longest segment the shared-memory sort handles
-constexpr int LENGTH_MAX = 262144;   // the reference stops at 131072 (binding.cpp:78); the global-memory sort goes on
+constexpr int LENGTH_MAX = 262144;   // the reference stops at 131072 (binding.cpp:78); the value-cut sort goes on
 constexpr int EMIT_ROWS = 0, EMIT_DOT = 1, EMIT_BOTH = 2;
 
 #define CU(expr)                                                   \
@@ -128,7 +128,7 @@ size_t walk_agg_floats(const WalkPlan& w, int nseg, int C4, bool laplace) {
 // scratch of one sort/rank run over nseg segments of N keys and M queries
 struct Records {
     uint32_t* xperm; float* xval; uint4* yrec; uint32_t* mstart; float* su0; float* su1;
-    void* large;          // extra scratch of the global-memory sort, only when max(N, M) > SMALL_MAX
+    void* large;          // extra scratch of the value-cut sort, only when max(N, M) > SMALL_MAX
     void carve(Bump& b, int nseg, int N, int M) {
         large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(nseg, N, M)) : nullptr;
         xperm  = b.take<uint32_t>((size_t)nseg * npad(N));
@@ -148,7 +148,7 @@ SortArgs sort_args(const Records& r, const float* x, const float* y, int nseg, i
     return s;
 }
 
-// the sort/rank stage: shared-memory kernel up to SMALL_MAX elements per segment, global-memory kernels above
+// the sort/rank stage: shared-memory kernel up to SMALL_MAX elements per segment, cut by value into its parts above
 cudaError_t launch_sort_rank(const SortArgs& s, const Records& r, cudaStream_t stream) {
     if (s.N <= SMALL_MAX && s.M <= SMALL_MAX) return launch_sort_rank_small(s, stream);
     return launch_sort_rank_large(s, r.large, stream);
@@ -281,8 +281,10 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
 
 // ------------------------------------------------------------------ short sequences: pair by pair
 // Whether the pairwise kernels beat the sorted walk, from two cost estimates fitted to measurements on a B200 (1 to 256 heads,
-// 64 to 4096 keys, 32 and 64 features, 32 to 128 channels). Both are good to about a fifth, and around the line the two
-// paths cost the same, so a case on the wrong side of it loses little.
+// 64 to 4096 keys, 32 and 64 features, 32 to 128 channels). The pairwise one is good to a tenth. The sorted one was fitted to slower walks
+// and lies 14 to 40 % above what they take now (64 features and channels, Laplace, estimate / measured: 96 heads x 256 keys 473 / 335 us,
+// 96 x 777 918 / 695, 48 x 1024 599 / 443, 48 x 4096 1911 / 1484), so near the line some calls run pair by pair that would be up to
+// a fifth faster sorted (96 x 777: 856 / 695 us).
 double dense_us(int kind, double P, int D, int N, int M, int C) {
     // picoseconds per pair and feature, and per pair and channel, with three CTAs on every SM
     const double per_d = kind == DENSE_LAPLACE ? 0.155 : kind == DENSE_BUMP ? 0.115 : 0.090, per_c = 0.027;
@@ -300,15 +302,22 @@ double sorted_us(int kind, double P, int D, int N, int M, int C) {
     const double keys = N * (0.022 + 0.045 * wide), queries = M * (0.022 + 0.050 * wide) * (kind == DENSE_BUMP ? 5.0 : 1.0);
     return 70.0 + segs * (30.0 + keys + queries) * 1e-3;               // (launches and tails; nanoseconds per segment)
 }
-// A key mask lets the pairwise kernels skip whole tiles of padding (a seventh is assumed) and costs the sorted path its bucket
-// sort: masked keys are zeros, too many in one bucket.
+// What a key mask does to either path is in its values, which are on the device; the factors are for the masks met in earnest. Measured at
+// 96 heads x 256 and 777 keys, 48 x 1024, 2048 and 4096 (64 features and channels) and 8 x 1500 (32), masked against unmasked:
+//   pairwise, texts padded to the longest (kept lengths N / 2 to N): forward 0.62 to 0.92, gradients 0.64 to 1.00 (tiles of padding are skipped);
+//     masked keys scattered, or 20 at the end: 0.91 to 1.06
+//   sorted (masked keys are zeros, too many in one bucket, so their segments take the radix sort), padded or scattered: Laplace and riesz
+//     forward 1.22 to 1.52, bump 1.13 to 1.50, Laplace gradients 1.14 to 1.94; 20 at the end: 1.03 to 1.13
+// 0.85 and 1.25 suit padded batches. They cost a call whose batch is hardly masked: 48 heads x 1024 keys, Laplace, 20 masked keys, runs
+// pair by pair in 711 us where the sorted path takes 493.
 bool dense_pays(int kind, long long P, int D, int N, int M, int C, bool masked = false) {
     if (D > DENSE_MAX_D) return false;
     return dense_us(kind, (double)P, D, N, M, C) * (masked ? 0.85 : 1.0) < sorted_us(kind, (double)P, D, N, M, C) * (masked ? 1.25 : 1.0);
 }
 
 // The same for the gradients: three kernels of the same tiling against two sorts and three walks (Laplace 0.43 ns per feature
-// and key, abs 0.30, measured at 4096 keys; the bump's are three abs gradients put together op by op).
+// and key, abs 0.30, measured at 4096 keys; the bump's are three abs gradients put together op by op). The Laplace estimate lies 39 % above
+// the present walks (48 heads x 1024 keys 1647 / 1188 us, x 4096 5705 / 4116).
 bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C, bool masked = false) {
     if (D > DENSE_MAX_D) return false;
     const double grad_d = kind == DENSE_LAPLACE ? 0.50 : kind == DENSE_BUMP ? 0.68 : 0.26, grad_c = 0.054;

@@ -90,6 +90,7 @@ struct Lists {
     size_t zeroed;
 };
 
+// The published integer hash "lowbias32" (Chris Wellons, found by search over xor-shift-multiply hashes for low bias; public domain).
 __device__ __forceinline__ uint32_t mix(uint32_t x) {
     x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; return x ^ (x >> 16);
 }

@@ -1,4 +1,4 @@
-"""Segments longer than the shared-memory sort holds (max(N, M) > 16384): the global-memory
+"""Segments longer than the shared-memory sort holds (max(N, M) > 16384): the value-cut
 sort/rank path, through the same operators, against the C checker."""
 
 import pytest
