@@ -192,7 +192,7 @@ def test_fused_attention_entry(shape, kernel, masked):
     assert rel_err(out, ref) < 2e-4, f"rel err {rel_err(out, ref)}"
     with torch.enable_grad():
         qg = q.clone().requires_grad_(True)
-        slow = attention(qg, k, v, kernel, tau, keep)                      # op-by-op route
+        slow = attention(qg, k, v, kernel, torch.tensor(tau, device="cuda", requires_grad=True), keep)      # op-by-op route (a trained temperature)
     assert rel_err(out, slow.double()) < 2e-4
 
 

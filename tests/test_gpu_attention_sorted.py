@@ -52,6 +52,23 @@ def call(q, k, v, grad, kernel, tau, keep, fn=None):
     return (out.detach(), *torch.autograd.grad(out, (q, k, v), grad.to(out.dtype)))
 
 
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("kernel", KERNELS)
+@pytest.mark.parametrize("B, H, S, C", [(1, 1, 1, 4), (2, 2, 64, 64), (1, 3, 129, 33), (2, 1, 300, 16), (1, 1, 700, 128), (3, 2, 90, 7)])
+def test_outputs_and_gradients(B, H, S, C, kernel, masked):
+    """Without autograd, with it, and its gradients, against the definition in float64."""
+    from kernel_attention import attention
+    q, k, v, grad, keep = inputs(B, H, S, SORTED, C, masked, S + C)
+    if kernel == "add_bump":        # at least 1 / 64 from every kink: 23 million pairs of smooth values have some within rounding of one, each off by a whole slope
+        q, k = (q * 64).round() / 64 + 1 / 128, (k * 64).round() / 64
+    got = call(q, k, v, grad, kernel, 0.5, keep)
+    want = call(q, k, v, grad, kernel, 0.5, keep, dense_attention)
+    assert rel_err(attention(q, k, v, kernel, 0.5, keep), want[0]) < 1e-4
+    assert rel_err(got[0], want[0]) < 1e-4
+    for a, b in zip(got[1:], want[1:]):      # (one key: the gradients of q and k are rounding)
+        assert two_norm(a, b) < 1e-4 or (S == 1 and (a.double() - b).abs().max().item() < 1e-6), two_norm(a, b)
+
+
 @pytest.mark.parametrize("D", [SORTED, PAIRWISE])
 @pytest.mark.parametrize("kernel", KERNELS)
 def test_queries_at_zero_beside_masked_keys(kernel, D):

@@ -85,7 +85,7 @@ def dense_attention(q, k, v, kernel, tau, keep):
 @pytest.mark.parametrize("kernel", ["add_laplace", "add_riesz", "add_bump"])
 @pytest.mark.parametrize("shape", [(2, 2, 64, 16, 64), (1, 3, 129, 30, 33), (2, 1, 300, 70, 16), (1, 1, 1500, 8, 64)])
 def test_attention_gradients(kernel, shape, masked):
-    """Forward and backward through autograd; the last shape takes the sorted kernels where those are the faster ones."""
+    """Forward and backward through autograd."""
     from kernel_attention import attention
     B, H, S, D, C = shape
     g = torch.Generator().manual_seed(S)

@@ -104,10 +104,12 @@ def test_argument_errors():
         weighted_laplace_sum(q, k, torch.zeros(1, 16, 129, device="cuda"))
 
 
-def test_host_pipeline_matches_device_call():
-    """Pinned host buffers in and out, heads streamed in chunks (ragged last chunk)."""
+@pytest.mark.parametrize("D", [4, 130])
+def test_host_pipeline_matches_device_call(D):
+    """Pinned host buffers in and out, heads streamed in chunks (ragged last chunk); pair by pair and, with more than 128 features,
+    sorted."""
     import qlka_native
-    P, D, N, M, C = 7, 4, 1200, 900, 32
+    P, N, M, C = 7, 1200, 900, 32
     q, k, v = make_inputs(P, D, N, M, C, seed=77, scale=2.0, device="cpu")
     q_h, k_h, v_h = q.pin_memory(), k.pin_memory(), v.pin_memory()
     out_w_h, out_u_h = torch.empty(P, M, C).pin_memory(), torch.empty(P, M).pin_memory()
@@ -141,7 +143,7 @@ def test_fused_attention_entry(shape, masked):
     assert rel_err(out, attention(q, k, v, "add_laplace", 0.5, keep).double()) < 1e-5     # same route without grad (atomics: order differs)
     with torch.enable_grad():
         qg = q.clone().requires_grad_(True)
-        slow = attention(qg, k, v, "add_laplace", 0.5, keep)                      # op-by-op route
+        slow = attention(qg, k, v, "add_laplace", torch.tensor(0.5, device="cuda", requires_grad=True), keep)      # op-by-op route (a trained temperature)
     assert rel_err(out, slow.double()) < 1e-5
 
 

@@ -93,7 +93,7 @@ def test_backward_global_memory_sort():
 
 
 def test_attention_add_laplace_trains():
-    """add_laplace attention with gradients: the sorted-walk backward against float64 autograd of the dense formula."""
+    """add_laplace attention with gradients (pair by pair at this length) against float64 autograd of the dense formula."""
     from kernel_attention import attention
     B, H, S, D = 1, 2, 192, 16
     g = torch.Generator().manual_seed(41)

@@ -1,6 +1,6 @@
 """More than 65535 batch*head problems in one call: every kernel carries the head (or segment) index in the x extent of
 its grid, whose limit is 2^31 - 1, never in y or z (limit 65535). Checked on the heads at both ends and around 65536
-against the float64 definitions."""
+against the float64 definitions. Few features run pair by pair, more than 128 through the sort and the walks."""
 
 import pytest
 import torch
@@ -9,11 +9,12 @@ from oracle import direct
 from util import rel_err
 
 pytestmark = pytest.mark.gpu
-P, D, N, M, C = 66000, 2, 24, 19, 4
+P, C = 66000, 4
+SIZES = [(2, 24, 19), (130, 9, 7)]       # D, N, M
 HEADS = [0, 1, 65534, 65535, 65536, 65537, P - 1]
 
 
-def _inputs():
+def _inputs(D, N, M):
     g = torch.Generator(device="cuda").manual_seed(11)
     q = torch.randn(P, D, M, device="cuda", generator=g)
     k = torch.randn(P, D, N, device="cuda", generator=g)
@@ -26,9 +27,10 @@ def _pick(*ts):
     return tuple(t.index_select(0, idx).contiguous() for t in ts)
 
 
-def test_laplace_forward_and_backward():
+@pytest.mark.parametrize("D, N, M", SIZES)
+def test_laplace_forward_and_backward(D, N, M):
     from weighted_laplace_sum import weighted_laplace_sum, weighted_laplace_sum_backward
-    q, k, v = _inputs()
+    q, k, v = _inputs(D, N, M)
     out_w, out_u = weighted_laplace_sum(q, k, v)
     g = torch.Generator(device="cuda").manual_seed(12)
     g_w = torch.randn(P, M, C, device="cuda", generator=g)
@@ -42,9 +44,10 @@ def test_laplace_forward_and_backward():
     assert rel_err(gqs, rq) < 1e-4 and rel_err(gks, rk) < 1e-4 and rel_err(gvs, rv) < 1e-4
 
 
-def test_abs_forward_backward_sgn():
+@pytest.mark.parametrize("D, N, M", SIZES)
+def test_abs_forward_backward_sgn(D, N, M):
     from weighted_abs_sum import weighted_abs_sum_full, weighted_sgn_sum
-    q, k, v = _inputs()
+    q, k, v = _inputs(D, N, M)
     q.requires_grad_(True); k.requires_grad_(True); v.requires_grad_(True)
     out_w, out_u = weighted_abs_sum_full(q, k, v)
     g = torch.Generator(device="cuda").manual_seed(13)

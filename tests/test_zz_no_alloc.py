@@ -2,8 +2,9 @@
 serving loops, hosts that own all device memory). Collected last on purpose.
 
 Called through the C ABI, twice in a row with different problems, and compared with the
-workspace entry point on the same inputs. The second call runs on scratch that still holds the
-first call's records, which must not matter."""
+workspace entry point on the same inputs. The second call runs on scratch that still holds what
+the first call left there, which must not matter. Pair by pair, and with more than 128 features
+sorted, where the scratch holds records."""
 
 import ctypes
 
@@ -28,13 +29,15 @@ def _call_noalloc(lib, q, k, v):
     return out_w, out_u
 
 
-def test_matches_workspace_entry_point_on_two_calls_in_a_row():
+@pytest.mark.parametrize("D", [(8, 4), (130, 140)])
+def test_matches_workspace_entry_point_on_two_calls_in_a_row(D):
     import qlka_native
     lib = qlka_native.lib()
     assert lib.qlka_noalloc_scratch_bytes() == 32 << 20
-    first = make_inputs(2, 8, 1500, 1200, 64, seed=31, scale=2.0)
-    second = make_inputs(3, 4, 700, 2100, 33, seed=32, scale=2.0)     # other sizes, padded channels
-    for q, k, v in (first, second):
+    few = D[0] > 128                                                  # heads, so that the records fit
+    first = make_inputs(1 if few else 2, D[0], 1200 if few else 1500, 1200, 64, seed=31, scale=2.0)
+    second = make_inputs(1 if few else 3, D[1], 700, 1400 if few else 2100, 33, seed=32, scale=2.0)     # other sizes, padded channels
+    for q, k, v in (first, second, first):
         got_w, got_u = _call_noalloc(lib, q, k, v)
         ref_w, ref_u = qlka_native.laplace_forward(q, k, v)
         torch.cuda.synchronize()
@@ -43,15 +46,15 @@ def test_matches_workspace_entry_point_on_two_calls_in_a_row():
         assert rel_err(got_u, ref_u.double()) < TOL
 
 
-def test_later_calls_leave_free_device_memory_unchanged():
+@pytest.mark.parametrize("P, D, N, M", [(2, 8, 1500, 1200), (1, 130, 1200, 1200)])
+def test_later_calls_leave_free_device_memory_unchanged(P, D, N, M):
     """The one claim of the entry point: once the scratch array exists (the first call on a device
     materialises it), a call takes no device memory - neither through the CUDA allocator nor
     through torch's. Outputs are preallocated so that the wrapper allocates nothing either."""
     import qlka_native
     lib = qlka_native.lib()
-    q, k, v = make_inputs(2, 8, 1500, 1200, 64, seed=33, scale=2.0)
-    P, D, M = q.shape
-    N, C = k.shape[2], v.shape[2]
+    C = 64
+    q, k, v = make_inputs(P, D, N, M, C, seed=33, scale=2.0)
     out_w = torch.empty(P, M, C, device="cuda")
     out_u = torch.empty(P, M, device="cuda")
     stream = torch.cuda.current_stream().cuda_stream
