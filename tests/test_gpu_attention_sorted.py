@@ -105,3 +105,16 @@ def test_masked_values_are_never_looked_at(kernel, D):
         assert a.masked_select(off.expand_as(a)).abs().max().item() == 0.0
     from kernel_attention import attention
     assert two_norm(attention(q, kj, vj, kernel, 0.5, keep), want[0]) < 1e-5
+
+
+@pytest.mark.parametrize("D", [SORTED, PAIRWISE])
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_batch_without_any_key(kernel, D):
+    """Every key of one batch entry masked: zeros come out there, no gradient goes in, and the other entry is not touched by it."""
+    q, k, v, grad, keep = inputs(2, 2, 150, D, 16, True, 3 * D)
+    keep[0] = False
+    got = call(q, k, v, grad, kernel, 0.5, keep)
+    alone = call(q[1:], k[1:], v[1:], grad[1:], kernel, 0.5, keep[1:])
+    for a, b in zip(got, alone):
+        assert a[0].abs().max().item() == 0.0
+        assert two_norm(a[1:], b) < 1e-5

@@ -103,3 +103,13 @@ def test_tensors_seen_by_hooks_stay_as_they_were():
         (model.embed if where == "embed" else model.blocks[0]).register_forward_hook(lambda m, i, o: kept.append((o, o.clone())))
         model(ids)
         assert torch.equal(*kept[0])
+
+
+def test_traced_and_compiled_models_hold_the_whole_computation():
+    from torch.fx.experimental.proxy_tensor import make_fx
+    model, ids = small("softmax")
+    other = ids.flip(0).flip(1).contiguous()
+    want = module_by_module(model, other)
+    for made in (torch.jit.trace(model, (ids,), check_trace=False), torch.compile(model, backend="eager", fullgraph=True), make_fx(model)(ids)):
+        assert ((made(other) - want).norm() / want.norm()).item() < 1e-5
+    assert ((torch.func.vmap(model)(other[:, None])[:, 0] - want).norm() / want.norm()).item() < 1e-5
