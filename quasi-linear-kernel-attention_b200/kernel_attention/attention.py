@@ -9,8 +9,8 @@ Two routes:
 * one native call forward and, where gradients are wanted, one backward (`qlka_native.attention`): layout change, tau,
   masking, the sums and the normalisation all happen inside the library;
 * the cases without such a call (gradients of add_riesz and add_bump at long lengths, add_bump beyond 5461 keys, training with a
-  temperature that is a tensor to broadcast or to train, or that is not above 0, or with a mask that wants a gradient) - the sums are
-  assembled here from the differentiable operators. Every kernel is described
+  temperature that is a tensor to broadcast or to train, or that is not above 0, or with a mask that wants a gradient; calls that
+  torch.jit.trace records) - the sums are assembled here from the differentiable operators. Every kernel is described
   by two small functions: `sums` returns the unnormalised numerator sum_j A_ij v_j and row sum sum_j A_ij over
   ALL S keys, and `at_origin` returns A(q_i, 0), the weight a key placed at the origin has. Masked keys are moved
   to the origin with a zero value row, so they add nothing to the numerator and exactly `at_origin` each to the
@@ -78,7 +78,9 @@ _ROUTES = {"add_laplace": (_laplace_sums, _laplace_at_origin),
 
 
 def _needs_operators(q, k, v, tau, keep):
-    """Whether a call asks for gradients that the native backward pass does not give, or for a temperature it does not take."""
+    """Whether a call asks for gradients that the native backward pass does not give, for a temperature it does not take, or for a record."""
+    if torch.jit.is_tracing():
+        return True
     by_tensor = isinstance(tau, torch.Tensor)
     trained = (by_tensor and tau.requires_grad) or (keep is not None and keep.requires_grad)
     if not (trained or q.requires_grad or k.requires_grad or v.requires_grad) or not torch.is_grad_enabled():

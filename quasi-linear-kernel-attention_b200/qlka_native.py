@@ -140,6 +140,41 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
+class _Recorded(torch.autograd.Function):
+    """The Laplace or the abs sum as a node that torch.jit.trace records. The nodes of the compiled binding are the same
+    without it, and a trace through them would hold their outputs as constants."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, name, *options):
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(q, k, v)
+        ctx.name = name
+        out_w, out_u = getattr(ext(), f"{name}_forward")(q, k, v, *options)
+        return out_w.clone() if out_u is None else (out_w.clone(), out_u.clone())      # (results of operations that the tracer saw)
+
+    @staticmethod
+    def backward(ctx, g_w, g_u=None):
+        q, k, v = ctx.saved_tensors
+        none = (None,) * (len(ctx.needs_input_grad) - 3)
+        if g_w is None and g_u is None:
+            return (None, None, None, *none)
+        g_w = q.new_zeros(q.shape[0], q.shape[2], v.shape[2]) if g_w is None else g_w.contiguous()
+        return (*getattr(ext(), f"{ctx.name}_backward")(q, k, v, g_w, None if g_u is None else g_u.contiguous()), *none)
+
+
+def laplace_sum(q, k, v):
+    """(out_w, out_u) of the weighted Laplace sum, differentiable."""
+    return _Recorded.apply(q, k, v, "laplace") if torch.jit.is_tracing() else ext().laplace_sum(q, k, v)
+
+
+def abs_sum(q, k, v, full, path=-1):
+    """(out_w, out_u), or (out_w,) unless `full`, of the weighted abs sum, differentiable."""
+    if torch.jit.is_tracing():
+        out = _Recorded.apply(q, k, v, "abs", full, path)
+        return out if full else (out,)
+    return ext().abs_sum(q, k, v, full, path)
+
+
 def laplace_forward(q, k, v):
     """(out_w, out_u) of the weighted Laplace sum, without autograd."""
     return ext().laplace_forward(q, k, v)

@@ -36,13 +36,13 @@ def weighted_abs_sum(q, k, v, backend="auto"):
 
     q: (P, D, M), k: (P, D, N), v: (P, N, C) -> (P, M, C). Differentiable.
     """
-    return _native.ext().abs_sum(q, k, v, False, _resolve(backend))[0]
+    return _native.abs_sum(q, k, v, False, _resolve(backend))[0]
 
 
 def weighted_abs_sum_full(q, k, v, backend="auto"):
     """Returns (out_w, out_u): the weighted abs sum (P, M, C) and the unweighted abs sum
     out_u[p,m] = sum_{n,d} |k[p,d,n] - q[p,d,m]| (P, M). Differentiable in both outputs."""
-    return tuple(_native.ext().abs_sum(q, k, v, True, _resolve(backend)))
+    return tuple(_native.abs_sum(q, k, v, True, _resolve(backend)))
 
 
 def weighted_abs_sum_shifted(q, k, v, shifts, weights):

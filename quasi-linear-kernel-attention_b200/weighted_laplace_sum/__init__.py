@@ -19,7 +19,7 @@ def weighted_laplace_sum(q, k, v):
     Differentiable in both outputs (where a key equals a query the one-sided derivative of the walk's
     tie side is taken). Padded keys: zero k and v there and subtract n_pad * sum_d exp(-|q_d|) from out_u.
     """
-    return _native.ext().laplace_sum(q, k, v)
+    return _native.laplace_sum(q, k, v)
 
 
 def weighted_laplace_sum_backward(q, k, v, g_w, g_u=None):

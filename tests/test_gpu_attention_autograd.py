@@ -130,3 +130,24 @@ def test_transforms_without_a_rule_are_refused():
             torch.func.jvp(lambda a: f(a, *args[1:]), (args[0],), (args[0],))
         with pytest.raises(Exception):
             torch.func.grad(lambda a: sum(t.sum() for t in f(a, *args[1:])))(args[0])
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("name", ["abs", "abs_full", "laplace", *KERNELS])
+def test_traced_calls_run_on_new_inputs(name, grad):
+    from kernel_attention import attention
+    from weighted_abs_sum import weighted_abs_sum, weighted_abs_sum_full
+    from weighted_laplace_sum import weighted_laplace_sum
+    call = {"abs": lambda q, k, v: weighted_abs_sum(q, k, v) * 2, "abs_full": lambda q, k, v: sum(t.sum(-1) if t.dim() == 3 else t for t in weighted_abs_sum_full(q, k, v)),
+            "laplace": lambda q, k, v: weighted_laplace_sum(q, k, v)[0] * 2}.get(name, lambda q, k, v: attention(q, k, v, name, 0.5) * 2)
+    g = torch.Generator(device="cuda").manual_seed(0)
+    shapes = ((1, 2, 40, 8), (1, 2, 40, 8), (1, 2, 40, 4)) if name in KERNELS else ((2, 3, 40), (2, 3, 50), (2, 50, 4))
+    first, second = ([torch.randn(*s, generator=g, device="cuda").requires_grad_(grad) for s in shapes] for _ in range(2))
+    made = torch.jit.trace(call, tuple(first), check_trace=False)
+    for compiled in (made, torch.compile(call, backend="aot_eager")):
+        got, want = compiled(*second), call(*second)
+        assert two_norm(got, want) < 1e-5
+        if grad:
+            for a, b in zip(torch.autograd.grad(got.sum(), second), torch.autograd.grad(want.sum(), second)):
+                assert two_norm(a, b) < 1e-5

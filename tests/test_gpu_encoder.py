@@ -105,6 +105,7 @@ def test_tensors_seen_by_hooks_stay_as_they_were():
         assert torch.equal(*kept[0])
 
 
+@pytest.mark.filterwarnings("ignore")
 def test_traced_and_compiled_models_hold_the_whole_computation():
     from torch.fx.experimental.proxy_tensor import make_fx
     model, ids = small("softmax")
