@@ -454,9 +454,9 @@ def run_ours(args, rank, world, local_rank):
 
 
 # figures from a profiler capture of the dominant kernel (dram__bytes_read + dram__bytes_write of one laplace_rows launch over
-# 12 heads: 837.6 MB + 41.3 MB) and from a bare gather / reduction loop with the walk's access pattern (two row gathers and one
-# row reduction per segment, 48 heads: 3.03 ms), both on a B200
-WALK_DRAM_BYTES_PER_HEAD = (837.61e6 + 41.28e6) / 12
+# 12 heads: 837.2 MB + 43.6 MB) and from a bare gather / reduction loop with the walk's access pattern (two row gathers and one
+# row reduction per segment, 48 heads: 3.03 ms), both on a B200; profiles/ has the captures
+WALK_DRAM_BYTES_PER_HEAD = (837.21e6 + 43.63e6) / 12
 L2_FLOOR_MS_PER_HEAD = 3.034 / 48
 
 

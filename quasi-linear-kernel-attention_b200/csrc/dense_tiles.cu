@@ -20,10 +20,10 @@
 // The first form leans on the FMA pipe, the second on the ALU pipe (minimum: half rate); half of the pairs take each.
 // That needs |q|, |k| <= LAP_RANGE (e^80 squared would overflow, and no product may be 0 * inf); tiles with larger values
 // are staged as they are and their pairs take the plain form.
-// Bound by instruction issue and the FMA / ALU pipes (Laplace at 2048 keys: 76 % of the issue slots, 54 % of the ALU pipe);
-// measured at B=4, H=12, D=C=64 as pairs x features per second: 5.3e12 (Laplace), 8.3e12 (abs), 6.7e12 (bump) at 2048 keys.
-// Times there, pairwise / sorted: 128 keys 33 / 218 us (abs), 512 keys 191 / 372 us (Laplace), 1024 keys 449 / 642 us (abs),
-// 549 / 1750 us (bump). On the way: 4 x 4 pairs per thread instead of 4 x 8 was bound by shared-memory reads (Laplace 4.1e12);
+// Bound by instruction issue and the FMA / ALU pipes (Laplace, 96 heads x 777 keys: 73 % of the issue slots, 52 % of the ALU pipe);
+// measured at B=4, H=12, D=C=64 as pairs x features per second: 5.2e12 (Laplace), 8.1e12 (riesz), 6.7e12 (bump) at 2048 keys.
+// Times of attention calls, pairwise / sorted: 96 heads x 256 keys 114 / 335 us (Laplace), 77 / 363 (riesz), 88 / 518 (bump); 48 x 1024
+// 710 / 443, 462 / 475, 552 / 892. On the way: 4 x 4 pairs per thread instead of 4 x 8 was bound by shared-memory reads (Laplace 4.1e12);
 // tiles transposed and exponentiated by the main kernel itself cost a quarter of its time (4.5e12); only the product form
 // or only the minimum form of the pair, two or four features unrolled: within 5 %.
 #include "qlka_common.cuh"

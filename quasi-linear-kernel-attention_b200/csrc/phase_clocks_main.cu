@@ -63,7 +63,7 @@ int main(int argc, char** argv) {
     CK(cudaMemcpyFromSymbol(clk, g_phase_clocks, sizeof(clk)));
     // marks in the order the kernel passes them
     const int   order[9] = {0, 1, 2, 3, 4, 7, 8, 5, 6};
-    const char* names[9] = {"load keys", "radix sort of the keys (4 passes)", "sorted keys to floats, xperm out, bucket index", "decays and scalar scans, xval / su out",
+    const char* names[9] = {"load keys", "sort of the keys (value buckets or radix)", "radix path's keys and buckets, xperm's tail", "decays and scalar scans, xval / su out",
                             "rank search", "rank histogram, scan, mstart, positions", "scalar side channel (out_u / out_s)",
                             "values and indices to record positions", "records built and written"};
     double total = 0.0;
