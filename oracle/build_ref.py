@@ -7,8 +7,8 @@ lacks (setup.py:6).
 
     python oracle/build_ref.py /path/to/reference
 
-`load_ref()` imports the built modules (on the GPU box the sources are absent; only the
-prebuilt .so files are used). They serve as a second parity checker for the GPU tests and
+`load_ref()` imports the built modules (on the GPU machine the sources are absent; only the
+prebuilt .so files are used). They serve as a second parity oracle for the GPU tests and
 as a GPU-side comparison point; the product never imports them.
 """
 

@@ -1,6 +1,6 @@
 """TEST INFRASTRUCTURE ONLY - fp64 direct O(N^2) evaluation of the additive-kernel sums.
 
-This module is the checker for the CUDA path: only tests, the smoke test and the
+This module is the oracle for the CUDA path: only tests, the smoke test and the
 CPU-baseline leg of the benchmark may import it. Nothing in the product package does.
 
 Every function restates a definition of the reference in float64, with the full

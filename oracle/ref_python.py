@@ -5,7 +5,7 @@ additive-kernel path needs (`__init__.py` is not taken: it would pull in nothing
 empty one keeps `nomic.py` / `vision_transformer.py` and their dependencies out) from a checkout into
 the git-ignored folder `baseline/_ref/Experiments/kernel_attention/`. Nothing of it enters the
 repository's history; like the compiled extensions of oracle/build_ref.py the folder only travels to the
-GPU box, where no checkout exists.
+GPU machine, where no checkout exists.
 
     python oracle/ref_python.py /path/to/reference
 

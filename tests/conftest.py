@@ -11,7 +11,7 @@ for p in (ROOT, PKG):
 
 
 def pytest_configure(config):
-    config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the GPU box)")
+    config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the GPU machine)")
 
 
 def pytest_collection_modifyitems(config, items):

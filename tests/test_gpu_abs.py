@@ -1,5 +1,5 @@
 """weighted_abs_sum (forward, backward, autograd) and weighted_sgn_sum on the GPU, through
-the C ABI, against the CPU checkers."""
+the C ABI, against the CPU oracles."""
 
 import os
 

@@ -1,5 +1,5 @@
 """The end-to-end encoder harness (the 12-layer pre-LN encoder, shrunk): the add_laplace encoder output equals
-the same network with its attention evaluated by the float64 O(N^2) checker, and the native blocks compute what calling the
+the same network with its attention evaluated by the float64 O(N^2) oracle, and the native blocks compute what calling the
 torch modules one by one does, hooks, replacements and casts included."""
 
 import pytest

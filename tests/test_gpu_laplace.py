@@ -1,4 +1,4 @@
-"""weighted_laplace_sum on the GPU (through the C ABI) against the CPU checkers."""
+"""weighted_laplace_sum on the GPU (through the C ABI) against the CPU oracles."""
 
 import os
 
@@ -10,7 +10,7 @@ from oracle import direct, sorted_scan
 from util import make_inputs, rel_err
 
 pytestmark = pytest.mark.gpu
-TOL = 1e-4          # max|a-b| / max|b| against float64; the north-star bound is 1e-3
+TOL = 1e-4          # max|a-b| / max|b| against float64; the bound asked for is 1e-3
 GOLD = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
 
 SHAPES = [
@@ -70,7 +70,7 @@ def test_config1_against_reference_golden():
 
 
 def test_linearity_and_sampled_head_at_full_size():
-    """B=4,H=12,N=16384,D=Dv=64 is too big for the checker as a whole: one head goes through the
+    """B=4,H=12,N=16384,D=Dv=64 is too big for the oracle as a whole: one head goes through the
     C restatement, and the full batch is checked through linearity in v."""
     from weighted_laplace_sum import weighted_laplace_sum
     P, D, N, C = 48, 64, 16384, 64

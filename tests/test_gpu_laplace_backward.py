@@ -1,7 +1,7 @@
-"""Gradients of weighted_laplace_sum on the GPU (through the C ABI) against float64 checkers.
+"""Gradients of weighted_laplace_sum on the GPU (through the C ABI) against float64 oracles.
 
 The reference has no Laplace backward (training goes through its chunked PyTorch route,
-Experiments/kernel_attention/attention.py:110-115), so the checkers are the direct float64
+Experiments/kernel_attention/attention.py:110-115), so the oracles are the direct float64
 formula with the walk's tie rule and, away from ties, torch autograd through exp(-|k - q|).
 """
 

@@ -1,5 +1,5 @@
 """Segments longer than the shared-memory sort holds (max(N, M) > 16384): the value-cut
-sort/rank path, through the same operators, against the C checker."""
+sort/rank path, through the same operators, against the C oracle."""
 
 import pytest
 import torch
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-4
 # Laplace with tens of thousands of keys per unit length: every prefix state is a product of thousands of
 # step decays that sit a few ulps below 1, and their fp32 rounding alone costs ~3e-5 at N = 65536 and
-# ~3e-4 at N = 262144 (measured with a correctly rounded CPU emulation); the north-star bound against
+# ~3e-4 at N = 262144 (measured with a correctly rounded CPU emulation); the bound asked for against
 # float64 is 1e-3
 TOL_DENSE = 1e-3
 
@@ -48,9 +48,9 @@ def test_abs_forward_backward_sgn(shape):
 
 
 # ---- long-context configuration as stated: B=1, H=16, D=Dv=64, N=M=65536 and 262144, q, k ~ N(0,1).
-# The whole problem runs on the GPU; one head goes through the C checker (all queries) and 256 sampled
+# The whole problem runs on the GPU; one head goes through the C oracle (all queries) and 256 sampled
 # query rows of another head through the float64 O(N^2) definition. Above 131072 the reference's own
-# extension refuses (Weighted_Laplace_Sum/csrc/binding.cpp:77-79), so these two are the only checkers there.
+# extension refuses (Weighted_Laplace_Sum/csrc/binding.cpp:77-79), so these two are the only oracles there.
 LONG = [65536, 262144]
 P_LONG, D_LONG, C_LONG = 16, 64, 64
 
@@ -71,10 +71,10 @@ def test_long_context_laplace_forward(N):
     q, k, v = make_inputs_cuda(P_LONG, D_LONG, N, N, C_LONG, seed=N)
     out_w, out_u = weighted_laplace_sum(q, k, v)
     torch.cuda.synchronize()
-    h = P_LONG - 1                                            # C checker: every query of one head
+    h = P_LONG - 1                                            # C oracle: every query of one head
     ref_w, ref_u = sorted_scan.laplace_sum(q[h:h + 1], k[h:h + 1], v[h:h + 1])
-    mw, pw = _report(f"laplace N={N} out_w vs C checker", out_w[h:h + 1], ref_w)
-    mu, pu = _report(f"laplace N={N} out_u vs C checker", out_u[h:h + 1], ref_u)
+    mw, pw = _report(f"laplace N={N} out_w vs C oracle", out_w[h:h + 1], ref_w)
+    mu, pu = _report(f"laplace N={N} out_u vs C oracle", out_u[h:h + 1], ref_u)
     assert mw < TOL_DENSE and mu < TOL_DENSE and pu < TOL_DENSE and pw < 5e-2
     rows = _sample_rows(N)                                    # float64 definition: sampled queries of another head
     dw, du = direct.laplace_sum(q[0:1][:, :, rows.cuda()], k[0:1], v[0:1])
@@ -91,8 +91,8 @@ def test_long_context_abs_forward(N):
     torch.cuda.synchronize()
     h = P_LONG - 1
     ref_w, ref_u = sorted_scan.abs_sum(q[h:h + 1], k[h:h + 1], v[h:h + 1])
-    mw, pw = _report(f"abs N={N} out_w vs C checker", out_w[h:h + 1], ref_w)
-    mu, pu = _report(f"abs N={N} out_u vs C checker", out_u[h:h + 1], ref_u)
+    mw, pw = _report(f"abs N={N} out_w vs C oracle", out_w[h:h + 1], ref_w)
+    mu, pu = _report(f"abs N={N} out_u vs C oracle", out_u[h:h + 1], ref_u)
     assert mw < TOL and mu < TOL and pu < TOL and pw < 5e-2
     rows = _sample_rows(N)
     dw, du = direct.abs_sum(q[0:1][:, :, rows.cuda()], k[0:1], v[0:1])
@@ -116,7 +116,7 @@ def test_long_context_abs_backward_and_sgn():
     rq, rk, rv = sorted_scan.abs_sum_backward(q[h], k[h], v[h], g_w[h], g_u[h])
     for name, got, want in (("grad_q", gq[h], rq), ("grad_k", gk[h], rk), ("grad_v", gv[h], rv),
                             ("sgn", sg[h], sorted_scan.sgn_sum(q[h], k[h], v[h], g_w[h]))):
-        mx, _ = _report(f"abs backward N={N} {name} vs C checker", got, want)
+        mx, _ = _report(f"abs backward N={N} {name} vs C oracle", got, want)
         assert mx < TOL, (name, mx)
 
 

@@ -1,6 +1,6 @@
 """Parity with the reference's own CUDA extensions, compiled for sm_100 by oracle/build_ref.py
 (binaries under oracle/_ref/; skipped when they are not there). Same seeded inputs, the bound of
-the north star: max|a - b| / max|b| <= 1e-4."""
+the bound asked for: max|a - b| / max|b| <= 1e-4."""
 
 import pytest
 import torch

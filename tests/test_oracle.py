@@ -1,4 +1,4 @@
-"""The checkers themselves: fp64 direct evaluation and the C sorted-scan restatement
+"""The oracles themselves: fp64 direct evaluation and the C sorted-scan restatement
 against the golden vectors produced by the reference's own Python code, and against
 each other (CPU only)."""
 
@@ -107,7 +107,7 @@ def test_backward_is_the_autograd_gradient_away_from_ties():
     gw, gu = torch.randn(P, M, C, generator=g, dtype=torch.float64), torch.randn(P, M, generator=g, dtype=torch.float64)
     A = (k[:, :, None, :] - q[:, :, :, None]).abs().sum(1)
     ((A @ v) * gw).sum().add((A.sum(2) * gu).sum()).backward()
-    # the checkers take fp32 inputs: compare on fp32-rounded copies
+    # the oracles take fp32 inputs: compare on fp32-rounded copies
     q32, k32, v32 = q.detach().float(), k.detach().float(), v.detach().float()
     got = direct.abs_sum_backward(q32, k32, v32, gw.float(), gu.float())
     for a, b in zip(got, (q.grad, k.grad, v.grad)):

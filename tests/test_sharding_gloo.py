@@ -1,5 +1,5 @@
 """The multi-GPU plumbing on CPU: two gloo ranks shard P, run a stand-in operator (the CPU
-checker) on their slices, and the gathered result equals the single-process one."""
+oracle) on their slices, and the gathered result equals the single-process one."""
 
 import os
 import sys

@@ -4,14 +4,14 @@ import torch
 
 
 def rel_err(a, b):
-    """max|a - b| / max|b| with b the checker's float64 result."""
+    """max|a - b| / max|b| with b the oracle's float64 result."""
     a = a.detach().to(torch.float64).cpu()
     b = b.detach().to(torch.float64).cpu()
     return ((a - b).abs().max() / b.abs().max().clamp_min(1e-6)).item()
 
 
 def err_stats(a, b, floor=1e-3):
-    """(max|a - b| / max|b|, 99.9th percentile of the element-wise relative error), b the checker's result.
+    """(max|a - b| / max|b|, 99.9th percentile of the element-wise relative error), b the oracle's result.
 
     The max-norm figure hides rows of small magnitude; the percentile figure looks at every element on its own,
     |a - b| / max(|b|, floor * max|b|) - the floor keeps elements where the sum cancels to nearly zero from
