@@ -62,14 +62,14 @@ inline int dense_split(long long ctas, int ntiles, int sms) {
 
 #ifdef __CUDACC__
 // The tiles of 64 keys that hold an unmasked one, in order, into `list` (shared memory, one entry per tile: twice the tile, plus 1 if
-// masked or absent keys are in it too); returns their number.
+// masked keys are in it too); returns their number.
 // Padding at the end of a sequence costs nothing that way. All threads of the block call it; `keep` has N entries.
 __device__ __forceinline__ int active_tiles(const float* __restrict__ keep, const int N, int* list, int* count) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, tiles = (N + 63) / 64;
     for (int t = warp; t < tiles; t += warps) {
         const int  n = t * 64 + lane;
         const bool a = n < N && __ldg(keep + n) != 0.0f, b = n + 32 < N && __ldg(keep + n + 32) != 0.0f;
-        const bool any = __any_sync(0xffffffffu, a || b), all = __all_sync(0xffffffffu, a && b);
+        const bool any = __any_sync(0xffffffffu, a || b), all = __all_sync(0xffffffffu, (a || n >= N) && (b || n + 32 >= N));
         if (lane == 0) list[t] = any ? (all ? 2 : 1) : 0;
     }
     __syncthreads();
