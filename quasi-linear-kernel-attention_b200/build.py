@@ -15,7 +15,7 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libqlka.so")
-SOURCES = ["qlka_api.cu", "sort_rank.cu", "sort_rank_large.cu", "walk_laplace.cu", "walk_prefix.cu", "dense_tiles.cu", "dense_gradient.cu", "encoder_linear.cu", "aux_kernels.cu"]
+SOURCES = ["qlka_api.cu", "sort_rank.cu", "sort_rank_large.cu", "walk_laplace.cu", "walk_prefix.cu", "walk_events.cu", "dense_tiles.cu", "dense_gradient.cu", "encoder_linear.cu", "aux_kernels.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
          "-Xcompiler", "-fPIC", "--threads", "4"]

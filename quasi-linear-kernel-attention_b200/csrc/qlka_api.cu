@@ -128,12 +128,16 @@ size_t walk_agg_floats(const WalkPlan& w, int nseg, int C4, bool laplace) {
 // scratch of one sort/rank run over nseg segments of N keys and M queries
 struct Records {
     uint32_t* xperm; float* xval; uint4* yrec; uint32_t* mstart; float* su0; float* su1;
+    uint32_t* eidx; float2* esc;      // the event list, where one is wanted
     void* large;          // extra scratch of the value-cut sort, only when max(N, M) > SMALL_MAX
-    void carve(Bump& b, int nseg, int N, int M) {
+    // records: of the queries, for the row walks; events: N' + M' of the longest list, for the walks with dots (0: none)
+    void carve(Bump& b, int nseg, int N, int M, bool records = true, int events = 0) {
         large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(nseg, N, M)) : nullptr;
         xperm  = b.take<uint32_t>((size_t)nseg * npad(N));
         xval   = b.take<float>((size_t)nseg * xstride(N));
-        yrec   = b.take<uint4>((size_t)nseg * (M + 1));
+        yrec   = records ? b.take<uint4>((size_t)nseg * (M + 1)) : nullptr;
+        eidx   = events ? b.take<uint32_t>((size_t)nseg * estride(events, 0)) : nullptr;
+        esc    = events ? b.take<float2>((size_t)nseg * estride(events, 0)) : nullptr;
         mstart = b.take<uint32_t>((size_t)nseg * mstride(N));
         su0    = b.take<float>((size_t)nseg * (N + 1));
         su1    = b.take<float>((size_t)nseg * (N + 1));
@@ -143,7 +147,7 @@ struct Records {
 SortArgs sort_args(const Records& r, const float* x, const float* y, int nseg, int D, int N, int M, int mode, int scal) {
     SortArgs s{};
     s.x = x; s.y = y;
-    s.xperm = r.xperm; s.xval = r.xval; s.yrec = r.yrec; s.mstart = r.mstart; s.su0 = r.su0; s.su1 = r.su1;
+    s.xperm = r.xperm; s.xval = r.xval; s.yrec = r.yrec; s.eidx = r.eidx; s.esc = r.esc; s.mstart = r.mstart; s.su0 = r.su0; s.su1 = r.su1;
     s.nseg = nseg; s.D = D; s.N = N; s.M = M; s.mode = mode; s.scal = scal;
     return s;
 }
@@ -156,7 +160,7 @@ cudaError_t launch_sort_rank(const SortArgs& s, const Records& r, cudaStream_t s
 
 WalkArgs walk_args(const Records& r, const float* rows, int nseg, int D, int N, int M, int C4) {
     WalkArgs a{};
-    a.rows = rows; a.xperm = r.xperm; a.xval = r.xval; a.yrec = r.yrec; a.mstart = r.mstart;
+    a.rows = rows; a.xperm = r.xperm; a.xval = r.xval; a.yrec = r.yrec; a.mstart = r.mstart; a.eidx = r.eidx; a.esc = r.esc;
     a.nseg = nseg; a.D = D; a.N = N; a.M = M; a.C4 = C4;
     a.sign = 1.0f;
     a.Mrows = M;
@@ -211,7 +215,9 @@ cudaError_t prefix_walk_chunked(WalkArgs w, int emit, int P, cudaStream_t stream
         w.rows   = all.rows + (size_t)p0 * all.N * all.C4;
         w.xperm  = all.xperm + s0 * npad(all.N);
         w.xval   = all.xval + s0 * xstride(all.N);
-        w.yrec   = all.yrec + s0 * (all.M + 1);
+        w.yrec   = all.yrec ? all.yrec + s0 * (all.M + 1) : nullptr;
+        w.eidx   = all.eidx ? all.eidx + s0 * estride(all.N, all.M) : nullptr;
+        w.esc    = all.esc ? all.esc + s0 * estride(all.N, all.M) : nullptr;
         w.mstart = all.mstart + s0 * mstride(all.N);
         w.out    = all.out ? all.out + (size_t)p0 * all.Mrows * all.C4 : nullptr;
         w.g      = all.g ? all.g + (size_t)p0 * all.M * all.C4 : nullptr;
@@ -224,32 +230,34 @@ cudaError_t prefix_walk_chunked(WalkArgs w, int emit, int P, cudaStream_t stream
     return cudaSuccess;
 }
 
-// The first walk pass leaves one suffix checkpoint per block of 8 keys and segment for the second pass: D / 8 times the
-// size of the row matrix. So that this scratch does not grow with the batch, a chunk's checkpoints also stay under
-// CKPT_BUDGET (the same chunks as the rows rule at D = 64).
+// The first walk pass leaves one suffix checkpoint per block and segment for the second pass: D / 8 times the size of the row matrix for
+// blocks of 8 keys, about twice that for blocks of 8 events (the walks with dots). So that this scratch does not grow with the batch, a chunk's
+// checkpoints also stay under CKPT_BUDGET (the same chunks as the rows rule at D = 64), twice that with dots.
 constexpr size_t CKPT_BUDGET = size_t(2) << 30;
 
-int laplace_chunk_heads(int P, int D, int N, int C4) {
-    const size_t per_head = (size_t)D * nblocks(N) * C4 * sizeof(float);
-    size_t h = CKPT_BUDGET / per_head;
+long long ckpt_blocks(int N, int M, bool dots) { return dots ? estride(N, M) / EB : nblocks(N); }
+
+int laplace_chunk_heads(int P, int D, int N, int M, int C4, bool dots) {
+    const size_t per_head = (size_t)D * ckpt_blocks(N, M, dots) * C4 * sizeof(float);
+    size_t h = (dots ? 2 : 1) * CKPT_BUDGET / per_head;
     if (h < 1) h = 1;
-    const int by_rows = walk_chunk_heads(P, N, C4);
+    const int by_rows = walk_chunk_heads(P, N > M || !dots ? N : M, C4);
     return (int)(h < (size_t)by_rows ? h : (size_t)by_rows);
 }
 
 struct LapWalkScratch {
     float *ckpt, *wck, *agg; int heads;
-    void carve(Bump& b, int P, int D, int N, int C4) {
-        heads = laplace_chunk_heads(P, D, N, C4);
+    // dots: for the streams of either side, N keys and M queries or the other way round
+    void carve(Bump& b, int P, int D, int N, int M, int C4, bool dots) {
+        heads = laplace_chunk_heads(P, D, N, M, C4, dots);
         const int nseg_c = heads * D;
-        ckpt = b.take<float>((size_t)nseg_c * nblocks(N) * C4);
-        wck  = b.take<float>((size_t)nseg_c * nblocks(N));
-        // the aggregate table of the larger of the two chunk sizes that occur (full chunks and the remainder)
-        size_t a = walk_agg_floats(plan_walk(nseg_c, N, C4, true), nseg_c, C4, true);
-        if (const int rem = P % heads) {
-            const size_t a2 = walk_agg_floats(plan_walk(rem * D, N, C4, true), rem * D, C4, true);
-            if (a2 > a) a = a2;
-        }
+        ckpt = b.take<float>((size_t)nseg_c * ckpt_blocks(N, M, dots) * C4);
+        wck  = b.take<float>((size_t)nseg_c * ckpt_blocks(N, M, dots) * (dots ? 2 : 1));
+        // the aggregate table of the largest of the chunks that occur (full chunks and the remainder)
+        size_t a = 0;
+        for (const int h : {heads, P % heads})
+            for (const int keys : {N, dots ? M : N})
+                if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, keys, C4, true), h * D, C4, true));
         agg = b.take<float>(a);
     }
 };
@@ -266,7 +274,9 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
         WalkArgs a{};
         a.rows = rows + (size_t)p0 * N * C4;
         a.xperm = r.xperm + s0 * npad(N); a.xval = r.xval + s0 * xstride(N);
-        a.yrec = r.yrec + s0 * (M + 1);   a.mstart = r.mstart + s0 * mstride(N);
+        if (emit == EMIT_ROWS) a.yrec = r.yrec + s0 * (M + 1);
+        else { a.eidx = r.eidx + s0 * estride(N, M); a.esc = r.esc + s0 * estride(N, M); }
+        a.mstart = r.mstart + s0 * mstride(N);
         a.ckpt = sc.ckpt; a.wck = sc.wck; a.agg = sc.agg;
         a.out   = out ? out + (size_t)p0 * M * C4 : nullptr;
         a.g     = g ? g + (size_t)p0 * M * C4 : nullptr;
@@ -376,7 +386,7 @@ struct LaplaceWs {
         vpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         opad = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         rec.carve(b, nseg, N, M);
-        walk.carve(b, P, D, N, C4);
+        walk.carve(b, P, D, N, M, C4, false);
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
@@ -391,8 +401,8 @@ struct LaplaceBwdWs {
         gpad  = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         gvpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         const int mx = N > M ? N : M;
-        rec.carve(b, nseg, mx, mx);
-        walk.carve(b, P, D, mx, C4);            // one scratch for both walks (stream of keys k, then stream of keys q): sized for the longer
+        rec.carve(b, nseg, mx, mx, false, N + M);
+        walk.carve(b, P, D, N, M, C4, true);     // one scratch for both walks (stream of keys k, then stream of keys q)
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
@@ -428,7 +438,7 @@ struct AbsBwdWs {
         gpad  = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         gvpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         const int mx = N > M ? N : M;
-        rec.carve(b, nseg, mx, mx);
+        rec.carve(b, nseg, mx, mx, false, N + M);
         qsumd = b.take<float>((size_t)P * M);
         sums  = b.take<float>((size_t)P * C4 * 3 + P);
         const size_t agg_k = prefix_agg_floats(P, D, N, C4), agg_q = prefix_agg_floats(P, D, M, C4);
@@ -1220,7 +1230,7 @@ int qlka_sort_rank_records(const float* x, const float* y,
     qlka_sort_rank_workspace_bytes(P, D, N, M, &need);
     if (!ws_ok(workspace, workspace_bytes, need)) return QLKA_ERR_WORKSPACE;
     Bump b(workspace);
-    Records r;
+    Records r{};
     r.xperm = xperm; r.xval = xval; r.yrec = reinterpret_cast<uint4*>(yrec); r.mstart = mstart;
     r.su0 = b.take<float>((size_t)P * D * (N + 1));
     r.su1 = b.take<float>((size_t)P * D * (N + 1));

@@ -13,6 +13,14 @@
 //                                  entry M is a sentinel with rank 0xffffffff
 //   mstart[seg][NBK + 1]   uint32  first query whose rank is >= b*KB, for every key block b
 //
+// The walks that need a row per query as well as per key (walk_events.cu) read keys and queries as one list in walk order
+// instead of yrec, a query before the first key that is not below it:
+//
+//   eidx  [seg][ES]        uint32  row index of the event; EVENT_QUERY is set in a query's
+//   esc   [seg][ES]        float2  key: {step decay, 0} (Laplace), {-2 key, 0} (abs); query: {e0, e1}
+//
+// with ES = estride(N + M); sorted key j is event j + (queries of rank <= j), query m of rank r event m + r.
+//
 // with KB = 8 keys per block, NBK = N/KB + 1 blocks and NP = NBK*KB padded keys, so that at
 // least one padded position follows the last key and every rank in [0, N] falls in a block.
 #pragma once
@@ -28,6 +36,10 @@ __host__ __device__ inline int       nblocks(int N)  { return N / KB + 1; }
 __host__ __device__ inline int       npad(int N)     { return nblocks(N) * KB; }
 __host__ __device__ inline long long xstride(int N)  { return (long long)npad(N) + KB; }
 __host__ __device__ inline long long mstride(int N)  { return (long long)((nblocks(N) + 1 + 3) & ~3); }
+
+constexpr int      EB = 8;                  // events per block of the walk over events
+constexpr uint32_t EVENT_QUERY = 0x80000000u;
+__host__ __device__ inline long long estride(int N, int M) { return ((long long)N + M + EB - 1) / EB * EB; }
 
 enum SortMode : int { MODE_LAPLACE = 0, MODE_ABS = 1, MODE_SGN = 2 };
 // scalar side channel of the sort/rank kernel
@@ -45,7 +57,9 @@ struct SortArgs {
     const float* y;          // (P, D, M) queries
     uint32_t*    xperm;
     float*       xval;
-    uint4*       yrec;
+    uint4*       yrec;       // or null
+    uint32_t*    eidx;       // the event list, or null
+    float2*      esc;
     uint32_t*    mstart;
     float*       su0;        // [seg][N + 1] scratch for the scalar scans
     float*       su1;
@@ -85,8 +99,10 @@ struct WalkArgs {
     const float*    xval;
     const uint4*    yrec;
     const uint32_t* mstart;
-    float*          ckpt;     // Laplace: [seg][NBK][C4] suffix checkpoints, written by the first pass
-    float*          wck;      // Laplace: [seg][NBK]
+    const uint32_t* eidx;
+    const float2*   esc;
+    float*          ckpt;     // Laplace: [seg][blocks][C4] suffix checkpoints, written by the first pass (blocks of keys; with dots of events)
+    float*          wck;      // Laplace: [seg][blocks], with dots [seg][blocks][2]
     float*          agg;      // [seg * sps + stream][...] per-stream aggregates of the first pass (layout per walk)
     float*          out;      // emit rows: (P, M, C4), accumulated with vector reductions
     const float*    g;        // emit dot: (P, M, C4) matrix contracted with the walk state

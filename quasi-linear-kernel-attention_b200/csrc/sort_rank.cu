@@ -314,13 +314,14 @@ __device__ __forceinline__ int lower_bound_f(const float* __restrict__ a, const 
 // cursor), which also yields mstart for free; the records are then built in position order. Queries of
 // equal rank come out in arbitrary order,
 // which the walk does not care about.
-// The kernel is compiled in four variants, so that each carries only the code of its own case (the whole kernel
+// The kernel is compiled in five variants, so that each carries only the code of its own case (the whole kernel
 // runs once per segment, straight through: instruction fetch is its most frequent stall, and dead branches cost):
 //   VAR_LAP         Laplace records, optional unit-column side channel
-//   VAR_LAP_SIGNED  Laplace records with the SCAL_SIGNED side channel (its scans run through shared memory)
-//   VAR_ABS         abs / sgn records, the queries as given
+//   VAR_LAP_SIGNED  Laplace events, optional SCAL_SIGNED side channel (its scans run through shared memory)
+//   VAR_ABS         abs records, the queries as given
 //   VAR_ABS_FOLD    abs records over folded (shifted, weighted) query copies
-enum SortVariant : int { VAR_LAP = 0, VAR_LAP_SIGNED = 1, VAR_ABS = 2, VAR_ABS_FOLD = 3 };
+//   VAR_ABS_SIGNED  abs / sgn events
+enum SortVariant : int { VAR_LAP = 0, VAR_LAP_SIGNED = 1, VAR_ABS = 2, VAR_ABS_FOLD = 3, VAR_ABS_SIGNED = 4 };
 
 // Value buckets per segment (see phase (1) of the kernel): the more, the shorter the in-bucket ranking and the rank search.
 // The 1024-thread kernel has its SM to itself and takes what its shared memory still holds (just under one bucket per
@@ -333,6 +334,7 @@ template <int THREADS, int E, int VAR, bool PART>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const SortArgs a, const PartArgs pa)
 {
     constexpr bool LAP = VAR == VAR_LAP || VAR == VAR_LAP_SIGNED, SIGNED = VAR == VAR_LAP_SIGNED, FOLD = VAR == VAR_ABS_FOLD;
+    constexpr bool EVENTS = VAR == VAR_LAP_SIGNED || VAR == VAR_ABS_SIGNED;
     constexpr int CAP = THREADS * E;
     constexpr int W   = THREADS / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -368,7 +370,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
 
     uint32_t* xperm  = a.xperm + (long long)seg * NP + ks;
     float*    xval   = a.xval + (long long)seg * xstride(NG) + ks;
-    uint4*    yrec   = a.yrec + (long long)seg * (MG + 1) + qs;
+    uint4*    yrec   = a.yrec + (long long)seg * (MG + 1) + qs;                             // (one of the two)
+    uint32_t* eidx   = a.eidx + (long long)seg * estride(NG, MG) + ks + qs;
+    float2*   esc    = a.esc + (long long)seg * estride(NG, MG) + ks + qs;
     uint32_t* mstart = a.mstart + (long long)seg * mstride(NG);
     float*    su0    = a.su0 ? a.su0 + (long long)seg * (NG + 1) + ks : nullptr;
     float*    su1    = a.su1 ? a.su1 + (long long)seg * (NG + 1) + ks : nullptr;
@@ -639,6 +643,13 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         }
         return make_uint4(__float_as_uint(e0), __float_as_uint(e1), (uint32_t)row, (uint32_t)(ks + r));
     };
+    auto store_record = [&](const int pos, const int r, const uint4& rec) {
+        if (!EVENTS) yrec[pos] = rec;
+        else {
+            eidx[pos + r] = rec.z | EVENT_QUERY;
+            esc[pos + r]  = make_float2(__uint_as_float(rec.x), __uint_as_float(rec.y));
+        }
+    };
     uint32_t rp[E];                                   // rank, later rank | position << 16 (both <= 16384)
     // Slot s of a thread is query tid + ((s + rot) mod E) * THREADS with rot the segment index: the D segments of a head
     // run at the same time and all add into the same out_u row, and with a common visiting order their atomics would
@@ -690,7 +701,16 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         for (int b = (ks + (first ? 0 : 1) + KB - 1) / KB + tid; b * KB <= ks + N; b += THREADS) mstart[b] = (uint32_t)qs + hist[b * KB - ks];
         if (first && tid == 0) {
             mstart[NBK] = (uint32_t)MG;
-            a.yrec[(long long)seg * (MG + 1) + MG] = make_uint4(0u, 0u, 0u, 0xffffffffu);      // sentinel: a rank no key position has
+            if (!EVENTS) a.yrec[(long long)seg * (MG + 1) + MG] = make_uint4(0u, 0u, 0u, 0xffffffffu);      // sentinel: a rank no key position has
+        }
+        if (EVENTS) {                                 // the keys' events: hist[j + 1] queries of this part precede key j
+            #pragma unroll 2
+            for (int j = tid; j < N; j += THREADS) {
+                const uint32_t e = (uint32_t)j + hist[j + 1];
+                eidx[e] = xperm[j];
+                if (LAP)                     esc[e] = make_float2(xval[j], 0.0f);
+                else if (a.mode == MODE_ABS) esc[e] = make_float2(-2.0f * xs[skew(j)], 0.0f);
+            }
         }
         __syncthreads();
     };
@@ -717,7 +737,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                     const int   r = (int)rank, row = query_row(m);
                     const float y = yval(m);
                     if (side) side_channel(m, row, r, y, su0s, lap ? su1 : su0);
-                    yrec[atomicAdd(&hist[r], 1u)] = record(m, row, r, y);
+                    store_record((int)atomicAdd(&hist[r], 1u), r, record(m, row, r, y));
                 }
             }
             if (sweep == 0) scan_ranks();
@@ -777,7 +797,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     for (int pos = tid; pos < M; pos += THREADS) {
         const uint32_t w = who[pos];
         const int      m = (int)(w & ((1u << WHO) - 1u)), r = (int)(w >> WHO);
-        yrec[pos] = record(m, FOLD ? m % MR : m, r, ypos[pos]);
+        store_record(pos, r, record(m, FOLD ? m % MR : m, r, ypos[pos]));
     }
     PHASE_MARK(6);
 }
@@ -801,7 +821,8 @@ template <int THREADS, int E>
 static cudaError_t launch_one(const SortArgs& a, cudaStream_t stream) {
     const PartArgs none{};
     if (a.mode == MODE_LAPLACE)
-        return a.scal == SCAL_SIGNED ? launch_inst<THREADS, E, VAR_LAP_SIGNED, false>(a, none, stream) : launch_inst<THREADS, E, VAR_LAP, false>(a, none, stream);
+        return a.eidx ? launch_inst<THREADS, E, VAR_LAP_SIGNED, false>(a, none, stream) : launch_inst<THREADS, E, VAR_LAP, false>(a, none, stream);
+    if (a.eidx) return launch_inst<THREADS, E, VAR_ABS_SIGNED, false>(a, none, stream);
     return a.fold ? launch_inst<THREADS, E, VAR_ABS_FOLD, false>(a, none, stream) : launch_inst<THREADS, E, VAR_ABS, false>(a, none, stream);
 }
 
@@ -809,7 +830,8 @@ static cudaError_t launch_one(const SortArgs& a, cudaStream_t stream) {
 cudaError_t launch_sort_rank_parts(const SortArgs& a, const PartArgs& pa, cudaStream_t stream) {
     constexpr int T = 512, E = PART_CAP / T;
     if (a.mode == MODE_LAPLACE)
-        return a.scal == SCAL_SIGNED ? launch_inst<T, E, VAR_LAP_SIGNED, true>(a, pa, stream) : launch_inst<T, E, VAR_LAP, true>(a, pa, stream);
+        return a.eidx ? launch_inst<T, E, VAR_LAP_SIGNED, true>(a, pa, stream) : launch_inst<T, E, VAR_LAP, true>(a, pa, stream);
+    if (a.eidx) return launch_inst<T, E, VAR_ABS_SIGNED, true>(a, pa, stream);
     return launch_inst<T, E, VAR_ABS, true>(a, pa, stream);
 }
 

@@ -1,12 +1,8 @@
 // Laplace walk: out[p, row_m, :] += e0_m * L_{r-1} + e1_m * R_r for every query m of every
 // segment, where r is the query's rank, L the decayed prefix sum of the gathered rows and R
 // the decayed suffix sum (recurrences of Weighted_Laplace_Sum/csrc/laplace_kernels.cu:5-13).
-// Two more emissions serve the gradients of the sum, which the reference does not have (its
-// training route is the chunked PyTorch path, Experiments/kernel_attention/attention.py:110-115):
-//   LAP_DOT   out_s[seg, row_m] += <g[p, row_m, :], e1_m * R_r - e0_m * L_{r-1}>   (d/dquery of the sum,
-//             contracted with the upstream gradient; one writer per element, added to the scalar
-//             term that the sort/rank kernel stored there)
-//   LAP_BOTH  the row reduction and the dot from one walk (grad_v and grad_k share stream and queries)
+// LAP_DOT and LAP_BOTH, the walks of the gradients of the sum, share the fold between the passes; their passes are in walk_events.cu.
+// (The reference's training route is the chunked PyTorch path, Experiments/kernel_attention/attention.py:110-115.)
 //
 // Replaces the reference's laplace_chunk / laplace_scan / laplace_walk trio
 // (laplace_kernels.cu:65-127, 134-188, 219-409) with two launches over independent work units:
@@ -28,14 +24,16 @@
 
 namespace qlka {
 
+cudaError_t launch_laplace_events1(const WalkArgs& a, int sms, cudaStream_t stream);      // walk_events.cu
+cudaError_t launch_laplace_events2(const WalkArgs& a, bool rows, int sms, cudaStream_t stream);
+
 enum { LAP_ROWS = 0, LAP_DOT = 1, LAP_BOTH = 2 };
 
 // resident CTAs per SM that the emitting pass is compiled for, and blocks in its rings: three CTAs with one stream per warp (two: 3.34
-// instead of 3.02 ms at 48 heads x 16384 keys; four leave 64 registers: 4.1 ms); two blocks where the emit-side rows want
-// shared memory and copies of their own (three: backward 4.1 -> 4.4 ms at 48 x 4096).
+// instead of 3.02 ms at 48 heads x 16384 keys; four leave 64 registers: 4.1 ms)
 constexpr int LAP_CTAS1 = 3, LAP_CTAS_ROWS = 2;
 __host__ __device__ constexpr int lap_ctas2(int cpl) { return cpl == 4 ? 2 : 3; }
-__host__ __device__ constexpr int lap_depth2(int emit) { return emit == LAP_ROWS ? 3 : 2; }
+constexpr int LAP_DEPTH2 = 3;
 
 // floats per stream in the aggregate table: forward aggregate | backward aggregate | decay forward, decay backward, pad
 __host__ __device__ inline int lap_agg_stride(int C4) { return 2 * C4 + 4; }
@@ -152,21 +150,20 @@ __global__ void __launch_bounds__(32 * FOLD_WARPS) laplace_fold(float* __restric
     }
 }
 
-template <int CPL, int EMIT>
+// The second pass with a warp per stream
+template <int CPL>
 __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(const WalkArgs a)
 {
-    constexpr bool DO_ROWS = EMIT != LAP_DOT, DO_DOT = EMIT != LAP_ROWS;
-    constexpr int  DEPTH = lap_depth2(EMIT);
-    using F2 = Feeder<CPL, true, DEPTH>;
+    using F2 = Feeder<CPL, true, LAP_DEPTH2>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = warp_index(), c0 = lane * CPL;
-    const int N = a.N, M = a.M, C4 = a.C4, NBK = nblocks(N);
+    const int N = a.N, C4 = a.C4, NBK = nblocks(N);
     const bool lane_on = c0 < C4;
     const int  c0l     = lane_on ? c0 : 0;         // idle lanes shadow lane 0's loads and store nothing
     const int  AGS     = lap_agg_stride(C4);
 
     F2 f;
-    f.init(smem_u32(smem) + warp * warp_bytes<CPL, DEPTH>(DO_DOT), lane, N, C4);
+    f.init(smem_u32(smem) + warp * warp_bytes<CPL, LAP_DEPTH2>(), lane, N, C4);
 
     // static round-robin over the work items (an atomic work counter was measured 10 % slower)
     for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
@@ -174,9 +171,7 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
         if (!st.on) break;
         const int b0 = st.b0, nblk = st.nblk;
         f.start(a, st.sg, st.p, b0);
-        char*  out   = DO_ROWS ? reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l) : nullptr;
-        float* out_s = DO_DOT ? a.out_s + (long long)st.sg * M : nullptr;
-        if (DO_DOT) f.start_dots(a, st.p);
+        char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
         const float* ck = a.ckpt + ((long long)st.sg * NBK + b0 + 1) * C4 + c0l;      // of the next block to fetch
         const float* wk = a.wck + (long long)st.sg * NBK + b0 + 1;
 
@@ -194,24 +189,14 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
         int cur = 0, j0 = b0 * KB;
         for (int t = 0; t < nblk; t++, j0 += KB, cur = F2::next_slot(cur)) {
             f.advance_range();
-            if (DO_DOT) {
-                // the block's copies have had whole iterations; once its records are readable the emit-side rows
-                // of its first G_SLOTS queries start, ahead of the next block's copies, and land during the arithmetic
-                cp_async_wait<F2::AHEAD - 1>();
-                __syncwarp();
-                f.issue_g(cur, j0, 0u);
-            } else {
-                __syncwarp();
-            }
+            __syncwarp();
             // suffix state entering the block from above: corrected checkpoint, or the stream's incoming state
             Vec<CPL> Rn = Rin;
             if (t + 1 < nblk) axpy(Rn, wnext, Rin, cnext);
             if (t + 2 < nblk) load_ckpt();
             f.step_issue(t, cur, nblk);
-            if (!DO_DOT) {
-                cp_async_wait<F2::AHEAD>();
-                __syncwarp();
-            }
+            cp_async_wait<F2::AHEAD>();
+            __syncwarp();
             float av[KB + 1];
             f.read_scalars(cur, av);
             Vec<CPL> v[KB], Rb[KB];
@@ -228,33 +213,12 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
                 v[i] = L;
                 axpy(L, av[i], L, row);
             }
-            if (DO_DOT) {
-                cp_async_wait<1>();               // the emit-side rows are in; the next block's copies may still fly
-                __syncwarp();                     // every lane has its rows in registers: the slot may hold partial dots
-            }
-            const uint32_t g_lane = DO_DOT ? f.g_lane() : 0u, part_lane = f.part_lane(cur);
-            auto emit = [&](const int i, const uint4& rec, const uint32_t n128) {
-                const float e0 = __uint_as_float(rec.x), e1 = __uint_as_float(rec.y);
-                if (DO_ROWS) {
-                    Vec<CPL> r;
-                    scale(r, e1, Rb[i]);
-                    axpy(r, e0, v[i], r);
-                    if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
-                }
-                if (DO_DOT) {
-                    const Vec<CPL> gq = vload_shared<CPL>(g_lane + n128 * CPL);
-                    float part = 0.0f;
-                    #pragma unroll
-                    for (int c = 0; c < CPL; c++) part = fmaf(gq.x[c], fmaf(e1, Rb[i].x[c], -e0 * v[i].x[c]), part);
-                    sts32f(part_lane + n128, lane_on ? part : 0.0f);
-                }
-            };
-            auto finish = [&](const uint32_t n0, const uint32_t n1) {
-                const float    sum = f.sum_parts(cur);
-                const uint32_t n   = n0 + (lane >> 2);
-                if ((lane & 3) == 0 && n < n1) atomicAdd(out_s + lds32u(f.records(cur) + n * 16 + 8), sum);
-            };
-            for_queries<DO_DOT>(f, cur, j0, emit, finish);
+            for_queries(f, cur, j0, [&](const int i, const uint4& rec) {
+                Vec<CPL> r;
+                scale(r, __uint_as_float(rec.y), Rb[i]);
+                axpy(r, __uint_as_float(rec.x), v[i], r);
+                if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
+            });
         }
         cp_async_wait<0>();
     }
@@ -341,40 +305,38 @@ static cudaError_t launch_lap_rows(const WalkArgs& a, int sms, cudaStream_t stre
     return cudaGetLastError();
 }
 
-template <int CPL, int EMIT>
+template <int CPL>
 static cudaError_t launch_lap_pass2(const WalkArgs& a, int sms, cudaStream_t stream) {
-    constexpr int smem = WALK_STREAMS * warp_bytes<CPL, lap_depth2(EMIT)>(EMIT != LAP_ROWS);
-    cudaError_t e = cudaFuncSetAttribute(laplace_pass2<CPL, EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int smem = WALK_STREAMS * warp_bytes<CPL, LAP_DEPTH2>();
+    cudaError_t e = cudaFuncSetAttribute(laplace_pass2<CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int cap = sms * lap_ctas2(CPL);
-    laplace_pass2<CPL, EMIT><<<a.nitems < cap ? a.nitems : cap, WALK_THREADS, smem, stream>>>(a);
+    laplace_pass2<CPL><<<a.nitems < cap ? a.nitems : cap, WALK_THREADS, smem, stream>>>(a);
     return cudaGetLastError();
 }
 
-template <int LPS, int CPL, int EMIT>
-static cudaError_t launch_lap(const WalkArgs& a, int sms, cudaStream_t stream, cudaEvent_t mid) {
-    constexpr int smem1 = sum_smem_bytes<LPS>();
-    cudaError_t e = cudaFuncSetAttribute(laplace_pass1<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
+template <int LPS>
+static cudaError_t launch_lap_pass1(const WalkArgs& a, int sms, cudaStream_t stream) {
+    constexpr int smem = sum_smem_bytes<LPS>();
+    cudaError_t e = cudaFuncSetAttribute(laplace_pass1<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const long long items1 = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
-    const int cap1 = sms * LAP_CTAS1;
-    laplace_pass1<LPS><<<items1 < cap1 ? (int)items1 : cap1, WALK_THREADS, smem1, stream>>>(a);
+    const long long items = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
+    const int cap = sms * LAP_CTAS1;
+    laplace_pass1<LPS><<<items < cap ? (int)items : cap, WALK_THREADS, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+template <int LPS, int CPL>
+static cudaError_t launch_lap(const WalkArgs& a, int emit, int sms, cudaStream_t stream, cudaEvent_t mid) {
+    cudaError_t e = emit == LAP_ROWS ? launch_lap_pass1<LPS>(a, sms, stream) : launch_laplace_events1(a, sms, stream);
+    if (e != cudaSuccess) return e;
     laplace_fold<<<fold_grid(a), 32 * FOLD_WARPS, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4, fold_share_warps(a));
     e = cudaGetLastError();
     if (e == cudaSuccess && mid) e = cudaEventRecord(mid, stream);
     if (e != cudaSuccess) return e;
-    if constexpr (EMIT == LAP_ROWS) {
-        if (CPL == 4 || rows_by_quads(a)) return launch_lap_rows<LPS>(a, sms, stream);
-    }
-    if constexpr (EMIT != LAP_ROWS || CPL < 4) return launch_lap_pass2<CPL, EMIT>(a, sms, stream);
-}
-
-template <int EMIT>
-static cudaError_t launch_lap_c(const WalkArgs& a, int sms, cudaStream_t stream, cudaEvent_t mid) {
-    if (a.C4 <= 32)  return launch_lap<8, 1, EMIT>(a, sms, stream, mid);
-    if (a.C4 <= 64)  return launch_lap<16, 2, EMIT>(a, sms, stream, mid);
-    if (a.C4 <= 128) return launch_lap<32, 4, EMIT>(a, sms, stream, mid);
-    return cudaErrorInvalidValue;
+    if (emit != LAP_ROWS) return launch_laplace_events2(a, emit == LAP_BOTH, sms, stream);
+    if (CPL == 4 || rows_by_quads(a)) return launch_lap_rows<LPS>(a, sms, stream);
+    if constexpr (CPL < 4) return launch_lap_pass2<CPL>(a, sms, stream);
 }
 
 int laplace_agg_stride(int C4) { return lap_agg_stride(C4); }
@@ -382,9 +344,9 @@ int laplace_agg_stride(int C4) { return lap_agg_stride(C4); }
 // emit: 0 = row reductions (the forward sum), 1 = dot, 2 = both;
 // mid: optional event recorded between the first pass (with the fold) and the second
 cudaError_t launch_laplace_walk(const WalkArgs& a, int emit, int sms, cudaStream_t stream, cudaEvent_t mid) {
-    if (emit == LAP_ROWS) return launch_lap_c<LAP_ROWS>(a, sms, stream, mid);
-    if (emit == LAP_DOT)  return launch_lap_c<LAP_DOT>(a, sms, stream, mid);
-    if (emit == LAP_BOTH) return launch_lap_c<LAP_BOTH>(a, sms, stream, mid);
+    if (a.C4 <= 32)  return launch_lap<8, 1>(a, emit, sms, stream, mid);
+    if (a.C4 <= 64)  return launch_lap<16, 2>(a, emit, sms, stream, mid);
+    if (a.C4 <= 128) return launch_lap<32, 4>(a, emit, sms, stream, mid);
     return cudaErrorInvalidValue;
 }
 

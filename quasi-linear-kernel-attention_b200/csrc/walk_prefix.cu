@@ -5,12 +5,8 @@
 //              with e0 = 2 * query and e1 = -2 this is the walk term 2 (q PV - PK) of the abs sum; folded
 //              queries (shifted, weighted copies that share a row) scale both by their weight
 //              (Weighted_Abs_Sum/csrc/abs_kernels.cu:9-18; abs_chunk :78-199, abs_prefix :202-405)
-//   EMIT_DOT   out_s[seg, row_m] = sign * ( <g[p, row_m, :], 2 PV - wtotal[p, :]> + e1_m )
-//              the signed-rank walk behind grad_q, grad_k and the public sgn op
-//              (Weighted_Abs_Sum/csrc/sgn_kernels.cu:8-15, sgn_prefix :17-192); one writer per
-//              output element, plain stores.
-//   EMIT_BOTH  both from one walk over the same stream, rows and queries (grad_v and grad_k); the rows are
-//              e0_m * (PV - wtotal[p, :] / 2) - 2 PK, the record's e1 belongs to the dot
+//
+// EMIT_DOT and EMIT_BOTH (the walks of the gradients) share the first launch and the fold; their emission is in walk_events.cu.
 //
 // Same mapping and staging as the Laplace walk (walk_ring.cuh; SPS independent streams per
 // segment numbered over all segments, persistent CTAs). The first launch sums each stream's rows into an aggregate
@@ -20,12 +16,14 @@
 
 namespace qlka {
 
+cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, int sms, cudaStream_t stream);      // walk_events.cu
+
 enum { EMIT_ROWS = 0, EMIT_DOT = 1, EMIT_BOTH = 2 };
 
 // resident CTAs per SM that the passes are compiled for, and blocks in the emitting pass's rings (as in the Laplace walk)
 constexpr int PREFIX_CTAS1 = 3, PREFIX_CTAS_ROWS = 2;
-__host__ __device__ constexpr int prefix_ctas2(int cpl, int emit) { return cpl == 4 ? 2 : emit == EMIT_BOTH ? 3 : 4; }
-__host__ __device__ constexpr int prefix_depth2(int emit) { return emit == EMIT_ROWS ? 3 : 2; }
+__host__ __device__ constexpr int prefix_ctas2(int cpl) { return cpl == 4 ? 2 : 4; }
+constexpr int PREFIX_DEPTH2 = 3;
 
 // floats per stream in the aggregate table: sum of the stream's rows | sum of key * row
 __host__ __device__ inline int prefix_agg_stride(int C4) { return 2 * C4; }
@@ -117,45 +115,33 @@ __global__ void __launch_bounds__(32 * FOLD_WARPS) prefix_fold(float* __restrict
     }
 }
 
-// Last launch: the walk with emission, every stream starting from its incoming prefix sums. With dots the walk carries
-// H = PV - wtotal / 2 and T = -2 PK, so that a query costs one fused multiply-add per channel for its dot (<g, H>, doubled when it is
-// written) and one for its row (e0 H + T: the caller's rows start without the - query * wtotal that H brings along). These walks are
-// bound by instruction issue; with PV and PK, and the whole record read for its rank, abs backward at 16 heads x 8192 keys x 128
-// channels took 3.98 instead of 3.63 ms, at 96 x 4096 x 64 6.75 instead of 6.64.
-template <int CPL, int EMIT>
-__global__ void __launch_bounds__(WALK_THREADS, prefix_ctas2(CPL, EMIT)) prefix_pass2(const WalkArgs a)
+// Last launch: the walk with row emission, every stream starting from its incoming prefix sums, one stream per warp.
+template <int CPL>
+__global__ void __launch_bounds__(WALK_THREADS, prefix_ctas2(CPL)) prefix_pass2(const WalkArgs a)
 {
-    constexpr bool DO_ROWS = EMIT != EMIT_DOT, DO_DOT = EMIT != EMIT_ROWS, WITH_K = DO_ROWS;
-    constexpr int  DEPTH = prefix_depth2(EMIT);
-    using F2 = Feeder<CPL, WITH_K, DEPTH>;
+    using F2 = Feeder<CPL, true, PREFIX_DEPTH2>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = warp_index(), c0 = lane * CPL;
-    const int N = a.N, M = a.M, C4 = a.C4, NBK = nblocks(N);
+    const int N = a.N, C4 = a.C4, NBK = nblocks(N);
     const bool lane_on = c0 < C4;
     const int  c0l     = lane_on ? c0 : 0;         // idle lanes shadow lane 0's loads and store nothing
 
     F2 f;
-    f.init(smem_u32(smem) + warp * warp_bytes<CPL, DEPTH>(DO_DOT), lane, N, C4);
+    f.init(smem_u32(smem) + warp * warp_bytes<CPL, PREFIX_DEPTH2>(), lane, N, C4);
 
     // static round-robin over the work items (an atomic work counter was measured 10 % slower)
     for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
         const StreamOf st(a, item, warp, NBK);
         if (!st.on) break;
         f.start(a, st.sg, st.p, st.b0);
-        char*  out   = DO_ROWS ? reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l) : nullptr;
-        float* out_s = DO_DOT ? a.out_s + (long long)st.sg * M : nullptr;
-        if (DO_DOT) f.start_dots(a, st.p);
+        char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
 
-        Vec<CPL> PV, PK;        // (with dots H and T)
+        Vec<CPL> PV, PK;
         PV.zero(); PK.zero();
         if (a.sps > 1) {        // incoming prefix sums (prefix_fold left them in the aggregate table)
             const float* ag = a.agg + st.g * prefix_agg_stride(C4) + c0l;
             PV = vload<CPL>(ag);
-            if (WITH_K) PK = vload<CPL>(ag + C4);
-        }
-        if (DO_DOT) {
-            axpy(PV, -0.5f, vload<CPL>(a.wtotal + (long long)st.p * C4 + c0l), PV);
-            if (WITH_K) scale(PK, -2.0f, PK);
+            PK = vload<CPL>(ag + C4);
         }
 
         __syncwarp();                              // every lane has left the previous item's slots
@@ -163,63 +149,29 @@ __global__ void __launch_bounds__(WALK_THREADS, prefix_ctas2(CPL, EMIT)) prefix_
         int cur = 0, j0 = st.b0 * KB;
         for (int t = 0; t < st.nblk; t++, j0 += KB, cur = F2::next_slot(cur)) {
             f.advance_range();
-            if (DO_DOT) {
-                // the block's copies have had whole iterations; once its records are readable the emit-side rows
-                // of its first G_SLOTS queries start, ahead of the next block's copies, and land during the arithmetic
-                cp_async_wait<F2::AHEAD - 1>();
-                __syncwarp();
-                f.issue_g(cur, j0, 0u);
-                f.step_issue(t, cur, st.nblk);
-            } else {
-                __syncwarp();
-                f.step_issue(t, cur, st.nblk);
-                cp_async_wait<F2::AHEAD>();
-                __syncwarp();
-            }
+            __syncwarp();
+            f.step_issue(t, cur, st.nblk);
+            cp_async_wait<F2::AHEAD>();
+            __syncwarp();
             float kv[KB + 1];
-            if (WITH_K) f.read_scalars(cur, kv);
-            Vec<CPL> v[KB], kb[WITH_K ? KB : 1];
+            f.read_scalars(cur, kv);
+            Vec<CPL> v[KB], kb[KB];
             f.read_rows(cur, j0, v);
             // prefix states before each key, in place of the rows
             #pragma unroll
             for (int i = 0; i < KB; i++) {
                 const Vec<CPL> row = v[i];
-                v[i] = PV;
+                v[i]  = PV;
+                kb[i] = PK;
                 vadd(PV, row);
-                if (WITH_K) {
-                    kb[i] = PK;
-                    axpy(PK, DO_DOT ? -2.0f * kv[i] : kv[i], row, PK);
-                }
+                axpy(PK, kv[i], row, PK);
             }
-            if (DO_DOT) {
-                cp_async_wait<1>();               // the emit-side rows are in; the next block's copies may still fly
-                __syncwarp();                     // every lane has its rows in registers: the slot may hold partial dots
-            }
-            const uint32_t g_lane = DO_DOT ? f.g_lane() : 0u, part_lane = f.part_lane(cur);
-            auto emit = [&](const int i, const uint4& rec, const uint32_t n128) {
-                if (DO_ROWS) {
-                    Vec<CPL> r = kb[WITH_K ? i : 0];
-                    if (!DO_DOT) scale(r, __uint_as_float(rec.y), r);
-                    axpy(r, __uint_as_float(rec.x), v[i], r);
-                    if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
-                }
-                if (DO_DOT) {
-                    const Vec<CPL> gq = vload_shared<CPL>(g_lane + n128 * CPL);
-                    float part = 0.0f;
-                    #pragma unroll
-                    for (int c = 0; c < CPL; c++) part = fmaf(gq.x[c], v[i].x[c], part);
-                    sts32f(part_lane + n128, lane_on ? part : 0.0f);
-                }
-            };
-            auto finish = [&](const uint32_t n0, const uint32_t n1) {
-                const float    sum = f.sum_parts(cur);
-                const uint32_t n   = n0 + (lane >> 2);
-                if ((lane & 3) == 0 && n < n1) {
-                    const uint4 r = lds128u(f.records(cur) + n * 16);
-                    out_s[r.z] = a.sign * fmaf(2.0f, sum, __uint_as_float(r.y));
-                }
-            };
-            for_queries<DO_DOT, DO_ROWS>(f, cur, j0, emit, finish);
+            for_queries(f, cur, j0, [&](const int i, const uint4& rec) {
+                Vec<CPL> r;
+                scale(r, __uint_as_float(rec.y), kb[i]);
+                axpy(r, __uint_as_float(rec.x), v[i], r);
+                if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
+            });
         }
         cp_async_wait<0>();
     }
@@ -294,11 +246,11 @@ static cudaError_t launch_rows(const WalkArgs& a, int sms, cudaStream_t stream) 
     return cudaGetLastError();
 }
 
-template <int CPL, int EMIT>
+template <int CPL>
 static cudaError_t launch_pass2(const WalkArgs& a, int sms, cudaStream_t stream) {
-    auto k2 = prefix_pass2<CPL, EMIT>;
-    constexpr int smem2 = WALK_STREAMS * warp_bytes<CPL, prefix_depth2(EMIT)>(EMIT != EMIT_ROWS);
-    const int cap2 = sms * prefix_ctas2(CPL, EMIT);
+    auto k2 = prefix_pass2<CPL>;
+    constexpr int smem2 = WALK_STREAMS * warp_bytes<CPL, PREFIX_DEPTH2>();
+    const int cap2 = sms * prefix_ctas2(CPL);
     cudaError_t e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
     if (e != cudaSuccess) return e;
     k2<<<a.nitems < cap2 ? a.nitems : cap2, WALK_THREADS, smem2, stream>>>(a);
@@ -324,12 +276,9 @@ static cudaError_t launch_pw(const WalkArgs& a, int emit, int sms, cudaStream_t 
         cudaError_t e = emit == EMIT_DOT ? launch_pass1<LPS, false>(a, sms, stream) : launch_pass1<LPS, true>(a, sms, stream);
         if (e != cudaSuccess) return e;
     }
-    if (emit == EMIT_ROWS) {
-        if (CPL == 4 || rows_by_quads(a)) return launch_rows<LPS>(a, sms, stream);
-        if constexpr (CPL < 4) return launch_pass2<CPL, EMIT_ROWS>(a, sms, stream);
-    }
-    if (emit == EMIT_DOT)  return launch_pass2<CPL, EMIT_DOT>(a, sms, stream);
-    return launch_pass2<CPL, EMIT_BOTH>(a, sms, stream);
+    if (emit != EMIT_ROWS) return launch_prefix_events(a, emit == EMIT_BOTH, sms, stream);
+    if (CPL == 4 || rows_by_quads(a)) return launch_rows<LPS>(a, sms, stream);
+    if constexpr (CPL < 4) return launch_pass2<CPL>(a, sms, stream);
 }
 
 int prefix_agg_stride_host(int C4) { return prefix_agg_stride(C4); }

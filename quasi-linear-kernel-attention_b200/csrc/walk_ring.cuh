@@ -2,9 +2,7 @@
 //
 // Emitting passes (Feeder): one warp walks one stream (a contiguous run of key blocks of a segment). Lane l owns the CPL
 // consecutive channels from l * CPL on, with CPL = 1, 2 or 4 for up to 32, 64 or 128 channels, so that every loop below is uniform
-// over the warp (two or four streams per warp, with 4 channels per lane whatever the width, spent half of their instructions on
-// diverged emission loops and left room for two CTAs per SM instead of three or four: Laplace backward at 48 heads x 4096 keys 5.6 ->
-// 4.1 ms, abs backward with 32 channels 4.2 -> 2.8 ms).
+// over the warp.
 // First passes (SumFeeder), which have nothing that diverges, keep 4 channels per lane and 1, 2 or 4 streams per warp: they are
 // bound by instruction issue, and a warp per stream took 1.35 instead of 1.02 ms at 48 heads x 16384 keys.
 //
@@ -15,13 +13,6 @@
 // a warp barrier at the top of the next iteration lets the slot be refilled. Blocks with QCAP queries or more read the further
 // records into the same place. The blocks' query ranges travel in registers. Shared memory is addressed with 32-bit
 // shared-window addresses throughout.
-//
-// Walks that contract their state with a row of a second matrix per query (the dot emissions) need that row, whose index is
-// only known once the query's record has arrived: the rows of up to G_SLOTS of the block's queries are copied into a third area
-// as soon as the block's records are readable, ahead of the next block's copies, and land during the block's arithmetic.
-// The dot of a query is a sum over the warp: each lane parks its part in shared memory (in the row slot in use, whose rows are
-// in registers by then), and after every G_SLOTS queries four lanes add up the parts of one query each: 16 instructions for 8
-// queries, where a shuffle tree per query takes 80.
 #pragma once
 #include "qlka_common.cuh"
 
@@ -31,7 +22,6 @@ constexpr int WALK_THREADS = 256;
 constexpr int WALK_STREAMS = WALK_THREADS / 32;      // streams per CTA
 constexpr int SX_STRIDE    = 12;     // floats per staged scalar slot: 8 decays / keys and the next four
 constexpr int QCAP         = 16;     // query records staged per block
-constexpr int G_SLOTS      = 8;      // emit-side rows staged per batch
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -173,13 +163,10 @@ __device__ __forceinline__ void vred(float* p, const Vec<CPL>& v) {
 // ------------------------------------------------------------------ shared memory of a warp
 template <int CPL> __host__ __device__ constexpr int row_pitch()  { return 128 * CPL; }
 template <int CPL> __host__ __device__ constexpr int slot_bytes() { return KB * row_pitch<CPL>(); }
-// row slots | scalar slots | record slots, and one more: a read may look one ahead | emit-side rows (dot emissions)
+// row slots | scalar slots | record slots, and one more: a read may look one ahead
 template <int CPL, int DEPTH> __host__ __device__ constexpr int sx_offset()  { return DEPTH * slot_bytes<CPL>(); }
 template <int CPL, int DEPTH> __host__ __device__ constexpr int rec_offset() { return sx_offset<CPL, DEPTH>() + DEPTH * SX_STRIDE * 4; }
-template <int CPL, int DEPTH> __host__ __device__ constexpr int g_offset()   { return rec_offset<CPL, DEPTH>() + (DEPTH * QCAP + 1) * 16; }
-template <int CPL, int DEPTH> __host__ __device__ constexpr int warp_bytes(const bool dots) {
-    return g_offset<CPL, DEPTH>() + (dots ? G_SLOTS * row_pitch<CPL>() : 0);
-}
+template <int CPL, int DEPTH> __host__ __device__ constexpr int warp_bytes() { return rec_offset<CPL, DEPTH>() + (DEPTH * QCAP + 1) * 16; }
 
 // the warp's index in its CTA, in a form the compiler knows to be uniform
 __device__ __forceinline__ int warp_index() { return __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0); }
@@ -200,7 +187,6 @@ struct Feeder {
     const char*     aux;       // lanes 0 .. 15: the segment's records; lanes 16 .. 18: the first block's scalars, + my 16 bytes
     uint32_t        aux_dst;   // shared address they go to in slot 0
     const uint4*    yrec;      // the segment's records
-    const char*     grows;     // dot emissions: + p * M * row_bytes + my 16 bytes
     // prefetched one block before its issue
     uint32_t idx[NCP], ms;
     // first query of the block in use and of the blocks in flight
@@ -222,9 +208,6 @@ struct Feeder {
         M      = a.M;
         aux    = lane < QCAP ? reinterpret_cast<const char*>(yrec)
                              : reinterpret_cast<const char*>(WITH_X ? a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * (lane - QCAP) : nullptr);
-    }
-    __device__ __forceinline__ void start_dots(const WalkArgs& a, const int p) {
-        grows = reinterpret_cast<const char*>(a.g + (long long)p * a.M * a.C4) + (lane % LR) * 16;
     }
 
     // t: the block's place in the stream
@@ -298,41 +281,13 @@ struct Feeder {
     }
 
     __device__ __forceinline__ uint32_t records(const int slot) const { return area + rec_offset<CPL, DEPTH>() + slot * QCAP * 16; }
-
-    // start the copies of the emit-side rows of the G_SLOTS staged records from n0 on, as far as they belong to the block of key j0;
-    // one commit group
-    __device__ __forceinline__ void issue_g(const int slot, const int j0, const uint32_t n0) const {
-        const uint32_t g   = area + g_offset<CPL, DEPTH>() + (lane / LR) * NCP * row_pitch<CPL>() + (lane % LR) * 16;
-        const uint32_t rec = records(slot) + (n0 + (lane / LR) * NCP) * 16;
-        #pragma unroll
-        for (int i = 0; i < NCP; i++) {
-            const uint2 zw = lds64u(rec + i * 16 + 8);
-            if (copy_on && zw.y - (uint32_t)j0 < (uint32_t)KB) cp_async16(g + i * row_pitch<CPL>(), grows + (unsigned long long)zw.x * row_bytes);
-        }
-        cp_async_commit();
-    }
-    // lane addresses of the emit-side row of query 0 of a batch and of this lane's part of its dot; query n: + n pitches, + n * 128
-    __device__ __forceinline__ uint32_t g_lane() const { return area + g_offset<CPL, DEPTH>() + lane * (4 * CPL); }
-    __device__ __forceinline__ uint32_t part_lane(const int slot) const { return area + slot * slot_bytes<CPL>() + lane * 4; }
-    // the dot of the batch's query lane / 4, in each of its four lanes
-    __device__ __forceinline__ float sum_parts(const int slot) const {
-        const int      q = lane >> 2, k = (lane & 3) ^ ((q & 1) * 4);      // (odd queries start in the other half: no bank conflicts)
-        const uint32_t p = area + slot * slot_bytes<CPL>() + q * 128;
-        const float4   a = lds128(p + k * 16), b = lds128(p + (k ^ 4) * 16);
-        float s = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
-        s += __shfl_xor_sync(FULL, s, 1);
-        return s + __shfl_xor_sync(FULL, s, 2);
-    }
 };
 
-// The queries of the block of key j0, in rank order: emit(i, rec, n128) for the queries that precede key i, n128 = 128 * (query's place
-// in its batch of G_SLOTS); finish(n0, n1) after every G_SLOTS queries and at the end (dot emissions; n0 counts from the staged
-// records). The staged records are followed by one of a later block (or the segment's sentinel), so a record's rank alone says
-// where the block ends; when the last staged record is still the block's, it goes QCAP - 1 queries at a time, with a terminator.
-// (Dots carry only the next query's rank: carrying its record costs them four moves a query; rows, with fewer registers in use,
-// are 3 % faster with the record. REC false: emit has no use for the record.)
-template <bool DO_DOT, bool REC = true, class F, class Emit, class Finish>
-__device__ __forceinline__ void for_queries(const F& f, const int slot, const int j0, Emit emit, Finish finish) {
+// The queries of the block of key j0, in rank order: emit(i, rec) for the queries that precede key i. The staged records are followed by one
+// of a later block (or the segment's sentinel), so a record's rank alone says where the block ends; when the last staged record is
+// still the block's, it goes QCAP - 1 queries at a time, with a terminator.
+template <class F, class Emit>
+__device__ __forceinline__ void for_queries(const F& f, const int slot, const int j0, Emit emit) {
     constexpr uint32_t BATCH = QCAP - 1;
     const uint32_t recs = f.records(slot);
     uint32_t at = f.m_lo;
@@ -343,50 +298,21 @@ __device__ __forceinline__ void for_queries(const F& f, const int slot, const in
             if (f.lane == 0) sts32f(recs + BATCH * 16 + 12, __uint_as_float(0xffffffffu));
             __syncwarp();
         }
-        uint32_t qa = recs, n128 = 0, n0 = 0;
-        uint4    rec;
-        uint32_t key;
-        auto fetch = [&]() {
-            if (DO_DOT) key = lds32u(qa + 12) - (uint32_t)j0;
-            else      { rec = lds128u(qa); key = rec.w - (uint32_t)j0; }
-        };
-        fetch();
+        uint32_t qa  = recs;
+        uint4    rec = lds128u(qa);
         #pragma unroll
         for (int i = 0; i < KB; i++) {
-            while (key == (uint32_t)i) {
-                const uint4 now = DO_DOT ? (REC ? lds128u(qa) : make_uint4(0u, 0u, 0u, 0u)) : rec;
+            while (rec.w - (uint32_t)j0 == (uint32_t)i) {
                 qa += 16;
-                if (DO_DOT) { fetch(); emit(i, now, n128); }
-                else        { emit(i, now, n128); fetch(); }
-                if (DO_DOT) {
-                    n128 += 128;
-                    if (n128 == G_SLOTS * 128) {
-                        __syncwarp();
-                        finish(n0, n0 + G_SLOTS);
-                        __syncwarp();
-                        n0 += G_SLOTS;
-                        n128 = 0;
-                        f.issue_g(slot, j0, n0);
-                        cp_async_wait<0>();
-                        __syncwarp();
-                    }
-                }
+                emit(i, rec);
+                rec = lds128u(qa);
             }
-        }
-        if (DO_DOT && n128 != 0) {
-            __syncwarp();
-            finish(n0, n0 + (n128 >> 7));
         }
         if (!more) break;
         at += BATCH;
         __syncwarp();
         if (f.lane < QCAP) sts128u(recs + f.lane * 16, __ldg(f.yrec + min(at + f.lane, (uint32_t)f.M)));
         __syncwarp();
-        if (DO_DOT) {
-            f.issue_g(slot, j0, 0u);
-            cp_async_wait<0>();
-            __syncwarp();
-        }
     }
 }
 

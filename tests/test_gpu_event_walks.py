@@ -1,0 +1,57 @@
+"""The walks over events (dots, and rows and dots) where their blocks, streams and channel groups begin and end."""
+
+import pytest
+import torch
+
+from oracle import direct, sorted_scan
+from util import rel_err
+
+pytestmark = pytest.mark.gpu
+
+D = 130        # more features than the pairwise gradients take: always the walks
+
+# keys, queries, channels: lone events, blocks of 8 events full and not, streams of several warps, every lane layout with idle lanes and without
+SIZES = [(1, 1, 1), (3, 5, 4), (8, 8, 33), (7, 10, 64), (16, 1, 40), (1, 41, 128), (130, 126, 32), (64, 300, 36), (515, 77, 100), (257, 1031, 64)]
+
+
+def _inputs(N, M, C, where):
+    g = torch.Generator().manual_seed(N * 7 + M * 3 + C)
+    r = lambda *s: torch.randn(*s, generator=g)
+    q, k = r(2, D, M), r(2, D, N)
+    if where == "apart":             # all queries of a feature on one side of its keys, or crowded between two of them
+        q[:, 0::3] = k[:, 0::3].amax(-1, keepdim=True) + 0.1 + q[:, 0::3].abs()
+        q[:, 1::3] = k[:, 1::3].amin(-1, keepdim=True) - 0.1 - q[:, 1::3].abs()
+        q[:, 2::3] = k[:, 2::3].mean(-1, keepdim=True) + 1e-3 * q[:, 2::3]
+    return q, k, r(2, N, C), r(2, M, C), r(2, M)
+
+
+def _tol(N, M):
+    """Every result is a sum over keys (or queries) and channels in fp32: its rounding grows with the number of additions in a row, here no
+    more than N + M + 128, each 2^-24 of sums that are at most a few times the largest result."""
+    return 4 * (N + M + 128) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("where", ["mixed", "apart"])
+@pytest.mark.parametrize("N,M,C", SIZES)
+def test_laplace(N, M, C, where):
+    import qlka_native
+    q, k, v, g_w, g_u = _inputs(N, M, C, where)
+    for gu in (g_u, None):
+        got = qlka_native.laplace_backward(q.cuda(), k.cuda(), v.cuda(), g_w.cuda(), gu.cuda() if gu is not None else None)
+        want = direct.laplace_sum_backward(q, k, v, g_w, gu if gu is not None else torch.zeros_like(g_u))
+        for name, a, b in zip(("q", "k", "v"), got, want):
+            assert rel_err(a, b) < _tol(N, M), (name, rel_err(a, b))
+
+
+@pytest.mark.parametrize("where", ["mixed", "apart"])
+@pytest.mark.parametrize("N,M,C", SIZES)
+def test_abs_and_sgn(N, M, C, where):
+    import qlka_native
+    from weighted_abs_sum import weighted_sgn_sum
+    q, k, v, g_w, g_u = _inputs(N, M, C, where)
+    got = qlka_native.abs_backward(q.cuda(), k.cuda(), v.cuda(), g_w.cuda(), g_u.cuda())
+    want = sorted_scan.abs_sum_backward(q, k, v, g_w, g_u)
+    for name, a, b in zip(("q", "k", "v"), got, want):
+        assert rel_err(a, b) < _tol(N, M), (name, rel_err(a, b))
+    out, ref = weighted_sgn_sum(q.cuda(), k.cuda(), v.cuda(), g_w.cuda()), sorted_scan.sgn_sum(q, k, v, g_w)
+    assert rel_err(out, ref) < _tol(N, M), rel_err(out, ref)
