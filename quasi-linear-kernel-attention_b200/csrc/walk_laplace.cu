@@ -31,68 +31,67 @@ enum { LAP_ROWS = 0, LAP_DOT = 1, LAP_BOTH = 2 };
 
 // resident CTAs per SM that the emitting pass is compiled for, and blocks in its rings: three CTAs with one stream per warp (two: 3.34
 // instead of 3.02 ms at 48 heads x 16384 keys; four leave 64 registers: 4.1 ms)
-constexpr int LAP_CTAS1 = 3, LAP_CTAS_ROWS = 2;
+constexpr int LAP_CTAS_ROWS = 2;
 __host__ __device__ constexpr int lap_ctas2(int cpl) { return cpl == 4 ? 2 : 3; }
 constexpr int LAP_DEPTH2 = 3;
 
 // floats per stream in the aggregate table: forward aggregate | backward aggregate | decay forward, decay backward, pad
 __host__ __device__ inline int lap_agg_stride(int C4) { return 2 * C4 + 4; }
 
-template <int LPS>
-__global__ void __launch_bounds__(WALK_THREADS, LAP_CTAS1) laplace_pass1(const WalkArgs a)
+template <int LPS, int CPL>
+__global__ void __launch_bounds__(KEY_THREADS, KEY_CTAS) laplace_pass1(const WalkArgs a)
 {
-    constexpr int STREAMS = WALK_THREADS / LPS;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int tid = threadIdx.x, ln = tid % LPS, c0 = ln * 4;
-    const int N = a.N, C4 = a.C4, NBK = nblocks(N);
-    const bool lane_on = c0 < C4;
-    const unsigned gmask = LPS == 32 ? FULL : (((1u << (LPS & 31)) - 1u) << ((tid & 31) & ~(LPS - 1)));
-
-    SumFeeder<LPS, true, -1> f;
-    f.init(smem_u32(smem), N, C4);
-
-    const int items = (int)(((long long)a.nseg * a.sps + STREAMS - 1) / STREAMS);
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const StreamOf st(a, item, tid / LPS, NBK, STREAMS);
-        const int b1 = st.b1, nblk = st.nblk;
-        f.start(a, st.sg, st.p, b1 - 1);
-        float* ck = a.ckpt + ((long long)st.sg * NBK + b1 - 1) * C4 + c0;      // of the block in use
-        float* wk = a.wck + (long long)st.sg * NBK + b1 - 1;
-
-        Vec<4> Rl, F;
-        Rl.zero(); F.zero();
-        float w = 1.0f, wprev = 1.0f;
-        const float a_j1 = b1 < NBK ? __ldg(a.xval + (long long)st.sg * xstride(N) + b1 * KB) : 0.0f;   // decay from the next stream's first key
-        __syncwarp(gmask);                         // every lane has left the previous item's slots
-        f.prologue(nblk);
-        int cur = 0, j0 = (b1 - 1) * KB;
-        for (int t = 0; t < nblk; t++, j0 -= KB, ck -= C4, wk--, cur ^= 1) {
-            __syncwarp(gmask);                     // every lane is done with the slot refilled below
-            f.step(t, cur, nblk);
-            __syncwarp(gmask);
-            float av[KB + 1];
-            f.read_scalars(cur, av);
-            Vec<4> v[KB];
-            f.read_rows(cur, j0, v);
+    using F = KeyFeeder<LPS, CPL, true, -1>;
+    __shared__ __align__(16) unsigned char smem[F::SMEM];
+    const int C4 = a.C4, NBK = nblocks(a.N);
+    F f;
+    f.init(smem_u32(smem), a.N, C4);
+    const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::STREAMS);
+    float* ck = a.ckpt + ((long long)st.sg * NBK + st.b1 - 1) * C4;               // of the block in use
+    float* wk = a.wck + (long long)st.sg * NBK + st.b1 - 1;
+    Vec<CPL> A, R;                                 // the stream's forward aggregate, its suffix state
+    A.zero(); R.zero();
+    float w = 1.0f, wr = 1.0f;                     // decay from the last key visited to the stream's last one, to the next stream's first
+    float anext = st.b1 < NBK ? __ldg(a.xval + (long long)st.sg * xstride(a.N) + st.b1 * KB) : 0.0f;
+    Vec<CPL> x[KB];
+    f.start(a, st, x);
+    const int steps = __reduce_max_sync(FULL, f.nblk);
+    for (int t = 0; t < steps; t++) {
+        f.step(t, x);
+        uint32_t n[KB];
+        float    av[KB];
+        f.scalars(av);
+        f.read_index(f.next, n);
+        if (t >= f.nblk) continue;                 // (the warp's other streams may be a block longer)
+        #pragma unroll
+        for (int h = KB - 4; h >= 0; h -= 4) {
             #pragma unroll
-            for (int i = KB - 1; i >= 0; i--) {
-                axpy(F, w, v[i], F);
-                axpy(Rl, av[i + 1], Rl, v[i]);
-                wprev = w;
-                w *= av[i];
+            for (int i = h + 3; i >= h; i--) {
+                axpy8(A, w, x[i], A);
+                axpy8(R, anext, R, x[i]);
+                wr *= anext; w *= av[i]; anext = av[i];
             }
-            if (lane_on) vstore_once(ck, Rl);      // (streaming: the second pass reads them long after, once)
-            if (ln == 0) *wk = wprev * a_j1;
-        }
-        cp_async_wait<0>();                        // (the trailing empty groups)
-        if (st.on) {
-            float* ag = a.agg + st.g * lap_agg_stride(C4);
-            if (lane_on) {
-                vstore(ag + c0, F);
-                vstore(ag + C4 + c0, Rl);
+            if (t + 1 < f.nblk) {
+                #pragma unroll
+                for (int i = h; i < h + 4; i++) x[i] = f.row(n[i]);
             }
-            if (ln == 0) { ag[2 * C4] = w; ag[2 * C4 + 1] = wprev * a_j1; }
         }
+        #pragma unroll
+        for (int q = 0; q < F::Q; q++)             // (streaming: the second pass reads them long after, once)
+            if (f.on[q]) __stcs(reinterpret_cast<float4*>(ck + f.channel(q)), make_float4(R.x[4 * q], R.x[4 * q + 1], R.x[4 * q + 2], R.x[4 * q + 3]));
+        if (f.ln == 0) *wk = wr;
+        ck -= C4; wk--;
+    }
+    cp_async_wait<0>();
+    if (st.on) {
+        float* ag = a.agg + st.g * lap_agg_stride(C4);
+        #pragma unroll
+        for (int q = 0; q < F::Q; q++) {
+            if (!f.on[q]) continue;
+            *reinterpret_cast<float4*>(ag + f.channel(q))      = make_float4(A.x[4 * q], A.x[4 * q + 1], A.x[4 * q + 2], A.x[4 * q + 3]);
+            *reinterpret_cast<float4*>(ag + C4 + f.channel(q)) = make_float4(R.x[4 * q], R.x[4 * q + 1], R.x[4 * q + 2], R.x[4 * q + 3]);
+        }
+        if (f.ln == 0) { ag[2 * C4] = w; ag[2 * C4 + 1] = wr; }
     }
 }
 
@@ -315,20 +314,16 @@ static cudaError_t launch_lap_pass2(const WalkArgs& a, int sms, cudaStream_t str
     return cudaGetLastError();
 }
 
-template <int LPS>
-static cudaError_t launch_lap_pass1(const WalkArgs& a, int sms, cudaStream_t stream) {
-    constexpr int smem = sum_smem_bytes<LPS>();
-    cudaError_t e = cudaFuncSetAttribute(laplace_pass1<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    const long long items = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
-    const int cap = sms * LAP_CTAS1;
-    laplace_pass1<LPS><<<items < cap ? (int)items : cap, WALK_THREADS, smem, stream>>>(a);
+template <int LPS, int CPL>
+static cudaError_t launch_lap_pass1(const WalkArgs& a, cudaStream_t stream) {
+    constexpr int streams = KEY_THREADS / LPS;
+    laplace_pass1<LPS, CPL><<<(unsigned)(((long long)a.nseg * a.sps + streams - 1) / streams), KEY_THREADS, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
 template <int LPS, int CPL>
 static cudaError_t launch_lap(const WalkArgs& a, int emit, int sms, cudaStream_t stream, cudaEvent_t mid) {
-    cudaError_t e = emit == LAP_ROWS ? launch_lap_pass1<LPS>(a, sms, stream) : launch_laplace_events1(a, sms, stream);
+    cudaError_t e = emit == LAP_ROWS ? launch_lap_pass1<LPS < 32 ? 8 : 16, LPS == 8 ? 4 : 8>(a, stream) : launch_laplace_events1(a, sms, stream);
     if (e != cudaSuccess) return e;
     laplace_fold<<<fold_grid(a), 32 * FOLD_WARPS, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4, fold_share_warps(a));
     e = cudaGetLastError();

@@ -21,7 +21,7 @@ cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, int sms, cudaStre
 enum { EMIT_ROWS = 0, EMIT_DOT = 1, EMIT_BOTH = 2 };
 
 // resident CTAs per SM that the passes are compiled for, and blocks in the emitting pass's rings (as in the Laplace walk)
-constexpr int PREFIX_CTAS1 = 3, PREFIX_CTAS_ROWS = 2;
+constexpr int PREFIX_CTAS_ROWS = 2;
 __host__ __device__ constexpr int prefix_ctas2(int cpl) { return cpl == 4 ? 2 : 4; }
 constexpr int PREFIX_DEPTH2 = 3;
 
@@ -29,49 +29,48 @@ constexpr int PREFIX_DEPTH2 = 3;
 __host__ __device__ inline int prefix_agg_stride(int C4) { return 2 * C4; }
 
 // First launch (only with more than one stream per segment): every stream sums its rows (and key * row).
-template <int LPS, bool WITH_K>
-__global__ void __launch_bounds__(WALK_THREADS, PREFIX_CTAS1) prefix_pass1(const WalkArgs a)
+template <int LPS, int CPL, bool WITH_K>
+__global__ void __launch_bounds__(KEY_THREADS, KEY_CTAS) prefix_pass1(const WalkArgs a)
 {
-    constexpr int STREAMS = WALK_THREADS / LPS;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int tid = threadIdx.x, ln = tid % LPS, c0 = ln * 4;
-    const int N = a.N, C4 = a.C4, NBK = nblocks(N);
-    const unsigned gmask = LPS == 32 ? FULL : (((1u << (LPS & 31)) - 1u) << ((tid & 31) & ~(LPS - 1)));
-
-    SumFeeder<LPS, WITH_K, 1> f;
-    f.init(smem_u32(smem), N, C4);
-
-    const int items = (int)(((long long)a.nseg * a.sps + STREAMS - 1) / STREAMS);
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const StreamOf st(a, item, tid / LPS, NBK, STREAMS);
-        f.start(a, st.sg, st.p, st.b0);
-
-        Vec<4> PV, PK;
-        PV.zero(); PK.zero();
-        __syncwarp(gmask);                         // every lane has left the previous item's slots
-        f.prologue(st.nblk);
-        int cur = 0, j0 = st.b0 * KB;
-        for (int t = 0; t < st.nblk; t++, j0 += KB, cur ^= 1) {
-            __syncwarp(gmask);                     // every lane is done with the slot refilled below
-            f.step(t, cur, st.nblk);
-            float kv[KB + 1];
-            if (WITH_K) {
-                __syncwarp(gmask);
-                f.read_scalars(cur, kv);
-            }
-            Vec<4> v[KB];
-            f.read_rows(cur, j0, v);
+    using F = KeyFeeder<LPS, CPL, WITH_K, 1>;
+    __shared__ __align__(16) unsigned char smem[F::SMEM];
+    const int C4 = a.C4, NBK = nblocks(a.N);
+    F f;
+    f.init(smem_u32(smem), a.N, C4);
+    const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::STREAMS);
+    Vec<CPL> PV, PK;
+    PV.zero(); PK.zero();
+    Vec<CPL> x[KB];
+    f.start(a, st, x);
+    const int steps = __reduce_max_sync(FULL, f.nblk);
+    for (int t = 0; t < steps; t++) {
+        f.step(t, x);
+        uint32_t n[KB];
+        float    kv[KB];
+        if (WITH_K) f.scalars(kv);
+        f.read_index(f.next, n);
+        if (t >= f.nblk) continue;                 // (the warp's other streams may be a block longer)
+        #pragma unroll
+        for (int h = 0; h < KB; h += 4) {
             #pragma unroll
-            for (int i = 0; i < KB; i++) {
-                vadd(PV, v[i]);
-                if (WITH_K) axpy(PK, kv[i], v[i], PK);
+            for (int i = h; i < h + 4; i++) {
+                vadd(PV, x[i]);
+                if (WITH_K) axpy8(PK, kv[i], x[i], PK);
+            }
+            if (t + 1 < f.nblk) {
+                #pragma unroll
+                for (int i = h; i < h + 4; i++) x[i] = f.row(n[i]);
             }
         }
-        cp_async_wait<0>();
-        if (st.on && c0 < C4) {
-            float* ag = a.agg + st.g * prefix_agg_stride(C4) + c0;
-            vstore(ag, PV);
-            if (WITH_K) vstore(ag + C4, PK);
+    }
+    cp_async_wait<0>();
+    if (st.on) {
+        float* ag = a.agg + st.g * prefix_agg_stride(C4);
+        #pragma unroll
+        for (int q = 0; q < F::Q; q++) {
+            if (!f.on[q]) continue;
+            *reinterpret_cast<float4*>(ag + f.channel(q)) = make_float4(PV.x[4 * q], PV.x[4 * q + 1], PV.x[4 * q + 2], PV.x[4 * q + 3]);
+            if (WITH_K) *reinterpret_cast<float4*>(ag + C4 + f.channel(q)) = make_float4(PK.x[4 * q], PK.x[4 * q + 1], PK.x[4 * q + 2], PK.x[4 * q + 3]);
         }
     }
 }
@@ -257,15 +256,10 @@ static cudaError_t launch_pass2(const WalkArgs& a, int sms, cudaStream_t stream)
     return cudaGetLastError();
 }
 
-template <int LPS, bool WITH_K>
-static cudaError_t launch_pass1(const WalkArgs& a, int sms, cudaStream_t stream) {
-    auto k1 = prefix_pass1<LPS, WITH_K>;
-    constexpr int smem1 = sum_smem_bytes<LPS>();
-    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
-    if (e != cudaSuccess) return e;
-    const long long items1 = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
-    const int cap1 = sms * PREFIX_CTAS1;
-    k1<<<items1 < cap1 ? (int)items1 : cap1, WALK_THREADS, smem1, stream>>>(a);
+template <int LPS, int CPL, bool WITH_K>
+static cudaError_t launch_pass1(const WalkArgs& a, cudaStream_t stream) {
+    constexpr int streams = KEY_THREADS / LPS;
+    prefix_pass1<LPS, CPL, WITH_K><<<(unsigned)(((long long)a.nseg * a.sps + streams - 1) / streams), KEY_THREADS, 0, stream>>>(a);
     prefix_fold<<<fold_grid(a), 32 * FOLD_WARPS, 0, stream>>>(a.agg, a.nseg, a.sps, a.C4, fold_share_warps(a), WITH_K ? 1 : 0);
     return cudaGetLastError();
 }
@@ -273,7 +267,8 @@ static cudaError_t launch_pass1(const WalkArgs& a, int sms, cudaStream_t stream)
 template <int LPS, int CPL>
 static cudaError_t launch_pw(const WalkArgs& a, int emit, int sms, cudaStream_t stream) {
     if (a.sps > 1) {                                                   // (a lone stream per segment has nothing before it)
-        cudaError_t e = emit == EMIT_DOT ? launch_pass1<LPS, false>(a, sms, stream) : launch_pass1<LPS, true>(a, sms, stream);
+        constexpr int L = LPS < 32 ? 8 : 16, W = LPS == 8 ? 4 : 8;         // lanes of a stream and channels of each in the first launch
+        cudaError_t e = emit == EMIT_DOT ? launch_pass1<L, W, false>(a, stream) : launch_pass1<L, W, true>(a, stream);
         if (e != cudaSuccess) return e;
     }
     if (emit != EMIT_ROWS) return launch_prefix_events(a, emit == EMIT_BOTH, sms, stream);

@@ -3,8 +3,7 @@
 // Emitting passes (Feeder): one warp walks one stream (a contiguous run of key blocks of a segment). Lane l owns the CPL
 // consecutive channels from l * CPL on, with CPL = 1, 2 or 4 for up to 32, 64 or 128 channels, so that every loop below is uniform
 // over the warp.
-// First passes (SumFeeder), which have nothing that diverges, keep 4 channels per lane and 1, 2 or 4 streams per warp: they are
-// bound by instruction issue, and a warp per stream took 1.35 instead of 1.02 ms at 48 heads x 16384 keys.
+// First passes (KeyFeeder), which have nothing that diverges, have 4 or 8 channels per lane and 2 or 4 streams per warp.
 //
 // Every warp owns a ring of DEPTH slots in shared memory; a slot holds the KB rows of one key block, the block's per-key
 // scalars (12 floats of which 9 are used) and its first QCAP query records. All of it is fetched with cp.async (global ->
@@ -99,6 +98,16 @@ __device__ __forceinline__ void scale(Vec<CPL>& d, const float a, const Vec<CPL>
         #pragma unroll
         for (int c = 0; c < CPL; c++) d.x[c] = a * x.x[c];
     }
+}
+// the same where a lane has 4 or 8 channels
+template <int CPL>
+__device__ __forceinline__ void axpy8(Vec<CPL>& d, const float a, const Vec<CPL>& x, const Vec<CPL>& y) {
+    #pragma unroll
+    for (int c = 0; c < CPL; c += 2)
+        asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+            "mov.b64 ra, {%2, %2};\n\tmov.b64 rb, {%3, %4};\n\tmov.b64 rc, {%5, %6};\n\t"
+            "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+            : "=f"(d.x[c]), "=f"(d.x[c + 1]) : "f"(a), "f"(x.x[c]), "f"(x.x[c + 1]), "f"(y.x[c]), "f"(y.x[c + 1]));
 }
 // d += x
 template <int CPL>
@@ -316,14 +325,14 @@ __device__ __forceinline__ void for_queries(const F& f, const int slot, const in
     }
 }
 
-// The first passes' staging: LPS lanes per stream (8, 16 or 32 for up to 32, 64 or 128 channels), 4 channels per lane. Every lane
+// Row emission by quads: LPS lanes per stream (8, 16 or 32 for up to 32, 64 or 128 channels), 4 channels per lane. Every lane
 // copies its own 16 bytes of each row into a private ring of two slots, and reads only those; the block's scalars are shared by
 // the lanes of the stream.
 constexpr int SUM_SLOT_BYTES = KB * WALK_THREADS * 16;
 template <int LPS> __host__ __device__ constexpr int sum_smem_bytes() { return 2 * SUM_SLOT_BYTES + (WALK_THREADS / LPS) * 2 * SX_STRIDE * 4; }
 
-template <int LPS, bool WITH_X, int DIR>
-struct SumFeeder {
+template <int LPS>
+struct QuadFeeder {
     uint32_t        ring, sx;  // shared addresses: this lane's 16 bytes of row 0 of slot 0, the stream's scalar slots
     uint32_t        row_bytes;
     int             ln, N;
@@ -342,13 +351,13 @@ struct SumFeeder {
     }
     __device__ __forceinline__ void start(const WalkArgs& a, const int sg, const int p, const int b) {
         xperm = a.xperm + (long long)sg * npad(a.N) + b * KB;
-        if (WITH_X) xval = a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * ln;
+        xval = a.xval + (long long)sg * xstride(a.N) + b * KB + 4 * ln;
         rows = reinterpret_cast<const char*>(a.rows + (long long)p * a.N * a.C4) + ln * 16;
     }
     __device__ __forceinline__ void prefetch_index() {
         p0 = __ldg(reinterpret_cast<const uint4*>(xperm));
         p1 = __ldg(reinterpret_cast<const uint4*>(xperm + 4));
-        xperm += DIR * KB;
+        xperm += KB;
     }
     __device__ __forceinline__ void issue(const int slot) {
         const uint32_t pr[KB] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
@@ -356,10 +365,8 @@ struct SumFeeder {
             #pragma unroll
             for (int i = 0; i < KB; i++) cp_async16(ring + slot * SUM_SLOT_BYTES + i * WALK_THREADS * 16, rows + (unsigned long long)pr[i] * row_bytes);
         }
-        if (WITH_X) {
-            if (ln < 3) cp_async16(sx + slot * SX_STRIDE * 4 + 16 * ln, xval);
-            xval += DIR * KB;
-        }
+        if (ln < 3) cp_async16(sx + slot * SX_STRIDE * 4 + 16 * ln, xval);
+        xval += KB;
         cp_async_commit();
     }
     __device__ __forceinline__ void prologue(const int nblk) {
@@ -395,8 +402,8 @@ struct SumFeeder {
 template <int LPS> __host__ __device__ constexpr int row_smem_bytes() { return sum_smem_bytes<LPS>() + WALK_THREADS * 2 * 16; }
 
 template <int LPS>
-struct RowFeeder : SumFeeder<LPS, true, 1> {
-    using Base = SumFeeder<LPS, true, 1>;
+struct RowFeeder : QuadFeeder<LPS> {
+    using Base = QuadFeeder<LPS>;
     uint32_t        recs;      // shared address of the stream's record slots [2][LPS]
     const uint4*    yrec;      // the segment's records
     const uint32_t* mstart;    // of the next block to prefetch
@@ -512,6 +519,90 @@ struct StreamOf {
         p  = sg / a.D;
         stream_blocks(s, a.sps, NBK, b0, b1);
         nblk = on ? b1 - b0 : 0;
+    }
+};
+
+// The first passes' staging: LPS lanes per stream with CPL = 4 or 8 channels each (quads ln, and LPS + ln, of the row). Rows go straight to
+// registers, those of the next block as soon as the block in use is done with (through shared memory, as above, the load/store pipe
+// moves them twice: Laplace at 48 heads x 16384 keys 1.12 -> 0.79 ms, abs at
+// 96 x 4096 0.43 -> 0.36; the gathers alone take 0.75 and 0.33). Indices and scalars are shared by the lanes of a stream and arrive in shared
+// memory a block ahead. Small CTAs, one item each: they spread over the SMs however few streams there are.
+constexpr int KEY_THREADS = 64, KEY_CTAS = 8, KEY_REC = KB * 8;
+
+template <int LPS, int CPL, bool WITH_X, int DIR>
+struct KeyFeeder {
+    static constexpr int STREAMS = KEY_THREADS / LPS, SMEM = STREAMS * 3 * KEY_REC, Q = CPL / 4;
+    uint32_t    rec, next, after;  // shared addresses: the indices and scalars of the block in use, the next one and the one after it
+    int         ln, N, j0;         // j0: first key of the block in use
+    bool        on[Q];             // quad q lies inside the row (idle ones read the first)
+    uint32_t    row_bytes, second; // from the first quad to the second
+    const char* rows;              // + p * N * row_bytes + my first quad
+    const char* aux;               // lanes 0, 1: the indices of the next block to copy; lanes 2, 3: its scalars, + my 16 bytes
+    int         nblk;
+
+    __device__ __forceinline__ int channel(const int q) const { return on[q] ? (q * LPS + ln) * 4 : 0; }
+    __device__ __forceinline__ void init(const uint32_t smem, const int N_, const int C4) {
+        ln = threadIdx.x % LPS; N = N_;
+        rec = smem + (threadIdx.x / LPS) * 3 * KEY_REC; next = rec + KEY_REC; after = next + KEY_REC;
+        #pragma unroll
+        for (int q = 0; q < Q; q++) on[q] = (q * LPS + ln) * 4 < C4;
+        second = Q > 1 && on[Q - 1] ? LPS * 16 : 0;
+        row_bytes = (uint32_t)C4 * 4u;
+    }
+    __device__ __forceinline__ void copy_records(const int t, const uint32_t dst) {
+        if (t < nblk && ln < (WITH_X ? 4 : 2)) { cp_async16(dst + ln * 16, aux); aux += DIR * KB * 4; }
+    }
+    __device__ __forceinline__ void read_index(const uint32_t r, uint32_t (&n)[KB]) const {
+        const uint4 a = lds128u(r), b = lds128u(r + 16);
+        n[0] = a.x; n[1] = a.y; n[2] = a.z; n[3] = a.w; n[4] = b.x; n[5] = b.y; n[6] = b.z; n[7] = b.w;
+    }
+    __device__ __forceinline__ void scalars(float (&s)[KB]) const {
+        const float4 a = lds128(rec + KB * 4), b = lds128(rec + KB * 4 + 16);
+        s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w; s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
+    }
+    __device__ __forceinline__ Vec<CPL> row(const uint32_t i) const {
+        const char* at = rows + (unsigned long long)i * row_bytes;
+        Vec<CPL> v;
+        #pragma unroll
+        for (int q = 0; q < Q; q++)
+            asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v.x[4 * q]), "=f"(v.x[4 * q + 1]), "=f"(v.x[4 * q + 2]), "=f"(v.x[4 * q + 3]) : "l"(at + (q ? second : 0u)));
+        return v;
+    }
+    // the stream's blocks in steps t = 0 .. nblk - 1; rows of the first under way, indices of the second as well
+    __device__ __forceinline__ void start(const WalkArgs& a, const StreamOf& st, Vec<CPL> (&x)[KB]) {
+        nblk = st.nblk;
+        const int b = DIR > 0 ? st.b0 : max(st.b1 - 1, 0);
+        j0   = (b - DIR) * KB;
+        rows = reinterpret_cast<const char*>(a.rows + (long long)st.p * a.N * a.C4 + channel(0));
+        aux  = ln < 2 ? reinterpret_cast<const char*>(a.xperm + (long long)st.sg * npad(a.N) + b * KB) + ln * 16
+                      : reinterpret_cast<const char*>(a.xval + (long long)st.sg * xstride(a.N) + b * KB) + (ln - 2) * 16;
+        copy_records(0, next);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncwarp();
+        copy_records(1, after);
+        cp_async_commit();
+        if (nblk > 0) {
+            uint32_t n[KB];
+            read_index(next, n);
+            #pragma unroll
+            for (int i = 0; i < KB; i++) x[i] = row(n[i]);
+        }
+    }
+    // the next block becomes the one in use; the indices after it are readable
+    __device__ __forceinline__ void step(const int t, Vec<CPL> (&x)[KB]) {
+        const uint32_t r = rec;
+        rec = next; next = after; after = r;
+        j0 += DIR * KB;
+        cp_async_wait<0>();
+        __syncwarp();                  // ... by every lane; and every lane has left block t - 1
+        copy_records(t + 2, after);
+        cp_async_commit();
+        if (j0 + KB > N) {             // (positions past the last key point at row 0)
+            #pragma unroll
+            for (int i = 0; i < KB; i++) if (j0 + i >= N) x[i].zero();
+        }
     }
 };
 

@@ -1,4 +1,4 @@
-"""The walks over events (dots, and rows and dots) where their blocks, streams and channel groups begin and end."""
+"""The walks over events (dots, and rows and dots) and the first passes of all walks where their blocks, streams and channel groups begin and end."""
 
 import pytest
 import torch
@@ -8,7 +8,7 @@ from util import rel_err
 
 pytestmark = pytest.mark.gpu
 
-D = 130        # more features than the pairwise gradients take: always the walks
+D = 130        # more features than the pairwise kernels take: always the walks
 
 # keys, queries, channels: lone events, blocks of 8 events full and not, streams of several warps, every lane layout with idle lanes and without
 SIZES = [(1, 1, 1), (3, 5, 4), (8, 8, 33), (7, 10, 64), (16, 1, 40), (1, 41, 128), (130, 126, 32), (64, 300, 36), (515, 77, 100), (257, 1031, 64)]
@@ -55,3 +55,13 @@ def test_abs_and_sgn(N, M, C, where):
         assert rel_err(a, b) < _tol(N, M), (name, rel_err(a, b))
     out, ref = weighted_sgn_sum(q.cuda(), k.cuda(), v.cuda(), g_w.cuda()), sorted_scan.sgn_sum(q, k, v, g_w)
     assert rel_err(out, ref) < _tol(N, M), rel_err(out, ref)
+
+
+@pytest.mark.parametrize("where", ["mixed", "apart"])
+@pytest.mark.parametrize("N,M,C", SIZES + [(1030, 515, 68), (2049, 2047, 8)])
+def test_forward(N, M, C, where):
+    import qlka_native
+    q, k, v, _, _ = _inputs(N, M, C, where)
+    for f, ref in ((qlka_native.laplace_forward, sorted_scan.laplace_sum), (lambda *x: qlka_native.abs_forward(*x, True), sorted_scan.abs_sum)):
+        for a, b in zip(f(q.cuda(), k.cuda(), v.cuda()), ref(q, k, v)):
+            assert rel_err(a, b) < _tol(N, M), rel_err(a, b)
