@@ -98,25 +98,30 @@ int sm_count() {
     return n;
 }
 
-// How a walk over `nseg` segments of N keys is cut into streams and work items (a CTA's worth of streams, one per warp). Streams are
-// independent work units (the passes exchange their states through memory), so a segment may be cut into any number of them:
-// more streams until the persistent CTAs of the second pass get about eight items each (sixteen: more aggregates to write, fold and read,
-// Laplace backward at 48 heads x 4096 keys 4.0 instead of 3.9 ms; four: tails, abs at 16 x 65536 8.45 instead of 8.25 ms), as long as a stream
-// keeps at least sixteen key blocks (the staging ring needs a few blocks to fill) - eight while there are fewer
-// items than CTAs. The prefix walks need no first pass with one stream per segment, which pays as soon as whole
-// segments alone give every CTA a few items.
+// How a walk over `nseg` segments of N keys is cut into streams and work items (eight streams). Streams are independent work units (the
+// passes exchange their states through memory), so a segment may be cut into any number of them, as long as a stream keeps at least
+// sixteen key blocks (a stream's start costs a few) - eight while there are fewer items than CTAs fit the GPU. The streams of a head are
+// neighbours, so the more of them, the fewer heads' rows are in use at a time and the better the L2 keeps them; against that, each leaves
+// aggregates to write, fold and read. Items per CTA of 256 threads, ms:        4      8      16     32
+//   Laplace sum, 4 x 12 heads x 16384 keys x 64 channels                       5.23   4.88   4.83   4.89
+//   abs training step, 8 x 12 x 4096 x 64                                      7.84   6.85   6.72   6.82
+//   abs sum, 16 x 262144 x 64                                                  38.2   36.4   35.4   35.9
+//   Laplace gradients, 48 x 4096 x 64 / 16 x 8192 x 128                        3.49   3.46   3.55   3.55 / 3.82   3.78   3.95   3.95
+//   Laplace sum, 16 x 8191 keys x 1030 queries x 128                           0.93   0.93   0.97   0.97
+// hence sixteen for row walks of up to 64 channels, else eight. The prefix walks need no first pass with one stream per segment, which
+// pays as soon as whole segments alone give every CTA a few items.
 struct WalkPlan { int sps, nitems; };
 
-WalkPlan plan_walk(int nseg, int N, int C4, bool laplace) {
-    constexpr int streams = 8;                        // warps of a walk CTA
+WalkPlan plan_walk(int nseg, int N, int C4, bool laplace, bool dots) {
+    constexpr int streams = 8;
     // resident CTAs, about (above 64 channels two per SM; planned for four, Laplace at 16 heads x 8191 keys x 1030 queries took 1.08
     // instead of 1.03 ms, its backward at 16 x 8192 4.71 instead of 4.45 ms)
-    const int cap = sm_count() * (C4 > 64 ? 2 : 4);
+    const int cap = sm_count() * (C4 > 64 ? 2 : 4), per_cta = dots || C4 > 64 ? 8 : 16;
     const int nbk = nblocks(N);
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
     if (laplace || items(1) < 2LL * cap)
-        while (items(sps) < 8LL * cap && nbk / (sps * 2) >= (items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
+        while (items(sps) < (long long)per_cta * cap && nbk / (sps * 2) >= (items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
     return {sps, (int)items(sps)};
 }
 
@@ -193,11 +198,11 @@ int walk_chunk_heads(int P, int N, int C4) {
 }
 
 // aggregate table of a prefix walk over P heads in chunks (the larger of the two chunk sizes that occur)
-size_t prefix_agg_floats(int P, int D, int N, int C4) {
+size_t prefix_agg_floats(int P, int D, int N, int C4, bool dots) {
     const int heads = walk_chunk_heads(P, N, C4);
-    size_t a = walk_agg_floats(plan_walk(heads * D, N, C4, false), heads * D, C4, false);
+    size_t a = walk_agg_floats(plan_walk(heads * D, N, C4, false, dots), heads * D, C4, false);
     if (const int rem = P % heads) {
-        const size_t a2 = walk_agg_floats(plan_walk(rem * D, N, C4, false), rem * D, C4, false);
+        const size_t a2 = walk_agg_floats(plan_walk(rem * D, N, C4, false, dots), rem * D, C4, false);
         if (a2 > a) a = a2;
     }
     return a;
@@ -211,7 +216,7 @@ cudaError_t prefix_walk_chunked(WalkArgs w, int emit, int P, cudaStream_t stream
     for (int p0 = 0; p0 < P; p0 += heads) {
         const int       pc = heads < P - p0 ? heads : P - p0;
         const long long s0 = (long long)p0 * all.D;
-        const WalkPlan  plan = plan_walk(pc * all.D, all.N, all.C4, false);
+        const WalkPlan  plan = plan_walk(pc * all.D, all.N, all.C4, false, emit != EMIT_ROWS);
         w.rows   = all.rows + (size_t)p0 * all.N * all.C4;
         w.xperm  = all.xperm + s0 * npad(all.N);
         w.xval   = all.xval + s0 * xstride(all.N);
@@ -257,7 +262,7 @@ struct LapWalkScratch {
         size_t a = 0;
         for (const int h : {heads, P % heads})
             for (const int keys : {N, dots ? M : N})
-                if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, keys, C4, true), h * D, C4, true));
+                if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, keys, C4, true, dots), h * D, C4, true));
         agg = b.take<float>(a);
     }
 };
@@ -270,7 +275,7 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
     for (int p0 = 0; p0 < P; p0 += sc.heads) {
         const int       pc = sc.heads < P - p0 ? sc.heads : P - p0, nseg = pc * D;
         const long long s0 = (long long)p0 * D;
-        const WalkPlan  plan = plan_walk(nseg, N, C4, true);
+        const WalkPlan  plan = plan_walk(nseg, N, C4, true, emit != EMIT_ROWS);
         WalkArgs a{};
         a.rows = rows + (size_t)p0 * N * C4;
         a.xperm = r.xperm + s0 * npad(N); a.xval = r.xval + s0 * xstride(N);
@@ -421,7 +426,7 @@ struct AbsFwdWs {
         vsum  = b.take<float>((size_t)P * C4 * 2 + P);     // vsum | ktot | ksr, zeroed together
         ktot  = vsum ? vsum + (size_t)P * C4 : nullptr;
         ksr   = vsum ? ktot + (size_t)P * C4 : nullptr;
-        agg   = b.take<float>(prefix_agg_floats(P, D, N, C4));
+        agg   = b.take<float>(prefix_agg_floats(P, D, N, C4, false));
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
@@ -441,7 +446,7 @@ struct AbsBwdWs {
         rec.carve(b, nseg, mx, mx, false, N + M);
         qsumd = b.take<float>((size_t)P * M);
         sums  = b.take<float>((size_t)P * C4 * 3 + P);
-        const size_t agg_k = prefix_agg_floats(P, D, N, C4), agg_q = prefix_agg_floats(P, D, M, C4);
+        const size_t agg_k = prefix_agg_floats(P, D, N, C4, true), agg_q = prefix_agg_floats(P, D, M, C4, true);
         agg   = b.take<float>(agg_k > agg_q ? agg_k : agg_q);
         bytes = (b.off + 255) & ~size_t(255);
     }

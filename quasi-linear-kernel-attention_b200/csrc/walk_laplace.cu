@@ -31,7 +31,7 @@ enum { LAP_ROWS = 0, LAP_DOT = 1, LAP_BOTH = 2 };
 
 // resident CTAs per SM that the emitting pass is compiled for, and blocks in its rings: three CTAs with one stream per warp (two: 3.34
 // instead of 3.02 ms at 48 heads x 16384 keys; four leave 64 registers: 4.1 ms)
-constexpr int LAP_CTAS_ROWS = 2;
+constexpr int LAP_CTAS_ROWS = 8;
 __host__ __device__ constexpr int lap_ctas2(int cpl) { return cpl == 4 ? 2 : 3; }
 constexpr int LAP_DEPTH2 = 3;
 
@@ -227,9 +227,9 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
 // some 120 registers. Bound by the L2 traffic of one row gathered and one row reduced per key and query (2.4 of its 2.8 ms
 // at 48 heads x 16384 keys and queries; with one stream per warp it took 3.0).
 template <int LPS>
-__global__ void __launch_bounds__(WALK_THREADS, LAP_CTAS_ROWS) laplace_rows(const WalkArgs a)
+__global__ void __launch_bounds__(ROW_THREADS, LAP_CTAS_ROWS) laplace_rows(const WalkArgs a)
 {
-    constexpr int STREAMS = WALK_THREADS / LPS;
+    constexpr int STREAMS = ROW_THREADS / LPS;
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, ln = tid % LPS, c0 = ln * 4;
     const int N = a.N, C4 = a.C4, NBK = nblocks(N);
@@ -298,9 +298,8 @@ static cudaError_t launch_lap_rows(const WalkArgs& a, int sms, cudaStream_t stre
     constexpr int smem = row_smem_bytes<LPS>();
     cudaError_t e = cudaFuncSetAttribute(laplace_rows<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const long long items = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
-    const int cap = sms * LAP_CTAS_ROWS;
-    laplace_rows<LPS><<<items < cap ? (int)items : cap, WALK_THREADS, smem, stream>>>(a);
+    const long long items = ((long long)a.nseg * a.sps * LPS + ROW_THREADS - 1) / ROW_THREADS;
+    laplace_rows<LPS><<<(unsigned)items, ROW_THREADS, smem, stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -21,7 +21,7 @@ cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, int sms, cudaStre
 enum { EMIT_ROWS = 0, EMIT_DOT = 1, EMIT_BOTH = 2 };
 
 // resident CTAs per SM that the passes are compiled for, and blocks in the emitting pass's rings (as in the Laplace walk)
-constexpr int PREFIX_CTAS_ROWS = 2;
+constexpr int PREFIX_CTAS_ROWS = 8;
 __host__ __device__ constexpr int prefix_ctas2(int cpl) { return cpl == 4 ? 2 : 4; }
 constexpr int PREFIX_DEPTH2 = 3;
 
@@ -178,9 +178,9 @@ __global__ void __launch_bounds__(WALK_THREADS, prefix_ctas2(CPL)) prefix_pass2(
 
 // Row emission with 4 channels per lane (RowFeeder; walk_ring.cuh's rows_by_quads says when)
 template <int LPS>
-__global__ void __launch_bounds__(WALK_THREADS, PREFIX_CTAS_ROWS) prefix_rows(const WalkArgs a)
+__global__ void __launch_bounds__(ROW_THREADS, PREFIX_CTAS_ROWS) prefix_rows(const WalkArgs a)
 {
-    constexpr int STREAMS = WALK_THREADS / LPS;
+    constexpr int STREAMS = ROW_THREADS / LPS;
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, ln = tid % LPS, c0 = ln * 4;
     const int N = a.N, C4 = a.C4, NBK = nblocks(N);
@@ -239,9 +239,8 @@ static cudaError_t launch_rows(const WalkArgs& a, int sms, cudaStream_t stream) 
     constexpr int smem = row_smem_bytes<LPS>();
     cudaError_t e = cudaFuncSetAttribute(prefix_rows<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const long long items = ((long long)a.nseg * a.sps * LPS + WALK_THREADS - 1) / WALK_THREADS;
-    const int cap = sms * PREFIX_CTAS_ROWS;
-    prefix_rows<LPS><<<items < cap ? (int)items : cap, WALK_THREADS, smem, stream>>>(a);
+    const long long items = ((long long)a.nseg * a.sps * LPS + ROW_THREADS - 1) / ROW_THREADS;
+    prefix_rows<LPS><<<(unsigned)items, ROW_THREADS, smem, stream>>>(a);
     return cudaGetLastError();
 }
 

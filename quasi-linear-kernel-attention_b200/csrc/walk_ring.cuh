@@ -328,8 +328,9 @@ __device__ __forceinline__ void for_queries(const F& f, const int slot, const in
 // Row emission by quads: LPS lanes per stream (8, 16 or 32 for up to 32, 64 or 128 channels), 4 channels per lane. Every lane
 // copies its own 16 bytes of each row into a private ring of two slots, and reads only those; the block's scalars are shared by
 // the lanes of the stream.
-constexpr int SUM_SLOT_BYTES = KB * WALK_THREADS * 16;
-template <int LPS> __host__ __device__ constexpr int sum_smem_bytes() { return 2 * SUM_SLOT_BYTES + (WALK_THREADS / LPS) * 2 * SX_STRIDE * 4; }
+constexpr int ROW_THREADS = 64;      // one item each: with 256, persistent, a stream that meets more queries than others kept its CTA's share waiting
+constexpr int SUM_SLOT_BYTES = KB * ROW_THREADS * 16;
+template <int LPS> __host__ __device__ constexpr int sum_smem_bytes() { return 2 * SUM_SLOT_BYTES + (ROW_THREADS / LPS) * 2 * SX_STRIDE * 4; }
 
 template <int LPS>
 struct QuadFeeder {
@@ -363,7 +364,7 @@ struct QuadFeeder {
         const uint32_t pr[KB] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
         if (on) {
             #pragma unroll
-            for (int i = 0; i < KB; i++) cp_async16(ring + slot * SUM_SLOT_BYTES + i * WALK_THREADS * 16, rows + (unsigned long long)pr[i] * row_bytes);
+            for (int i = 0; i < KB; i++) cp_async16(ring + slot * SUM_SLOT_BYTES + i * ROW_THREADS * 16, rows + (unsigned long long)pr[i] * row_bytes);
         }
         if (ln < 3) cp_async16(sx + slot * SX_STRIDE * 4 + 16 * ln, xval);
         xval += KB;
@@ -381,7 +382,7 @@ struct QuadFeeder {
     }
     __device__ __forceinline__ void read_rows(const int slot, const int j0, Vec<4> (&v)[KB]) const {
         #pragma unroll
-        for (int i = 0; i < KB; i++) v[i] = vload_shared<4>(ring + slot * SUM_SLOT_BYTES + i * WALK_THREADS * 16);
+        for (int i = 0; i < KB; i++) v[i] = vload_shared<4>(ring + slot * SUM_SLOT_BYTES + i * ROW_THREADS * 16);
         if (j0 + KB > N) {
             #pragma unroll
             for (int i = 0; i < KB; i++) if (j0 + i >= N) v[i].zero();
@@ -399,7 +400,7 @@ struct QuadFeeder {
 // The same mapping with the queries' records, for row emission where queries are few beside the keys or the rows are wide: what a
 // block costs besides its queries is then what counts, and 4 channels per lane halve (LPS = 16) or quarter (LPS = 8) it. The
 // streams of a warp go through their queries side by side, each in its own loop.
-template <int LPS> __host__ __device__ constexpr int row_smem_bytes() { return sum_smem_bytes<LPS>() + WALK_THREADS * 2 * 16; }
+template <int LPS> __host__ __device__ constexpr int row_smem_bytes() { return sum_smem_bytes<LPS>() + ROW_THREADS * 2 * 16; }
 
 template <int LPS>
 struct RowFeeder : QuadFeeder<LPS> {
