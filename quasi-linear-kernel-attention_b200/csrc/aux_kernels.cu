@@ -22,34 +22,52 @@ __global__ void colsum_d_kernel(const float* __restrict__ x, float* __restrict__
 // Per p over rows r of w (P, R, C4) with optional row scalars s (P, R):
 //   wsum[p, c] += sum_r w[r, c],  swsum[p, c] += sum_r s[r] w[r, c],  ssum[p] += sum_r s[r]
 // (outputs must be zeroed; partial sums of a row tile are added atomically). grid (tiles, P).
+// VEC: C4 is a multiple of four; 16 bytes per lane, eight rows of a thread in flight (one float per lane and row at a time: 0.064 -> 0.024 ms
+// for 96 heads x 4096 rows x 64 channels, 101 MB).
 constexpr int RS_THREADS = 256, RS_ROWS = 256;
+template <bool VEC>
 __global__ void __launch_bounds__(RS_THREADS) rowstat_kernel(
     const float* __restrict__ w, const float* __restrict__ s,
     float* __restrict__ wsum, float* __restrict__ swsum, float* __restrict__ ssum,
     const int R, const int C4)
 {
-    __shared__ float red_w[RS_THREADS], red_k[RS_THREADS];
+    constexpr int U = VEC ? 4 : 1;                                // channels of a lane
+    __shared__ float red_w[U][RS_THREADS], red_k[U][RS_THREADS];
     const int chunks = (R + RS_ROWS - 1) / RS_ROWS;               // (p rides in blockIdx.x: a grid's y extent stops at 65535)
     const int p  = blockIdx.x / chunks;
     const int r0 = (blockIdx.x % chunks) * RS_ROWS, r1 = min(R, r0 + RS_ROWS);
-    const int CW = C4 <= 32 ? 32 : (C4 <= 64 ? 64 : 128);
-    const int c  = threadIdx.x % CW, lane_r = threadIdx.x / CW, nr = RS_THREADS / CW;
-    float aw = 0.0f, ak = 0.0f, as = 0.0f;
+    const int CW = (C4 <= 32 ? 32 : (C4 <= 64 ? 64 : 128)) / U;   // lanes of a row
+    const int c  = threadIdx.x % CW * U, lane_r = threadIdx.x / CW, nr = RS_THREADS / CW;
+    const float* rows = w + (long long)p * R * C4 + c;
+    const float* sp   = s ? s + (long long)p * R : nullptr;
+    float aw[U], ak[U], as = 0.0f;
+    #pragma unroll
+    for (int u = 0; u < U; u++) aw[u] = ak[u] = 0.0f;
     if (c < C4) {
+        #pragma unroll 8
         for (int r = r0 + lane_r; r < r1; r += nr) {
-            const float x  = w[((long long)p * R + r) * C4 + c];
-            const float sc = s ? s[(long long)p * R + r] : 0.0f;
-            aw += x;
-            ak = fmaf(sc, x, ak);
-            if (c == 0) as += sc;
+            float x[U];
+            if constexpr (VEC) { const float4 t = ldg4(rows + (long long)r * C4); x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w; }
+            else               x[0] = rows[(long long)r * C4];
+            const float sc = sp ? __ldg(sp + r) : 0.0f;
+            #pragma unroll
+            for (int u = 0; u < U; u++) { aw[u] += x[u]; ak[u] = fmaf(sc, x[u], ak[u]); }
+            as += sc;
         }
     }
-    red_w[threadIdx.x] = aw; red_k[threadIdx.x] = ak;
+    #pragma unroll
+    for (int u = 0; u < U; u++) { red_w[u][threadIdx.x] = aw[u]; red_k[u][threadIdx.x] = ak[u]; }
     __syncthreads();
     if (lane_r == 0 && c < C4) {
-        for (int j = 1; j < nr; j++) { aw += red_w[j * CW + c]; ak += red_k[j * CW + c]; }
-        atomicAdd(wsum + (long long)p * C4 + c, aw);
-        if (swsum) atomicAdd(swsum + (long long)p * C4 + c, ak);
+        for (int j = 1; j < nr; j++) {
+            #pragma unroll
+            for (int u = 0; u < U; u++) { aw[u] += red_w[u][j * CW + threadIdx.x]; ak[u] += red_k[u][j * CW + threadIdx.x]; }
+        }
+        #pragma unroll
+        for (int u = 0; u < U; u++) {
+            atomicAdd(wsum + (long long)p * C4 + c + u, aw[u]);
+            if (swsum) atomicAdd(swsum + (long long)p * C4 + c + u, ak[u]);
+        }
     }
     if (ssum && c == 0) atomicAdd(ssum + p, as);
 }
@@ -72,23 +90,31 @@ __global__ void __launch_bounds__(256) vecsum_kernel(const float* __restrict__ x
 // out[p, m, c] = A * ktot[p, c] - (A * qsum[p, m] + Bq) * vsum[p, c];  out_u[p, m] = A * ksr[p] - Nk * (A * qsum[p, m] + Bq)
 // (A = 1, Bq = 0 for the plain abs sum; a folded sum over shifted queries has A = sum of weights, Bq = D * sum w_s shift_s; without
 // qsum the query terms are left out)
-__global__ void abs_init_kernel(
+// The kernels over rows take ROW_TILE rows per CTA, so that what depends on the row is worked out once per CTA, not by a division per element.
+constexpr int ROW_TILE = 64;
+__global__ void __launch_bounds__(256) abs_init_kernel(
     const float* __restrict__ ktot, const float* __restrict__ vsum, const float* __restrict__ qsum,
     const float* __restrict__ ksr, float* __restrict__ out, float* __restrict__ out_u,
-    const int M, const int C4, const float Nk, const long long total4, const float A, const float Bq)
+    const int M, const int C4, const float Nk, const long long rows, const float A, const float Bq)
 {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total4) return;
-    const int       q4 = C4 >> 2;
-    const int       c  = (int)(i % q4) * 4;
-    const long long pm = i / q4;
-    const long long p  = pm / M;
-    const float4 kt = *reinterpret_cast<const float4*>(ktot + p * C4 + c);
-    const float4 vs = *reinterpret_cast<const float4*>(vsum + p * C4 + c);
-    const float  qs = qsum ? fmaf(A, qsum[pm], Bq) : 0.0f;
-    *reinterpret_cast<float4*>(out + pm * C4 + c) =
-        make_float4(fmaf(-qs, vs.x, A * kt.x), fmaf(-qs, vs.y, A * kt.y), fmaf(-qs, vs.z, A * kt.z), fmaf(-qs, vs.w, A * kt.w));
-    if (out_u && c == 0) out_u[pm] = A * ksr[p] - Nk * qs;
+    __shared__ float qs[ROW_TILE];
+    __shared__ int   head[ROW_TILE];
+    const long long r0 = (long long)blockIdx.x * ROW_TILE;
+    const int n = (int)min((long long)ROW_TILE, rows - r0), q4 = C4 >> 2, tid = threadIdx.x;
+    if (tid < n) {
+        const int p = (int)((r0 + tid) / M);
+        head[tid] = p;
+        qs[tid]   = qsum ? fmaf(A, qsum[r0 + tid], Bq) : 0.0f;
+        if (out_u) out_u[r0 + tid] = A * ksr[p] - Nk * qs[tid];
+    }
+    __syncthreads();
+    #pragma unroll 4
+    for (int i = tid; i < n * q4; i += 256) {
+        const int r = i / q4, c = (i - r * q4) * 4;
+        const float4 kt = ldg4(ktot + (long long)head[r] * C4 + c), vs = ldg4(vsum + (long long)head[r] * C4 + c);
+        *reinterpret_cast<float4*>(out + r0 * C4 + 4 * i) =
+            make_float4(fmaf(-qs[r], vs.x, A * kt.x), fmaf(-qs[r], vs.y, A * kt.y), fmaf(-qs[r], vs.z, A * kt.z), fmaf(-qs[r], vs.w, A * kt.w));
+    }
 }
 
 // dst (rows, C4) <- src (rows, C), zero filled
@@ -177,22 +203,34 @@ __global__ void __launch_bounds__(256) transpose_back_kernel(const float* __rest
 }
 
 // dn[row, :] = g[row, :] / max(den[row], clamp),  dd[row] = den[row] >= clamp ? -<dn[row, :], out[row, :]> : 0; one warp per row
+template <bool VEC>
 __global__ void __launch_bounds__(256) attention_gradient_rows_kernel(const float* __restrict__ g, const float* __restrict__ out, const float* __restrict__ den,
                                                                       float* __restrict__ dn, float* __restrict__ dd, const int C, const float clamp, const long long rows)
 {
-    const long long row  = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int       lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const float d = den[row], inv = 1.0f / fmaxf(d, clamp);
-    float dot = 0.0f;
-    for (int c = lane; c < C; c += 32) {
-        const float x = g[row * C + c] * inv;
-        dn[row * C + c] = x;
-        dot = fmaf(x, out[row * C + c], dot);
+    constexpr int U = VEC ? 4 : 1;
+    const int lanes = VEC ? (C <= 32 ? 8 : C <= 64 ? 16 : 32) : 32, step = 256 / lanes, ln = threadIdx.x % lanes;
+    const long long r0 = (long long)blockIdx.x * ROW_TILE, r1 = min(rows, r0 + ROW_TILE);
+    #pragma unroll 4
+    for (long long r = r0 + threadIdx.x / lanes; r - threadIdx.x / lanes < r1; r += step) {      // (all lanes of a warp stay for the shuffles)
+        const long long row = min(r, rows - 1);
+        const float d = __ldg(den + row), inv = 1.0f / fmaxf(d, clamp);
+        float dot = 0.0f;
+        for (int c = ln * U; c < C; c += lanes * U) {
+            if constexpr (VEC) {
+                float4 x = ldg4(g + row * C + c);
+                const float4 o = ldg4(out + row * C + c);
+                x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
+                if (r < r1) *reinterpret_cast<float4*>(dn + row * C + c) = x;
+                dot = fmaf(x.x, o.x, fmaf(x.y, o.y, fmaf(x.z, o.z, fmaf(x.w, o.w, dot))));
+            } else {
+                const float x = g[row * C + c] * inv;
+                if (r < r1) dn[row * C + c] = x;
+                dot = fmaf(x, out[row * C + c], dot);
+            }
+        }
+        for (int off = lanes / 2; off > 0; off >>= 1) dot += __shfl_xor_sync(FULL, dot, off);
+        if (ln == 0 && r < r1) dd[row] = d >= clamp ? -dot : 0.0f;
     }
-    #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(FULL, dot, off);
-    if (lane == 0) dd[row] = d >= clamp ? -dot : 0.0f;
 }
 
 // dst[p, s, :] = src[p, s, :] * keep[p / H, s]   (src may be dst)
@@ -224,40 +262,59 @@ __global__ void __launch_bounds__(256) npad_kernel(const float* __restrict__ kee
 // out[p, m, :] /= max(out_u[p, m] - n_pad[p / H] * sum_d f(qt[p, d, m]), clamp): the row normalisation of _add_laplace
 // (BUMP = false, f(x) = exp(-|x|)) and of _add_bump (BUMP = true, f(x) = max(0, 1 - |x|)), with the row sum corrected for
 // the masked keys (each sits at k = 0 with v = 0 and adds f(q_d) per dimension); the corrected sum goes to den_out if given.
-// One warp per row.
+// A warp per row took 53 us for 24 heads x 8192 rows x 64 channels (101 MB moved), this 15.
 template <bool BUMP>
 __global__ void __launch_bounds__(256) normalise_kernel(float* __restrict__ out, const float* __restrict__ out_u,
                                                         const float* __restrict__ qt, const float* __restrict__ n_pad,
                                                         const int M, const int D, const int C, const int H,
                                                         const float clamp, const long long rows, float* __restrict__ den_out)
 {
-    const long long row  = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int       lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const long long p = row / M, m = row % M;
-    float den = out_u[row];
-    if (n_pad) {
-        const float np = n_pad[p / H];
-        if (np != 0.0f) {
+    __shared__ float part[4][ROW_TILE], inv[ROW_TILE];
+    const long long r0 = (long long)blockIdx.x * ROW_TILE;
+    const int n = (int)min((long long)ROW_TILE, rows - r0), tid = threadIdx.x, t = tid % ROW_TILE;
+    if (n_pad) {                                       // the weights of a masked key, whose coordinates are 0: neighbouring lanes on neighbouring rows
+        if (t < n) {
+            const int p = (int)((r0 + t) / M), m = (int)((r0 + t) - (long long)p * M);
             float acc = 0.0f;
-            for (int d = lane; d < D; d += 32) {
-                const float x = fabsf(qt[(p * D + d) * M + m]);
-                acc += BUMP ? fmaxf(0.0f, 1.0f - x) : __expf(-x);
+            if (n_pad[p / H] != 0.0f) {
+                #pragma unroll 8
+                for (int d = tid / ROW_TILE; d < D; d += 4) {
+                    const float x = fabsf(__ldg(qt + ((long long)p * D + d) * M + m));
+                    acc += BUMP ? fmaxf(0.0f, 1.0f - x) : __expf(-x);
+                }
             }
-            #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(FULL, acc, off);
-            den -= np * acc;
+            part[tid / ROW_TILE][t] = acc;
         }
+        __syncthreads();
     }
-    if (den_out && lane == 0) den_out[row] = den;
-    const float inv = 1.0f / fmaxf(den, clamp);
-    float* o = out + row * C;
-    for (int c = lane; c < C; c += 32) o[c] *= inv;
+    if (tid < n) {
+        float den = out_u[r0 + tid];
+        if (n_pad) {
+            const float np = n_pad[(int)((r0 + tid) / M) / H];
+            if (np != 0.0f) den -= np * ((part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]));
+        }
+        if (den_out) den_out[r0 + tid] = den;
+        inv[tid] = 1.0f / fmaxf(den, clamp);
+    }
+    __syncthreads();
+    float* o = out + r0 * C;
+    if (C % 4 == 0) {
+        const int q = C >> 2;
+        #pragma unroll 4
+        for (int i = tid; i < n * q; i += 256) {
+            float4 x = *reinterpret_cast<const float4*>(o + 4 * i);
+            const float f = inv[i / q];
+            x.x *= f; x.y *= f; x.z *= f; x.w *= f;
+            *reinterpret_cast<float4*>(o + 4 * i) = x;
+        }
+    } else {
+        for (int i = tid; i < n * C; i += 256) o[i] *= inv[i / C];
+    }
 }
 
 // The add_riesz epilogue (Experiments/kernel_attention/attention.py:75-81), in place on out = the weighted abs sum:
 //   a = aq[p, m] + eps;  num = a * vsum[p, :] + akv[p, :] - out;  den = a * S + aksum[p] - out_u[p, m] - eps * n_pad[p / H]
-//   out = num / max(den, clamp).   One warp per row.
+//   out = num / max(den, clamp).
 __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__ out, const float* __restrict__ out_u,
                                                              const float* __restrict__ aq, const float* __restrict__ vsum,
                                                              const float* __restrict__ akv, const float* __restrict__ aksum,
@@ -265,17 +322,38 @@ __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__
                                                              const int M, const int C, const int C4, const int H,
                                                              const float eps, const float clamp, const long long rows, float* __restrict__ den_out)
 {
-    const long long row  = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int       lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const long long p = row / M;
-    const float a   = aq[row] + eps;
-    const float np  = n_pad ? n_pad[p / H] : 0.0f;
-    const float den = a * (float)M + aksum[p] - out_u[row] - eps * np;
-    if (den_out && lane == 0) den_out[row] = den;
-    const float inv = 1.0f / fmaxf(den, clamp);
-    float* o = out + row * C;
-    for (int c = lane; c < C; c += 32) o[c] = (fmaf(a, vsum[p * C4 + c], akv[p * C4 + c]) - o[c]) * inv;
+    __shared__ float as[ROW_TILE], inv[ROW_TILE];
+    __shared__ int   head[ROW_TILE];
+    const long long r0 = (long long)blockIdx.x * ROW_TILE;
+    const int n = (int)min((long long)ROW_TILE, rows - r0), tid = threadIdx.x;
+    if (tid < n) {
+        const int   p   = (int)((r0 + tid) / M);
+        const float a   = aq[r0 + tid] + eps;
+        const float np  = n_pad ? n_pad[p / H] : 0.0f;
+        const float den = a * (float)M + aksum[p] - out_u[r0 + tid] - eps * np;
+        if (den_out) den_out[r0 + tid] = den;
+        as[tid] = a; head[tid] = p; inv[tid] = 1.0f / fmaxf(den, clamp);
+    }
+    __syncthreads();
+    float* o = out + r0 * C;
+    if (C % 4 == 0 && C4 == C) {
+        const int q = C >> 2;
+        #pragma unroll 4
+        for (int i = tid; i < n * q; i += 256) {
+            const int r = i / q, c = (i - r * q) * 4;
+            const float4 vs = ldg4(vsum + (long long)head[r] * C4 + c), kv = ldg4(akv + (long long)head[r] * C4 + c);
+            const float  a = as[r], f = inv[r];
+            float4 x = *reinterpret_cast<const float4*>(o + 4 * i);
+            x.x = (fmaf(a, vs.x, kv.x) - x.x) * f; x.y = (fmaf(a, vs.y, kv.y) - x.y) * f;
+            x.z = (fmaf(a, vs.z, kv.z) - x.z) * f; x.w = (fmaf(a, vs.w, kv.w) - x.w) * f;
+            *reinterpret_cast<float4*>(o + 4 * i) = x;
+        }
+    } else {
+        for (int i = tid; i < n * C; i += 256) {
+            const int r = i / C, c = i - r * C;
+            o[i] = (fmaf(as[r], vsum[(long long)head[r] * C4 + c], akv[(long long)head[r] * C4 + c]) - o[i]) * inv[r];
+        }
+    }
 }
 
 static inline unsigned blocks_for(long long total, int threads) { return (unsigned)((total + threads - 1) / threads); }
@@ -292,7 +370,8 @@ cudaError_t launch_abscolsum_d(const float* x, float* out, int P, int D, int L, 
 }
 cudaError_t launch_rowstat(const float* w, const float* s, float* wsum, float* swsum, float* ssum, int P, int R, int C4, cudaStream_t st) {
     const unsigned grid = (unsigned)((R + RS_ROWS - 1) / RS_ROWS) * (unsigned)P;
-    rowstat_kernel<<<grid, RS_THREADS, 0, st>>>(w, s, wsum, swsum, ssum, R, C4);
+    if (C4 % 4 == 0) rowstat_kernel<true><<<grid, RS_THREADS, 0, st>>>(w, s, wsum, swsum, ssum, R, C4);
+    else             rowstat_kernel<false><<<grid, RS_THREADS, 0, st>>>(w, s, wsum, swsum, ssum, R, C4);
     return cudaGetLastError();
 }
 cudaError_t launch_vecsum(const float* x, float* out, int P, int L, cudaStream_t st) {
@@ -301,8 +380,8 @@ cudaError_t launch_vecsum(const float* x, float* out, int P, int L, cudaStream_t
 }
 cudaError_t launch_abs_init(const float* ktot, const float* vsum, const float* qsum, const float* ksr,
                             float* out, float* out_u, int P, int M, int C4, int Nk, float A, float Bq, cudaStream_t st) {
-    const long long total4 = (long long)P * M * (C4 >> 2);
-    abs_init_kernel<<<blocks_for(total4, 256), 256, 0, st>>>(ktot, vsum, qsum, ksr, out, out_u, M, C4, (float)Nk, total4, A, Bq);
+    const long long rows = (long long)P * M;
+    abs_init_kernel<<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(ktot, vsum, qsum, ksr, out, out_u, M, C4, (float)Nk, rows, A, Bq);
     return cudaGetLastError();
 }
 cudaError_t launch_pad_rows(const float* src, float* dst, long long rows, int C, int C4, cudaStream_t st) {
@@ -328,7 +407,8 @@ cudaError_t launch_transpose_back(const float* src, float* dst, const float* kee
     return cudaGetLastError();
 }
 cudaError_t launch_attention_gradient_rows(const float* g, const float* out, const float* den, float* dn, float* dd, long long rows, int C, float clamp, cudaStream_t st) {
-    attention_gradient_rows_kernel<<<blocks_for(rows, 8), 256, 0, st>>>(g, out, den, dn, dd, C, clamp, rows);
+    if (C % 4 == 0) attention_gradient_rows_kernel<true><<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(g, out, den, dn, dd, C, clamp, rows);
+    else            attention_gradient_rows_kernel<false><<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(g, out, den, dn, dd, C, clamp, rows);
     return cudaGetLastError();
 }
 cudaError_t launch_mask_rows(const float* src, float* dst, const float* keep, int P, int S, int C, int H, cudaStream_t st) {
@@ -343,15 +423,15 @@ cudaError_t launch_npad(const float* keep, float* n_pad, int B, int S, cudaStrea
 cudaError_t launch_normalise(float* out, const float* out_u, const float* qt, const float* n_pad,
                              int P, int M, int D, int C, int H, float clamp, bool bump, float* den_out, cudaStream_t st) {
     const long long rows = (long long)P * M;
-    if (bump) normalise_kernel<true><<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows, den_out);
-    else      normalise_kernel<false><<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows, den_out);
+    if (bump) normalise_kernel<true><<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows, den_out);
+    else      normalise_kernel<false><<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(out, out_u, qt, n_pad, M, D, C, H, clamp, rows, den_out);
     return cudaGetLastError();
 }
 cudaError_t launch_riesz_epilogue(float* out, const float* out_u, const float* aq, const float* vsum, const float* akv,
                                   const float* aksum, const float* n_pad, int P, int M, int C, int C4, int H,
                                   float eps, float clamp, float* den_out, cudaStream_t st) {
     const long long rows = (long long)P * M;
-    riesz_epilogue_kernel<<<blocks_for(rows, 8), 256, 0, st>>>(out, out_u, aq, vsum, akv, aksum, n_pad, M, C, C4, H, eps, clamp, rows, den_out);
+    riesz_epilogue_kernel<<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(out, out_u, aq, vsum, akv, aksum, n_pad, M, C, C4, H, eps, clamp, rows, den_out);
     return cudaGetLastError();
 }
 
