@@ -98,7 +98,8 @@ __global__ void __launch_bounds__(KEY_THREADS, KEY_CTAS) laplace_pass1(const Wal
 // Between the passes: per segment and channel, the aggregates of the SPS streams become the states entering each
 // stream - in place, forward aggregate -> prefix state before the stream (L = decay * L + aggregate over the earlier
 // streams), backward aggregate -> suffix state after it. A warp's share of the streams is one such step itself: its aggregate and the
-// product of its decays.
+// product of its decays. Bound by latency: with the share in registers, read once and at once, 26 -> 12 us for 24576 streams of 64 channels
+// (48 heads x 1024 keys).
 __global__ void __launch_bounds__(32 * FOLD_WARPS) laplace_fold(float* __restrict__ agg, const int nseg, const int SPS, const int C4, const int warps)
 {
     __shared__ float4 total[FOLD_WARPS][32];       // forward and backward aggregate, forward and backward decay of a share
@@ -106,6 +107,41 @@ __global__ void __launch_bounds__(32 * FOLD_WARPS) laplace_fold(float* __restric
     const int lane = threadIdx.x & 31, c = f.c, first = f.first, last = f.last, AGS = lap_agg_stride(C4);
     float* ag = agg + f.sg * SPS * AGS;
     float L = 0.0f, R = 0.0f;
+    if ((SPS + warps - 1) / warps <= FOLD_CHUNK) {         // the share fits registers: read once, everything in flight together
+        float fv[FOLD_CHUNK], bv[FOLD_CHUNK], af[FOLD_CHUNK], ab[FOLD_CHUNK];
+        #pragma unroll
+        for (int k = 0; k < FOLD_CHUNK; k++) {
+            fv[k] = bv[k] = 0.0f; af[k] = ab[k] = 1.0f;
+            if (first + k < last) {
+                const float* at = ag + (long long)(first + k) * AGS;
+                fv[k] = at[c]; bv[k] = at[C4 + c];
+                const float2 d = *reinterpret_cast<const float2*>(at + 2 * C4);
+                af[k] = d.x; ab[k] = d.y;
+            }
+        }
+        if (warps > 1) {
+            float dl = 1.0f, dr = 1.0f;
+            #pragma unroll
+            for (int k = 0; k < FOLD_CHUNK; k++) {
+                L = fmaf(af[k], L, fv[k]);
+                R = fmaf(dr, bv[k], R);
+                dl *= af[k]; dr *= ab[k];
+            }
+            total[threadIdx.x >> 5][lane] = make_float4(L, R, dl, dr);
+            __syncthreads();
+            L = R = 0.0f;
+            for (int u = f.group; u < f.group + f.share; u++)             { const float4 t = total[u][lane]; L = fmaf(t.z, L, t.x); }
+            for (int u = f.group + warps - 1; u > f.group + f.share; u--) { const float4 t = total[u][lane]; R = fmaf(t.w, R, t.y); }
+        }
+        if (!f.on) return;
+        #pragma unroll
+        for (int k = 0; k < FOLD_CHUNK; k++)
+            if (first + k < last) { ag[(long long)(first + k) * AGS + c] = L; L = fmaf(af[k], L, fv[k]); }
+        #pragma unroll
+        for (int k = FOLD_CHUNK - 1; k >= 0; k--)
+            if (first + k < last) { ag[(long long)(first + k) * AGS + C4 + c] = R; R = fmaf(ab[k], R, bv[k]); }
+        return;
+    }
     if (warps > 1) {
         float dl = 1.0f, dr = 1.0f;
         #pragma unroll FOLD_CHUNK
