@@ -19,7 +19,8 @@
 //   eidx  [seg][ES]        uint32  row index of the event; EVENT_QUERY is set in a query's
 //   esc   [seg][ES]        float2  key: {step decay, 0} (Laplace), {-2 key, 0} (abs); query: {e0, e1}
 //
-// with ES = estride(N + M); sorted key j is event j + (queries of rank <= j), query m of rank r event m + r.
+// with ES = estride(N + M); sorted key j is event j + (queries of rank <= j), query m of rank r event m + r. In xperm (Laplace),
+// KEY_FIRST marks the keys that are the first one of their block of EB events, KEY_LATER those whose block begins after the key before.
 //
 // with KB = 8 keys per block, NBK = N/KB + 1 blocks and NP = NBK*KB padded keys, so that at
 // least one padded position follows the last key and every rank in [0, N] falls in a block.
@@ -38,7 +39,7 @@ __host__ __device__ inline long long xstride(int N)  { return (long long)npad(N)
 __host__ __device__ inline long long mstride(int N)  { return (long long)((nblocks(N) + 1 + 3) & ~3); }
 
 constexpr int      EB = 8;                  // events per block of the walk over events
-constexpr uint32_t EVENT_QUERY = 0x80000000u;
+constexpr uint32_t EVENT_QUERY = 0x80000000u, KEY_FIRST = 0x80000000u, KEY_LATER = 0x40000000u;
 __host__ __device__ inline long long estride(int N, int M) { return ((long long)N + M + EB - 1) / EB * EB; }
 
 enum SortMode : int { MODE_LAPLACE = 0, MODE_ABS = 1, MODE_SGN = 2 };

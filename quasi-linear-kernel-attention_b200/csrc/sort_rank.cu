@@ -706,9 +706,16 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         if (EVENTS) {                                 // the keys' events: hist[j + 1] queries of this part precede key j
             #pragma unroll 2
             for (int j = tid; j < N; j += THREADS) {
-                const uint32_t e = (uint32_t)j + hist[j + 1];
-                eidx[e] = xperm[j];
-                if (LAP)                     esc[e] = make_float2(xval[j], 0.0f);
+                const uint32_t e = (uint32_t)j + hist[j + 1], row = xperm[j];
+                eidx[e] = row;
+                if (LAP) {
+                    esc[e] = make_float2(xval[j], 0.0f);
+                    const uint32_t at = (uint32_t)(ks + qs), from = at + (uint32_t)j + hist[j];      // (from: right after the key before)
+                    uint32_t marks = 0u;
+                    if (ks + j > 0 && (at + e) / EB != (from - 1u) / EB) marks |= KEY_FIRST;
+                    if ((at + e) / EB != from / EB) marks |= KEY_LATER;
+                    if (marks) xperm[j] = row | marks;
+                }
                 else if (a.mode == MODE_ABS) esc[e] = make_float2(-2.0f * xs[skew(j)], 0.0f);
             }
         }

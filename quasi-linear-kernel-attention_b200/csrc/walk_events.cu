@@ -51,8 +51,8 @@ __device__ __forceinline__ f2 mul2(const f2 a, const f2 b) { f2 r; asm("mul.rn.f
 __device__ __forceinline__ f2 fma2(const f2 a, const f2 b, const f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ bool is_query(const uint32_t e) { return (int)e < 0; }
 
-// A stream's events: LPS lanes, blocks visited in steps t = 0 .. nblk-1, forwards (DIR 1) or backwards (DIR -1).
-template <int LPS, int CPL, int DIR>
+// A stream's events: LPS lanes, block t = 0 .. nblk-1.
+template <int LPS, int CPL>
 struct EventFeeder {
     using S = Shape<LPS, CPL>;
     static constexpr int LPE = LPS / EB;       // lanes that add up an event's parts
@@ -94,13 +94,11 @@ struct EventFeeder {
         inner = __reduce_min_sync(FULL, nblk) - 1;
         krows = (unsigned long long)__cvta_generic_to_global(a.rows + (long long)st.p * a.N * a.C4 + channel(0));
         qrows = (unsigned long long)__cvta_generic_to_global(a.g + (long long)st.p * a.M * a.C4 + channel(0)) - (unsigned long long)EVENT_QUERY * row_bytes;
-        const long long at = first + (DIR > 0 ? 0 : max(nblk - 1, 0) * EB);
-        aux = ln < 2 ? reinterpret_cast<const char*>(a.eidx + at) + ln * 16 : reinterpret_cast<const char*>(a.esc + at) + (ln - 2) * 16;
-        aux_step = DIR * EB * (ln < 2 ? 4 : 8);
+        aux = ln < 2 ? reinterpret_cast<const char*>(a.eidx + first) + ln * 16 : reinterpret_cast<const char*>(a.esc + first) + (ln - 2) * 16;
+        aux_step = EB * (ln < 2 ? 4 : 8);
         return first;
     }
-    __device__ __forceinline__ int  block(const int t) const { return DIR > 0 ? t : nblk - 1 - t; }
-    __device__ __forceinline__ bool has(const int t, const int i) const { const int at = block(t) * EB + i; return t < nblk && at >= ev0 && at < ev1; }
+    __device__ __forceinline__ bool has(const int t, const int i) const { const int at = t * EB + i; return t < nblk && at >= ev0 && at < ev1; }
     __device__ __forceinline__ bool edge(const int t) const { return t == 0 || t >= inner; }
     __device__ __forceinline__ void copy_records(const int t, const uint32_t dst) {
         if (t < nblk && ln < 6) { cp_async16(dst + ln * 16, aux); aux += aux_step; }
@@ -123,8 +121,7 @@ struct EventFeeder {
                          : "=f"(v.x[4 * q]), "=f"(v.x[4 * q + 1]), "=f"(v.x[4 * q + 2]), "=f"(v.x[4 * q + 3]) : "l"(at + (q ? second : 0u)));
         return v;
     }
-    // rows of block 0 under way (KEYS: the keys' only), records of block 1 as well
-    template <bool KEYS>
+    // rows of block 0 under way, records of block 1 as well
     __device__ __forceinline__ void prologue(Vec<CPL> (&x)[EB], uint32_t (&e)[EB]) {
         __syncwarp();                  // every lane has left the previous item's slots
         copy_records(0, next);
@@ -136,7 +133,7 @@ struct EventFeeder {
         cp_async_commit();
         read_index(next, e);
         #pragma unroll
-        for (int i = 0; i < EB; i++) if (!KEYS || !is_query(e[i])) x[i] = row(e[i]);
+        for (int i = 0; i < EB; i++) x[i] = row(e[i]);
     }
     // block t becomes the block in use; the indices of block t + 1 are readable
     __device__ __forceinline__ void step(const int t) {
@@ -198,7 +195,7 @@ __device__ __forceinline__ void red_if_query(const bool on, const uint32_t e, co
 template <int LPS, int CPL, bool ROWS>
 __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) prefix_events(const WalkArgs a)
 {
-    using F = EventFeeder<LPS, CPL, 1>;
+    using F = EventFeeder<LPS, CPL>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int C4 = a.C4, NBK = nblocks(a.N);
     F f;
@@ -229,7 +226,7 @@ __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) prefix_events(const WalkA
         }
         Vec<CPL> x[EB];
         uint32_t e[EB];
-        f.template prologue<false>(x, e);
+        f.prologue(x, e);
         const int steps = __reduce_max_sync(FULL, f.nblk);
         for (int t = 0; t < steps; t++) {
             f.step(t);
@@ -285,77 +282,14 @@ cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, int sms, cudaStre
     return cudaErrorInvalidValue;
 }
 
-// The Laplace walk with dots goes over its streams twice, as the row walk does: backwards over the keys for the streams' aggregates and the
-// suffix state at the start of every block, then forwards. There a block is swept twice in registers: backwards with the suffix state, which
-// the next block's checkpoint gives, forwards with the prefix state. (Dots with the stream's own suffix state in the first walk, corrected by
-// the second with what comes from beyond, needs no checkpoints but gathers the queries' rows twice: 0.35 against 0.33 ms at 48 x 1024.)
-// Per block of events: {decay from its first key on to the next stream's first key, decay of its first key}, and the state at that key.
-template <int LPS, int CPL>
-__global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events1(const WalkArgs a)
-{
-    using F = EventFeeder<LPS, CPL, -1>;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int C4 = a.C4, NBK = nblocks(a.N);
-    F f;
-    f.init(smem_u32(smem), C4);
-
-    {
-        const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::S::STREAMS);
-        const long long block0 = f.start(a, st, NBK) / EB;
-        Vec<CPL> A, R;                                    // the stream's forward aggregate, its suffix state
-        A.zero(); R.zero();
-        float w = 1.0f, wr = 1.0f;                        // decay from the last key visited to the stream's last one, to the next stream's first
-        float anext = st.on && st.b1 < NBK ? __ldg(a.xval + (long long)st.sg * xstride(a.N) + st.b1 * KB) : 0.0f;
-        Vec<CPL> x[EB];
-        uint32_t e[EB];
-        f.template prologue<true>(x, e);
-        const int steps = __reduce_max_sync(FULL, f.nblk);
-        for (int t = 0; t < steps; t++) {
-            f.step(t);
-            uint32_t n[EB];
-            f.read_index(f.next, n);
-            #pragma unroll
-            for (int h = EB - EV_GROUP; h >= 0; h -= EV_GROUP) {
-                #pragma unroll
-                for (int i = h + EV_GROUP - 1; i >= h; i--) {
-                    const float s = f.scalars(i).x;
-                    if (!is_query(e[i])) {
-                        #pragma unroll
-                        for (int c = 0; c < CPL; c++) { A.x[c] = fmaf(w, x[i].x[c], A.x[c]); R.x[c] = fmaf(anext, R.x[c], x[i].x[c]); }
-                        wr *= anext; w *= s; anext = s;
-                    }
-                }
-                #pragma unroll
-                for (int i = h; i < h + EV_GROUP; i++) if (!is_query(n[i])) x[i] = f.row(n[i]);
-            }
-            const int b = f.block(t);
-            if (b > 0) {                                  // (streaming: the second pass reads them long after, once)
-                #pragma unroll
-                for (int q = 0; q < F::Q; q++)
-                    if (f.on[q]) __stcs(reinterpret_cast<float4*>(a.ckpt + (block0 + b) * C4 + f.channel(q)), make_float4(R.x[4 * q], R.x[4 * q + 1], R.x[4 * q + 2], R.x[4 * q + 3]));
-                if (f.ln == 0) *reinterpret_cast<float2*>(a.wck + (block0 + b) * 2) = make_float2(wr, anext);
-            }
-            #pragma unroll
-            for (int i = 0; i < EB; i++) e[i] = n[i];
-        }
-        cp_async_wait<0>();
-        if (st.on) {
-            float* ag = a.agg + st.g * (2 * C4 + 4);
-            #pragma unroll
-            for (int q = 0; q < F::Q; q++) {
-                if (!f.on[q]) continue;
-                *reinterpret_cast<float4*>(ag + f.channel(q))      = make_float4(A.x[4 * q], A.x[4 * q + 1], A.x[4 * q + 2], A.x[4 * q + 3]);
-                *reinterpret_cast<float4*>(ag + C4 + f.channel(q)) = make_float4(R.x[4 * q], R.x[4 * q + 1], R.x[4 * q + 2], R.x[4 * q + 3]);
-            }
-            if (f.ln == 0) { ag[2 * C4] = w; ag[2 * C4 + 1] = wr; }
-        }
-    }
-}
-
+// The Laplace walk with dots goes over its streams twice, as the row walk does: backwards over the keys (laplace_pass1, with marks), then
+// forwards over the events. There a block is swept twice in registers: backwards with the suffix state, which the checkpoint of the
+// first key after the block gives, forwards with the prefix state. (Dots with the stream's own suffix state in the first walk, corrected by
+// the second with what comes from beyond, need no checkpoints but gather the queries' rows twice: 0.35 against 0.33 ms at 48 x 1024.)
 template <int LPS, int CPL, bool ROWS>
-__global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events2(const WalkArgs a)
+__global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events(const WalkArgs a)
 {
-    using F = EventFeeder<LPS, CPL, 1>;
+    using F = EventFeeder<LPS, CPL>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int C4 = a.C4, NBK = nblocks(a.N);
     F f;
@@ -369,24 +303,25 @@ __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events2(const Wal
         const float* ag = a.agg + (st.on ? st.g : 0) * (2 * C4 + 4);       // incoming states (laplace_fold left them in the aggregate table)
         Vec<CPL> L = f.vector(ag);
         const float alast = st.on && st.b1 < NBK ? __ldg(a.xval + (long long)st.sg * xstride(a.N) + st.b1 * KB) : 0.0f;
-        const float* ck = a.ckpt + (block0 + 1) * C4;            // of the next block to fetch
-        const float* wk = a.wck + (block0 + 1) * 2;
-        // the checkpoint after the block in use, fetched one block early, into registers that the backward sweep leaves
+        // checkpoints: of the first keys of the blocks after the first that have any, in the places of the stream's last blocks
+        int       left = st.on ? __float_as_int(__ldg(ag + 2 * C4 + 2)) : 0;
+        long long at   = block0 + f.nblk - left;
+        // the checkpoint of the first key after the block in use, fetched one block early, into registers that the backward sweep leaves
         Vec<CPL> cnext;
         float2   wnext = make_float2(0.0f, 0.0f);
         cnext.zero();
-        auto load_ckpt = [&]() { wnext = __ldg(reinterpret_cast<const float2*>(wk)); wk += 2; cnext = f.vector(ck); ck += C4; };
-        if (f.nblk > 1) load_ckpt();
+        auto load_ckpt = [&]() { wnext = __ldg(reinterpret_cast<const float2*>(a.wck + 2 * at)); cnext = f.vector(a.ckpt + at * C4); };
+        if (left > 0) load_ckpt();
         Vec<CPL> x[EB];
         uint32_t e[EB];
-        f.template prologue<false>(x, e);
+        f.prologue(x, e);
         const int steps = __reduce_max_sync(FULL, f.nblk);
         for (int t = 0; t < steps; t++) {
             f.step(t);
             // the state at the first key after the block, that key's decay
             Vec<CPL> R = f.vector(ag + C4);
             float anext = alast;
-            if (t + 1 < f.nblk) {
+            if (left > 0) {
                 #pragma unroll
                 for (int c = 0; c < CPL; c++) R.x[c] = fmaf(wnext.x, R.x[c], cnext.x[c]);
                 anext = wnext.y;
@@ -408,9 +343,15 @@ __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events2(const Wal
                     anext = s.x;
                 }
             }
-            if (t + 2 < f.nblk) load_ckpt();
             uint32_t n[EB];
             f.read_index(f.next, n);
+            if (left > 0) {                               // (the last one read stays until its block comes)
+                bool keys = false;
+                #pragma unroll
+                for (int i = 0; i < EB; i++) keys |= !is_query(n[i]);
+                if (keys) { left--; at++; }
+                if (left > 0) load_ckpt();
+            }
             #pragma unroll
             for (int h = 0; h < EB; h += EV_GROUP) {
                 #pragma unroll
@@ -448,31 +389,18 @@ __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events2(const Wal
     }
 }
 
-template <int LPS, int CPL>
-static cudaError_t launch_lap1(const WalkArgs& a, int sms, cudaStream_t stream) {
-    const long long items = ((long long)a.nseg * a.sps * LPS + EV_THREADS - 1) / EV_THREADS;
-    laplace_events1<LPS, CPL><<<(unsigned)items, EV_THREADS, Shape<LPS, CPL>::SMEM, stream>>>(a);
-    return cudaGetLastError();
-}
 template <int LPS, int CPL, bool ROWS>
-static cudaError_t launch_lap2(const WalkArgs& a, int sms, cudaStream_t stream) {
+static cudaError_t launch_lap(const WalkArgs& a, cudaStream_t stream) {
     const long long items = ((long long)a.nseg * a.sps * LPS + EV_THREADS - 1) / EV_THREADS;
-    laplace_events2<LPS, CPL, ROWS><<<(unsigned)items, EV_THREADS, Shape<LPS, CPL>::SMEM, stream>>>(a);
+    laplace_events<LPS, CPL, ROWS><<<(unsigned)items, EV_THREADS, Shape<LPS, CPL>::SMEM, stream>>>(a);
     return cudaGetLastError();
 }
 
-// the first pass of the Laplace walk with dots
-cudaError_t launch_laplace_events1(const WalkArgs& a, int sms, cudaStream_t stream) {
-    if (a.C4 <= 32)  return launch_lap1<8, 4>(a, sms, stream);
-    if (a.C4 <= 64)  return launch_lap1<8, 8>(a, sms, stream);
-    if (a.C4 <= 128) return launch_lap1<16, 8>(a, sms, stream);
-    return cudaErrorInvalidValue;
-}
-// ... and, after laplace_fold, the second: dots, or rows and dots
-cudaError_t launch_laplace_events2(const WalkArgs& a, bool rows, int sms, cudaStream_t stream) {
-    if (a.C4 <= 32)  return rows ? launch_lap2<8, 4, true>(a, sms, stream) : launch_lap2<8, 4, false>(a, sms, stream);
-    if (a.C4 <= 64)  return rows ? launch_lap2<16, 4, true>(a, sms, stream) : launch_lap2<16, 4, false>(a, sms, stream);
-    if (a.C4 <= 128) return rows ? launch_lap2<32, 4, true>(a, sms, stream) : launch_lap2<32, 4, false>(a, sms, stream);
+// the second pass of the Laplace walk with dots, after laplace_pass1 and laplace_fold: dots, or rows and dots
+cudaError_t launch_laplace_events(const WalkArgs& a, bool rows, cudaStream_t stream) {
+    if (a.C4 <= 32)  return rows ? launch_lap<8, 4, true>(a, stream) : launch_lap<8, 4, false>(a, stream);
+    if (a.C4 <= 64)  return rows ? launch_lap<16, 4, true>(a, stream) : launch_lap<16, 4, false>(a, stream);
+    if (a.C4 <= 128) return rows ? launch_lap<32, 4, true>(a, stream) : launch_lap<32, 4, false>(a, stream);
     return cudaErrorInvalidValue;
 }
 

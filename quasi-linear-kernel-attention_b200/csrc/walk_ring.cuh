@@ -523,6 +523,11 @@ struct StreamOf {
     }
 };
 
+// where the events of key blocks before b end, among all events of all segments
+__device__ __forceinline__ long long events_end(const WalkArgs& a, const int sg, const int b) {
+    return (long long)sg * estride(a.N, a.M) + min(b * KB, a.N) + (int)__ldg(a.mstart + (long long)sg * mstride(a.N) + b);
+}
+
 // The first passes' staging: LPS lanes per stream with CPL = 4 or 8 channels each (quads ln, and LPS + ln, of the row). Rows go straight to
 // registers, those of the next block as soon as the block in use is done with (through shared memory, as above, the load/store pipe
 // moves them twice: Laplace at 48 heads x 16384 keys 1.12 -> 0.79 ms, abs at
@@ -562,7 +567,7 @@ struct KeyFeeder {
         s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w; s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
     }
     __device__ __forceinline__ Vec<CPL> row(const uint32_t i) const {
-        const char* at = rows + (unsigned long long)i * row_bytes;
+        const char* at = rows + (unsigned long long)(i & ~(KEY_FIRST | KEY_LATER)) * row_bytes;
         Vec<CPL> v;
         #pragma unroll
         for (int q = 0; q < Q; q++)
