@@ -92,14 +92,15 @@ __device__ __forceinline__ void tmem_load32(const uint32_t addr, float (&r)[32])
                  : "r"(addr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void split3(const float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
-    a = __float2bfloat16_rn(x);
-    const float r = x - __bfloat162float(a);
-    b = __float2bfloat16_rn(r);
-    c = __float2bfloat16_rn(r - __bfloat162float(b));
-}
-__device__ __forceinline__ uint32_t pack2(const __nv_bfloat16 lo, const __nv_bfloat16 hi) {
-    return (uint32_t)__bfloat16_as_ushort(lo) | (uint32_t)__bfloat16_as_ushort(hi) << 16;
+// the three parts of two neighbouring values, one word each (two conversions per instruction)
+__device__ __forceinline__ void split3(const float x, const float y, uint32_t (&p)[3]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(x, y);
+    const float rx = x - __low2float(a), ry = y - __high2float(a);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(rx, ry);
+    const __nv_bfloat162 c = __floats2bfloat162_rn(rx - __low2float(b), ry - __high2float(b));
+    p[0] = *reinterpret_cast<const uint32_t*>(&a);
+    p[1] = *reinterpret_cast<const uint32_t*>(&b);
+    p[2] = *reinterpret_cast<const uint32_t*>(&c);
 }
 
 }  // namespace
@@ -278,16 +279,20 @@ __global__ void __launch_bounds__(LIN_THREADS, 1) linear_kernel(const __grid_con
                         #pragma unroll
                         for (int j = 0; j < 32; j += 8) {
                             uint32_t p[3][4];
+                            const float4 b0 = ldg4(g.bias + n + j), b1 = ldg4(g.bias + n + j + 4);
+                            const float  bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
                             #pragma unroll
                             for (int e = 0; e < 8; e += 2) {
-                                __nv_bfloat16 u[2][3];
+                                float z[2];
                                 #pragma unroll
                                 for (int f = 0; f < 2; f++) {
-                                    const float y = r[c][j + e + f] + __ldg(g.bias + n + j + e + f);
-                                    split3(0.5f * y * (1.0f + erff(y * 0.70710678118654752440f)), u[f][0], u[f][1], u[f][2]);
+                                    const float y = r[c][j + e + f] + bias[e + f];
+                                    z[f] = 0.5f * y * (1.0f + erff(y * 0.70710678118654752440f));
                                 }
+                                uint32_t u[3];
+                                split3(z[0], z[1], u);
                                 #pragma unroll
-                                for (int i = 0; i < 3; i++) p[i][e / 2] = pack2(u[0][i], u[1][i]);
+                                for (int i = 0; i < 3; i++) p[i][e / 2] = u[i];
                             }
                             #pragma unroll
                             for (int i = 0; i < 3; i++) *reinterpret_cast<uint4*>(o + i * part + j) = make_uint4(p[i][0], p[i][1], p[i][2], p[i][3]);
@@ -342,33 +347,31 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
             y[0] = fmaf((y[0] - mean) * inv, w4.x, b4.x); y[1] = fmaf((y[1] - mean) * inv, w4.y, b4.y);
             y[2] = fmaf((y[2] - mean) * inv, w4.z, b4.z); y[3] = fmaf((y[3] - mean) * inv, w4.w, b4.w);
         }
-        __nv_bfloat16 u[4][3];
+        uint32_t lo[3], hi[3];
+        split3(y[0], y[1], lo);
+        split3(y[2], y[3], hi);
         #pragma unroll
-        for (int e = 0; e < 4; e++) split3(y[e], u[e][0], u[e][1], u[e][2]);
-        #pragma unroll
-        for (int i = 0; i < 3; i++)
-            *reinterpret_cast<uint2*>(out + (i * rows + row) * K + c) = make_uint2(pack2(u[0][i], u[1][i]), pack2(u[2][i], u[3][i]));
+        for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(out + (i * rows + row) * K + c) = make_uint2(lo[i], hi[i]);
     }
 }
 
-// o (B, H, S, D) -> parts of (B, S, H * D)
-__global__ void __launch_bounds__(256) split_heads_kernel(const float* __restrict__ o, __nv_bfloat16* __restrict__ out, const int H, const int S, const int D, const long long total4)
+// o (B, H, S, D) -> parts of (B, S, H * D); a CTA per (b, h) and run of positions, so that no thread divides but by D / 4
+constexpr int SPLIT_POS = 64;
+__global__ void __launch_bounds__(256) split_heads_kernel(const float* __restrict__ o, __nv_bfloat16* __restrict__ out, const int H, const int S, const int D, const int runs, const long long total)
 {
-    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (i >= total4) return;
-    const int d4 = D >> 2, d = (int)(i % d4) * 4;
-    const long long bsh = i / d4;
-    const int h = (int)(bsh % H);
-    const long long bs = bsh / H;
-    const long long b = bs / S, s = bs % S;
-    const float4 v = ldg4(o + ((b * H + h) * S + s) * D + d);
-    const float  y[4] = {v.x, v.y, v.z, v.w};
-    __nv_bfloat16 u[4][3];
-    #pragma unroll
-    for (int e = 0; e < 4; e++) split3(y[e], u[e][0], u[e][1], u[e][2]);
-    #pragma unroll
-    for (int p = 0; p < 3; p++)
-        *reinterpret_cast<uint2*>(out + p * total4 * 4 + bsh * D + d) = make_uint2(pack2(u[0][p], u[1][p]), pack2(u[2][p], u[3][p]));
+    const int bh = blockIdx.x / runs, s0 = (blockIdx.x % runs) * SPLIT_POS, n = min(SPLIT_POS, S - s0), d4 = D >> 2;
+    const float* src = o + ((long long)bh * S + s0) * D;
+    const long long dst = (((long long)(bh / H) * S + s0) * H + bh % H) * D;
+    #pragma unroll 4
+    for (int i = threadIdx.x; i < n * d4; i += 256) {
+        const int s = i / d4, d = (i - s * d4) * 4;
+        const float4 v = ldg4(src + 4 * i);
+        uint32_t lo[3], hi[3];
+        split3(v.x, v.y, lo);
+        split3(v.z, v.w, hi);
+        #pragma unroll
+        for (int p = 0; p < 3; p++) *reinterpret_cast<uint2*>(out + p * total + dst + (long long)s * H * D + d) = make_uint2(lo[p], hi[p]);
+    }
 }
 
 cudaError_t launch_split_rows(const float* x, const float* w, const float* b, void* out, long long rows, int K, float eps, cudaStream_t st) {
@@ -379,8 +382,8 @@ cudaError_t launch_split_rows(const float* x, const float* w, const float* b, vo
 }
 
 cudaError_t launch_split_heads(const float* o, void* out, int B, int H, int S, int D, cudaStream_t st) {
-    const long long total4 = (long long)B * H * S * D / 4;
-    split_heads_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, st>>>(o, static_cast<__nv_bfloat16*>(out), H, S, D, total4);
+    const int runs = (S + SPLIT_POS - 1) / SPLIT_POS;
+    split_heads_kernel<<<(unsigned)B * H * runs, 256, 0, st>>>(o, static_cast<__nv_bfloat16*>(out), H, S, D, runs, (long long)B * H * S * D);
     return cudaGetLastError();
 }
 
