@@ -331,9 +331,12 @@ bool dense_pays(int kind, long long P, int D, int N, int M, int C, bool masked =
     return dense_us(kind, (double)P, D, N, M, C) * (masked ? 0.85 : 1.0) < sorted_us(kind, (double)P, D, N, M, C) * (masked ? 1.25 : 1.0);
 }
 
-// The same for the gradients: three kernels of the same tiling against two sorts and three walks (Laplace 0.43 ns per feature
-// and key, abs 0.30, measured at 4096 keys; the bump's are three abs gradients put together op by op). The Laplace estimate lies 39 % above
-// the present walks (48 heads x 1024 keys 1647 / 1188 us, x 4096 5705 / 4116).
+// The same for the gradients: three kernels of the same tiling against two sorts and three walks. The abs estimate is fitted to the present
+// walks (within a tenth; pairwise / sorted in us: 48 heads x 300 keys 227 / 316, x 450 490 / 401, x 600 759 / 512, 8 x 800 300 / 172,
+// 48 x 600 with 32 features and channels 584 / 212), which are no less accurate (2-norm against float64, grad_q and grad_v at 600 keys: 1.3e-7 and
+// 2.0e-7 pairwise, 1.2e-7 and 1.3e-7 sorted). The Laplace one lies 70 % above the walks (48 x 1024 1647 / 957 us): the sorted sums
+// round more (grad_q at 900 keys 5.0e-7 against 1.6e-7 pairwise), so calls stay where they were. (The bump's are three abs
+// gradients put together op by op, and so is the sorted riesz.)
 bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C, bool masked = false) {
     if (D > DENSE_MAX_D) return false;
     const double grad_d = kind == DENSE_LAPLACE ? 0.50 : kind == DENSE_BUMP ? 0.68 : 0.26, grad_c = 0.054;
@@ -341,6 +344,7 @@ bool dense_gradient_pays(int kind, long long P, int D, int N, int M, int C, bool
     const double tile = 4096e-6 * sm_count() * (D * grad_d + cw * grad_c);
     const double per_sm = std::ceil((double)P * ((M + N + 127) / 128) / sm_count());
     const double dense = 20.0 + std::max(per_sm, 1.0) * ((M + N + 127) / 128) * tile * (per_sm < 2 ? 0.5 : 1.0) + dense_us(kind, (double)P, D, M, N, C);
+    if (kind == DENSE_ABS) return dense < 100.0 + (double)P * D * (15.0 + 0.19 * (C <= 32 ? 0.55 : C <= 64 ? 1.0 : 1.6) * 0.5 * (N + M)) * 1e-3;
     const double wide = C <= 32 ? 0.8 : C <= 64 ? 1.0 : 1.4, pair = kind == DENSE_LAPLACE ? 0.43 : kind == DENSE_BUMP ? 1.45 : 0.30;
     const double sorted = (kind == DENSE_BUMP ? 250.0 : 110.0) + (double)P * D * (60.0 + pair * wide * 0.5 * (N + M)) * 1e-3;
     return dense * (masked ? 0.85 : 1.0) < sorted * (masked ? 1.25 : 1.0);
