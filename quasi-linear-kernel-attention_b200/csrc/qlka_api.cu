@@ -113,16 +113,17 @@ int sm_count() {
 // pays as soon as whole segments alone give every CTA a few items.
 struct WalkPlan { int sps, nitems; };
 
-WalkPlan plan_walk(int nseg, int N, int C4, bool laplace, bool dots) {
+// lean: as few streams as serve, for scratch that the usual number of aggregates would not fit
+WalkPlan plan_walk(int nseg, int N, int C4, bool laplace, bool dots, bool lean = false) {
     constexpr int streams = 8;
     // resident CTAs, about (above 64 channels two per SM; planned for four, Laplace at 16 heads x 8191 keys x 1030 queries took 1.08
     // instead of 1.03 ms, its backward at 16 x 8192 4.71 instead of 4.45 ms)
-    const int cap = sm_count() * (C4 > 64 ? 2 : 4), per_cta = dots || C4 > 64 ? 8 : 16;
+    const int cap = sm_count() * (C4 > 64 ? 2 : 4), per_cta = dots || lean || C4 > 64 ? 8 : 16;
     const int nbk = nblocks(N);
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
     if (laplace || items(1) < 2LL * cap)
-        while (items(sps) < (long long)per_cta * cap && nbk / (sps * 2) >= (items(sps) < cap / 4 ? 4 : items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
+        while (items(sps) < (long long)per_cta * cap && nbk / (sps * 2) >= (items(sps) < cap / 4 && !lean ? 4 : items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
     return {sps, (int)items(sps)};
 }
 
@@ -252,9 +253,10 @@ int laplace_chunk_heads(int P, int D, int N, int M, int C4, bool dots) {
 }
 
 struct LapWalkScratch {
-    float *ckpt, *wck, *agg; int heads;
+    float *ckpt, *wck, *agg; int heads; bool lean;
     // dots: for the streams of either side, N keys and M queries or the other way round
-    void carve(Bump& b, int P, int D, int N, int M, int C4, bool dots) {
+    void carve(Bump& b, int P, int D, int N, int M, int C4, bool dots, bool lean_ = false) {
+        lean  = lean_;
         heads = laplace_chunk_heads(P, D, N, M, C4, dots);
         const int nseg_c = heads * D;
         ckpt = b.take<float>((size_t)nseg_c * ckpt_blocks(N, M, dots) * C4);
@@ -263,7 +265,7 @@ struct LapWalkScratch {
         size_t a = 0;
         for (const int h : {heads, P % heads})
             for (const int keys : {N, dots ? M : N})
-                if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, keys, C4, true, dots), h * D, C4, true));
+                if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, keys, C4, true, dots, lean), h * D, C4, true));
         agg = b.take<float>(a);
     }
 };
@@ -276,7 +278,7 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
     for (int p0 = 0; p0 < P; p0 += sc.heads) {
         const int       pc = sc.heads < P - p0 ? sc.heads : P - p0, nseg = pc * D;
         const long long s0 = (long long)p0 * D;
-        const WalkPlan  plan = plan_walk(nseg, N, C4, true, emit != EMIT_ROWS);
+        const WalkPlan  plan = plan_walk(nseg, N, C4, true, emit != EMIT_ROWS, sc.lean);
         WalkArgs a{};
         a.rows = rows + (size_t)p0 * N * C4;
         a.xperm = r.xperm + s0 * npad(N); a.xval = r.xval + s0 * xstride(N);
@@ -390,13 +392,13 @@ DenseArgs dense_attention_args(const float* q, const float* k, const float* v, c
 // ------------------------------------------------------------------ Laplace forward
 struct LaplaceWs {
     float* vpad; float* opad; Records rec; LapWalkScratch walk; size_t bytes;
-    LaplaceWs(void* base, int P, int D, int N, int M, int C) {
+    LaplaceWs(void* base, int P, int D, int N, int M, int C, bool lean = false) {
         Bump b(base);
         const int C4 = round4(C), nseg = P * D;
         vpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         opad = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         rec.carve(b, nseg, N, M);
-        walk.carve(b, P, D, N, M, C4, false);
+        walk.carve(b, P, D, N, M, C4, false, lean);
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
@@ -507,7 +509,10 @@ static int laplace_forward_impl(const float* q, const float* k, const float* v,
         return QLKA_OK;
     }
     LaplaceWs ws(workspace, P, D, N, M, C);
-    if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
+    if (!ws_ok(workspace, workspace_bytes, ws.bytes)) {
+        ws = LaplaceWs(workspace, P, D, N, M, C, true);
+        if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
+    }
     const int C4 = round4(C), nseg = P * D;
 
     const float* rows = v;
@@ -916,7 +921,7 @@ int qlka_weighted_laplace_sum_forward_noalloc(const float* q, const float* k, co
     if (st) return st;
     if (!q || !k || !v || !out_w || !out_u) return QLKA_ERR_NULL;
     if (!aligned16(v, out_w)) return QLKA_ERR_ALIGNMENT;
-    if (LaplaceWs(nullptr, P, D, N, M, C).bytes > QLKA_NOALLOC_SCRATCH_BYTES) return QLKA_ERR_NO_ALLOC_LIMIT;
+    if (LaplaceWs(nullptr, P, D, N, M, C, true).bytes > QLKA_NOALLOC_SCRATCH_BYTES) return QLKA_ERR_NO_ALLOC_LIMIT;
     void* scratch = nullptr;
     st = noalloc_scratch(&scratch);
     if (st) return st;

@@ -88,3 +88,16 @@ def test_refuses_problems_beyond_the_fixed_scratch():
     with pytest.raises(RuntimeError, match="32 MiB"):
         q, k, v = make_inputs(48, 64, 2048, 2048, 8, seed=1)
         qlka_native.laplace_forward_noalloc(q, k, v)
+
+
+def test_fits_with_fewer_streams():
+    """A problem whose scratch only fits with the smaller number of streams per segment is taken, with the same results."""
+    import ctypes as ct
+    import qlka_native
+    lib = qlka_native.lib()
+    P, D, N, M, C = 4, 129, 114, 3465, 100
+    size = ct.c_size_t()
+    assert lib.qlka_laplace_forward_workspace_bytes(P, D, N, M, C, ct.byref(size)) == 0 and size.value > lib.qlka_noalloc_scratch_bytes()
+    q, k, v = make_inputs(P, D, N, M, C, seed=34)
+    for a, b in zip(_call_noalloc(lib, q, k, v), qlka_native.laplace_forward(q, k, v)):
+        assert rel_err(a, b.double()) < TOL
