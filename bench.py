@@ -454,9 +454,9 @@ def run_ours(args, rank, world, local_rank):
 
 
 # figures from a profiler capture of the dominant kernel (dram__bytes_read + dram__bytes_write of one laplace_rows launch over
-# 12 heads: 837.2 MB + 43.6 MB) and from a bare gather / reduction loop with the walk's access pattern (two row gathers and one
+# 12 heads: 845.1 MB + 46.6 MB) and from a bare gather / reduction loop with the walk's access pattern (two row gathers and one
 # row reduction per segment, 48 heads: 3.03 ms), both on a B200; profiles/ has the captures
-WALK_DRAM_BYTES_PER_HEAD = (837.21e6 + 43.63e6) / 12
+WALK_DRAM_BYTES_PER_HEAD = (845.06e6 + 46.57e6) / 12
 L2_FLOOR_MS_PER_HEAD = 3.034 / 48
 
 
