@@ -242,6 +242,14 @@ int qlka_sort_rank_records(const float* x, const float* y,
                            uint32_t* xperm, float* xval, uint32_t* yrec, uint32_t* mstart,
                            void* workspace, size_t workspace_bytes,
                            int P, int D, int N, int M, int mode, qlka_stream_t stream);
+/* The same for the walks of the gradients, which read keys and queries as one list in walk order: eidx (P*D, ES) uint32, the event's
+ * row, bit 31 set in a query's; esc (P*D, ES) 2 x float, {step decay, 0} (Laplace) or {-2 key, 0} (abs) of a key, {e0, e1} of a query;
+ * ES = N + M rounded up to a multiple of 8. In xperm (Laplace) bit 31 marks the keys that are the first one of their 8 events, the
+ * segment's first apart, bit 30 those whose 8 events begin after the key before. */
+int qlka_sort_rank_events(const float* x, const float* y,
+                          uint32_t* xperm, float* xval, uint32_t* eidx, float* esc, uint32_t* mstart,
+                          void* workspace, size_t workspace_bytes,
+                          int P, int D, int N, int M, int mode, qlka_stream_t stream);
 
 #ifdef __cplusplus
 }

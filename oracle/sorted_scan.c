@@ -19,6 +19,10 @@
  *            + g_u (2 rank - N); grad_k the same with the roles of q and k swapped;
  *            grad_v the abs sum with q as keys and g_w as weights. A tie belongs to the
  *            ">=" side in both walks, i.e. sub-gradient -1.
+ *   Laplace backward: the same states contracted. A query with k_j < q <= k_{j+1} has
+ *            d out / d q = exp(-(k_{j+1} - q)) R_{j+1} - exp(-(q - k_j)) L_j, so grad_q is that row times g_w (and, with
+ *            the v == 1 channel, times g_u); grad_k the same with the roles of q and k swapped; grad_v the sum with q as
+ *            keys and g_w as weights. (The reference has no Laplace backward.)
  *
  * Everything is accumulated in double. Written from those formulas, not from the kernels.
  * Parity pin: tests/test_oracle.py checks this file against oracle/direct.py (fp64 O(N^2))
@@ -94,6 +98,80 @@ int oracle_laplace_forward(const float* q, const float* k, const float* v,
             }
         }
         free(it); free(L); free(R);
+    }
+    return fail;
+}
+
+/* the states of oracle_laplace_forward over a sorted stream with rows w; channel C is w == u_i */
+static void laplace_states(const item_t* it, int n, const float* w, const float* u, int C, double* L, double* R) {
+    const int C1 = C + 1;
+    for (int c = 0; c < C1; c++) { L[c] = 0.0; R[(size_t)n * C1 + c] = 0.0; }
+    for (int j = 0; j < n; j++) {
+        const double a = j ? exp(-((double)it[j].key - (double)it[j - 1].key)) : 0.0;
+        const float* wr = w + (size_t)it[j].idx * C;
+        for (int c = 0; c < C; c++) L[(size_t)(j + 1) * C1 + c] = a * L[(size_t)j * C1 + c] + wr[c];
+        L[(size_t)(j + 1) * C1 + C] = a * L[(size_t)j * C1 + C] + u[it[j].idx];
+    }
+    for (int j = n - 1; j >= 0; j--) {
+        const double a = (j + 1 < n) ? exp(-((double)it[j + 1].key - (double)it[j].key)) : 0.0;
+        const float* wr = w + (size_t)it[j].idx * C;
+        for (int c = 0; c < C; c++) R[(size_t)j * C1 + c] = a * R[(size_t)(j + 1) * C1 + c] + wr[c];
+        R[(size_t)j * C1 + C] = a * R[(size_t)(j + 1) * C1 + C] + u[it[j].idx];
+    }
+}
+
+/* grad_q (P,D,M), grad_k (P,D,N), grad_v (P,N,C); g_u may be NULL */
+int oracle_laplace_backward(const float* q, const float* k, const float* v,
+                            const float* g_w, const float* g_u,
+                            double* grad_q, double* grad_k, double* grad_v,
+                            int P, int D, int N, int M, int C)
+{
+    memset(grad_v, 0, sizeof(double) * (size_t)P * N * C);
+    int fail = 0;
+    #pragma omp parallel for schedule(dynamic)
+    for (int p = 0; p < P; p++) {
+        const int C1 = C + 1;
+        const int X  = N > M ? N : M;
+        item_t* it = (item_t*)malloc(sizeof(item_t) * (size_t)X);
+        double* L  = (double*)malloc(sizeof(double) * (size_t)(X + 1) * C1);
+        double* R  = (double*)malloc(sizeof(double) * (size_t)(X + 1) * C1);
+        float*  ones = (float*)malloc(sizeof(float) * (size_t)N);
+        float*  zero = (float*)calloc((size_t)M, sizeof(float));
+        if (!it || !L || !R || !ones || !zero) { fail = 1; free(it); free(L); free(R); free(ones); free(zero); continue; }
+        for (int n = 0; n < N; n++) ones[n] = 1.0f;
+        const float* vp = v + (size_t)p * N * C;
+        const float* gp = g_w + (size_t)p * M * C;
+        const float* up = g_u ? g_u + (size_t)p * M : zero;
+        for (int d = 0; d < D; d++) {
+            const float* kk = k + ((size_t)p * D + d) * N;
+            const float* qq = q + ((size_t)p * D + d) * M;
+            sort_items(kk, N, it);
+            laplace_states(it, N, vp, ones, C, L, R);
+            for (int m = 0; m < M; m++) {
+                const int     j = rank_below(it, N, qq[m]);
+                const double  dl = j > 0 ? exp(-((double)qq[m] - (double)it[j - 1].key)) : 0.0, dr = j < N ? exp(-((double)it[j].key - (double)qq[m])) : 0.0;
+                const double *l = L + (size_t)j * C1, *r = R + (size_t)j * C1;
+                double acc = (double)up[m] * (dr * r[C] - dl * l[C]);
+                for (int c = 0; c < C; c++) acc += (double)gp[(size_t)m * C + c] * (dr * r[c] - dl * l[c]);
+                grad_q[((size_t)p * D + d) * M + m] = acc;
+            }
+            /* grad_k and grad_v: stream = queries with rows g_w (channel C carries g_u) */
+            sort_items(qq, M, it);
+            laplace_states(it, M, gp, up, C, L, R);
+            for (int n = 0; n < N; n++) {
+                const int     j = rank_below(it, M, kk[n]);
+                const double  dl = j > 0 ? exp(-((double)kk[n] - (double)it[j - 1].key)) : 0.0, dr = j < M ? exp(-((double)it[j].key - (double)kk[n])) : 0.0;
+                const double *l = L + (size_t)j * C1, *r = R + (size_t)j * C1;
+                double  acc = dr * r[C] - dl * l[C];
+                double* gv  = grad_v + ((size_t)p * N + n) * C;
+                for (int c = 0; c < C; c++) {
+                    acc += (double)vp[(size_t)n * C + c] * (dr * r[c] - dl * l[c]);
+                    gv[c] += dl * l[c] + dr * r[c];
+                }
+                grad_k[((size_t)p * D + d) * N + n] = acc;
+            }
+        }
+        free(it); free(L); free(R); free(ones); free(zero);
     }
     return fail;
 }

@@ -63,17 +63,25 @@ def abs_sum(q, k, v):
     return torch.from_numpy(ow), torch.from_numpy(ou)
 
 
-def abs_sum_backward(q, k, v, g_w, g_u=None):
+def _backward(name, q, k, v, g_w, g_u):
     q, k, v, g_w = _f32(q), _f32(k), _f32(v), _f32(g_w)
     P, D, N, M, C = _dims(q, k, v)
     gu = None if g_u is None else _f32(g_u)
     gq = np.empty((P, D, M), np.float64)
     gk = np.empty((P, D, N), np.float64)
     gv = np.empty((P, N, C), np.float64)
-    rc = _load().oracle_abs_backward(_ptr(q), _ptr(k), _ptr(v), _ptr(g_w), None if gu is None else _ptr(gu),
-                                     _ptr(gq), _ptr(gk), _ptr(gv), P, D, N, M, C)
+    rc = getattr(_load(), name)(_ptr(q), _ptr(k), _ptr(v), _ptr(g_w), None if gu is None else _ptr(gu),
+                                _ptr(gq), _ptr(gk), _ptr(gv), P, D, N, M, C)
     assert rc == 0
     return torch.from_numpy(gq), torch.from_numpy(gk), torch.from_numpy(gv)
+
+
+def laplace_sum_backward(q, k, v, g_w, g_u=None):
+    return _backward("oracle_laplace_backward", q, k, v, g_w, g_u)
+
+
+def abs_sum_backward(q, k, v, g_w, g_u=None):
+    return _backward("oracle_abs_backward", q, k, v, g_w, g_u)
 
 
 def sgn_sum(q, k, v, g):

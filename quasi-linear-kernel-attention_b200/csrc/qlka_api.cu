@@ -1232,27 +1232,50 @@ int qlka_sort_rank_workspace_bytes(int P, int D, int N, int M, size_t* bytes) {
     return QLKA_OK;
 }
 
-int qlka_sort_rank_records(const float* x, const float* y,
-                           uint32_t* xperm, float* xval, uint32_t* yrec, uint32_t* mstart,
-                           void* workspace, size_t workspace_bytes,
-                           int P, int D, int N, int M, int mode, qlka_stream_t stream_)
+// r: the output arrays, either of queries' records or of events
+static int sort_rank_diagnostic(const float* x, const float* y, Records r, void* workspace, size_t workspace_bytes,
+                                int P, int D, int N, int M, int mode, qlka_stream_t stream)
 {
     int st = check_dims(P, D, N, M, 1);
     if (st) return st;
-    if (!x || !y || !xperm || !xval || !yrec || !mstart) return QLKA_ERR_NULL;
+    if (!x || !y || !r.xperm || !r.xval || !r.mstart) return QLKA_ERR_NULL;
     if (mode != MODE_LAPLACE && mode != MODE_ABS) return QLKA_ERR_PATH;
     size_t need = 0;
     qlka_sort_rank_workspace_bytes(P, D, N, M, &need);
     if (!ws_ok(workspace, workspace_bytes, need)) return QLKA_ERR_WORKSPACE;
     Bump b(workspace);
-    Records r{};
-    r.xperm = xperm; r.xval = xval; r.yrec = reinterpret_cast<uint4*>(yrec); r.mstart = mstart;
     r.su0 = b.take<float>((size_t)P * D * (N + 1));
     r.su1 = b.take<float>((size_t)P * D * (N + 1));
     r.large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(P * D, N, M)) : nullptr;
     SortArgs s = sort_args(r, x, y, P * D, D, N, M, mode, SCAL_NONE);
-    CU(launch_sort_rank(s, r, reinterpret_cast<cudaStream_t>(stream_)));
+    CU(launch_sort_rank(s, r, reinterpret_cast<cudaStream_t>(stream)));
     return QLKA_OK;
+}
+
+int qlka_sort_rank_records(const float* x, const float* y,
+                           uint32_t* xperm, float* xval, uint32_t* yrec, uint32_t* mstart,
+                           void* workspace, size_t workspace_bytes,
+                           int P, int D, int N, int M, int mode, qlka_stream_t stream)
+{
+    Records r{};
+    r.xperm = xperm; r.xval = xval; r.yrec = reinterpret_cast<uint4*>(yrec); r.mstart = mstart;
+    int st = check_dims(P, D, N, M, 1);
+    if (st) return st;
+    if (!yrec) return QLKA_ERR_NULL;
+    return sort_rank_diagnostic(x, y, r, workspace, workspace_bytes, P, D, N, M, mode, stream);
+}
+
+int qlka_sort_rank_events(const float* x, const float* y,
+                          uint32_t* xperm, float* xval, uint32_t* eidx, float* esc, uint32_t* mstart,
+                          void* workspace, size_t workspace_bytes,
+                          int P, int D, int N, int M, int mode, qlka_stream_t stream)
+{
+    Records r{};
+    r.xperm = xperm; r.xval = xval; r.eidx = eidx; r.esc = reinterpret_cast<float2*>(esc); r.mstart = mstart;
+    int st = check_dims(P, D, N, M, 1);
+    if (st) return st;
+    if (!eidx || !esc) return QLKA_ERR_NULL;
+    return sort_rank_diagnostic(x, y, r, workspace, workspace_bytes, P, D, N, M, mode, stream);
 }
 
 }  // extern "C"

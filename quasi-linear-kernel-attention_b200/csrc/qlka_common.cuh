@@ -42,6 +42,11 @@ constexpr int      EB = 8;                  // events per block of the walk over
 constexpr uint32_t EVENT_QUERY = 0x80000000u, KEY_FIRST = 0x80000000u, KEY_LATER = 0x40000000u;
 __host__ __device__ inline long long estride(int N, int M) { return ((long long)N + M + EB - 1) / EB * EB; }
 
+// the marks of the key at event `own`, `after` being the event right after the key before (0 for the segment's first)
+__device__ __forceinline__ uint32_t key_marks(const uint32_t after, const uint32_t own) {
+    return (after > 0u && own / EB != (after - 1u) / EB ? KEY_FIRST : 0u) | (own / EB != after / EB ? KEY_LATER : 0u);
+}
+
 enum SortMode : int { MODE_LAPLACE = 0, MODE_ABS = 1, MODE_SGN = 2 };
 // scalar side channel of the sort/rank kernel
 enum ScalMode : int {
@@ -91,6 +96,7 @@ struct PartArgs {
     const float*    qval;                   // [seg][M] queries grouped by part
     const uint32_t* qidx;                   // [seg][M]
     const PartInfo* info;                   // [seg][maxparts], n = 0 beyond the last part
+    uint2* ends;                            // [seg][maxparts], Laplace events: queries of the part not above its smallest key, above its largest
     int maxparts;
 };
 

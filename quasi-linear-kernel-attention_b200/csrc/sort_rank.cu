@@ -703,6 +703,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
             mstart[NBK] = (uint32_t)MG;
             if (!EVENTS) a.yrec[(long long)seg * (MG + 1) + MG] = make_uint4(0u, 0u, 0u, 0xffffffffu);      // sentinel: a rank no key position has
         }
+        if (PART && EVENTS && LAP && tid == 0) pa.ends[blockIdx.x] = make_uint2(hist[1], (uint32_t)M - hist[N]);
         if (EVENTS) {                                 // the keys' events: hist[j + 1] queries of this part precede key j
             #pragma unroll 2
             for (int j = tid; j < N; j += THREADS) {
@@ -710,10 +711,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
                 eidx[e] = row;
                 if (LAP) {
                     esc[e] = make_float2(xval[j], 0.0f);
-                    const uint32_t at = (uint32_t)(ks + qs), from = at + (uint32_t)j + hist[j];      // (from: right after the key before)
-                    uint32_t marks = 0u;
-                    if (ks + j > 0 && (at + e) / EB != (from - 1u) / EB) marks |= KEY_FIRST;
-                    if ((at + e) / EB != from / EB) marks |= KEY_LATER;
+                    // (a part's first key: where the key before is, only the part before it knows; mark_part_starts puts both together)
+                    const uint32_t at = (uint32_t)(ks + qs), marks = j > 0 || first ? key_marks(at + (uint32_t)j + hist[j], at + e) : 0u;
                     if (marks) xperm[j] = row | marks;
                 }
                 else if (a.mode == MODE_ABS) esc[e] = make_float2(-2.0f * xs[skew(j)], 0.0f);

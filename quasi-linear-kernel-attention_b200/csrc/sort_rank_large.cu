@@ -14,6 +14,7 @@
 //   part_stats        per part: smallest and largest key and the part's own scalar sums; the last CTA of a segment chains them
 //                     into what enters each part from below and from above.
 //   sort_rank_small<..., PART>   the parts.
+//   mark_part_starts  Laplace events: the marks of the parts' first keys.
 //
 // An exact bin count is what bounds a part, not the sample: a part overflows only if a single bin does, that is if more than
 // PART_CAP consecutive keys held no more than SAMPLES_PER_BIN of the samples although 64 or more are expected (below 1e-16
@@ -366,6 +367,17 @@ __global__ void __launch_bounds__(256) part_stats(const SortArgs a, const Lists 
     }
 }
 
+// The marks of the first keys of a segment's parts but the first: the key before is as many events before the part as the part before
+// has queries above its largest key. A thread per part.
+__global__ void __launch_bounds__(256) mark_part_starts(const SortArgs a, const PartArgs pa)
+{
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= (long long)a.nseg * pa.maxparts || i % pa.maxparts == 0 || pa.info[i].n == 0) return;
+    const int ks = pa.info[i].ks;
+    const uint32_t at = (uint32_t)(ks + pa.info[i].qs);
+    a.xperm[i / pa.maxparts * npad(a.N) + ks] |= key_marks(at - pa.ends[i - 1].y, at + pa.ends[i].x);
+}
+
 }  // namespace
 
 size_t sort_rank_large_scratch_bytes(int nseg, int N, int M) { return Lists(nullptr, nseg, N, M).bytes; }
@@ -385,7 +397,11 @@ cudaError_t launch_sort_rank_large(const SortArgs& a, void* scratch, cudaStream_
     if (e != cudaSuccess) return e;
     PartArgs pa{};
     pa.kkey = l.kkey; pa.kidx = l.kidx; pa.qval = l.qval; pa.qidx = l.qidx; pa.info = l.info; pa.maxparts = l.mp;
-    return launch_sort_rank_parts(a, pa, stream);
+    pa.ends = reinterpret_cast<uint2*>(l.stats);            // (chained into info by now)
+    e = launch_sort_rank_parts(a, pa, stream);
+    if (e != cudaSuccess || !a.eidx || a.mode != MODE_LAPLACE) return e;
+    mark_part_starts<<<(parts + 255) / 256, 256, 0, stream>>>(a, pa);
+    return cudaGetLastError();
 }
 
 }  // namespace qlka

@@ -70,6 +70,8 @@ def lib():
         L.qlka_weighted_sgn_sum_forward.argtypes = [_vp] * 5 + [_vp, _sz] + [_i] * 5 + [_vp]
         L.qlka_sort_rank_records.restype = _i
         L.qlka_sort_rank_records.argtypes = [_vp] * 6 + [_vp, _sz] + [_i] * 5 + [_vp]
+        L.qlka_sort_rank_events.restype = _i
+        L.qlka_sort_rank_events.argtypes = [_vp] * 7 + [_vp, _sz] + [_i] * 5 + [_vp]
         _lib = L
     return _lib
 
@@ -361,15 +363,16 @@ def laplace_attention(q, k, v, tau, keep=None):
     return fused_attention("add_laplace", q, k, v, tau, keep)
 
 
-def sort_rank_records(x, y, mode):
-    """Diagnostic: the walk records of the sort/rank stage (see include/qlka.h)."""
+def sort_rank_records(x, y, mode, events=False):
+    """Diagnostic: the walk records of the sort/rank stage (see include/qlka.h): (xperm, xval, yrec, mstart), or
+    (xperm, xval, eidx, esc, mstart) with keys and queries as one list of events."""
     _check(x.is_cuda and y.is_cuda and x.dtype == y.dtype == torch.float32 and x.is_contiguous() and y.is_contiguous(),
            "x and y must be contiguous float32 CUDA tensors")
     P, D, N = x.shape
     M = y.shape[2]
     L = lib()
     NBK = N // 8 + 1
-    NP, MS = NBK * 8, (NBK + 1 + 3) // 4 * 4
+    NP, MS, ES = NBK * 8, (NBK + 1 + 3) // 4 * 4, (N + M + 7) // 8 * 8
     dev = x.device
     with torch.cuda.device(dev):
         n = _sz(0)
@@ -379,10 +382,12 @@ def sort_rank_records(x, y, mode):
         ws = torch.empty(int(n.value), dtype=torch.uint8, device=dev)
         xperm = torch.zeros(P * D, NP, dtype=torch.int32, device=dev)
         xval = torch.zeros(P * D, NP + 8, dtype=torch.float32, device=dev)
-        yrec = torch.zeros(P * D, M + 1, 4, dtype=torch.int32, device=dev)
+        lists = [torch.zeros(P * D, ES, dtype=torch.int32, device=dev), torch.zeros(P * D, ES, 2, dtype=torch.float32, device=dev)] if events \
+            else [torch.zeros(P * D, M + 1, 4, dtype=torch.int32, device=dev)]
         mstart = torch.zeros(P * D, MS, dtype=torch.int32, device=dev)
-        st = L.qlka_sort_rank_records(x.data_ptr(), y.data_ptr(), xperm.data_ptr(), xval.data_ptr(), yrec.data_ptr(),
-                                      mstart.data_ptr(), ws.data_ptr(), int(n.value), P, D, N, M, int(mode), _stream())
+        out = (xperm, xval, *lists, mstart)
+        st = (L.qlka_sort_rank_events if events else L.qlka_sort_rank_records)(
+            x.data_ptr(), y.data_ptr(), *[t.data_ptr() for t in out], ws.data_ptr(), int(n.value), P, D, N, M, int(mode), _stream())
     if st:
         _raise(st)
-    return xperm, xval, yrec, mstart
+    return out

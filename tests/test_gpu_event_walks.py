@@ -65,3 +65,59 @@ def test_forward(N, M, C, where):
     for f, ref in ((qlka_native.laplace_forward, sorted_scan.laplace_sum), (lambda *x: qlka_native.abs_forward(*x, True), sorted_scan.abs_sum)):
         for a, b in zip(f(q.cuda(), k.cuda(), v.cuda()), ref(q, k, v)):
             assert rel_err(a, b) < _tol(N, M), rel_err(a, b)
+
+
+# Above 16384 keys or queries a segment is cut by value into parts; 64 features, so that there are hundreds of part boundaries.
+LONG = [(2, 64, 20000, 20000, 64), (1, 64, 65536, 65536, 32), (2, 64, 8192, 40000, 64), (2, 64, 40000, 8192, 64)]
+
+
+def _long_inputs(P, D, N, M, C):
+    g = torch.Generator().manual_seed(N + 3 * M)
+    r = lambda *s: torch.randn(*s, generator=g)
+    return r(P, D, M), r(P, D, N), r(P, N, C), r(P, M, C), r(P, M)
+
+
+def _off(got, want, dim):
+    """Largest relative error in the 2-norm over `dim` (a feature's whole gradient, or a row of grad_v's head)."""
+    got, want = got.detach().double().cpu(), want
+    return ((got - want).norm(dim=dim) / want.norm(dim=dim)).max().item()
+
+
+def _long_tol(N, M, C):
+    """Prefix sums: a state takes one rounded addition per key and a dot C more, twice N + M + C roundings of 2^-25 in the root mean square, which
+    come together as their square root; products with keys, and sums whose terms cancel, are worth a factor of four."""
+    return 4 * (2 * (N + M + C)) ** 0.5 * 2.0 ** -25
+
+
+def _decay_tol(N, M):
+    """Laplace: a step decay is rounded once, by 2^-25 at most and half of that on average, and these roundings need not cancel: between close keys
+    the gaps are multiples of the keys' own spacing, so ties between two decays all go the same way. A state remembers
+    keys about one unit back, 0.4 of all where N(0, 1) is densest. That bias (1.2e-4 at 20000) outgrows the rounding of the sums."""
+    return 0.4 * max(N, M) * 2.0 ** -26
+
+
+@pytest.mark.parametrize("with_u", [True, False])
+@pytest.mark.parametrize("P,D_,N,M,C", LONG)
+def test_long_laplace(P, D_, N, M, C, with_u):
+    from weighted_laplace_sum import weighted_laplace_sum_backward
+    q, k, v, g_w, g_u = _long_inputs(P, D_, N, M, C)
+    g_u = g_u if with_u else None
+    got = weighted_laplace_sum_backward(q.cuda(), k.cuda(), v.cuda(), g_w.cuda(), g_u.cuda() if with_u else None)
+    want = sorted_scan.laplace_sum_backward(q, k, v, g_w, g_u)
+    off = {name: _off(a, b, dim) for name, a, b, dim in zip(("q", "k", "v"), got, want, (-1, -1, 1))}
+    assert max(off.values()) < _decay_tol(N, M), off
+
+
+@pytest.mark.parametrize("with_u", [True, False])
+@pytest.mark.parametrize("P,D_,N,M,C", LONG)
+def test_long_abs_and_sgn(P, D_, N, M, C, with_u):
+    from weighted_abs_sum import weighted_sgn_sum
+    import qlka_native
+    q, k, v, g_w, g_u = _long_inputs(P, D_, N, M, C)
+    g_u = g_u if with_u else None
+    got = qlka_native.abs_backward(q.cuda(), k.cuda(), v.cuda(), g_w.cuda(), g_u.cuda() if with_u else None)
+    want = sorted_scan.abs_sum_backward(q, k, v, g_w, g_u)
+    off = {name: _off(a, b, dim) for name, a, b, dim in zip(("q", "k", "v"), got, want, (-1, -1, 1))}
+    if with_u:
+        off["sgn"] = _off(weighted_sgn_sum(q.cuda(), k.cuda(), v.cuda(), g_w.cuda()), sorted_scan.sgn_sum(q, k, v, g_w), -1)
+    assert max(off.values()) < _long_tol(N, M, C), off

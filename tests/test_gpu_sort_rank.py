@@ -107,6 +107,63 @@ def test_records_more_queries_than_keys(shape, kind):
         check_records(x, y, mode)
 
 
+# The list of events that the walks of the gradients read, and the marks at the keys where their first pass leaves checkpoints; above 16384
+# keys or queries the segment is cut into parts, whose boundaries the blocks of 8 events do not respect.
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 3, 7, 5), (1, 2, 8, 40), (1, 2, 257, 300), (1, 2, 1025, 1500), (1, 2, 64, 4000), (1, 2, 4000, 9), (1, 2, 16384, 16384),
+                                   (2, 4, 20000, 20000), (1, 4, 65536, 65536), (1, 4, 40000, 8192), (1, 4, 8192, 40000), (2, 1, 5, 40000), (1, 1, 512, 70000), (1, 1, 2000, 262144)])
+@pytest.mark.parametrize("kind", ["plain", "narrow", "few_values", "one_key_value"])
+def test_events(shape, kind):
+    P, D, N, M = shape
+    g = torch.Generator().manual_seed(N * 5 + M)
+    x, y = torch.randn(P, D, N, generator=g), torch.randn(P, D, M, generator=g)
+    if kind == "narrow":             # queries crowd between few keys: more of them in a part than a CTA holds
+        y *= 0.01
+    elif kind == "few_values":
+        x, y = (x * 2).round() / 2, (y * 2).round() / 2
+    elif kind == "one_key_value":
+        x[:] = 0.25
+    for mode in (0, 1):
+        check_events(x, y, mode)
+
+
+def check_events(x, y, mode):
+    import qlka_native
+    P, D, N = x.shape
+    M = y.shape[2]
+    xperm, xval, eidx, esc, mstart = (t.cpu().numpy() for t in qlka_native.sort_rank_records(x.cuda(), y.cuda(), mode, events=True))
+    _, _, yrec, want_ms = (t.cpu().numpy() for t in qlka_native.sort_rank_records(x.cuda(), y.cuda(), mode))      # (checked above)
+    for s in range(P * D):
+        xs, ys = x.numpy().reshape(P * D, N)[s], y.numpy().reshape(P * D, M)[s]
+        word = xperm[s, :N].view(np.uint32)
+        perm = (word & 0x3fffffff).astype(np.int64)
+        sx = xs[perm]
+        assert sorted(perm.tolist()) == list(range(N)) and np.all(sx[1:] >= sx[:-1])
+        assert np.array_equal(mstart[s], want_ms[s])
+        rank = np.sort(np.searchsorted(sx, ys, side="left"))                          # of the queries in walk order
+        key_at, query_at = np.arange(N) + np.searchsorted(rank, np.arange(N), side="right"), np.arange(M) + rank
+        e = eidx[s, :N + M].view(np.uint32)
+        assert np.array_equal(e[key_at], perm.astype(np.uint32)), "a key's event"
+        assert np.all(e[query_at] >> 31), "a query's event"
+        rows = (e[query_at] & 0x7fffffff).astype(np.int64)
+        assert sorted(rows.tolist()) == list(range(M))
+        assert np.array_equal(np.searchsorted(sx, ys[rows], side="left"), rank), "queries not in rank order"
+        # the queries' weights: those of their records, whichever of equal rank comes first
+        by_row = np.empty((M, 2), np.int32)
+        by_row[yrec[s, :M, 2]] = yrec[s, :M, :2]
+        got = np.ascontiguousarray(esc[s, query_at]).view(np.int32)
+        assert np.array_equal(got if mode == 0 else got[:, :1], by_row[rows] if mode == 0 else by_row[rows, :1])
+        if mode == 1:
+            assert np.array_equal(esc[s, key_at], np.stack([-2.0 * sx, np.zeros_like(sx)], 1))
+            assert np.all(word >> 30 == 0)
+            continue
+        assert np.array_equal(esc[s, key_at], np.stack([xval[s, :N], np.zeros_like(sx)], 1))
+        after = np.concatenate([[0], key_at[:-1] + 1])                                # the event right after the key before
+        first = (np.arange(N) > 0) & (key_at // 8 != (after - 1) // 8)
+        later = key_at // 8 != after // 8
+        assert np.array_equal(word >> 31, first), f"{np.count_nonzero((word >> 31) != first)} marks of first keys"
+        assert np.array_equal(word >> 30 & 1, later), f"{np.count_nonzero((word >> 30 & 1) != later)} marks of later keys"
+
+
 def check_records(x, y, mode):
     import qlka_native
     P, D, N = x.shape

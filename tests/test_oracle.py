@@ -95,6 +95,9 @@ def test_sorted_scan_against_direct(shape):
         assert rel(a, b) < 1e-12
     for a, b in zip(sorted_scan.abs_sum_backward(q, k, v, gw), direct.abs_sum_backward(q, k, v, gw)):
         assert rel(a, b) < 1e-12
+    for u in (gu, None):
+        for a, b in zip(sorted_scan.laplace_sum_backward(q, k, v, gw, u), direct.laplace_sum_backward(q, k, v, gw, u)):
+            assert rel(a, b) < 1e-12
     assert rel(sorted_scan.sgn_sum(q, k, v, gw), direct.sgn_sum(q, k, v, gw)) < 1e-12
 
 
