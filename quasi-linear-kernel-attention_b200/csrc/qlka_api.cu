@@ -132,19 +132,40 @@ size_t walk_agg_floats(const WalkPlan& w, int nseg, int C4, bool laplace) {
     return (size_t)nseg * w.sps * (laplace ? laplace_agg_stride(C4) : prefix_agg_stride_host(C4));
 }
 
-// scratch of one sort/rank run over nseg segments of N keys and M queries
+// scratch of sort/rank runs over nseg segments
 struct Records {
     uint32_t* xperm; float* xval; uint4* yrec; uint32_t* mstart; float* su0; float* su1;
     uint32_t* eidx; float2* esc;      // the event list, where one is wanted
-    void* large;          // extra scratch of the value-cut sort, only when max(N, M) > SMALL_MAX
-    // records: of the queries, for the row walks; events: N' + M' of the longest list, for the walks with dots (0: none)
-    void carve(Bump& b, int nseg, int N, int M, bool records = true, int events = 0) {
-        large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(nseg, N, M)) : nullptr;
-        xperm  = b.take<uint32_t>((size_t)nseg * npad(N));
-        xval   = b.take<float>((size_t)nseg * xstride(N));
-        yrec   = records ? b.take<uint4>((size_t)nseg * (M + 1)) : nullptr;
-        eidx   = events ? b.take<uint32_t>((size_t)nseg * estride(events, 0)) : nullptr;
-        esc    = events ? b.take<float2>((size_t)nseg * estride(events, 0)) : nullptr;
+    void* large; size_t large_bytes;  // extra scratch of the value-cut sort, only when max(N, M) > SMALL_MAX
+    // for the row walks: N keys, the records of M queries
+    void carve(Bump& b, int nseg, int N, int M) {
+        carve_large(b, nseg, N, M, false);
+        carve_keys(b, nseg, N);
+        yrec = b.take<uint4>((size_t)nseg * (M + 1));
+        eidx = nullptr; esc = nullptr;
+        carve_scans(b, nseg, N);
+    }
+    // for the walks with dots: the events of N keys and M queries, then of the other way round
+    void carve_events(Bump& b, int nseg, int N, int M) {
+        carve_large(b, nseg, N, M, true);
+        carve_keys(b, nseg, std::max(N, M));
+        yrec = nullptr;
+        eidx = b.take<uint32_t>((size_t)nseg * estride(N, M));
+        esc  = b.take<float2>((size_t)nseg * estride(N, M));
+        carve_scans(b, nseg, std::max(N, M));
+    }
+    // (its layout is neither symmetric in N and M nor bounded by that of the longer side twice: parts are cut by queries too where there are more of them)
+    void carve_large(Bump& b, int nseg, int N, int M, bool both) {
+        large_bytes = N > SMALL_MAX || M > SMALL_MAX ? sort_rank_large_scratch_bytes(nseg, N, M) : 0;
+        if (large_bytes && both) large_bytes = std::max(large_bytes, sort_rank_large_scratch_bytes(nseg, M, N));
+        large = large_bytes ? b.take<unsigned char>(large_bytes) : nullptr;
+    }
+private:
+    void carve_keys(Bump& b, int nseg, int N) {
+        xperm = b.take<uint32_t>((size_t)nseg * npad(N));
+        xval  = b.take<float>((size_t)nseg * xstride(N));
+    }
+    void carve_scans(Bump& b, int nseg, int N) {
         mstart = b.take<uint32_t>((size_t)nseg * mstride(N));
         su0    = b.take<float>((size_t)nseg * (N + 1));
         su1    = b.take<float>((size_t)nseg * (N + 1));
@@ -162,6 +183,7 @@ SortArgs sort_args(const Records& r, const float* x, const float* y, int nseg, i
 // the sort/rank stage: shared-memory kernel up to SMALL_MAX elements per segment, cut by value into its parts above
 cudaError_t launch_sort_rank(const SortArgs& s, const Records& r, cudaStream_t stream) {
     if (s.N <= SMALL_MAX && s.M <= SMALL_MAX) return launch_sort_rank_small(s, stream);
+    if (sort_rank_large_scratch_bytes(s.nseg, s.N, s.M) > r.large_bytes) return cudaErrorInvalidValue;
     return launch_sort_rank_large(s, r.large, stream);
 }
 
@@ -412,8 +434,7 @@ struct LaplaceBwdWs {
         vpad  = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         gpad  = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         gvpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
-        const int mx = N > M ? N : M;
-        rec.carve(b, nseg, mx, mx, false, N + M);
+        rec.carve_events(b, nseg, N, M);
         walk.carve(b, P, D, N, M, C4, true);     // one scratch for both walks (stream of keys k, then stream of keys q)
         bytes = (b.off + 255) & ~size_t(255);
     }
@@ -449,8 +470,7 @@ struct AbsBwdWs {
         vpad  = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         gpad  = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         gvpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
-        const int mx = N > M ? N : M;
-        rec.carve(b, nseg, mx, mx, false, N + M);
+        rec.carve_events(b, nseg, N, M);
         qsumd = b.take<float>((size_t)P * M);
         sums  = b.take<float>((size_t)P * C4 * 3 + P);
         const size_t agg_k = prefix_agg_floats(P, D, N, C4, true), agg_q = prefix_agg_floats(P, D, M, C4, true);
@@ -1246,7 +1266,7 @@ static int sort_rank_diagnostic(const float* x, const float* y, Records r, void*
     Bump b(workspace);
     r.su0 = b.take<float>((size_t)P * D * (N + 1));
     r.su1 = b.take<float>((size_t)P * D * (N + 1));
-    r.large = (N > SMALL_MAX || M > SMALL_MAX) ? b.take<unsigned char>(sort_rank_large_scratch_bytes(P * D, N, M)) : nullptr;
+    r.carve_large(b, P * D, N, M, false);
     SortArgs s = sort_args(r, x, y, P * D, D, N, M, mode, SCAL_NONE);
     CU(launch_sort_rank(s, r, reinterpret_cast<cudaStream_t>(stream)));
     return QLKA_OK;

@@ -67,6 +67,32 @@ def test_workspace_grows_with_the_problem(lib):
         assert a.value % 256 == 0
 
 
+@pytest.mark.parametrize("N,M", [(n, n + d) for n in (16384, 20000, 65535, 131000, 262044) for d in (1, 10, 100)] + [(8192, 40000), (512, 70000), (1, 16385), (20000, 20000)])
+def test_gradient_workspaces_hold_the_long_sorts_of_both_orders(lib, N, M):
+    """Above 16384 the sort's own scratch depends on which side is the longer one, by no rule that the longer side alone would bound. What the
+    gradients reserve for it is worked out from their sizes at two channel counts: all else is known, or proportional to the channels."""
+    D = 64
+
+    def size(name, *dims):
+        n = ctypes.c_size_t(0)
+        assert getattr(lib, f"qlka_{name}_workspace_bytes")(*dims, ctypes.byref(n)) == 0
+        return n.value
+
+    sort = max(size("sort_rank", 1, D, a, b) - 8 * D * (a + 1) - 1024 for a, b in ((N, M), (M, N)))
+    most = max(N, M)
+    blocks, events = most // 8 + 1, (N + M + 7) // 8 * 8
+    records = D * (8 * blocks * 4 + (8 * blocks + 8) * 4 + 12 * events + (blocks + 4) // 4 * 16 + 2 * 4 * (most + 1))
+    rounding = 16 * 256                                  # arrays start at multiples of 256 bytes
+    for a, b in ((N, M), (M, N)):
+        for name in ("abs_backward", "sgn_forward"):
+            flat = 2 * size(name, 1, D, a, b, 4) - size(name, 1, D, a, b, 8)          # without what the channels take
+            assert flat + rounding >= sort + records + 4 * b, (name, flat - sort - records)
+        four = size("laplace_backward", 1, D, a, b, 8) - size("laplace_backward", 1, D, a, b, 4)
+        aggregates = (four - D * events // 8 * 16) // 32 * 16                          # two rows of channels and four scalars per stream
+        flat = size("laplace_backward", 1, D, a, b, 4) - four
+        assert flat + rounding >= sort + records + D * events // 8 * 8 + aggregates, flat - sort - records
+
+
 def test_ops_fail_loudly_without_cuda_tensors(lib):
     import torch
     from weighted_abs_sum import weighted_abs_sum

@@ -67,8 +67,9 @@ def test_forward(N, M, C, where):
             assert rel_err(a, b) < _tol(N, M), rel_err(a, b)
 
 
-# Above 16384 keys or queries a segment is cut by value into parts; 64 features, so that there are hundreds of part boundaries.
-LONG = [(2, 64, 20000, 20000, 64), (1, 64, 65536, 65536, 32), (2, 64, 8192, 40000, 64), (2, 64, 40000, 8192, 64)]
+# Above 16384 keys or queries a segment is cut by value into parts; 64 features, so that there are hundreds of part boundaries. Nearly equal
+# lengths: the parts of the one order need more room than those of the longer side twice.
+LONG = [(2, 64, 20000, 20000, 64), (1, 64, 65536, 65536, 32), (2, 64, 8192, 40000, 64), (2, 64, 40000, 8192, 64), (1, 64, 65535, 65536, 32), (2, 64, 16394, 16384, 64)]
 
 
 def _long_inputs(P, D, N, M, C):
