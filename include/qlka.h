@@ -5,7 +5,9 @@
  * with a status code; nothing throws and no host synchronisation happens. Outputs are
  * written to caller-allocated buffers. Scratch memory is a caller-allocated workspace whose
  * size the matching *_workspace_bytes function reports; its contents are meaningless between
- * calls. Inputs are never modified.
+ * calls. Inputs are never modified. The sums, the signed sum, the attention and the sorted gradients
+ * take smaller workspaces too, as far as they can do with them: the gradients and the signed sum go
+ * over their heads, or one head's features, in pieces, down to a segment at a time.
  *
  * Shapes (row-major): q (P, D, M) queries, k (P, D, N) keys, v (P, N, C) values,
  * g_w / g (P, M, C), g_u (P, M), with P = batch * heads.

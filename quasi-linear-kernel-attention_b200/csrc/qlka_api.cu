@@ -208,6 +208,49 @@ bool ws_ok(const void* ws, size_t have, size_t need) {
     return need == 0 || (ws != nullptr && (reinterpret_cast<uintptr_t>(ws) & 255) == 0 && have >= need);
 }
 
+// ------------------------------------------------------------------ gradients, piece by piece
+// The gradients' records and checkpoints grow with the batch, to several times the inputs. So a gradient can go over its heads in pieces, and over
+// the features of one head: whole while that takes no more than PIECE_BUDGET, in halves and so on where it takes more, or where
+// the caller's workspace is smaller. Pieces cost launches and tails (48 heads x 4096 keys, Laplace: 1.4 GB and 3.36 ms whole, 0.7 and 3.62 in
+// two; abs 2.28, 2.51), above the budget nothing (48 x 16384, Laplace: 5.4 GB and 14.5 ms whole, 2.8 and 14.4 in two).
+constexpr size_t PIECE_BUDGET = size_t(4) << 30;
+constexpr size_t ANY_SIZE = ~size_t(0);
+
+struct Piece {
+    int heads, features;                    // features: all of them but where heads is 1
+    Piece half() const { return heads > 1 ? Piece{(heads + 1) / 2, features} : Piece{1, (features + 1) / 2}; }
+    bool  least() const { return heads == 1 && features == 1; }
+};
+
+// the sizes that the pieces of P heads with D features come in
+struct PieceSizes {
+    Piece p[3]; int n = 0;
+    PieceSizes(int P, int D, const Piece& piece) {
+        for (const Piece& c : {piece, Piece{P % piece.heads, piece.features}, Piece{piece.heads, D % piece.features}})
+            if (c.heads && c.features) p[n++] = c;
+    }
+    const Piece* begin() const { return p; }
+    const Piece* end() const { return p + n; }
+};
+
+// the workspace of the largest pieces that suit the budget (whole heads) and `have` bytes, as far as there are such
+template <class Ws>
+Ws in_pieces(void* base, size_t have, int P, int D, int N, int M, int C) {
+    Piece piece{P, D};
+    while (piece.heads > 1 && Ws(nullptr, P, D, N, M, C, piece).bytes > PIECE_BUDGET) piece = piece.half();
+    while (!piece.least() && Ws(nullptr, P, D, N, M, C, piece).bytes > have) piece = piece.half();
+    return Ws(base, P, D, N, M, C, piece);
+}
+
+// run(p0, pc, d0, dc): features d0 .. d0 + dc - 1 of heads p0 .. p0 + pc - 1
+template <class Run>
+int for_pieces(int P, int D, const Piece& piece, Run run) {
+    for (int p0 = 0; p0 < P; p0 += piece.heads)
+        for (int d0 = 0; d0 < D; d0 += piece.features)
+            if (int st = run(p0, std::min(piece.heads, P - p0), d0, std::min(piece.features, D - d0))) return st;
+    return QLKA_OK;
+}
+
 // ------------------------------------------------------------------ walks, a few heads at a time
 // A walk gathers the rows of a head in 64 different orders and adds into its output rows; once the heads in flight no
 // longer fit the L2 (long sequences) it pays to finish a few heads before starting the next ones, so every walk runs over
@@ -222,25 +265,23 @@ int walk_chunk_heads(int P, int N, int C4) {
 }
 
 // aggregate table of a prefix walk over P heads in chunks (the larger of the two chunk sizes that occur)
-size_t prefix_agg_floats(int P, int D, int N, int C4, bool dots) {
+size_t prefix_agg_floats(int P, int D, int N, int C4, bool dots, bool lean = false) {
     const int heads = walk_chunk_heads(P, N, C4);
-    size_t a = walk_agg_floats(plan_walk(heads * D, N, C4, false, dots), heads * D, C4, false);
-    if (const int rem = P % heads) {
-        const size_t a2 = walk_agg_floats(plan_walk(rem * D, N, C4, false, dots), rem * D, C4, false);
-        if (a2 > a) a = a2;
-    }
+    size_t a = 0;
+    for (const int h : {heads, P % heads})
+        if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, N, C4, false, dots, lean), h * D, C4, false));
     return a;
 }
 
 // `w` describes the whole problem (pointers of head 0, nseg = P * D); every chunk gets its own plan
-cudaError_t prefix_walk_chunked(WalkArgs w, int emit, int P, cudaStream_t stream)
+cudaError_t prefix_walk_chunked(WalkArgs w, int emit, int P, cudaStream_t stream, bool lean = false)
 {
     const int heads = walk_chunk_heads(P, w.N, w.C4);
     const WalkArgs all = w;
     for (int p0 = 0; p0 < P; p0 += heads) {
         const int       pc = heads < P - p0 ? heads : P - p0;
         const long long s0 = (long long)p0 * all.D;
-        const WalkPlan  plan = plan_walk(pc * all.D, all.N, all.C4, false, emit != EMIT_ROWS);
+        const WalkPlan  plan = plan_walk(pc * all.D, all.N, all.C4, false, emit != EMIT_ROWS, lean);
         w.rows   = all.rows + (size_t)p0 * all.N * all.C4;
         w.xperm  = all.xperm + s0 * npad(all.N);
         w.xval   = all.xval + s0 * xstride(all.N);
@@ -276,18 +317,19 @@ int laplace_chunk_heads(int P, int D, int N, int M, int C4, bool dots) {
 
 struct LapWalkScratch {
     float *ckpt, *wck, *agg; int heads; bool lean;
-    // dots: for the streams of either side, N keys and M queries or the other way round
-    void carve(Bump& b, int P, int D, int N, int M, int C4, bool dots, bool lean_ = false) {
+    // dots: for the streams of either side, N keys and M queries or the other way round. sizes: heads and features of the walks to come
+    void carve(Bump& b, const PieceSizes& sizes, int N, int M, int C4, bool dots, bool lean_ = false) {
         lean  = lean_;
-        heads = laplace_chunk_heads(P, D, N, M, C4, dots);
-        const int nseg_c = heads * D;
+        heads = laplace_chunk_heads(sizes.p[0].heads, sizes.p[0].features, N, M, C4, dots);
+        const int nseg_c = heads * sizes.p[0].features;
         ckpt = b.take<float>((size_t)nseg_c * ckpt_blocks(N, M, dots) * C4);
         wck  = b.take<float>((size_t)nseg_c * ckpt_blocks(N, M, dots) * (dots ? 2 : 1));
         // the aggregate table of the largest of the chunks that occur (full chunks and the remainder)
         size_t a = 0;
-        for (const int h : {heads, P % heads})
-            for (const int keys : {N, dots ? M : N})
-                if (h) a = std::max(a, walk_agg_floats(plan_walk(h * D, keys, C4, true, dots, lean), h * D, C4, true));
+        for (const Piece& size : sizes)
+            for (const int h : {std::min(heads, size.heads), size.heads % heads})
+                for (const int keys : {N, dots ? M : N})
+                    if (h) a = std::max(a, walk_agg_floats(plan_walk(h * size.features, keys, C4, true, dots, lean), h * size.features, C4, true));
         agg = b.take<float>(a);
     }
 };
@@ -420,30 +462,30 @@ struct LaplaceWs {
         vpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         opad = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         rec.carve(b, nseg, N, M);
-        walk.carve(b, P, D, N, M, C4, false, lean);
+        walk.carve(b, PieceSizes(P, D, Piece{P, D}), N, M, C4, false, lean);
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
 
 // ------------------------------------------------------------------ Laplace backward
 struct LaplaceBwdWs {
-    float *vpad, *gpad, *gvpad; Records rec; LapWalkScratch walk; size_t bytes;
-    LaplaceBwdWs(void* base, int P, int D, int N, int M, int C) {
+    float *vpad, *gpad, *gvpad; Records rec; LapWalkScratch walk; Piece piece; size_t bytes;
+    LaplaceBwdWs(void* base, int P, int D, int N, int M, int C, const Piece& piece_) : piece(piece_) {
         Bump b(base);
-        const int C4 = round4(C), nseg = P * D;
+        const int C4 = round4(C), nseg = piece.heads * piece.features;
         vpad  = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         gpad  = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         gvpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         rec.carve_events(b, nseg, N, M);
-        walk.carve(b, P, D, N, M, C4, true);     // one scratch for both walks (stream of keys k, then stream of keys q)
+        walk.carve(b, PieceSizes(P, D, piece), N, M, C4, true);     // one scratch for both walks (stream of keys k, then stream of keys q)
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
 
 // ------------------------------------------------------------------ abs forward
 struct AbsFwdWs {
-    float* vpad; float* opad; Records rec; float *qsum, *ksumd, *vsum, *ktot, *ksr, *agg; size_t bytes;
-    AbsFwdWs(void* base, int P, int D, int N, int M, int C) {
+    float* vpad; float* opad; Records rec; float *qsum, *ksumd, *vsum, *ktot, *ksr, *agg; bool lean; size_t bytes;
+    AbsFwdWs(void* base, int P, int D, int N, int M, int C, bool lean_ = false) : lean(lean_) {
         Bump b(base);
         const int C4 = round4(C), nseg = P * D;
         vpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
@@ -454,7 +496,7 @@ struct AbsFwdWs {
         vsum  = b.take<float>((size_t)P * C4 * 2 + P);     // vsum | ktot | ksr, zeroed together
         ktot  = vsum ? vsum + (size_t)P * C4 : nullptr;
         ksr   = vsum ? ktot + (size_t)P * C4 : nullptr;
-        agg   = b.take<float>(prefix_agg_floats(P, D, N, C4, false));
+        agg   = b.take<float>(prefix_agg_floats(P, D, N, C4, false, lean));
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
@@ -463,18 +505,20 @@ struct AbsFwdWs {
 struct AbsBwdWs {
     float *vpad, *gpad, *gvpad; Records rec;
     float *qsumd, *sums /* vsum | gwsum | qtotg | gu_total */, *agg;
-    size_t bytes;
-    AbsBwdWs(void* base, int P, int D, int N, int M, int C) {
+    Piece piece; size_t bytes;
+    AbsBwdWs(void* base, int P, int D, int N, int M, int C, const Piece& piece_) : piece(piece_) {
         Bump b(base);
-        const int C4 = round4(C), nseg = P * D;
+        const int C4 = round4(C), nseg = piece.heads * piece.features;
         vpad  = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         gpad  = C4 != C ? b.take<float>((size_t)P * M * C4) : nullptr;
         gvpad = C4 != C ? b.take<float>((size_t)P * N * C4) : nullptr;
         rec.carve_events(b, nseg, N, M);
         qsumd = b.take<float>((size_t)P * M);
         sums  = b.take<float>((size_t)P * C4 * 3 + P);
-        const size_t agg_k = prefix_agg_floats(P, D, N, C4, true), agg_q = prefix_agg_floats(P, D, M, C4, true);
-        agg   = b.take<float>(agg_k > agg_q ? agg_k : agg_q);
+        size_t a = 0;
+        for (const Piece& size : PieceSizes(P, D, piece))
+            for (const int keys : {N, M}) a = std::max(a, prefix_agg_floats(size.heads, size.features, keys, C4, true));
+        agg   = b.take<float>(a);
         bytes = (b.off + 255) & ~size_t(255);
     }
 };
@@ -591,7 +635,7 @@ int qlka_laplace_backward_workspace_bytes(int P, int D, int N, int M, int C, siz
     if (!bytes) return QLKA_ERR_NULL;
     int st = check_dims(P, D, N, M, C);
     if (st) return st;
-    *bytes = std::max(LaplaceBwdWs(nullptr, P, D, N, M, C).bytes, dense_gradient_bytes(DENSE_LAPLACE, P, D, N, M, C, false));
+    *bytes = std::max(in_pieces<LaplaceBwdWs>(nullptr, ANY_SIZE, P, D, N, M, C).bytes, dense_gradient_bytes(DENSE_LAPLACE, P, D, N, M, C, false));
     return QLKA_OK;
 }
 
@@ -611,7 +655,7 @@ int qlka_weighted_laplace_sum_backward(const float* q, const float* k, const flo
                                  reinterpret_cast<cudaStream_t>(stream_)));
         return QLKA_OK;
     }
-    LaplaceBwdWs ws(workspace, P, D, N, M, C);
+    const LaplaceBwdWs ws = in_pieces<LaplaceBwdWs>(workspace, workspace_bytes, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int C4 = round4(C), nseg = P * D;
@@ -630,19 +674,25 @@ int qlka_weighted_laplace_sum_backward(const float* q, const float* k, const flo
         CU(cudaMemsetAsync(grad_q, 0, sizeof(float) * (size_t)nseg * M, stream));
         CU(cudaMemsetAsync(grad_k, 0, sizeof(float) * (size_t)nseg * N, stream));
     }
-    {   // grad_q[d, m] = <g_w[m], e1 R_r - e0 L_{r-1}> + g_u[m] (e1 Ru_r - e0 Lu_{r-1}): queries q walk the key stream k
-        SortArgs s = sort_args(ws.rec, k, q, nseg, D, N, M, MODE_LAPLACE, full ? SCAL_SIGNED : SCAL_NONE);
-        s.uq = g_u; s.out_s = grad_q;
-        CU(launch_sort_rank(s, ws.rec, stream));
-        CU(laplace_walk_chunked(ws.rec, ws.walk, vrows, nullptr, grows, grad_q, EMIT_DOT, P, D, N, M, C4, stream, nullptr));
-    }
-    {   // roles swapped: queries k walk the stream q whose rows are g_w (and whose per-key scalar is g_u);
-        // the row emission is grad_v, the dot with the v rows is grad_k
-        SortArgs s = sort_args(ws.rec, q, k, nseg, D, M, N, MODE_LAPLACE, full ? SCAL_SIGNED : SCAL_NONE);
-        s.us = g_u; s.out_s = grad_k;
-        CU(launch_sort_rank(s, ws.rec, stream));
-        CU(laplace_walk_chunked(ws.rec, ws.walk, grows, gv, vrows, grad_k, EMIT_BOTH, P, D, M, N, C4, stream, nullptr));
-    }
+    st = for_pieces(P, D, ws.piece, [&](const int p0, const int pc, const int d0, const int dc) -> int {
+        const size_t s0 = (size_t)p0 * D + d0;
+        const float *qp = q + s0 * M, *kp = k + s0 * N, *vp = vrows + (size_t)p0 * N * C4, *gp = grows + (size_t)p0 * M * C4, *up = full ? g_u + (size_t)p0 * M : nullptr;
+        {   // grad_q[d, m] = <g_w[m], e1 R_r - e0 L_{r-1}> + g_u[m] (e1 Ru_r - e0 Lu_{r-1}): queries q walk the key stream k
+            SortArgs s = sort_args(ws.rec, kp, qp, pc * dc, dc, N, M, MODE_LAPLACE, full ? SCAL_SIGNED : SCAL_NONE);
+            s.uq = up; s.out_s = grad_q + s0 * M;
+            CU(launch_sort_rank(s, ws.rec, stream));
+            CU(laplace_walk_chunked(ws.rec, ws.walk, vp, nullptr, gp, grad_q + s0 * M, EMIT_DOT, pc, dc, N, M, C4, stream, nullptr));
+        }
+        {   // roles swapped: queries k walk the stream q whose rows are g_w (and whose per-key scalar is g_u);
+            // the row emission is grad_v, the dot with the v rows is grad_k
+            SortArgs s = sort_args(ws.rec, qp, kp, pc * dc, dc, M, N, MODE_LAPLACE, full ? SCAL_SIGNED : SCAL_NONE);
+            s.us = up; s.out_s = grad_k + s0 * N;
+            CU(launch_sort_rank(s, ws.rec, stream));
+            CU(laplace_walk_chunked(ws.rec, ws.walk, gp, gv + (size_t)p0 * N * C4, vp, grad_k + s0 * N, EMIT_BOTH, pc, dc, M, N, C4, stream, nullptr));
+        }
+        return QLKA_OK;
+    });
+    if (st) return st;
     if (C4 != C) CU(launch_unpad_rows(gv, grad_v, (long long)P * N, C, C4, stream));
     return QLKA_OK;
 }
@@ -650,7 +700,7 @@ int qlka_weighted_laplace_sum_backward(const float* q, const float* k, const flo
 // ---------------------------------------------------------------- add_laplace attention on (B, H, S, D)
 namespace {
 struct LaplaceAttnWs {
-    float *qt, *kt, *vm, *out_u, *n_pad; void* inner; size_t inner_bytes, bytes;
+    float *qt, *kt, *vm, *out_u, *n_pad; void* inner; size_t fixed, bytes, least;      // inner: what lies beyond `fixed`
     LaplaceAttnWs(void* base, int B, int H, int S, int D, int C, bool masked) {
         Bump b(base);
         const size_t P = (size_t)B * H;
@@ -659,9 +709,10 @@ struct LaplaceAttnWs {
         vm    = masked ? b.take<float>(P * S * C) : nullptr;
         out_u = b.take<float>(P * S);
         n_pad = masked ? b.take<float>((size_t)B) : nullptr;
-        inner_bytes = LaplaceWs(nullptr, (int)P, D, S, S, C).bytes;
-        inner = b.take<unsigned char>(inner_bytes);
-        bytes = (b.off + 255) & ~size_t(255);
+        inner = b.take<unsigned char>(0);
+        fixed = b.off;
+        bytes = fixed + LaplaceWs(nullptr, (int)P, D, S, S, C).bytes;
+        least = fixed + LaplaceWs(nullptr, (int)P, D, S, S, C, true).bytes;
     }
 };
 }  // namespace
@@ -697,7 +748,7 @@ static int laplace_attention_impl(const float* q, const float* k, const float* v
     }
     const bool masked = keep != nullptr;
     LaplaceAttnWs ws(workspace, B, H, S, D, Dv, masked);
-    if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
+    if (!ws_ok(workspace, workspace_bytes, ws.least)) return QLKA_ERR_WORKSPACE;
     const int P = B * H;
 
     CU(launch_transpose_scale(q, ws.qt, nullptr, 1.0f / tau, P, S, D, H, stream));
@@ -708,7 +759,7 @@ static int laplace_attention_impl(const float* q, const float* k, const float* v
         CU(launch_npad(keep, ws.n_pad, B, S, stream));
         rows = ws.vm;
     }
-    st = laplace_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, stream, nullptr);
+    st = laplace_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, workspace_bytes - ws.fixed, P, D, S, S, Dv, stream, nullptr);
     if (st) return st;
     CU(launch_normalise(out, ws.out_u, ws.qt, ws.n_pad, P, S, D, Dv, H, 1e-6f, false, den, stream));
     return QLKA_OK;
@@ -729,7 +780,7 @@ namespace {
 constexpr float BUMP_SHIFTS[3]  = {0.0f, 1.0f, -1.0f};     // max(0, 1 - |x|) = |x + 1| / 2 + |x - 1| / 2 - |x|
 constexpr float BUMP_WEIGHTS[3] = {-1.0f, 0.5f, 0.5f};
 struct AbsAttnWs {
-    float *qt, *kt, *vm, *out_u, *n_pad, *aq, *ak, *sums /* vsum | akv | aksum */; void* inner; size_t inner_bytes, bytes;
+    float *qt, *kt, *vm, *out_u, *n_pad, *aq, *ak, *sums /* vsum | akv | aksum */; void* inner; size_t fixed, bytes, least;
     AbsAttnWs(void* base, int B, int H, int S, int D, int C, bool masked, bool bump) {
         Bump b(base);
         const size_t P = (size_t)B * H;
@@ -741,9 +792,10 @@ struct AbsAttnWs {
         aq    = bump ? nullptr : b.take<float>(P * S);
         ak    = bump ? nullptr : b.take<float>(P * S);
         sums  = bump ? nullptr : b.take<float>(P * C * 2 + P);
-        inner_bytes = AbsFwdWs(nullptr, (int)P, D, S, bump ? 3 * S : S, C).bytes;
-        inner = b.take<unsigned char>(inner_bytes);
-        bytes = (b.off + 255) & ~size_t(255);
+        inner = b.take<unsigned char>(0);
+        fixed = b.off;
+        bytes = fixed + AbsFwdWs(nullptr, (int)P, D, S, bump ? 3 * S : S, C).bytes;
+        least = fixed + AbsFwdWs(nullptr, (int)P, D, S, bump ? 3 * S : S, C, true).bytes;
     }
 };
 }  // namespace
@@ -780,7 +832,7 @@ static int abs_attention_impl(int kind, const float* q, const float* k, const fl
         return QLKA_OK;
     }
     AbsAttnWs ws(workspace, B, H, S, D, Dv, masked, bump);
-    if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
+    if (!ws_ok(workspace, workspace_bytes, ws.least)) return QLKA_ERR_WORKSPACE;
     const int P = B * H;
 
     CU(launch_transpose_scale(q, ws.qt, nullptr, 1.0f / tau, P, S, D, H, stream));
@@ -793,7 +845,7 @@ static int abs_attention_impl(int kind, const float* q, const float* k, const fl
     }
     if (bump) {
         // numerator and row sum of the three shifted abs sums from one sort, then the row normalisation
-        st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, 3, BUMP_SHIFTS, BUMP_WEIGHTS, stream);
+        st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, workspace_bytes - ws.fixed, P, D, S, S, Dv, 3, BUMP_SHIFTS, BUMP_WEIGHTS, stream);
         if (st) return st;
         CU(launch_normalise(out, ws.out_u, ws.qt, ws.n_pad, P, S, D, Dv, H, 1e-6f, true, den, stream));
     } else {
@@ -805,7 +857,7 @@ static int abs_attention_impl(int kind, const float* q, const float* k, const fl
         CU(launch_abscolsum_d(ws.kt, ws.ak, P, D, S, stream));
         CU(cudaMemsetAsync(ws.sums, 0, sizeof(float) * ((size_t)P * Dv * 2 + P), stream));
         CU(launch_rowstat(rows, ws.ak, vsum, akv, aksum, P, S, Dv, stream));
-        st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, ws.inner_bytes, P, D, S, S, Dv, 0, nullptr, nullptr, stream, true);
+        st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, workspace_bytes - ws.fixed, P, D, S, S, Dv, 0, nullptr, nullptr, stream, true);
         if (st) return st;
         CU(launch_riesz_epilogue(out, ws.out_u, ws.aq, vsum, akv, aksum, ws.n_pad, P, S, Dv, Dv, H, 1e-3f, 1e-6f, den, stream));
     }
@@ -825,7 +877,7 @@ constexpr int ATTN_LAPLACE = 2;
 int dense_kind_of(int kind) { return kind == ATTN_LAPLACE ? DENSE_LAPLACE : kind == 1 ? DENSE_BUMP : DENSE_RIESZ; }
 
 struct LaplaceAttnBwdWs {
-    float *qt, *kt, *vm, *dn, *dd, *gqt, *gkt, *n_pad; void* inner; size_t inner_bytes, bytes;
+    float *qt, *kt, *vm, *dn, *dd, *gqt, *gkt, *n_pad; void* inner; size_t fixed, bytes, least;
     LaplaceAttnBwdWs(void* base, int B, int H, int S, int D, int C, bool masked) {
         Bump b(base);
         const size_t P = (size_t)B * H;
@@ -837,9 +889,10 @@ struct LaplaceAttnBwdWs {
         dn    = b.take<float>(P * S * C);
         dd    = b.take<float>(P * S);
         n_pad = masked ? b.take<float>((size_t)B) : nullptr;
-        inner_bytes = LaplaceBwdWs(nullptr, (int)P, D, S, S, C).bytes;
-        inner = b.take<unsigned char>(inner_bytes);
-        bytes = (b.off + 255) & ~size_t(255);
+        inner = b.take<unsigned char>(0);
+        fixed = b.off;
+        bytes = fixed + in_pieces<LaplaceBwdWs>(nullptr, ANY_SIZE, (int)P, D, S, S, C).bytes;
+        least = fixed + in_pieces<LaplaceBwdWs>(nullptr, 0, (int)P, D, S, S, C).bytes;
     }
 };
 }  // namespace
@@ -881,16 +934,17 @@ int qlka_attention_backward(int kind, const float* q, const float* k, const floa
     if (!q || !k || !v || !out || !den || !grad_out || !grad_q || !grad_k || !grad_v) return QLKA_ERR_NULL;
     if (!aligned16(v, out, grad_out, grad_v)) return QLKA_ERR_ALIGNMENT;
     if (!(tau > 0.0f)) return QLKA_ERR_BAD_SHAPE;
-    if (!ws_ok(workspace, workspace_bytes, need)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int P = B * H, dk = dense_kind_of(kind);
     if (dense_gradient_pays(dk, P, D, S, S, Dv, masked)) {
+        if (!ws_ok(workspace, workspace_bytes, need)) return QLKA_ERR_WORKSPACE;
         DenseGradArgs g = dense_grad_args(q, k, v, grad_out, nullptr, grad_q, grad_k, grad_v, workspace, P, D, S, S, Dv);
         g.attention = true; g.H = H; g.scale = 1.0f / tau; g.eps = 1e-3f; g.clamp = 1e-6f; g.keep = keep; g.out = out; g.den = den;
         CU(launch_dense_gradient(g, dk, sm_count(), stream));
         return QLKA_OK;
     }
     LaplaceAttnBwdWs ws(workspace, B, H, S, D, Dv, masked);
+    if (!ws_ok(workspace, workspace_bytes, ws.least)) return QLKA_ERR_WORKSPACE;
     CU(launch_transpose_scale(q, ws.qt, nullptr, 1.0f / tau, P, S, D, H, stream));
     CU(launch_transpose_scale(k, ws.kt, keep, 1.0f / tau, P, S, D, H, stream));
     const float* rows = v;
@@ -900,7 +954,7 @@ int qlka_attention_backward(int kind, const float* q, const float* k, const floa
         rows = ws.vm;
     }
     CU(launch_attention_gradient_rows(grad_out, out, den, ws.dn, ws.dd, (long long)P * S, Dv, 1e-6f, stream));
-    st = qlka_weighted_laplace_sum_backward(ws.qt, ws.kt, rows, ws.dn, ws.dd, ws.gqt, ws.gkt, grad_v, ws.inner, ws.inner_bytes, P, D, S, S, Dv, stream_);
+    st = qlka_weighted_laplace_sum_backward(ws.qt, ws.kt, rows, ws.dn, ws.dd, ws.gqt, ws.gkt, grad_v, ws.inner, workspace_bytes - ws.fixed, P, D, S, S, Dv, stream_);
     if (st) return st;
     CU(launch_transpose_back(ws.gqt, grad_q, nullptr, 1.0f / tau, masked ? ws.qt : nullptr, ws.dd, ws.n_pad, P, S, D, H, stream));
     CU(launch_transpose_back(ws.gkt, grad_k, keep, 1.0f / tau, nullptr, nullptr, nullptr, P, S, D, H, stream));
@@ -973,7 +1027,10 @@ static int abs_forward_impl(const float* q, const float* k, const float* v, floa
     }
     const int MQ = ns ? ns * M : M;                 // queries per segment
     AbsFwdWs ws(workspace, P, D, N, MQ, C);
-    if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
+    if (!ws_ok(workspace, workspace_bytes, ws.bytes)) {
+        ws = AbsFwdWs(workspace, P, D, N, MQ, C, true);
+        if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
+    }
     const int C4 = round4(C), nseg = P * D;
     const bool full = out_u != nullptr;
     float A = 1.0f, Bq = 0.0f;
@@ -999,7 +1056,7 @@ static int abs_forward_impl(const float* q, const float* k, const float* v, floa
 
     WalkArgs w = walk_args(ws.rec, rows, nseg, D, N, MQ, C4);
     w.out = out; w.Mrows = M; w.agg = ws.agg;
-    CU(prefix_walk_chunked(w, EMIT_ROWS, P, stream));
+    CU(prefix_walk_chunked(w, EMIT_ROWS, P, stream, ws.lean));
 
     if (C4 != C) CU(launch_unpad_rows(out, out_w, (long long)P * M, C, C4, stream));
     return QLKA_OK;
@@ -1049,7 +1106,7 @@ int qlka_abs_backward_workspace_bytes(int P, int D, int N, int M, int C, size_t*
     if (!bytes) return QLKA_ERR_NULL;
     int st = check_dims(P, D, N, M, C);
     if (st) return st;
-    *bytes = std::max(AbsBwdWs(nullptr, P, D, N, M, C).bytes, dense_gradient_bytes(DENSE_ABS, P, D, N, M, C, false));
+    *bytes = std::max(in_pieces<AbsBwdWs>(nullptr, ANY_SIZE, P, D, N, M, C).bytes, dense_gradient_bytes(DENSE_ABS, P, D, N, M, C, false));
     return QLKA_OK;
 }
 
@@ -1069,7 +1126,7 @@ int qlka_weighted_abs_sum_backward(const float* q, const float* k, const float* 
                                  reinterpret_cast<cudaStream_t>(stream_)));
         return QLKA_OK;
     }
-    AbsBwdWs ws(workspace, P, D, N, M, C);
+    const AbsBwdWs ws = in_pieces<AbsBwdWs>(workspace, workspace_bytes, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int C4 = round4(C), nseg = P * D;
@@ -1093,25 +1150,31 @@ int qlka_weighted_abs_sum_backward(const float* q, const float* k, const float* 
     CU(launch_rowstat(grows, ws.qsumd, gwsum, qtotg, nullptr, P, M, C4, stream));
     if (full) CU(launch_vecsum(g_u, gu_total, P, M, stream));
 
-    {   // grad_q: queries q walk the key stream k; prefix of v rows contracted with g_w rows
-        SortArgs s = sort_args(ws.rec, k, q, nseg, D, N, M, MODE_SGN, full ? SCAL_RANK : SCAL_NONE);
-        s.uq = g_u;
-        CU(launch_sort_rank(s, ws.rec, stream));
-        WalkArgs w = walk_args(ws.rec, vrows, nseg, D, N, M, C4);
-        w.g = grows; w.wtotal = vsum; w.out_s = grad_q; w.agg = ws.agg;
-        CU(prefix_walk_chunked(w, EMIT_DOT, P, stream));
-    }
-    {   // roles swapped: queries k walk the stream q whose rows are g_w
-        SortArgs s = sort_args(ws.rec, q, k, nseg, D, M, N, MODE_ABS, full ? SCAL_PREFIX : SCAL_NONE);
-        s.us = g_u; s.us_total = gu_total;
-        CU(launch_sort_rank(s, ws.rec, stream));
-        // one walk for both: grad_v = abs sum with keys q, weights g_w, evaluated at the keys k (row reductions on
-        // top of a constant row per head); grad_k = prefix of g_w rows contracted with v rows (+ the g_u term in e1)
-        CU(launch_abs_init(qtotg, gwsum, nullptr, nullptr, gv, nullptr, P, N, C4, M, 1.0f, 0.0f, stream));
-        WalkArgs w = walk_args(ws.rec, grows, nseg, D, M, N, C4);
-        w.g = vrows; w.wtotal = gwsum; w.out_s = grad_k; w.out = gv; w.agg = ws.agg;
-        CU(prefix_walk_chunked(w, EMIT_BOTH, P, stream));
-    }
+    // grad_v starts from a constant row per head
+    CU(launch_abs_init(qtotg, gwsum, nullptr, nullptr, gv, nullptr, P, N, C4, M, 1.0f, 0.0f, stream));
+    st = for_pieces(P, D, ws.piece, [&](const int p0, const int pc, const int d0, const int dc) -> int {
+        const size_t s0 = (size_t)p0 * D + d0;
+        const float *qp = q + s0 * M, *kp = k + s0 * N, *vp = vrows + (size_t)p0 * N * C4, *gp = grows + (size_t)p0 * M * C4, *up = full ? g_u + (size_t)p0 * M : nullptr;
+        {   // grad_q: queries q walk the key stream k; prefix of v rows contracted with g_w rows
+            SortArgs s = sort_args(ws.rec, kp, qp, pc * dc, dc, N, M, MODE_SGN, full ? SCAL_RANK : SCAL_NONE);
+            s.uq = up;
+            CU(launch_sort_rank(s, ws.rec, stream));
+            WalkArgs w = walk_args(ws.rec, vp, pc * dc, dc, N, M, C4);
+            w.g = gp; w.wtotal = vsum + (size_t)p0 * C4; w.out_s = grad_q + s0 * M; w.agg = ws.agg;
+            CU(prefix_walk_chunked(w, EMIT_DOT, pc, stream));
+        }
+        {   // roles swapped: queries k walk the stream q whose rows are g_w. One walk for both: grad_v = abs sum with keys q, weights
+            // g_w, evaluated at the keys k (row reductions); grad_k = prefix of g_w rows contracted with v rows (+ the g_u term in e1)
+            SortArgs s = sort_args(ws.rec, qp, kp, pc * dc, dc, M, N, MODE_ABS, full ? SCAL_PREFIX : SCAL_NONE);
+            s.us = up; s.us_total = gu_total + p0;
+            CU(launch_sort_rank(s, ws.rec, stream));
+            WalkArgs w = walk_args(ws.rec, gp, pc * dc, dc, M, N, C4);
+            w.g = vp; w.wtotal = gwsum + (size_t)p0 * C4; w.out_s = grad_k + s0 * N; w.out = gv + (size_t)p0 * N * C4; w.agg = ws.agg;
+            CU(prefix_walk_chunked(w, EMIT_BOTH, pc, stream));
+        }
+        return QLKA_OK;
+    });
+    if (st) return st;
     if (C4 != C) CU(launch_unpad_rows(gv, grad_v, (long long)P * N, C, C4, stream));
     return QLKA_OK;
 }
@@ -1129,7 +1192,7 @@ int qlka_weighted_sgn_sum_forward(const float* q, const float* k, const float* v
     if (st) return st;
     if (!q || !k || !v || !g || !out) return QLKA_ERR_NULL;
     if (!aligned16(v, g)) return QLKA_ERR_ALIGNMENT;
-    AbsBwdWs ws(workspace, P, D, N, M, C);
+    const AbsBwdWs ws = in_pieces<AbsBwdWs>(workspace, workspace_bytes, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     const int C4 = round4(C), nseg = P * D;
@@ -1145,12 +1208,15 @@ int qlka_weighted_sgn_sum_forward(const float* q, const float* k, const float* v
     CU(cudaMemsetAsync(vsum, 0, sizeof(float) * (size_t)P * C4, stream));
     CU(launch_rowstat(vrows, nullptr, vsum, nullptr, nullptr, P, N, C4, stream));
 
-    SortArgs s = sort_args(ws.rec, k, q, nseg, D, N, M, MODE_SGN, SCAL_NONE);
-    CU(launch_sort_rank(s, ws.rec, stream));
-    WalkArgs w = walk_args(ws.rec, vrows, nseg, D, N, M, C4);
-    w.g = grows; w.wtotal = vsum; w.out_s = out; w.sign = -1.0f; w.agg = ws.agg;
-    CU(prefix_walk_chunked(w, EMIT_DOT, P, stream));
-    return QLKA_OK;
+    return for_pieces(P, D, ws.piece, [&](const int p0, const int pc, const int d0, const int dc) -> int {
+        const size_t s0 = (size_t)p0 * D + d0;
+        SortArgs s = sort_args(ws.rec, k + s0 * N, q + s0 * M, pc * dc, dc, N, M, MODE_SGN, SCAL_NONE);
+        CU(launch_sort_rank(s, ws.rec, stream));
+        WalkArgs w = walk_args(ws.rec, vrows + (size_t)p0 * N * C4, pc * dc, dc, N, M, C4);
+        w.g = grows + (size_t)p0 * M * C4; w.wtotal = vsum + (size_t)p0 * C4; w.out_s = out + s0 * M; w.sign = -1.0f; w.agg = ws.agg;
+        CU(prefix_walk_chunked(w, EMIT_DOT, pc, stream));
+        return QLKA_OK;
+    });
 }
 
 // ---------------------------------------------------------------- linear layers of the encoder

@@ -123,19 +123,27 @@ Tensor floats(const at::IntArrayRef shape, const Tensor& like) {
     return at::detail::empty_cuda(shape, at::kFloat, like.device(), std::nullopt);
 }
 
-struct Workspace {
-    Tensor t;
+// call(workspace, bytes) with a workspace of the size that `size` gives for these dimensions. Where the device has not that much left, the call is
+// offered less and less: most take some, and go over their heads in pieces. What none takes is the allocator's error.
+template <class Size, class... Args, class Call>
+void with_workspace(const Tensor& like, Call call, Size size, Args... dims) {
     size_t bytes = 0;
-    void*  ptr() const { return t.mutable_data_ptr(); }
-    void   take(const Tensor& like) { t = at::detail::empty_cuda({(int64_t)std::max<size_t>(bytes, 256)}, at::kByte, like.device(), std::nullopt); }
-};
-
-template <class Size, class... Args>
-Workspace workspace(const Tensor& like, Size size, Args... dims) {
-    Workspace w;
-    check_status(size(dims..., &w.bytes));
-    w.take(like);
-    return w;
+    check_status(size(dims..., &bytes));
+    std::exception_ptr refused;
+    for (const int sixteenths : {16, 15, 14, 12, 8, 4, 2, 1}) {
+        const size_t have = bytes / 16 * sixteenths + (sixteenths == 16 ? bytes % 16 : 0);
+        Tensor ws;
+        try {
+            ws = at::detail::empty_cuda({(int64_t)std::max<size_t>(have, 256)}, at::kByte, like.device(), std::nullopt);
+        } catch (const c10::OutOfMemoryError&) {
+            if (!refused) refused = std::current_exception();
+            continue;
+        }
+        const int st = call(ws.mutable_data_ptr(), have);
+        if (refused && st == QLKA_ERR_WORKSPACE) break;
+        return check_status(st);
+    }
+    std::rethrow_exception(refused);
 }
 
 // ------------------------------------------------------------------ operators
@@ -143,10 +151,10 @@ std::tuple<Tensor, Tensor> laplace_forward(const Tensor& q, const Tensor& k, con
     const Dims d = check_qkv(q, k, v_, "q, k and v");
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor v = aligned(v_);
-    const Workspace ws = workspace(q, api.qlka_laplace_forward_workspace_bytes, d.P, d.D, d.N, d.M, d.C);
     Tensor out_w = floats({d.P, d.M, d.C}, q), out_u = floats({d.P, d.M}, q);
-    check_status(api.qlka_weighted_laplace_sum_forward(ptr(q), ptr(k), ptr(v), out_ptr(out_w), out_ptr(out_u), ws.ptr(), ws.bytes,
-                                                       d.P, d.D, d.N, d.M, d.C, current_stream()));
+    with_workspace(q, [&](void* ws, size_t bytes) {
+        return api.qlka_weighted_laplace_sum_forward(ptr(q), ptr(k), ptr(v), out_ptr(out_w), out_ptr(out_u), ws, bytes, d.P, d.D, d.N, d.M, d.C, current_stream());
+    }, api.qlka_laplace_forward_workspace_bytes, d.P, d.D, d.N, d.M, d.C);
     return {out_w, out_u};
 }
 
@@ -157,10 +165,10 @@ std::tuple<Tensor, Tensor, Tensor> backward(Size size, Call call, const Tensor& 
     if (g_u.defined()) check_like(g_u, "g_u", {d.P, d.M}, q);
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor v = aligned(v_), g_w = aligned(g_w_);
-    const Workspace ws = workspace(q, size, d.P, d.D, d.N, d.M, d.C);
     Tensor gq = floats({d.P, d.D, d.M}, q), gk = floats({d.P, d.D, d.N}, q), gv = floats({d.P, d.N, d.C}, q);
-    check_status(call(ptr(q), ptr(k), ptr(v), ptr(g_w), ptr(g_u), out_ptr(gq), out_ptr(gk), out_ptr(gv), ws.ptr(), ws.bytes,
-                      d.P, d.D, d.N, d.M, d.C, current_stream()));
+    with_workspace(q, [&](void* ws, size_t bytes) {
+        return call(ptr(q), ptr(k), ptr(v), ptr(g_w), ptr(g_u), out_ptr(gq), out_ptr(gk), out_ptr(gv), ws, bytes, d.P, d.D, d.N, d.M, d.C, current_stream());
+    }, size, d.P, d.D, d.N, d.M, d.C);
     return {gq, gk, gv};
 }
 
@@ -176,11 +184,11 @@ std::tuple<Tensor, std::optional<Tensor>> abs_forward(const Tensor& q, const Ten
     const Dims d = check_qkv(q, k, v_, "q, k, and v");
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor v = aligned(v_);
-    const Workspace ws = workspace(q, api.qlka_abs_forward_workspace_bytes, d.P, d.D, d.N, d.M, d.C);
     Tensor out_w = floats({d.P, d.M, d.C}, q), out_u;
     if (full) out_u = floats({d.P, d.M}, q);
-    check_status(api.qlka_weighted_abs_sum_forward(ptr(q), ptr(k), ptr(v), out_ptr(out_w), out_ptr(out_u), ws.ptr(), ws.bytes,
-                                                   d.P, d.D, d.N, d.M, d.C, (int)path, current_stream()));
+    with_workspace(q, [&](void* ws, size_t bytes) {
+        return api.qlka_weighted_abs_sum_forward(ptr(q), ptr(k), ptr(v), out_ptr(out_w), out_ptr(out_u), ws, bytes, d.P, d.D, d.N, d.M, d.C, (int)path, current_stream());
+    }, api.qlka_abs_forward_workspace_bytes, d.P, d.D, d.N, d.M, d.C);
     return {out_w, full ? std::optional<Tensor>(out_u) : std::nullopt};
 }
 
@@ -189,10 +197,10 @@ Tensor sgn_forward(const Tensor& q, const Tensor& k, const Tensor& v_, const Ten
     check_like(g_, "g", {d.P, d.M, d.C}, q);
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor v = aligned(v_), g = aligned(g_);
-    const Workspace ws = workspace(q, api.qlka_sgn_forward_workspace_bytes, d.P, d.D, d.N, d.M, d.C);
     Tensor out = floats({d.P, d.D, d.M}, q);
-    check_status(api.qlka_weighted_sgn_sum_forward(ptr(q), ptr(k), ptr(v), ptr(g), out_ptr(out), ws.ptr(), ws.bytes,
-                                                   d.P, d.D, d.N, d.M, d.C, current_stream()));
+    with_workspace(q, [&](void* ws, size_t bytes) {
+        return api.qlka_weighted_sgn_sum_forward(ptr(q), ptr(k), ptr(v), ptr(g), out_ptr(out), ws, bytes, d.P, d.D, d.N, d.M, d.C, current_stream());
+    }, api.qlka_sgn_forward_workspace_bytes, d.P, d.D, d.N, d.M, d.C);
     return out;
 }
 
@@ -276,11 +284,12 @@ Tensor keep_floats(const std::optional<Tensor>& keep, const Tensor& q) {
 }
 
 Tensor attention_forward(const int64_t kind, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& keep, const double tau, const AttnDims& d, Tensor* den) {
-    const Workspace ws = workspace(q, api.qlka_attention_workspace_bytes, (int)kind, d.B, d.H, d.S, d.D, d.C, (int)keep.defined());
     Tensor out = floats({d.B, d.H, d.S, d.C}, q);
     if (den) *den = floats({d.B, d.H, d.S}, q);
-    check_status(api.qlka_attention_forward((int)kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, out_ptr(out), den ? out_ptr(*den) : nullptr,
-                                            ws.ptr(), ws.bytes, d.B, d.H, d.S, d.D, d.C, current_stream()));
+    with_workspace(q, [&](void* ws, size_t bytes) {
+        return api.qlka_attention_forward((int)kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, out_ptr(out), den ? out_ptr(*den) : nullptr,
+                                          ws, bytes, d.B, d.H, d.S, d.D, d.C, current_stream());
+    }, api.qlka_attention_workspace_bytes, (int)kind, d.B, d.H, d.S, d.D, d.C, (int)keep.defined());
     return out;
 }
 
@@ -322,10 +331,11 @@ public:
         const double tau = ctx->saved_data["tau"].toDouble();
         const bool   changed = static_cast<const OutputVersion*>(ctx->saved_data["out"].toCapsule().get())->changed();
         const Tensor out = changed ? attention_forward(kind, q, k, v, keep, tau, d, nullptr) : saved_out;
-        const Workspace ws = workspace(q, api.qlka_attention_backward_workspace_bytes, kind, d.B, d.H, d.S, d.D, d.C, (int)keep.defined());
         Tensor gq = floats(q.sizes(), q), gk = floats(k.sizes(), q), gv = floats(v.sizes(), q);
-        check_status(api.qlka_attention_backward(kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, ptr(out), ptr(den), ptr(grad),
-                                                 out_ptr(gq), out_ptr(gk), out_ptr(gv), ws.ptr(), ws.bytes, d.B, d.H, d.S, d.D, d.C, current_stream()));
+        with_workspace(q, [&](void* ws, size_t bytes) {
+            return api.qlka_attention_backward(kind, ptr(q), ptr(k), ptr(v), ptr(keep), (float)tau, ptr(out), ptr(den), ptr(grad),
+                                               out_ptr(gq), out_ptr(gk), out_ptr(gv), ws, bytes, d.B, d.H, d.S, d.D, d.C, current_stream());
+        }, api.qlka_attention_backward_workspace_bytes, kind, d.B, d.H, d.S, d.D, d.C, (int)keep.defined());
         return {gq, gk, gv, Tensor(), Tensor(), Tensor()};
     }
 };

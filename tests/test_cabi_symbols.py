@@ -93,6 +93,17 @@ def test_gradient_workspaces_hold_the_long_sorts_of_both_orders(lib, N, M):
         assert flat + rounding >= sort + records + D * events // 8 * 8 + aggregates, flat - sort - records
 
 
+def test_gradient_workspaces_are_bounded(lib):
+    """Large batches go over their heads in pieces: the scratch of a gradient stays under 4 GiB, or what a single head takes."""
+    def size(name, *dims):
+        n = ctypes.c_size_t(0)
+        assert getattr(lib, f"qlka_{name}_workspace_bytes")(*dims, ctypes.byref(n)) == 0
+        return n.value
+    for dims in ((48, 64, 16384, 16384, 64), (16, 64, 262144, 262144, 64), (2000, 64, 4096, 4096, 64), (16, 64, 65536, 8192, 128)):
+        for name in ("laplace_backward", "abs_backward", "sgn_forward"):
+            assert size(name, *dims) <= max(4 << 30, size(name, 1, *dims[1:])), (name, dims)
+
+
 def test_ops_fail_loudly_without_cuda_tensors(lib):
     import torch
     from weighted_abs_sum import weighted_abs_sum
