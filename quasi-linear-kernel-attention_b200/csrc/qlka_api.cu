@@ -101,7 +101,9 @@ int sm_count() {
 // How a walk over `nseg` segments of N keys is cut into streams and work items (eight streams). Streams are independent work units (the
 // passes exchange their states through memory), so a segment may be cut into any number of them, as long as a stream keeps at least
 // sixteen key blocks (a stream's start costs a few) - eight while there are fewer items than CTAs fit the GPU, four while there are fewer
-// than a quarter of that (attention training, one head of 376 keys x 96 features 193 -> 168 us, of 2000 x 64 281 -> 245). The streams of a head are
+// than a quarter of that (attention training, one head of 376 keys x 96 features 193 -> 168 us, of 2000 x 64 281 -> 245), with dots than a half: those
+// streams share a warp, so the few of a head or two leave SMs idle (Laplace gradients, heads x features x keys x channels, four instead of eight
+// at a half: 4 x 16 x 3000 x 16 187 -> 161 us, 1 x 64 x 3000 x 33 215 -> 189, 2 x 64 x 1024 x 64 123 -> 107; abs 158 -> 145, 194 -> 175, 122 -> 110). The streams of a head are
 // neighbours, so the more of them, the fewer heads' rows are in use at a time and the better the L2 keeps them; against that, each leaves
 // aggregates to write, fold and read. Items per CTA of 256 threads, ms:        4      8      16     32
 //   Laplace sum, 4 x 12 heads x 16384 keys x 64 channels                       5.23   4.88   4.83   4.89
@@ -123,7 +125,7 @@ WalkPlan plan_walk(int nseg, int N, int C4, bool laplace, bool dots, bool lean =
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
     if (laplace || items(1) < 2LL * cap)
-        while (items(sps) < (long long)per_cta * cap && nbk / (sps * 2) >= (items(sps) < cap / 4 && !lean ? 4 : items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
+        while (items(sps) < (long long)per_cta * cap && nbk / (sps * 2) >= (items(sps) < cap / (dots ? 2 : 4) && !lean ? 4 : items(sps) < cap ? 8 : 16) && sps < 4096) sps *= 2;
     return {sps, (int)items(sps)};
 }
 
