@@ -22,8 +22,9 @@ __global__ void colsum_d_kernel(const float* __restrict__ x, float* __restrict__
 // Per p over rows r of w (P, R, C4) with optional row scalars s (P, R):
 //   wsum[p, c] += sum_r w[r, c],  swsum[p, c] += sum_r s[r] w[r, c],  ssum[p] += sum_r s[r]
 // (outputs must be zeroed; partial sums of a row tile are added atomically). grid (tiles, P).
-// VEC: C4 is a multiple of four; 16 bytes per lane, eight rows of a thread in flight (one float per lane and row at a time: 0.064 -> 0.024 ms
-// for 96 heads x 4096 rows x 64 channels, 101 MB).
+// VEC: C4 is a multiple of four; 16 bytes per lane, eight rows of a thread in flight (one float per lane and row at a time: 0.064 -> 0.022 ms
+// for 96 heads x 4096 rows x 64 channels, 101 MB). A CTA adds each of its sums once: with an atomic per row lane for ssum, and the partial sums added up one after
+// the other, narrow rows took longer than one float per lane (48 heads x 9000 rows, 16 channels 39 us, then 59, now 12; 32 channels 40, 60, 15).
 constexpr int RS_THREADS = 256, RS_ROWS = 256;
 template <bool VEC>
 __global__ void __launch_bounds__(RS_THREADS) rowstat_kernel(
@@ -32,7 +33,7 @@ __global__ void __launch_bounds__(RS_THREADS) rowstat_kernel(
     const int R, const int C4)
 {
     constexpr int U = VEC ? 4 : 1;                                // channels of a lane
-    __shared__ float red_w[U][RS_THREADS], red_k[U][RS_THREADS];
+    __shared__ float red_w[U][RS_THREADS], red_k[U][RS_THREADS], red_s[RS_THREADS];
     const int chunks = (R + RS_ROWS - 1) / RS_ROWS;               // (p rides in blockIdx.x: a grid's y extent stops at 65535)
     const int p  = blockIdx.x / chunks;
     const int r0 = (blockIdx.x % chunks) * RS_ROWS, r1 = min(R, r0 + RS_ROWS);
@@ -55,21 +56,29 @@ __global__ void __launch_bounds__(RS_THREADS) rowstat_kernel(
             as += sc;
         }
     }
+    for (int off = CW; off < 32; off <<= 1) {                     // the rows of a warp
+        #pragma unroll
+        for (int u = 0; u < U; u++) { aw[u] += __shfl_xor_sync(FULL, aw[u], off); ak[u] += __shfl_xor_sync(FULL, ak[u], off); }
+        as += __shfl_xor_sync(FULL, as, off);
+    }
     #pragma unroll
     for (int u = 0; u < U; u++) { red_w[u][threadIdx.x] = aw[u]; red_k[u][threadIdx.x] = ak[u]; }
+    red_s[threadIdx.x] = as;
     __syncthreads();
     if (lane_r == 0 && c < C4) {
-        for (int j = 1; j < nr; j++) {
+        const int apart = max(CW, 32);                            // threads from one partial sum to the next
+        for (int j = apart + threadIdx.x; j < RS_THREADS; j += apart) {
             #pragma unroll
-            for (int u = 0; u < U; u++) { aw[u] += red_w[u][j * CW + threadIdx.x]; ak[u] += red_k[u][j * CW + threadIdx.x]; }
+            for (int u = 0; u < U; u++) { aw[u] += red_w[u][j]; ak[u] += red_k[u][j]; }
+            as += red_s[j];
         }
         #pragma unroll
         for (int u = 0; u < U; u++) {
             atomicAdd(wsum + (long long)p * C4 + c + u, aw[u]);
             if (swsum) atomicAdd(swsum + (long long)p * C4 + c + u, ak[u]);
         }
+        if (ssum && c == 0) atomicAdd(ssum + p, as);
     }
-    if (ssum && c == 0) atomicAdd(ssum + p, as);
 }
 
 // out[p] = sum_l x[p, l]; one CTA per p
