@@ -111,7 +111,9 @@ int sm_count() {
 //   abs sum, 16 x 262144 x 64                                                  38.2   36.4   35.4   35.9
 //   Laplace gradients, 48 x 4096 x 64 / 16 x 8192 x 128                        3.49   3.46   3.55   3.55 / 3.82   3.78   3.95   3.95
 //   Laplace sum, 16 x 8191 keys x 1030 queries x 128                           0.93   0.93   0.97   0.97
-// hence sixteen for row walks of up to 64 channels, else eight. The prefix walks need no first pass with one stream per segment, which
+//   abs sum / Laplace sum, 48 x 4096 x 32                                             0.95 / 1.02   0.98 / 1.04
+//   abs sum / Laplace sum, 16 x 16384 x 32                                            1.32 / 1.34   1.34 / 1.40
+// hence sixteen for row walks of 33 to 64 channels, else eight. The prefix walks need no first pass with one stream per segment, which
 // pays as soon as whole segments alone give every CTA a few items.
 struct WalkPlan { int sps, nitems; };
 
@@ -120,7 +122,7 @@ WalkPlan plan_walk(int nseg, int N, int C4, bool laplace, bool dots, bool lean =
     constexpr int streams = 8;
     // resident CTAs, about (above 64 channels two per SM; planned for four, Laplace at 16 heads x 8191 keys x 1030 queries took 1.08
     // instead of 1.03 ms, its backward at 16 x 8192 4.71 instead of 4.45 ms)
-    const int cap = sm_count() * (C4 > 64 ? 2 : 4), per_cta = dots || lean || C4 > 64 ? 8 : 16;
+    const int cap = sm_count() * (C4 > 64 ? 2 : 4), per_cta = dots || lean || C4 <= 32 || C4 > 64 ? 8 : 16;
     const int nbk = nblocks(N);
     auto items = [&](long long sps) { return (long long)(((long long)nseg * sps + streams - 1) / streams); };
     int sps = 1;
