@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) transpose_back_kernel(const float* __rest
     }
 }
 
-// dn[row, :] = g[row, :] / max(den[row], clamp),  dd[row] = den[row] >= clamp ? -<dn[row, :], out[row, :]> : 0; one warp per row
+// dn[row, :] = g[row, :] / max(den[row], clamp),  dd[row] = den[row] >= clamp ? -<dn[row, :], out[row, :]> : 0; 8, 16 or 32 lanes per row with VEC (C a multiple of four), else a warp
 template <bool VEC>
 __global__ void __launch_bounds__(256) attention_gradient_rows_kernel(const float* __restrict__ g, const float* __restrict__ out, const float* __restrict__ den,
                                                                       float* __restrict__ dn, float* __restrict__ dd, const int C, const float clamp, const long long rows)
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__
                                                              const float* __restrict__ aq, const float* __restrict__ vsum,
                                                              const float* __restrict__ akv, const float* __restrict__ aksum,
                                                              const float* __restrict__ n_pad,
-                                                             const int M, const int C, const int C4, const int H,
+                                                             const int M, const int C, const int H,
                                                              const float eps, const float clamp, const long long rows, float* __restrict__ den_out)
 {
     __shared__ float as[ROW_TILE], inv[ROW_TILE];
@@ -345,12 +345,12 @@ __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__
     }
     __syncthreads();
     float* o = out + r0 * C;
-    if (C % 4 == 0 && C4 == C) {
+    if (C % 4 == 0) {
         const int q = C >> 2;
         #pragma unroll 4
         for (int i = tid; i < n * q; i += 256) {
             const int r = i / q, c = (i - r * q) * 4;
-            const float4 vs = ldg4(vsum + (long long)head[r] * C4 + c), kv = ldg4(akv + (long long)head[r] * C4 + c);
+            const float4 vs = ldg4(vsum + (long long)head[r] * C + c), kv = ldg4(akv + (long long)head[r] * C + c);
             const float  a = as[r], f = inv[r];
             float4 x = *reinterpret_cast<const float4*>(o + 4 * i);
             x.x = (fmaf(a, vs.x, kv.x) - x.x) * f; x.y = (fmaf(a, vs.y, kv.y) - x.y) * f;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(256) riesz_epilogue_kernel(float* __restrict__
     } else {
         for (int i = tid; i < n * C; i += 256) {
             const int r = i / C, c = i - r * C;
-            o[i] = (fmaf(as[r], vsum[(long long)head[r] * C4 + c], akv[(long long)head[r] * C4 + c]) - o[i]) * inv[r];
+            o[i] = (fmaf(as[r], vsum[(long long)head[r] * C + c], akv[(long long)head[r] * C + c]) - o[i]) * inv[r];
         }
     }
 }
@@ -437,10 +437,10 @@ cudaError_t launch_normalise(float* out, const float* out_u, const float* qt, co
     return cudaGetLastError();
 }
 cudaError_t launch_riesz_epilogue(float* out, const float* out_u, const float* aq, const float* vsum, const float* akv,
-                                  const float* aksum, const float* n_pad, int P, int M, int C, int C4, int H,
+                                  const float* aksum, const float* n_pad, int P, int M, int C, int H,
                                   float eps, float clamp, float* den_out, cudaStream_t st) {
     const long long rows = (long long)P * M;
-    riesz_epilogue_kernel<<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(out, out_u, aq, vsum, akv, aksum, n_pad, M, C, C4, H, eps, clamp, rows, den_out);
+    riesz_epilogue_kernel<<<blocks_for(rows, ROW_TILE), 256, 0, st>>>(out, out_u, aq, vsum, akv, aksum, n_pad, M, C, H, eps, clamp, rows, den_out);
     return cudaGetLastError();
 }
 

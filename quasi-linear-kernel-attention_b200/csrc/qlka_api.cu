@@ -42,7 +42,7 @@ cudaError_t launch_normalise(float* out, const float* out_u, const float* qt, co
                              int P, int M, int D, int C, int H, float clamp, bool bump, float* den_out, cudaStream_t st);
 cudaError_t launch_abscolsum_d(const float* x, float* out, int P, int D, int L, cudaStream_t st);
 cudaError_t launch_riesz_epilogue(float* out, const float* out_u, const float* aq, const float* vsum, const float* akv,
-                                  const float* aksum, const float* n_pad, int P, int M, int C, int C4, int H,
+                                  const float* aksum, const float* n_pad, int P, int M, int C, int H,
                                   float eps, float clamp, float* den_out, cudaStream_t st);
 }  // namespace qlka
 
@@ -863,7 +863,7 @@ static int abs_attention_impl(int kind, const float* q, const float* k, const fl
         CU(launch_rowstat(rows, ws.ak, vsum, akv, aksum, P, S, Dv, stream));
         st = abs_forward_impl(ws.qt, ws.kt, rows, out, ws.out_u, ws.inner, workspace_bytes - ws.fixed, P, D, S, S, Dv, 0, nullptr, nullptr, stream, true);
         if (st) return st;
-        CU(launch_riesz_epilogue(out, ws.out_u, ws.aq, vsum, akv, aksum, ws.n_pad, P, S, Dv, Dv, H, 1e-3f, 1e-6f, den, stream));
+        CU(launch_riesz_epilogue(out, ws.out_u, ws.aq, vsum, akv, aksum, ws.n_pad, P, S, Dv, H, 1e-3f, 1e-6f, den, stream));
     }
     return QLKA_OK;
 }

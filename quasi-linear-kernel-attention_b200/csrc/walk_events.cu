@@ -123,7 +123,6 @@ struct EventFeeder {
     }
     // rows of block 0 under way, records of block 1 as well
     __device__ __forceinline__ void prologue(Vec<CPL> (&x)[EB], uint32_t (&e)[EB]) {
-        __syncwarp();                  // every lane has left the previous item's slots
         copy_records(0, next);
         cp_async_commit();
         cp_async_wait<0>();
@@ -201,73 +200,71 @@ __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) prefix_events(const WalkA
     F f;
     f.init(smem_u32(smem), C4);
 
-    {
-        const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::S::STREAMS);
-        f.start(a, st, NBK);
-        float* out_s = a.out_s + (long long)st.sg * a.M;
-        const unsigned long long out = ROWS ? (unsigned long long)__cvta_generic_to_global(a.out + (long long)st.p * a.Mrows * C4 + f.channel(0)) - (unsigned long long)EVENT_QUERY * f.row_bytes : 0ull;
-        Vec<CPL> H, T;
-        H.zero(); T.zero();
-        #pragma unroll
-        for (int q = 0; q < F::Q; q++) {
-            const int c = f.channel(q);
-            if (a.sps > 1) {           // incoming prefix sums (prefix_fold left them in the aggregate table)
-                const float* ag = a.agg + (st.on ? st.g : 0) * 2 * C4 + c;
-                const float4 h = ldg4(ag);
-                H.x[4 * q] = h.x; H.x[4 * q + 1] = h.y; H.x[4 * q + 2] = h.z; H.x[4 * q + 3] = h.w;
-                if (ROWS) {
-                    const float4 u = ldg4(ag + C4);
-                    T.x[4 * q] = -2.0f * u.x; T.x[4 * q + 1] = -2.0f * u.y; T.x[4 * q + 2] = -2.0f * u.z; T.x[4 * q + 3] = -2.0f * u.w;
-                }
+    const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::S::STREAMS);
+    f.start(a, st, NBK);
+    float* out_s = a.out_s + (long long)st.sg * a.M;
+    const unsigned long long out = ROWS ? (unsigned long long)__cvta_generic_to_global(a.out + (long long)st.p * a.Mrows * C4 + f.channel(0)) - (unsigned long long)EVENT_QUERY * f.row_bytes : 0ull;
+    Vec<CPL> H, T;
+    H.zero(); T.zero();
+    #pragma unroll
+    for (int q = 0; q < F::Q; q++) {
+        const int c = f.channel(q);
+        if (a.sps > 1) {           // incoming prefix sums (prefix_fold left them in the aggregate table)
+            const float* ag = a.agg + (st.on ? st.g : 0) * 2 * C4 + c;
+            const float4 h = ldg4(ag);
+            H.x[4 * q] = h.x; H.x[4 * q + 1] = h.y; H.x[4 * q + 2] = h.z; H.x[4 * q + 3] = h.w;
+            if (ROWS) {
+                const float4 u = ldg4(ag + C4);
+                T.x[4 * q] = -2.0f * u.x; T.x[4 * q + 1] = -2.0f * u.y; T.x[4 * q + 2] = -2.0f * u.z; T.x[4 * q + 3] = -2.0f * u.w;
             }
-            const float4 w = ldg4(a.wtotal + (long long)st.p * C4 + c);
-            H.x[4 * q] = fmaf(-0.5f, w.x, H.x[4 * q]);         H.x[4 * q + 1] = fmaf(-0.5f, w.y, H.x[4 * q + 1]);
-            H.x[4 * q + 2] = fmaf(-0.5f, w.z, H.x[4 * q + 2]); H.x[4 * q + 3] = fmaf(-0.5f, w.w, H.x[4 * q + 3]);
         }
-        Vec<CPL> x[EB];
-        uint32_t e[EB];
-        f.prologue(x, e);
-        const int steps = __reduce_max_sync(FULL, f.nblk);
-        for (int t = 0; t < steps; t++) {
-            f.step(t);
-            uint32_t n[EB];
-            f.read_index(f.next, n);
-            #pragma unroll
-            for (int h = 0; h < EB; h += EV_GROUP) {
-                #pragma unroll
-                for (int i = h; i < h + EV_GROUP; i++) {
-                    const Vec<CPL> y = x[i];
-                    f.park(i, f.dot(y, H));
-                    const float s = ROWS ? f.scalars(i).x : 0.0f;
-                    if (ROWS) {
-                        float r[CPL];
-                        #pragma unroll
-                        for (int c = 0; c < CPL; c++) r[c] = fmaf(s, H.x[c], T.x[c]);
-                        const bool write = !f.edge(t) || f.has(t, i);
-                        #pragma unroll
-                        for (int q = 0; q < F::Q; q++) red_if_query(f.on[q] && write, e[i], out + (q ? f.second : 0u), f.row_bytes, r + 4 * q);
-                    }
-                    if (!is_query(e[i])) {
-                        #pragma unroll
-                        for (int c = 0; c < CPL; c++) { if (ROWS) T.x[c] = fmaf(s, y.x[c], T.x[c]); H.x[c] += y.x[c]; }
-                    }
-                }
-                // the next block's rows into the registers that are free now
-                #pragma unroll
-                for (int i = h; i < h + EV_GROUP; i++) x[i] = f.row(n[i]);
-            }
-            f.finish(t, [&](const float sum, const uint32_t row, const uint32_t sc) {
-                out_s[row] = a.sign * fmaf(2.0f, sum, lds_f2(sc).y);
-            });
-            #pragma unroll
-            for (int i = 0; i < EB; i++) e[i] = n[i];
-        }
-        cp_async_wait<0>();
+        const float4 w = ldg4(a.wtotal + (long long)st.p * C4 + c);
+        H.x[4 * q] = fmaf(-0.5f, w.x, H.x[4 * q]);         H.x[4 * q + 1] = fmaf(-0.5f, w.y, H.x[4 * q + 1]);
+        H.x[4 * q + 2] = fmaf(-0.5f, w.z, H.x[4 * q + 2]); H.x[4 * q + 3] = fmaf(-0.5f, w.w, H.x[4 * q + 3]);
     }
+    Vec<CPL> x[EB];
+    uint32_t e[EB];
+    f.prologue(x, e);
+    const int steps = __reduce_max_sync(FULL, f.nblk);
+    for (int t = 0; t < steps; t++) {
+        f.step(t);
+        uint32_t n[EB];
+        f.read_index(f.next, n);
+        #pragma unroll
+        for (int h = 0; h < EB; h += EV_GROUP) {
+            #pragma unroll
+            for (int i = h; i < h + EV_GROUP; i++) {
+                const Vec<CPL> y = x[i];
+                f.park(i, f.dot(y, H));
+                const float s = ROWS ? f.scalars(i).x : 0.0f;
+                if (ROWS) {
+                    float r[CPL];
+                    #pragma unroll
+                    for (int c = 0; c < CPL; c++) r[c] = fmaf(s, H.x[c], T.x[c]);
+                    const bool write = !f.edge(t) || f.has(t, i);
+                    #pragma unroll
+                    for (int q = 0; q < F::Q; q++) red_if_query(f.on[q] && write, e[i], out + (q ? f.second : 0u), f.row_bytes, r + 4 * q);
+                }
+                if (!is_query(e[i])) {
+                    #pragma unroll
+                    for (int c = 0; c < CPL; c++) { if (ROWS) T.x[c] = fmaf(s, y.x[c], T.x[c]); H.x[c] += y.x[c]; }
+                }
+            }
+            // the next block's rows into the registers that are free now
+            #pragma unroll
+            for (int i = h; i < h + EV_GROUP; i++) x[i] = f.row(n[i]);
+        }
+        f.finish(t, [&](const float sum, const uint32_t row, const uint32_t sc) {
+            out_s[row] = a.sign * fmaf(2.0f, sum, lds_f2(sc).y);
+        });
+        #pragma unroll
+        for (int i = 0; i < EB; i++) e[i] = n[i];
+    }
+    cp_async_wait<0>();
 }
 
 template <int LPS, int CPL, bool ROWS>
-static cudaError_t launch_prefix(const WalkArgs& a, int sms, cudaStream_t stream) {
+static cudaError_t launch_prefix(const WalkArgs& a, cudaStream_t stream) {
     constexpr int smem = Shape<LPS, CPL>::SMEM;
     const long long items = ((long long)a.nseg * a.sps * LPS + EV_THREADS - 1) / EV_THREADS;
     prefix_events<LPS, CPL, ROWS><<<(unsigned)items, EV_THREADS, smem, stream>>>(a);
@@ -275,10 +272,10 @@ static cudaError_t launch_prefix(const WalkArgs& a, int sms, cudaStream_t stream
 }
 
 // dots, or rows and dots, of a prefix walk whose streams' incoming sums are in a.agg
-cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, int sms, cudaStream_t stream) {
-    if (a.C4 <= 32)  return rows ? launch_prefix<8, 4, true>(a, sms, stream) : launch_prefix<8, 4, false>(a, sms, stream);
-    if (a.C4 <= 64)  return rows ? launch_prefix<8, 8, true>(a, sms, stream) : launch_prefix<8, 8, false>(a, sms, stream);
-    if (a.C4 <= 128) return rows ? launch_prefix<16, 8, true>(a, sms, stream) : launch_prefix<16, 8, false>(a, sms, stream);
+cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, cudaStream_t stream) {
+    if (a.C4 <= 32)  return rows ? launch_prefix<8, 4, true>(a, stream) : launch_prefix<8, 4, false>(a, stream);
+    if (a.C4 <= 64)  return rows ? launch_prefix<8, 8, true>(a, stream) : launch_prefix<8, 8, false>(a, stream);
+    if (a.C4 <= 128) return rows ? launch_prefix<16, 8, true>(a, stream) : launch_prefix<16, 8, false>(a, stream);
     return cudaErrorInvalidValue;
 }
 
@@ -295,98 +292,96 @@ __global__ void __launch_bounds__(EV_THREADS, EV_CTAS) laplace_events(const Walk
     F f;
     f.init(smem_u32(smem), C4);
 
-    {
-        const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::S::STREAMS);
-        const long long block0 = f.start(a, st, NBK) / EB;
-        float* out_s = a.out_s + (long long)st.sg * a.M;
-        const unsigned long long out = ROWS ? (unsigned long long)__cvta_generic_to_global(a.out + (long long)st.p * a.Mrows * C4 + f.channel(0)) - (unsigned long long)EVENT_QUERY * f.row_bytes : 0ull;
-        const float* ag = a.agg + (st.on ? st.g : 0) * (2 * C4 + 4);       // incoming states (laplace_fold left them in the aggregate table)
-        Vec<CPL> L = f.vector(ag);
-        const float alast = st.on && st.b1 < NBK ? __ldg(a.xval + (long long)st.sg * xstride(a.N) + st.b1 * KB) : 0.0f;
-        // checkpoints: of the first keys of the blocks after the first that have any, in the places of the stream's last blocks
-        int       left = st.on ? __float_as_int(__ldg(ag + 2 * C4 + 2)) : 0;
-        long long at   = block0 + f.nblk - left;
-        // the checkpoint of the first key after the block in use, fetched one block early, into registers that the backward sweep leaves
-        Vec<CPL> cnext;
-        float2   wnext = make_float2(0.0f, 0.0f);
-        cnext.zero();
-        auto load_ckpt = [&]() { wnext = __ldg(reinterpret_cast<const float2*>(a.wck + 2 * at)); cnext = f.vector(a.ckpt + at * C4); };
-        if (left > 0) load_ckpt();
-        Vec<CPL> x[EB];
-        uint32_t e[EB];
-        f.prologue(x, e);
-        const int steps = __reduce_max_sync(FULL, f.nblk);
-        for (int t = 0; t < steps; t++) {
-            f.step(t);
-            // the state at the first key after the block, that key's decay
-            Vec<CPL> R = f.vector(ag + C4);
-            float anext = alast;
-            if (left > 0) {
-                #pragma unroll
-                for (int c = 0; c < CPL; c++) R.x[c] = fmaf(wnext.x, R.x[c], cnext.x[c]);
-                anext = wnext.y;
-            }
-            float dr[ROWS ? 1 : EB];                      // dots with the suffix state ...
-            f2    r[ROWS ? EB : 1][CPL / 2];              // ... or that state, for rows and dots
+    const StreamOf st(a, blockIdx.x, threadIdx.x / LPS, NBK, F::S::STREAMS);
+    const long long block0 = f.start(a, st, NBK) / EB;
+    float* out_s = a.out_s + (long long)st.sg * a.M;
+    const unsigned long long out = ROWS ? (unsigned long long)__cvta_generic_to_global(a.out + (long long)st.p * a.Mrows * C4 + f.channel(0)) - (unsigned long long)EVENT_QUERY * f.row_bytes : 0ull;
+    const float* ag = a.agg + (st.on ? st.g : 0) * (2 * C4 + 4);       // incoming states (laplace_fold left them in the aggregate table)
+    Vec<CPL> L = f.vector(ag);
+    const float alast = st.on && st.b1 < NBK ? __ldg(a.xval + (long long)st.sg * xstride(a.N) + st.b1 * KB) : 0.0f;
+    // checkpoints: of the first keys of the blocks after the first that have any, in the places of the stream's last blocks
+    int       left = st.on ? __float_as_int(__ldg(ag + 2 * C4 + 2)) : 0;
+    long long at   = block0 + f.nblk - left;
+    // the checkpoint of the first key after the block in use, fetched one block early, into registers that the backward sweep leaves
+    Vec<CPL> cnext;
+    float2   wnext = make_float2(0.0f, 0.0f);
+    cnext.zero();
+    auto load_ckpt = [&]() { wnext = __ldg(reinterpret_cast<const float2*>(a.wck + 2 * at)); cnext = f.vector(a.ckpt + at * C4); };
+    if (left > 0) load_ckpt();
+    Vec<CPL> x[EB];
+    uint32_t e[EB];
+    f.prologue(x, e);
+    const int steps = __reduce_max_sync(FULL, f.nblk);
+    for (int t = 0; t < steps; t++) {
+        f.step(t);
+        // the state at the first key after the block, that key's decay
+        Vec<CPL> R = f.vector(ag + C4);
+        float anext = alast;
+        if (left > 0) {
             #pragma unroll
-            for (int i = EB - 1; i >= 0; i--) {
-                const float2 s = f.scalars(i);
+            for (int c = 0; c < CPL; c++) R.x[c] = fmaf(wnext.x, R.x[c], cnext.x[c]);
+            anext = wnext.y;
+        }
+        float dr[ROWS ? 1 : EB];                      // dots with the suffix state ...
+        f2    r[ROWS ? EB : 1][CPL / 2];              // ... or that state, for rows and dots
+        #pragma unroll
+        for (int i = EB - 1; i >= 0; i--) {
+            const float2 s = f.scalars(i);
+            if (ROWS) {
+                #pragma unroll
+                for (int c = 0; c < CPL / 2; c++) r[ROWS ? i : 0][c] = mul2(pack2(s.y, s.y), pack2(R.x[2 * c], R.x[2 * c + 1]));
+            } else {
+                dr[ROWS ? 0 : i] = s.y * f.dot(x[i], R);
+            }
+            if (!is_query(e[i])) {
+                #pragma unroll
+                for (int c = 0; c < CPL; c++) R.x[c] = fmaf(anext, R.x[c], x[i].x[c]);
+                anext = s.x;
+            }
+        }
+        uint32_t n[EB];
+        f.read_index(f.next, n);
+        if (left > 0) {                               // (the last one read stays until its block comes)
+            bool keys = false;
+            #pragma unroll
+            for (int i = 0; i < EB; i++) keys |= !is_query(n[i]);
+            if (keys) { left--; at++; }
+            if (left > 0) load_ckpt();
+        }
+        #pragma unroll
+        for (int h = 0; h < EB; h += EV_GROUP) {
+            #pragma unroll
+            for (int i = h; i < h + EV_GROUP; i++) {
+                const float s = f.scalars(i).x;
                 if (ROWS) {
+                    float row[CPL];
+                    Vec<CPL> z;                       // e1 R - e0 L
                     #pragma unroll
-                    for (int c = 0; c < CPL / 2; c++) r[ROWS ? i : 0][c] = mul2(pack2(s.y, s.y), pack2(R.x[2 * c], R.x[2 * c + 1]));
+                    for (int c = 0; c < CPL / 2; c++) {
+                        const f2 l = pack2(L.x[2 * c], L.x[2 * c + 1]), suf = r[ROWS ? i : 0][c];
+                        unpack2(fma2(pack2(s, s), l, suf), row[2 * c], row[2 * c + 1]);
+                        unpack2(fma2(pack2(-s, -s), l, suf), z.x[2 * c], z.x[2 * c + 1]);
+                    }
+                    f.park(i, f.dot(x[i], z));
+                    #pragma unroll
+                    for (int q = 0; q < F::Q; q++) red_if_query(f.on[q] && (!f.edge(t) || f.has(t, i)), e[i], out + (q ? f.second : 0u), f.row_bytes, row + 4 * q);
                 } else {
-                    dr[ROWS ? 0 : i] = s.y * f.dot(x[i], R);
+                    f.park(i, fmaf(-s, f.dot(x[i], L), dr[ROWS ? 0 : i]));
                 }
                 if (!is_query(e[i])) {
                     #pragma unroll
-                    for (int c = 0; c < CPL; c++) R.x[c] = fmaf(anext, R.x[c], x[i].x[c]);
-                    anext = s.x;
+                    for (int c = 0; c < CPL; c++) L.x[c] = fmaf(s, L.x[c], x[i].x[c]);
                 }
             }
-            uint32_t n[EB];
-            f.read_index(f.next, n);
-            if (left > 0) {                               // (the last one read stays until its block comes)
-                bool keys = false;
-                #pragma unroll
-                for (int i = 0; i < EB; i++) keys |= !is_query(n[i]);
-                if (keys) { left--; at++; }
-                if (left > 0) load_ckpt();
-            }
+            // the next block's rows into the registers that are free now
             #pragma unroll
-            for (int h = 0; h < EB; h += EV_GROUP) {
-                #pragma unroll
-                for (int i = h; i < h + EV_GROUP; i++) {
-                    const float s = f.scalars(i).x;
-                    if (ROWS) {
-                        float row[CPL];
-                        Vec<CPL> z;                       // e1 R - e0 L
-                        #pragma unroll
-                        for (int c = 0; c < CPL / 2; c++) {
-                            const f2 l = pack2(L.x[2 * c], L.x[2 * c + 1]), suf = r[ROWS ? i : 0][c];
-                            unpack2(fma2(pack2(s, s), l, suf), row[2 * c], row[2 * c + 1]);
-                            unpack2(fma2(pack2(-s, -s), l, suf), z.x[2 * c], z.x[2 * c + 1]);
-                        }
-                        f.park(i, f.dot(x[i], z));
-                        #pragma unroll
-                        for (int q = 0; q < F::Q; q++) red_if_query(f.on[q] && (!f.edge(t) || f.has(t, i)), e[i], out + (q ? f.second : 0u), f.row_bytes, row + 4 * q);
-                    } else {
-                        f.park(i, fmaf(-s, f.dot(x[i], L), dr[ROWS ? 0 : i]));
-                    }
-                    if (!is_query(e[i])) {
-                        #pragma unroll
-                        for (int c = 0; c < CPL; c++) L.x[c] = fmaf(s, L.x[c], x[i].x[c]);
-                    }
-                }
-                // the next block's rows into the registers that are free now
-                #pragma unroll
-                for (int i = h; i < h + EV_GROUP; i++) x[i] = f.row(n[i]);
-            }
-            f.finish(t, [&](const float sum, const uint32_t row, const uint32_t) { atomicAdd(out_s + row, sum); });
-            #pragma unroll
-            for (int i = 0; i < EB; i++) e[i] = n[i];
+            for (int i = h; i < h + EV_GROUP; i++) x[i] = f.row(n[i]);
         }
-        cp_async_wait<0>();
+        f.finish(t, [&](const float sum, const uint32_t row, const uint32_t) { atomicAdd(out_s + row, sum); });
+        #pragma unroll
+        for (int i = 0; i < EB; i++) e[i] = n[i];
     }
+    cp_async_wait<0>();
 }
 
 template <int LPS, int CPL, bool ROWS>

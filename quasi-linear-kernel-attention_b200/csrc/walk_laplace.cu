@@ -7,7 +7,7 @@
 // Replaces the reference's laplace_chunk / laplace_scan / laplace_walk trio
 // (laplace_kernels.cu:65-127, 134-188, 219-409) with two launches over independent work units:
 //   * a "stream" is a contiguous run of key blocks of one segment; a segment is cut into SPS of them
-//     (any number: the host picks it so that the persistent CTAs stay balanced) and the streams of all
+//     (any number: the host picks it so that every SM gets its share) and the streams of all
 //     segments are numbered consecutively (walk_ring.cuh: how lanes share a stream); nothing couples the
 //     streams of a CTA.
 //   * laplace_pass1 walks every stream backwards once: the local suffix state at every block start goes
@@ -15,7 +15,7 @@
 //     across it to the aggregate table.
 //   * laplace_fold turns the aggregates of a segment's streams into the prefix state entering each stream
 //     and the suffix state entering it from above (serial over the streams, parallel over channels).
-//   * laplace_pass2 walks every stream forward from those states: per
+//   * laplace_rows or laplace_pass2 (persistent CTAs) walks every stream forward from those states: per
 //     block of 8 keys the suffix states are rebuilt in registers from the next checkpoint, the prefix
 //     states overwrite the row registers, and the block's queries are emitted in rank order.
 // The rows are therefore gathered twice (the reference gathers them three times) and every
@@ -273,8 +273,8 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
     }
 }
 
-// The second pass's row emission with 4 channels per lane (RowFeeder; rows_by_quads says when). Two CTAs per SM: its state takes
-// some 120 registers. Bound by the L2 traffic of one row gathered and one row reduced per key and query (2.4 of its 2.8 ms
+// The second pass's row emission with 4 channels per lane (RowFeeder; rows_by_quads says when). A CTA per item, eight of them (16 warps) on an
+// SM: its state takes some 120 registers. Bound by the L2 traffic of one row gathered and one row reduced per key and query (2.4 of its 2.8 ms
 // at 48 heads x 16384 keys and queries; with one stream per warp it took 3.0).
 template <int LPS>
 __global__ void __launch_bounds__(ROW_THREADS, LAP_CTAS_ROWS) laplace_rows(const WalkArgs a)
@@ -290,61 +290,57 @@ __global__ void __launch_bounds__(ROW_THREADS, LAP_CTAS_ROWS) laplace_rows(const
     RowFeeder<LPS> f;
     f.init(smem_u32(smem), N, a.M, C4);
 
-    const int items = (int)(((long long)a.nseg * a.sps + STREAMS - 1) / STREAMS);
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const StreamOf st(a, item, tid / LPS, NBK, STREAMS);
-        const int nblk = st.nblk;
-        f.start(a, st.sg, st.p, st.b0);
-        char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
-        const float* ck = a.ckpt + ((long long)st.sg * NBK + st.b0 + 1) * C4 + c0l;      // of the next block to fetch
-        const float* wk = a.wck + (long long)st.sg * NBK + st.b0 + 1;
-        const float* ag = a.agg + (st.on ? st.g : 0) * lap_agg_stride(C4) + c0l;
-        Vec<4> L = vload<4>(ag), Rin = vload<4>(ag + C4);
+    const StreamOf st(a, blockIdx.x, tid / LPS, NBK, STREAMS);
+    const int nblk = st.nblk;
+    f.start(a, st.sg, st.p, st.b0);
+    char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
+    const float* ck = a.ckpt + ((long long)st.sg * NBK + st.b0 + 1) * C4 + c0l;      // of the next block to fetch
+    const float* wk = a.wck + (long long)st.sg * NBK + st.b0 + 1;
+    const float* ag = a.agg + (st.on ? st.g : 0) * lap_agg_stride(C4) + c0l;
+    Vec<4> L = vload<4>(ag), Rin = vload<4>(ag + C4);
 
-        __syncwarp(gmask);                         // every lane has left the previous item's slots
-        f.prologue(nblk);
-        Vec<4> cnext; cnext.zero();
-        float  wnext = 0.0f;
-        auto load_ckpt = [&]() { wnext = *wk++; cnext = vload_once<4>(ck); ck += C4; };
-        if (nblk > 1) load_ckpt();
-        int cur = 0, j0 = st.b0 * KB;
-        for (int t = 0; t < nblk; t++, j0 += KB, cur ^= 1) {
-            __syncwarp(gmask);                     // every lane is done with the slot refilled below
-            // suffix state entering the block from above: corrected checkpoint, or the stream's incoming state
-            Vec<4> Rn = Rin;
-            if (t + 1 < nblk) axpy(Rn, wnext, Rin, cnext);
-            if (t + 2 < nblk) load_ckpt();
-            f.step(t, cur, nblk);
-            __syncwarp(gmask);
-            float av[KB + 1];
-            f.read_scalars(cur, av);
-            Vec<4> v[KB], Rb[KB];
-            f.read_rows(cur, j0, v);
-            #pragma unroll
-            for (int i = KB - 1; i >= 0; i--) {
-                axpy(Rn, av[i + 1], Rn, v[i]);
-                Rb[i] = Rn;
-            }
-            // prefix state before each key, in place of the rows
-            #pragma unroll
-            for (int i = 0; i < KB; i++) {
-                const Vec<4> row = v[i];
-                v[i] = L;
-                axpy(L, av[i], L, row);
-            }
-            f.for_queries(cur, j0, [&](const int i, const uint4& rec) {
-                Vec<4> r;
-                scale(r, __uint_as_float(rec.y), Rb[i]);
-                axpy(r, __uint_as_float(rec.x), v[i], r);
-                if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
-            });
+    f.prologue(nblk);
+    Vec<4> cnext; cnext.zero();
+    float  wnext = 0.0f;
+    auto load_ckpt = [&]() { wnext = *wk++; cnext = vload_once<4>(ck); ck += C4; };
+    if (nblk > 1) load_ckpt();
+    int cur = 0, j0 = st.b0 * KB;
+    for (int t = 0; t < nblk; t++, j0 += KB, cur ^= 1) {
+        __syncwarp(gmask);                     // every lane is done with the slot refilled below
+        // suffix state entering the block from above: corrected checkpoint, or the stream's incoming state
+        Vec<4> Rn = Rin;
+        if (t + 1 < nblk) axpy(Rn, wnext, Rin, cnext);
+        if (t + 2 < nblk) load_ckpt();
+        f.step(t, cur, nblk);
+        __syncwarp(gmask);
+        float av[KB + 1];
+        f.read_scalars(cur, av);
+        Vec<4> v[KB], Rb[KB];
+        f.read_rows(cur, j0, v);
+        #pragma unroll
+        for (int i = KB - 1; i >= 0; i--) {
+            axpy(Rn, av[i + 1], Rn, v[i]);
+            Rb[i] = Rn;
         }
-        cp_async_wait<0>();
+        // prefix state before each key, in place of the rows
+        #pragma unroll
+        for (int i = 0; i < KB; i++) {
+            const Vec<4> row = v[i];
+            v[i] = L;
+            axpy(L, av[i], L, row);
+        }
+        f.for_queries(cur, j0, [&](const int i, const uint4& rec) {
+            Vec<4> r;
+            scale(r, __uint_as_float(rec.y), Rb[i]);
+            axpy(r, __uint_as_float(rec.x), v[i], r);
+            if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
+        });
     }
+    cp_async_wait<0>();
 }
 
 template <int LPS>
-static cudaError_t launch_lap_rows(const WalkArgs& a, int sms, cudaStream_t stream) {
+static cudaError_t launch_lap_rows(const WalkArgs& a, cudaStream_t stream) {
     constexpr int smem = row_smem_bytes<LPS>();
     cudaError_t e = cudaFuncSetAttribute(laplace_rows<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
@@ -380,7 +376,7 @@ static cudaError_t launch_lap(const WalkArgs& a, int emit, int sms, cudaStream_t
     if (e == cudaSuccess && mid) e = cudaEventRecord(mid, stream);
     if (e != cudaSuccess) return e;
     if (emit != LAP_ROWS) return launch_laplace_events(a, emit == LAP_BOTH, stream);
-    if (CPL == 4 || rows_by_quads(a)) return launch_lap_rows<LPS>(a, sms, stream);
+    if (CPL == 4 || rows_by_quads(a)) return launch_lap_rows<LPS>(a, stream);
     if constexpr (CPL < 4) return launch_lap_pass2<CPL>(a, sms, stream);
 }
 

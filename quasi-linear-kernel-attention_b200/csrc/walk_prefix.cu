@@ -9,14 +9,14 @@
 // EMIT_DOT and EMIT_BOTH (the walks of the gradients) share the first launch and the fold; their emission is in walk_events.cu.
 //
 // Same mapping and staging as the Laplace walk (walk_ring.cuh; SPS independent streams per
-// segment numbered over all segments, persistent CTAs). The first launch sums each stream's rows into an aggregate
+// segment numbered over all segments). The first launch sums each stream's rows into an aggregate
 // table, a small kernel turns the table into exclusive prefix sums over each segment's streams, the last launch walks
 // every stream forward from its incoming prefix and emits. With one stream per segment only the last one runs.
 #include "walk_ring.cuh"
 
 namespace qlka {
 
-cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, int sms, cudaStream_t stream);      // walk_events.cu
+cudaError_t launch_prefix_events(const WalkArgs& a, bool rows, cudaStream_t stream);      // walk_events.cu
 
 enum { EMIT_ROWS = 0, EMIT_DOT = 1, EMIT_BOTH = 2 };
 
@@ -191,51 +191,47 @@ __global__ void __launch_bounds__(ROW_THREADS, PREFIX_CTAS_ROWS) prefix_rows(con
     RowFeeder<LPS> f;
     f.init(smem_u32(smem), N, a.M, C4);
 
-    const int items = (int)(((long long)a.nseg * a.sps + STREAMS - 1) / STREAMS);
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const StreamOf st(a, item, tid / LPS, NBK, STREAMS);
-        f.start(a, st.sg, st.p, st.b0);
-        char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
-        Vec<4> PV, PK;
-        PV.zero(); PK.zero();
-        if (a.sps > 1) {        // incoming prefix sums (prefix_fold left them in the aggregate table)
-            const float* ag = a.agg + (st.on ? st.g : 0) * prefix_agg_stride(C4) + c0l;
-            PV = vload<4>(ag);
-            PK = vload<4>(ag + C4);
-        }
-        __syncwarp(gmask);                         // every lane has left the previous item's slots
-        f.prologue(st.nblk);
-        int cur = 0, j0 = st.b0 * KB;
-        for (int t = 0; t < st.nblk; t++, j0 += KB, cur ^= 1) {
-            __syncwarp(gmask);                     // every lane is done with the slot refilled below
-            f.step(t, cur, st.nblk);
-            __syncwarp(gmask);
-            float kv[KB + 1];
-            f.read_scalars(cur, kv);
-            Vec<4> v[KB], kb[KB];
-            f.read_rows(cur, j0, v);
-            // prefix states before each key, in place of the rows
-            #pragma unroll
-            for (int i = 0; i < KB; i++) {
-                const Vec<4> row = v[i];
-                v[i]  = PV;
-                kb[i] = PK;
-                vadd(PV, row);
-                axpy(PK, kv[i], row, PK);
-            }
-            f.for_queries(cur, j0, [&](const int i, const uint4& rec) {
-                Vec<4> r;
-                scale(r, __uint_as_float(rec.y), kb[i]);
-                axpy(r, __uint_as_float(rec.x), v[i], r);
-                if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
-            });
-        }
-        cp_async_wait<0>();
+    const StreamOf st(a, blockIdx.x, tid / LPS, NBK, STREAMS);
+    f.start(a, st.sg, st.p, st.b0);
+    char* out = reinterpret_cast<char*>(a.out + (long long)st.p * a.Mrows * C4 + c0l);
+    Vec<4> PV, PK;
+    PV.zero(); PK.zero();
+    if (a.sps > 1) {        // incoming prefix sums (prefix_fold left them in the aggregate table)
+        const float* ag = a.agg + (st.on ? st.g : 0) * prefix_agg_stride(C4) + c0l;
+        PV = vload<4>(ag);
+        PK = vload<4>(ag + C4);
     }
+    f.prologue(st.nblk);
+    int cur = 0, j0 = st.b0 * KB;
+    for (int t = 0; t < st.nblk; t++, j0 += KB, cur ^= 1) {
+        __syncwarp(gmask);                     // every lane is done with the slot refilled below
+        f.step(t, cur, st.nblk);
+        __syncwarp(gmask);
+        float kv[KB + 1];
+        f.read_scalars(cur, kv);
+        Vec<4> v[KB], kb[KB];
+        f.read_rows(cur, j0, v);
+        // prefix states before each key, in place of the rows
+        #pragma unroll
+        for (int i = 0; i < KB; i++) {
+            const Vec<4> row = v[i];
+            v[i]  = PV;
+            kb[i] = PK;
+            vadd(PV, row);
+            axpy(PK, kv[i], row, PK);
+        }
+        f.for_queries(cur, j0, [&](const int i, const uint4& rec) {
+            Vec<4> r;
+            scale(r, __uint_as_float(rec.y), kb[i]);
+            axpy(r, __uint_as_float(rec.x), v[i], r);
+            if (lane_on) vred(reinterpret_cast<float*>(out + (unsigned long long)rec.z * f.row_bytes), r);
+        });
+    }
+    cp_async_wait<0>();
 }
 
 template <int LPS>
-static cudaError_t launch_rows(const WalkArgs& a, int sms, cudaStream_t stream) {
+static cudaError_t launch_rows(const WalkArgs& a, cudaStream_t stream) {
     constexpr int smem = row_smem_bytes<LPS>();
     cudaError_t e = cudaFuncSetAttribute(prefix_rows<LPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
@@ -270,8 +266,8 @@ static cudaError_t launch_pw(const WalkArgs& a, int emit, int sms, cudaStream_t 
         cudaError_t e = emit == EMIT_DOT ? launch_pass1<L, W, false>(a, stream) : launch_pass1<L, W, true>(a, stream);
         if (e != cudaSuccess) return e;
     }
-    if (emit != EMIT_ROWS) return launch_prefix_events(a, emit == EMIT_BOTH, sms, stream);
-    if (CPL == 4 || rows_by_quads(a)) return launch_rows<LPS>(a, sms, stream);
+    if (emit != EMIT_ROWS) return launch_prefix_events(a, emit == EMIT_BOTH, stream);
+    if (CPL == 4 || rows_by_quads(a)) return launch_rows<LPS>(a, stream);
     if constexpr (CPL < 4) return launch_pass2<CPL>(a, sms, stream);
 }
 

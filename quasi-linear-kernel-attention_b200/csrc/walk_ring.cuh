@@ -41,11 +41,6 @@ __device__ __forceinline__ uint32_t lds32u(const uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ uint2 lds64u(const uint32_t addr) {
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
-    return v;
-}
 __device__ __forceinline__ void sts32f(const uint32_t addr, const float v) {
     asm volatile("st.shared.f32 [%0], %1;" :: "r"(addr), "f"(v) : "memory");
 }
@@ -140,7 +135,7 @@ __device__ __forceinline__ Vec<CPL> vload(const float* p) {
     else                         v.x[0] = __ldg(p);
     return v;
 }
-// loads and stores of data that is used once, long after or long before
+// loads of data that is used once, long after it was written
 template <int CPL>
 __device__ __forceinline__ Vec<CPL> vload_once(const float* p) {
     Vec<CPL> v;
@@ -148,18 +143,6 @@ __device__ __forceinline__ Vec<CPL> vload_once(const float* p) {
     else if constexpr (CPL == 2) { const float2 t = __ldcs(reinterpret_cast<const float2*>(p)); v.x[0] = t.x; v.x[1] = t.y; }
     else                         v.x[0] = __ldcs(p);
     return v;
-}
-template <int CPL>
-__device__ __forceinline__ void vstore_once(float* p, const Vec<CPL>& v) {
-    if constexpr (CPL == 4)      __stcs(reinterpret_cast<float4*>(p), make_float4(v.x[0], v.x[1], v.x[2], v.x[3]));
-    else if constexpr (CPL == 2) __stcs(reinterpret_cast<float2*>(p), make_float2(v.x[0], v.x[1]));
-    else                         __stcs(p, v.x[0]);
-}
-template <int CPL>
-__device__ __forceinline__ void vstore(float* p, const Vec<CPL>& v) {
-    if constexpr (CPL == 4)      *reinterpret_cast<float4*>(p) = make_float4(v.x[0], v.x[1], v.x[2], v.x[3]);
-    else if constexpr (CPL == 2) *reinterpret_cast<float2*>(p) = make_float2(v.x[0], v.x[1]);
-    else                         *p = v.x[0];
 }
 // vector reduction into global memory (no return value): a row of the output per warp
 template <int CPL>
@@ -369,16 +352,6 @@ struct QuadFeeder {
         if (ln < 3) cp_async16(sx + slot * SX_STRIDE * 4 + 16 * ln, xval);
         xval += KB;
         cp_async_commit();
-    }
-    __device__ __forceinline__ void prologue(const int nblk) {
-        if (nblk > 0) { prefetch_index(); issue(0); }
-        if (nblk > 1) prefetch_index();
-    }
-    __device__ __forceinline__ void step(const int t, const int cur, const int nblk) {
-        if (t + 1 < nblk) issue(cur ^ 1);
-        else cp_async_commit();
-        if (t + 2 < nblk) prefetch_index();
-        cp_async_wait<1>();
     }
     __device__ __forceinline__ void read_rows(const int slot, const int j0, Vec<4> (&v)[KB]) const {
         #pragma unroll
