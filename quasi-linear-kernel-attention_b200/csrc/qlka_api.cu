@@ -368,9 +368,11 @@ cudaError_t laplace_walk_chunked(const Records& r, const LapWalkScratch& sc, con
 // ------------------------------------------------------------------ short sequences: pair by pair
 // Whether the pairwise kernels beat the sorted walk, from two cost estimates fitted to measurements on a B200 (1 to 256 heads,
 // 64 to 4096 keys, 32 and 64 features, 32 to 128 channels). The pairwise one is good to a tenth. The sorted one was fitted to slower walks
-// and lies 14 to 40 % above what they take now (64 features and channels, Laplace, estimate / measured: 96 heads x 256 keys 473 / 335 us,
-// 96 x 777 918 / 695, 48 x 1024 599 / 443, 48 x 4096 1911 / 1484), so near the line some calls run pair by pair that would be up to
-// a fifth faster sorted (96 x 777: 856 / 695 us).
+// and lies 43 to 68 % above what they take now (64 features and channels, estimate / measured in us: Laplace sum of 96 heads x 256 keys 473 / 285,
+// 96 x 777 918 / 576, 48 x 1024 599 / 372, 48 x 4096 1911 / 1250; riesz 327, 615, 420, 1314; bump of 48 x 1024 1505 / 897), so near the line some calls
+// run pair by pair that would be up to a third faster sorted (Laplace 96 x 777 873 / 576, abs 542 / 566, riesz 546 / 615). The sorted forward sums
+// round no more (2-norm against float64, sorted / pairwise, 96 x 777: Laplace 1.3e-7 / 4.9e-7, abs 1.4e-7 / 4.9e-7, riesz 5.7e-7 / 5.7e-7, bump 4.1e-7 /
+// 4.9e-7): accuracy is no reason for where this line lies, as it is for the Laplace gradients below.
 double dense_us(int kind, double P, int D, int N, int M, int C) {
     // picoseconds per pair and feature, and per pair and channel, with three CTAs on every SM
     const double per_d = kind == DENSE_LAPLACE ? 0.155 : kind == DENSE_BUMP ? 0.115 : 0.090, per_c = 0.027;
