@@ -13,21 +13,6 @@
 
 namespace qlka {
 
-// Diagnostic build only (-DQLKA_PHASE_CLOCKS, see phase_clocks_main.cu): thread 0 of every CTA adds the cycles it spent
-// between two marks to a global table, so that the kernel's phases can be weighed against each other.
-#ifdef QLKA_PHASE_CLOCKS
-__device__ unsigned long long g_phase_clocks[16];
-#define PHASE_BEGIN() long long phase_t_ = clock64()
-#define PHASE_MARK(i)                                                                                        \
-    do {                                                                                                     \
-        __syncthreads();                                                                                     \
-        if (threadIdx.x == 0) { const long long t_ = clock64(); atomicAdd(&g_phase_clocks[i], (unsigned long long)(t_ - phase_t_)); phase_t_ = t_; } \
-    } while (0)
-#else
-#define PHASE_BEGIN()
-#define PHASE_MARK(i)
-#endif
-
 // ------------------------------------------------------------------ block radix sort
 // Elements are held in registers, E per thread, in warp-blocked order: the element at
 // array position warp*32*E + s*32 + lane sits in slot s of that lane. One pass ranks each
@@ -378,7 +363,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     float*    su1    = a.su1 ? a.su1 + (long long)seg * (NG + 1) + ks : nullptr;
     auto key_row = [&](const uint32_t i) -> uint32_t { return PART ? __ldg(kidx + i) : i; };
     auto query_row = [&](const int m) -> int { return PART ? (int)__ldg(qidx + m) : m; };
-    PHASE_BEGIN();
     // ---- (1) keys
     // NB equal-width value buckets between the smallest and the largest key; the bucket of a value is a monotone
     // function of it. They serve twice. Sorting: when no bucket holds more than RUN_LIMIT keys (any smooth
@@ -398,7 +382,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         uint32_t key[E], idx[E];
         if (PART) load_part<THREADS, E>(kkey, N, key, idx);
         else      load_segment<THREADS, E>(a.x + (long long)seg * N, N, key, idx);
-        PHASE_MARK(0);
         const int warp = tid >> 5, lane = tid & 31;
         uint32_t* hw = reinterpret_cast<uint32_t*>(bst);           // the bucket counters: NB + 1 of 16 bits, two to a word
         {
@@ -494,7 +477,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
             sorted = sidx;
         }
     }
-    PHASE_MARK(1);
     if (by_radix) {
         // sorted keys to floats; the bucket starts again, now from the sorted order: key j starts every bucket above its
         // predecessor's up to its own
@@ -516,7 +498,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     if (PART || by_radix) for (int j = tid; j < N; j += THREADS) xperm[j] = PART ? skey[sorted[j]] : (uint32_t)sorted[j];
     if (last) for (int j = N + tid; j < NP - ks; j += THREADS) xperm[j] = 0u;
     __syncthreads();
-    PHASE_MARK(2);
     // ---- (2) per-key scalars; my run of keys is [i0, i0 + cntk). The run length is odd so that the
     // strided shared-memory accesses below are bank-conflict free; results leave through a staging
     // buffer (the idle sort buffer) so that the global stores are coalesced.
@@ -596,7 +577,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         }
     }
     __syncthreads();          // the su arrays are complete; skey becomes the rank histogram
-    PHASE_MARK(3);
     // ---- (3) queries: rank, counting sort by rank, records
     uint32_t* hist = skey;                                         // N + 1 bins
     for (int i = tid; i <= N; i += THREADS) hist[i] = 0;
@@ -722,7 +702,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     };
     if constexpr (!PART) {
         rank_queries(0);
-        PHASE_MARK(4);
         count_ranks(0);
         scan_ranks();
     } else {
@@ -754,7 +733,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
     for (int s = 0; s < E; s++)
         if (mq(s) < M) rp[s] |= atomicAdd(&hist[rp[s]], 1u) << 16;       // final position of the record
     __syncthreads();
-    PHASE_MARK(7);
     // The histogram is spent. Three steps from here, so that every access indexed by the query (its value, the
     // scalar side inputs, the out_u / out_s updates) is coalesced and every record leaves in position order as
     // full lines:
@@ -784,7 +762,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         }
     }
     __syncthreads();
-    PHASE_MARK(8);
     constexpr int WHO = PART ? 18 : 16;               // row (a part's: below 2^18) and rank (at most 16384, a part's 8192) in one word
     uint32_t* who  = skey;
     float*    ypos = su0s;
@@ -798,14 +775,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) sort_rank_small(const
         }
     }
     __syncthreads();
-    PHASE_MARK(5);
     #pragma unroll 4
     for (int pos = tid; pos < M; pos += THREADS) {
         const uint32_t w = who[pos];
         const int      m = (int)(w & ((1u << WHO) - 1u)), r = (int)(w >> WHO);
         store_record(pos, r, record(m, FOLD ? m % MR : m, r, ypos[pos]));
     }
-    PHASE_MARK(6);
 }
 
 

@@ -14,7 +14,7 @@
 // lane. A loop over each key's queries, one stream per warp, with the queries' rows fetched once their records had arrived, took 60
 // instructions per key and query where this takes 20 (dots) to 45. At 96 heads x 4096 keys x 64 features and channels: prefix dots
 // 1.94 -> 0.78 ms, rows and dots 2.78 -> 1.69; Laplace at 24 heads x 4096, both passes: dots 0.79 -> 0.65, rows and dots 0.93 -> 0.79.
-// A row gathered per event is 0.65 ms of the first at the L2's rate (l2_row_traffic_main.cu), with a row reduced 1.5 of the second.
+// A row gathered per event is 0.65 ms of the first at the L2's rate (a bare loop over the same gathers), with a row reduced 1.5 of the second.
 // Rows go straight to registers, block t + 1's as soon as block t's are done with: through shared memory (cp.async) the load/store
 // pipe moved every row twice and was 77 % busy (dots 1.20 ms); with L1::no_allocate on the loads the L2 did not keep them (7.4 instead of
 // 0.9 GB from memory, 1.23 ms); bulk copies go at half the rate. 16 warps per SM: 24, with registers spilled, are slower.
