@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(WALK_THREADS, lap_ctas2(CPL)) laplace_pass2(co
 }
 
 // The second pass's row emission with 4 channels per lane (RowFeeder; rows_by_quads says when). A CTA per item, eight of them (16 warps) on an
-// SM: its state takes some 120 registers. Bound by the L2 traffic of one row gathered and one row reduced per key and query (2.4 of its 2.8 ms
+// SM: its state takes some 120 registers. Bound by the L2 traffic of one row gathered and one row reduced per key and query (2.38 of its 2.64 ms
 // at 48 heads x 16384 keys and queries; with one stream per warp it took 3.0).
 template <int LPS>
 __global__ void __launch_bounds__(ROW_THREADS, LAP_CTAS_ROWS) laplace_rows(const WalkArgs a)
