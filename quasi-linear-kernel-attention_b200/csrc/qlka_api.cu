@@ -1135,7 +1135,7 @@ int qlka_weighted_abs_sum_backward(const float* q, const float* k, const float* 
     const AbsBwdWs ws = in_pieces<AbsBwdWs>(workspace, workspace_bytes, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    const int C4 = round4(C), nseg = P * D;
+    const int C4 = round4(C);
     const bool full = g_u != nullptr;
 
     const float* vrows = v;
@@ -1201,7 +1201,7 @@ int qlka_weighted_sgn_sum_forward(const float* q, const float* k, const float* v
     const AbsBwdWs ws = in_pieces<AbsBwdWs>(workspace, workspace_bytes, P, D, N, M, C);
     if (!ws_ok(workspace, workspace_bytes, ws.bytes)) return QLKA_ERR_WORKSPACE;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    const int C4 = round4(C), nseg = P * D;
+    const int C4 = round4(C);
 
     const float* vrows = v;
     const float* grows = g;
